@@ -442,8 +442,151 @@ __device__ __noinline__ void certain_collection(const CellArgs& a, CellSmem S, i
   collect_once(a, &S, imin, imax, lo_i ? i : j, lo_i ? j : i, Tc, use_E);
 }
 
+// One event of a cell's sequential order, taken by a whole warp: the pair of
+// slots (l0, l1) with draw r, either placed certainly in an ordinary collection
+// by the FP32 bounds (certain) or evaluated exactly.  Even lanes hold SIP l0,
+// odd lanes SIP l1 (lanes 0 and 1 write): both SIPs' loads, densities and
+// radii run side by side, and the updated masses stay in registers for the
+// FP32 copies instead of being read back, so an event costs one round of
+// loads and one chain of FP64 operations (its latency is what a raining cell
+// waits for).  Same decisions and operation order as exact_pair and
+// collect_once.  Returns 0 (no collision), 1 (one collection) or 2 (multiple
+// collection), the same in all lanes.
+__device__ __noinline__ int warp_event(const CellArgs& a, CellSmem S, int l0, int l1, double Tc,
+                                       bool use_E, double r, bool certain) {
+  constexpr unsigned FULL = 0xffffffffu;
+  const int lane = threadIdx.x & 31, me = lane & 1;
+  const bool writes = lane < 2;
+  const int l = me ? l1 : l0;
+  const int32_t id = S.sid[l];
+  // one round of independent loads
+  double xi = a.xi[id];
+  double mw = a.m_w[id], ms = a.m_s[id];
+  int32_t gk = a.gk[id];
+  double R = a.gR[id], rho = a.grho[id];
+  const double u = certain ? 0.0 : a.vel[id], w = certain ? 0.0 : a.vel[a.n + id];
+  const double xo = __shfl_xor_sync(FULL, xi, 1);
+  // imin is l0's SIP when XI[ii] <= XI[jj], else l1's
+  const double x0 = me ? xo : xi, x1 = me ? xi : xo;
+  const bool lo0 = x0 <= x1;
+  const bool is_min = (me == 0) == lo0;
+  if (gk == GK_NONE && (!certain || is_min)) {
+    rho = density_of(a, R, rho, Tc);   // R, rho held the step-start m_p, m_s
+    gk = GK_STALE;
+    if (writes) { a.grho[id] = rho; a.gk[id] = gk; }
+  }
+  double p_crit = 0.0;
+  if (!certain) {
+    if (gk < 0) {
+      R = col_radius(mw + ms, rho);
+      gk = use_E ? col_bin_f(R, a.lo, a.bl, a.nb, a.lo_f, a.inv_bl_f, a.bin_margin) : 0;
+      if (writes) { a.gR[id] = R; a.gk[id] = gk; }
+    }
+    const int32_t go = __shfl_xor_sync(FULL, gk, 1);
+    const double Ro = __shfl_xor_sync(FULL, R, 1);
+    const double e = use_E ? __ldg(a.E + (int64_t)(me ? go : gk) * a.nb + (me ? gk : go))
+                           : a.E_const;
+    const double du = u - __shfl_xor_sync(FULL, u, 1), dw = w - __shfl_xor_sync(FULL, w, 1);
+    const double dv = sqrt(du * du + dw * dw);
+    const double Rs = R + Ro;
+    const double xi_max = lo0 ? x1 : x0;
+    p_crit = xi_max * a.dtdv * (LC_PI * Rs * Rs * e * dv * 1.0E-12);
+    if (!(p_crit > 1.0) && !(p_crit > r)) {
+      __syncwarp();   // orders the scratch writes before the next event's loads
+      return 0;
+    }
+  }
+  const double mwo = __shfl_xor_sync(FULL, mw, 1), mso = __shfl_xor_sync(FULL, ms, 1);
+  const int32_t ido = __shfl_xor_sync(FULL, id, 1);
+  const int32_t imin = is_min ? id : ido, imax = is_min ? ido : id;
+  const double xi_min = lo0 ? x0 : x1, xi_max = lo0 ? x1 : x0;
+  int out = 1;
+  bool split = false;
+  if (p_crit > 1.0) {
+    out = 2;
+    if (a.log && lane == 0) log_event(a, imin, imax, 2, p_crit, 0.0);
+    if (is_min) {
+      mw = mw + p_crit * mwo;
+      ms = ms + p_crit * mso;
+    } else {
+      xi -= p_crit * xi_min;
+    }
+  } else {
+    // xi_rel_dev < 1e-5; clear of the limit, a product decides
+    const double d = xi_max - xi_min;
+    split = !(xi_max > 0.0 && d > 2.0E-5 * xi_max) && d / xi_max < 1.0E-5;
+    if (!split) {
+      if (a.log && lane == 0) log_event(a, imin, imax, 0, 0.0, 0.0);
+      if (is_min) {
+        mw += mwo;
+        ms += mso;
+      } else {
+        xi -= xi_min;
+      }
+    } else {
+      if (a.log && lane == 0) log_event(a, imin, imax, 1, xi_min, xi_max);
+      if (gk == GK_NONE) {
+        // imax's density belongs to its step-start masses
+        rho = density_of(a, R, rho, Tc);
+        if (writes) a.grho[id] = rho;
+      }
+      const double rhoo = __shfl_xor_sync(FULL, rho, 1);
+      const double xi_ges = xi_min + xi_max;
+      const double w_min = is_min ? mw : mwo, w_max = is_min ? mwo : mw;
+      const double s_min = is_min ? ms : mso, s_max = is_min ? mso : ms;
+      mw = 2.0 * (xi_min * w_min + xi_max * w_max) / xi_ges;
+      ms = 2.0 * (xi_min * s_min + xi_max * s_max) / xi_ges;
+      // both radii follow from imin's density (all_or_nothing.py:615-624)
+      R = col_radius(mw + ms, is_min ? rho : rhoo);
+      const double xm = 0.5 * 0.7 * xi_ges;
+      xi = is_min ? 0.5 * xi_ges - xm : xm;
+      gk = use_E ? col_bin_f(R, a.lo, a.bl, a.nb, a.lo_f, a.inv_bl_f, a.bin_margin) : 0;
+    }
+  }
+  if (writes) {
+    if (is_min || split) { a.m_w[id] = mw; a.m_s[id] = ms; }
+    if (!is_min || split) { a.xi[id] = xi; S.v[l].x = d2f_rn(xi); }
+    if (split) {
+      a.gR[id] = R;
+      a.gk[id] = gk;
+      S.v[l].y = d2f_rn(R);
+      S.sk[l] = gk;
+    } else if (is_min) {
+      // the exact radius and bin become stale; the FP32 copies follow now
+      // (masses_changed)
+      const float Rf = lt_cbrtf((float)LC_FOUR_PI_OVER_THREE_INV * d2f_rn(mw + ms) / d2f_rn(rho));
+      int32_t kb = 0;
+      gk = GK_STALE;
+      if (use_E) {
+        const float v = (__logf(Rf) - a.lo_f) * a.inv_bl_f + 0.5f;
+        const float fl = floorf(v);
+        if (v - fl > a.bin_margin && (fl + 1.0f) - v > a.bin_margin && v > -1e6f && v < 1e6f &&
+            Rf > 0.f) {
+          kb = __float2int_rz(fl);
+          kb = kb < 0 ? 0 : (kb > a.nb - 1 ? (int32_t)a.nb - 1 : kb);
+        } else {
+          R = col_radius(mw + ms, rho);
+          a.gR[id] = R;
+          kb = gk = col_bin_f(R, a.lo, a.bl, a.nb, a.lo_f, a.inv_bl_f, a.bin_margin);
+        }
+      }
+      a.gk[id] = gk;
+      S.v[l].y = Rf;
+      S.sk[l] = kb;
+    }
+  }
+  __threadfence_block();
+  __syncwarp();
+  return out;
+}
+
 __device__ __noinline__ double philox_from_bits(uint64_t k53) {
   return (double)k53 * (1.0 / 9007199254740992.0);
+}
+// a pair's draw from its two words: an injected double's bits, or Philox's
+__device__ __forceinline__ double draw_of(bool injected, uint64_t w) {
+  if (injected) return __longlong_as_double((long long)w);
+  return philox_from_bits((w >> 37) * 67108864ull + (uint64_t)((uint32_t)w >> 6));
 }
 
 // FP32 screen of the pair (i, j): 0 = certainly no collision, 1 = certainly
@@ -494,6 +637,29 @@ __device__ __forceinline__ void injected_interval(double r, float& r_lo, float& 
   r_hi = in01 ? r_lo + 0x1p-24f : -1.0f;
 }
 
+// First screen of the per-pair draws, without a table look-up: the pair of
+// SIPs vi and vj is certainly no collision when screen_pair's upper bound with
+// the table's largest efficiency (folded into cmax with dt/dV, pi 1e-12 and the
+// bound's 2^-14 slack) lies below r, a lower bound of the draw that is 0 or at
+// least 2^-24 (a product flushed to zero belongs to a p_crit far below that).
+// NaN and non-positive multiplicities never pass.
+__device__ __forceinline__ bool surely_skips(float4 vi, float4 vj, float cmax, float r) {
+  const float dv = fabsf(vi.z - vj.z) + fabsf(vi.w - vj.w);
+  const float sl = (fabsf(vi.z) + fabsf(vi.w)) + (fabsf(vj.z) + fabsf(vj.w));
+  const float rs = vi.y + vj.y;
+  const float p = ((fmaxf(vi.x, vj.x) * cmax) * (rs * rs)) * (dv + 0x1p-21f * sl) + 1e-36f;
+  return p < r && vi.x > 0.0f && vj.x > 0.0f;
+}
+// the lower bound of a draw surely_skips takes: from the top word of a Philox
+// draw (23 bits), or of an injected one
+__device__ __forceinline__ float low_of_word(uint32_t x) {
+  return __uint_as_float(0x3f800000u | (x >> 9)) - 1.0f;
+}
+__device__ __forceinline__ float low_of_double(double r) {
+  const uint64_t b = (uint64_t)__double_as_longlong(r);
+  return b < 0x3ff0000000000000ull && b >= 0x3e70000000000000ull ? d2f_down_pos(r) : 0.0f;
+}
+
 // the exact data of a cell's SIPs, computed lazily from the step-start masses
 __device__ __forceinline__ void init_exact_scratch(const CellArgs& a, const CellSmem& S, int n,
                                                    int lane) {
@@ -504,23 +670,6 @@ __device__ __forceinline__ void init_exact_scratch(const CellArgs& a, const Cell
     a.gk[id] = -1;
   }
   __syncwarp();
-}
-
-// one pair with draw r: the screen on the FP32 copies, else the exact
-// evaluation; returns 0 (no change) or the outcome counters it adds
-__device__ __forceinline__ void decide_pair(const CellArgs& a, const CellSmem& S, bool use_E,
-                                            int i, int j, double r, float r_lo, float r_hi,
-                                            double Tc, int64_t& c0, int64_t& c1) {
-  const int sc = screen_pair(a, use_E, S.v[i], S.sk[i], S.v[j], S.sk[j], r_lo, r_hi);
-  if (sc == 0) return;
-  if (sc == 1) {
-    certain_collection(a, S, i, j, Tc, use_E);
-    c0 += 1;
-    return;
-  }
-  const int o = exact_pair(a, S, S.sid[i], S.sid[j], i, j, Tc, use_E, r);
-  c0 += o == 1;
-  c1 += o == 2;
 }
 
 // order-preserving keys of non-NaN floats (for warp min/max reductions)
@@ -680,25 +829,15 @@ __device__ __forceinline__ int2 thin_cell(const CellArgs& a, const CellSmem S, i
           bool col_now = false;
           while (cand) {
             const int t = __ffs(cand) - 1;
-            int col = 0;
+            const int o = warp_event(a, S, ei, ej + t, Tc, use_E,
+                                     philox_from_bits(__shfl_sync(FULL, k53, t)),
+                                     __shfl_sync(FULL, sc, t) == 1);
             if (lane == t) {
-              if (sc == 1) {
-                certain_collection(a, S, ei, q, Tc, use_E);
-                c0 += 1;
-                col = 1;
-              } else {
-                const int o = exact_pair(a, S, S.sid[ei], S.sid[q], ei, q, Tc, use_E,
-                                         philox_from_bits(k53));
-                c0 += o == 1;
-                c1 += o == 2;
-                col = o != 0;
-              }
+              c0 += o == 1;
+              c1 += o == 2;
             }
-            col = __shfl_sync(FULL, col, t);
-            __threadfence_block();
-            __syncwarp();
             todo &= ~((2u << t) - 1u);   // pairs up to t are done
-            if (col) { col_now = true; break; }
+            if (o) { col_now = true; break; }
             cand &= cand - 1u;   // no change: the later screens still hold
           }
           if (!col_now) break;
@@ -715,24 +854,23 @@ __device__ __forceinline__ int2 thin_cell(const CellArgs& a, const CellSmem S, i
         const unsigned bal = __ballot_sync(FULL, succ);
         const int g = bal ? __ffs(bal) - 1 : m - 1;
         const uint32_t jd = g < m - 1 ? (uint32_t)(g + 2) : (uint32_t)m;
-        int col = 0;
-        if (lane == 0) {
-          const double r = ldexp((double)lt_bits53(a.seed, chunk, esub, jd, pc1) *
-                                     (1.0 / 9007199254740992.0), -ee);
-          // a float interval around r: truncation and the next float up
-          // (below the normal range: [0, 2^-126])
-          const bool normal = r >= 0x1p-126;
-          const float r_lo = normal ? d2f_down_pos(r) : 0.0f;
-          const float r_hi = normal ? __uint_as_float(__float_as_uint(r_lo) + 1u) : 0x1p-126f;
-          int64_t d0 = 0, d1 = 0;
-          decide_pair(a, S, use_E, ei, ej + g, r, r_lo, r_hi, Tc, d0, d1);
-          c0 += (int)d0;
-          c1 += (int)d1;
-          col = (d0 | d1) != 0;
+        const double r = ldexp((double)lt_bits53(a.seed, chunk, esub, jd, pc1) *
+                                   (1.0 / 9007199254740992.0), -ee);
+        // a float interval around r: truncation and the next float up
+        // (below the normal range: [0, 2^-126])
+        const bool normal = r >= 0x1p-126;
+        const float r_lo = normal ? d2f_down_pos(r) : 0.0f;
+        const float r_hi = normal ? __uint_as_float(__float_as_uint(r_lo) + 1u) : 0x1p-126f;
+        const int hj = ej + g;
+        const int sc = screen_pair(a, use_E, S.v[ei], S.sk[ei], S.v[hj], S.sk[hj], r_lo, r_hi);
+        if (sc != 0) {
+          const int o = warp_event(a, S, ei, hj, Tc, use_E, r, sc == 1);
+          if (lane == 0) {
+            c0 += o == 1;
+            c1 += o == 2;
+          }
+          changed = o != 0;
         }
-        changed = __shfl_sync(FULL, col, 0) != 0;
-        __threadfence_block();
-        __syncwarp();
         next_j = ej + g + 1;
       }
       const bool part_left = !eind && next_j < eend;
@@ -801,6 +939,19 @@ __global__ void __launch_bounds__(CELL_WARPS * 32, MINB)
   const uint64_t cstep = (uint64_t)*a.col_step;
   const bool use_E = a.E != nullptr;
   const float c43 = (float)LC_FOUR_PI_OVER_THREE_INV;
+  float cmax = 0.0f;   // surely_skips' factor
+  if constexpr (!THIN) {
+    float em = a.E_const_f;
+    if (use_E) {
+      // the largest of the row maxima (infinity without them: every pair is screened)
+      em = a.erow ? 0.0f : __uint_as_float(0x7f800000u);
+      if (a.erow) {
+        for (int64_t q = lane; q < a.nb; q += 32) em = fmaxf(em, __ldg(a.erow + q));
+        em = __uint_as_float(__reduce_max_sync(0xffffffffu, __float_as_uint(em)));
+      }
+    }
+    cmax = ((a.dtdv_f * (float)(LC_PI * 1.0E-12)) * fmaxf(em, 0.0f)) * (1.0f + 0x1p-13f);
+  }
   int64_t c0 = 0, c1 = 0;
   // persistent warps take the member's cells, largest first, from a counter
   for (;;) {
@@ -879,99 +1030,106 @@ __global__ void __launch_bounds__(CELL_WARPS * 32, MINB)
       __syncwarp();
       continue;
     }
-    // Speculative sequential order.  From rank pos on, the lanes screen the
-    // pairs in parallel with the current state: lane l takes the couples
-    // (p0 + 2l + 64t, p0 + 2l + 64t + 1), p0 = pos rounded down to even, in
-    // lexicographic order, one Philox block per couple.  The first pair p*
-    // the screen does not skip is the next event of the sequential order:
-    // every pair before it is skipped with the very state it would see.  The
-    // lane that found p* processes it (certain collection or exact FP64
-    // evaluation), then screening resumes at p* + 1.  Most cells have no
-    // event at all.  A cell with many events finishes with the anti-diagonal
-    // schedule from its current position.
-    const int event_limit = 16 + P / 64;
+    // Speculative sequential order, one window of 64 pairs (lexicographic
+    // order) at a time: lane l draws the couple of ranks (w0 + 2l, w0 + 2l + 1),
+    // one Philox block per couple, and screens both pairs with the current
+    // state (surely_skips, then screen_pair for the few left).  The first pair
+    // the screens do not skip is the next event of the sequential order (every
+    // pair before it is skipped with the very state it would see), processed by
+    // the warp.  An event that changes nothing leaves the later screens valid;
+    // after a collection the window's later pairs are screened again with the
+    // draws they already have.  So an event costs one more screen of its
+    // window, where letting every lane run on to its own first hit cost a screen
+    // of the whole rest of the cell: a step of a raining 75 x 75 x 128 state (14
+    // collections per cell on average, 190 in the heaviest) went from 10.6 ms to
+    // 1.1 ms; a fresh 75 x 75 x 64 state stays at 125 us (the Philox blocks).
+    // A cell with many events finishes with the anti-diagonal schedule from its
+    // current position: the sequence costs a chain of some 4 us per event, the
+    // 2n - 3 diagonals about as much each.
+    const int event_limit = 64 + 2 * n;
     int pos = 0;           // first rank not processed yet
-    int bi = 0, bj = 1;    // the pair of rank pos & ~1
     int events = 0;
     bool diagonal = false;
-    for (;;) {
-      int my_p = 0x7fffffff, my_i = 0, my_j = 0, my_sc = 0;
-      uint64_t my_k53 = 0;
-      {
-        int i = bi, j = bj + 2 * lane, p = (pos & ~1) + 2 * lane;
-        for (;;) {
-          while (j > n - 1 && i < n - 2) { j += i + 2 - n; ++i; }
-          if (j > n - 1) break;
-          // the next pair in lexicographic order (absent past the last pair)
-          int i2 = i, j2 = j + 1;
-          if (j2 > n - 1) { i2 = i + 1; j2 = i + 2; }
-          const bool has2 = i2 < n - 1;
-          float rl0, rh0, rl1 = 0.f, rh1 = 0.f;
-          uint64_t k0 = 0, k1 = 0;
-          if (rnd) {
-            injected_interval(rnd[p], rl0, rh0);
-            if (has2) injected_interval(rnd[p + 1], rl1, rh1);
-          } else {
-            const PhiloxBlock blk = philox_block(a.seed, (uint64_t)(p >> 1), pc1);
-            k0 = philox_half53(blk, false);
-            k1 = philox_half53(blk, true);
-            philox_interval(k0, rl0, rh0);
-            philox_interval(k1, rl1, rh1);
-          }
-          const float4 vi = S.v[i], vj = S.v[j];
-          const int32_t ki = S.sk[i], kj = S.sk[j];
-          if (p >= pos) {
-            const int sc = screen_pair(a, use_E, vi, ki, vj, kj, rl0, rh0);
-            if (sc != 0) { my_p = p; my_i = i; my_j = j; my_sc = sc; my_k53 = k0; break; }
-          }
-          if (has2) {
-            // the couple's second pair shares SIP i unless it starts a new row
-            const bool same = i2 == i;
-            const float4 vi2 = same ? vi : S.v[i2];
-            const int32_t ki2 = same ? ki : S.sk[i2];
-            const int sc = screen_pair(a, use_E, vi2, ki2, S.v[j2], S.sk[j2], rl1, rh1);
-            if (sc != 0) { my_p = p + 1; my_i = i2; my_j = j2; my_sc = sc; my_k53 = k1; break; }
-          }
-          j += 64;
-          p += 64;
+    int i = 0, j = 1 + 2 * lane;   // the pair of rank w0 + 2 lane
+    float4 vi = S.v[0];
+    for (int w0 = 0; w0 < P && !diagonal; w0 += 64, j += 64) {
+      if (j > n - 1) {
+        while (j > n - 1 && i < n - 2) { j += i + 2 - n; ++i; }
+        vi = S.v[i];
+      }
+      const int p = w0 + 2 * lane;
+      const bool has0 = p < P, has1 = p + 1 < P;
+      // the next pair in lexicographic order: the same row, or the next one's first
+      const bool same = j < n - 1;
+      const int i2 = same ? i : i + 1, j2 = same ? j + 1 : i + 2;
+      PhiloxBlock x = {0, 0, 0, 0};   // the couple's draws (injected ones as their bits)
+      if (rnd) {
+        if (has0) {
+          const uint64_t q = (uint64_t)__double_as_longlong(rnd[p]);
+          x.x0 = (uint32_t)(q >> 32); x.x1 = (uint32_t)q;
         }
-      }
-      const int pstar = __reduce_min_sync(0xffffffffu, my_p);
-      if (pstar == 0x7fffffff) break;   // no further event in this cell
-      if (events == 0) {
-        // exact data of the cell's SIPs, computed lazily from the step-start masses
-        for (int q = lane; q < n; q += 32) {
-          const int32_t id = S.sid[q];
-          a.gR[id] = a.m_w[id] + a.m_s[id];
-          a.grho[id] = a.m_s[id];
-          a.gk[id] = -1;
+        if (has1) {
+          const uint64_t q = (uint64_t)__double_as_longlong(rnd[p + 1]);
+          x.x2 = (uint32_t)(q >> 32); x.x3 = (uint32_t)q;
         }
-        __syncwarp();
+      } else {
+        x = philox_block(a.seed, (uint64_t)(p >> 1), pc1);
       }
-      const int L = __ffs(__ballot_sync(0xffffffffu, my_p == pstar)) - 1;
-      if (lane == L) {
-        if (my_sc == 1) {
-          certain_collection(a, S, my_i, my_j, Tc, use_E);
-          c0 += 1;
-        } else {
-          const int o = exact_pair(a, S, S.sid[my_i], S.sid[my_j], my_i, my_j, Tc,
-                                   use_E, rnd ? rnd[pstar] : philox_from_bits(my_k53));
-          c0 += o == 1;
-          c1 += o == 2;
+      const float r0 = rnd ? low_of_double(__hiloint2double((int)x.x0, (int)x.x1))
+                           : low_of_word(x.x0);
+      const float r1 = rnd ? low_of_double(__hiloint2double((int)x.x2, (int)x.x3))
+                           : low_of_word(x.x2);
+      int done = w0;   // ranks below it are done
+      for (;;) {       // screen the window's pairs from rank `done` on
+        bool m0 = false, m1 = false;
+        if (has0) m0 = p >= done && !surely_skips(vi, S.v[j], cmax, r0);
+        if (has1)
+          m1 = p + 1 >= done && !surely_skips(same ? vi : S.v[i2], S.v[j2], cmax, r1);
+        if (!__any_sync(0xffffffffu, m0 | m1)) break;
+        uint32_t sc = 0;   // screen_pair's answers, two bits per pair
+        float r_lo, r_hi;
+        if (m0) {
+          if (rnd) injected_interval(__hiloint2double((int)x.x0, (int)x.x1), r_lo, r_hi);
+          else philox_interval(philox_half53(x, false), r_lo, r_hi);
+          sc = (uint32_t)screen_pair(a, use_E, vi, S.sk[i], S.v[j], S.sk[j], r_lo, r_hi);
         }
+        if (m1) {
+          if (rnd) injected_interval(__hiloint2double((int)x.x2, (int)x.x3), r_lo, r_hi);
+          else philox_interval(philox_half53(x, true), r_lo, r_hi);
+          sc |= (uint32_t)screen_pair(a, use_E, S.v[i2], S.sk[i2], S.v[j2], S.sk[j2], r_lo, r_hi)
+                << 2;
+        }
+        bool changed = false;
+        unsigned hits;
+        while (!changed && (hits = __ballot_sync(0xffffffffu, sc != 0)) != 0) {
+          if (events == 0) {
+            // exact data of the cell's SIPs, computed lazily from the step-start masses
+            init_exact_scratch(a, S, n, lane);
+            events = 1;
+          }
+          const int L = __ffs(hits) - 1;
+          const uint32_t scL = __shfl_sync(0xffffffffu, sc, L);
+          const bool sec = (scL & 3u) == 0;
+          const uint64_t dr = ((uint64_t)(sec ? x.x2 : x.x0) << 32) | (sec ? x.x3 : x.x1);
+          const int o = warp_event(
+              a, S, __shfl_sync(0xffffffffu, sec ? i2 : i, L),
+              __shfl_sync(0xffffffffu, sec ? j2 : j, L), Tc, use_E,
+              draw_of(rnd != nullptr, __shfl_sync(0xffffffffu, dr, L)),
+              (sec ? scL >> 2 : scL & 3u) == 1u);
+          if (lane == L) {
+            c0 += o == 1;
+            c1 += o == 2;
+            sc &= sec ? 3u : 12u;
+          }
+          done = w0 + 2 * L + (sec ? 2 : 1);
+          changed = o != 0;
+          if (changed && ++events > event_limit) diagonal = true;
+        }
+        if (!changed) break;
+        vi = S.v[i];   // SIP i may have changed
+        if (diagonal) break;
       }
-      __threadfence_block();
-      __syncwarp();
-      const int si = __shfl_sync(0xffffffffu, my_i, L), sj = __shfl_sync(0xffffffffu, my_j, L);
-      pos = pstar + 1;
-      if (pstar & 1) {   // rank pos is even: the successor of p*
-        bi = si; bj = sj + 1;
-        if (bj > n - 1) { bi = si + 1; bj = si + 2; }
-      } else {           // rank pos is odd: its couple starts at p* itself
-        bi = si; bj = sj;
-      }
-      if (pos >= P) break;
-      if (++events >= event_limit) { diagonal = true; break; }
+      pos = diagonal ? done : w0 + 64;
     }
     if (diagonal) {
       // anti-diagonal schedule of the pairs from rank pos on
@@ -1293,16 +1451,13 @@ static inline int nblk(int64_t n, int t) {
 }
 static const size_t CELL_SMEM_BYTES = (size_t)CELL_WARPS * CELL_WARP_BYTES;
 
-__global__ void k_table_to_float(const double* __restrict__ E, float* __restrict__ Ef, int64_t m) {
-  for (int64_t k = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; k < m;
-       k += (int64_t)gridDim.x * blockDim.x)
-    Ef[k] = (float)E[k];
-}
-// largest FP32 efficiency of each row, one warp per row: the maximum of the
-// row's positive values by a warp reduction; a row with a NaN, or whose
-// largest value is not positive (where the sign of a zero or the place of a
-// NaN decides), is taken in column order by one lane, as the oracle does
-__global__ void k_table_rowmax(const double* __restrict__ E, float* __restrict__ erow, int64_t nb) {
+// The FP32 copy of the efficiency table and the largest FP32 efficiency of
+// each row, one warp per row: the maximum of the row's positive values by a
+// warp reduction; a row with a NaN, or whose largest value is not positive
+// (where the sign of a zero or the place of a NaN decides), is taken in column
+// order by one lane, as the oracle does
+__global__ void k_table_float(const double* __restrict__ E, float* __restrict__ Ef,
+                              float* __restrict__ erow, int64_t nb) {
   const int lane = threadIdx.x & 31;
   const int64_t warps = (int64_t)gridDim.x * (blockDim.x >> 5);
   for (int64_t k = blockIdx.x * (int64_t)(blockDim.x >> 5) + (threadIdx.x >> 5); k < nb;
@@ -1312,6 +1467,7 @@ __global__ void k_table_rowmax(const double* __restrict__ E, float* __restrict__
     bool odd = false;
     for (int64_t q = lane; q < nb; q += 32) {
       const float v = (float)__ldg(row + q);
+      Ef[k * nb + q] = v;
       odd |= v != v;
       if (v > 0.0f) mk = max(mk, __float_as_uint(v));   // positive floats order as integers
     }
@@ -1402,16 +1558,12 @@ cudaError_t launch_collide_cells(const Bt& B, const lacmo_params_t& p, const lac
   cc.erow = nullptr;
   float* Ef = B.one.w.Ef;   // member 0's slot serves the whole batch
   if (p.E_col_grid && Ef && p.no_kernel_bins <= LACMO_MAX_KERNEL_BINS) {
-    const int64_t m = p.no_kernel_bins * p.no_kernel_bins;
-    k_table_to_float<<<nblk(m, 256), 256, 0, s>>>(p.E_col_grid, Ef, m); note_launches(1);
+    float* erow = Ef + (int64_t)LACMO_MAX_KERNEL_BINS * LACMO_MAX_KERNEL_BINS;
+    k_table_float<<<nblk(p.no_kernel_bins * 32, 128), 128, 0, s>>>(p.E_col_grid, Ef, erow,
+                                                                   p.no_kernel_bins);
+    note_launches(1);
     cc.Ef = Ef;
-    if (p.thin_draws) {
-      float* erow = Ef + (int64_t)LACMO_MAX_KERNEL_BINS * LACMO_MAX_KERNEL_BINS;
-      k_table_rowmax<<<nblk(p.no_kernel_bins * 32, 128), 128, 0, s>>>(p.E_col_grid, erow,
-                                                                      p.no_kernel_bins);
-      note_launches(1);
-      cc.erow = erow;
-    }
+    cc.erow = erow;
   }
   // thinned draws need the row maxima of a tabulated efficiency
   cc.thin = (p.thin_draws != 0 && d.draws == nullptr && (!p.E_col_grid || cc.erow)) ? 1 : 0;
