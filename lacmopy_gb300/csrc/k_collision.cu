@@ -19,121 +19,9 @@
 
 #include <atomic>
 
-#include "lacmo_crmath.h"
-#include "lacmo_internal.cuh"
-#include "lacmo_physics.cuh"
-#include "lacmo_thin.h"
+#include "lacmo_colmath.cuh"
 
 namespace lacmo {
-
-// x^(1/3 rounded to double) correctly rounded, fast path.  With c = double(1/3)
-// = 1/3 - d, d = 2^-54/3, the value is cbrt(x) * exp(-d ln x).  y = cbrt(x)
-// (faithful) is refined by one Newton step whose residual x - y^3 is formed in
-// double-double, and exp(-d ln x) = 1 - d L + (d L)^2/2 to far below 2^-100.
-// So z = y + t with t computed to ~2^-100 |y|.  The rounded sum y + t is the
-// correctly-rounded result unless y + t lies within 2^-85 |y| of a rounding
-// midpoint; then (or for non-normal x) the full routine decides.  The margin
-// is wider than the full routine's own uncertainty, so both always agree.
-__device__ __forceinline__ double cr_pow13_dd(double x) {
-  if (!(x >= 0x1p-1000 && x <= 0x1p1000)) return lacmo_cr_pow(x, LC_ONE_THIRD);
-  const double y = cbrt(x);
-  const lacmo_dd y2 = lacmo_two_prod(y, y);
-  const lacmo_dd y3 = lacmo_dd_mul_d(y2, y);
-  const double r = (x - y3.hi) - y3.lo;           // x - y3.hi is exact (Sterbenz)
-  const double corr = r / (3.0 * y2.hi);
-  const double dL = 0x1.5555555555555p-56 * log(x);  // d * ln x, d = 2^-54 / 3
-  const double t = corr - y * dL + y * (0.5 * dL * dL);
-  const double s = y + t;
-  const double e = (y - s) + t;                   // y + t = s + e exactly
-  const uint64_t b = lacmo_as_u64(s);
-  const int64_t ex = (int64_t)((b >> 52) & 0x7ff);
-  double half_ulp = lacmo_as_f64((uint64_t)(ex - 53) << 52);
-  if (e < 0.0 && (b & 0x000fffffffffffffULL) == 0) half_ulp *= 0.5;
-  if (fabs(fabs(e) - half_ulp) <= 0x1p-85 * s) return lacmo_cr_pow(x, LC_ONE_THIRD);
-  return s;
-}
-
-// The same value with most of the FP64 work moved to FP32 (GB300's FP64 pipe
-// is narrow, and the collision events run on single lanes).  For x in
-// [2^-40, 2^40] (every radius from 1 nm to 1 cm in micrometres):
-//  - y: the FP32 cube root (a few ulp) refined by two Newton steps
-//    y += (x - y^3) / (3 y^2), the residual in FP64 and the quotient in FP32:
-//    the error goes 2^-21 -> 2^-43 -> within about an ulp (FP64 rounding of
-//    the residual);
-//  - t = r / (3 y^2) - y d ln x with r = x - y^3 in double-double as above,
-//    both terms in FP32: |r / (3 y^2)| < 2^-50 y and |y d ln x| < 2^-46 y,
-//    each within 2^-22 relative, their sum within 2^-24 of the larger, and the
-//    neglected (d ln x)^2 / 2 below 2^-92: t is within 2^-67 y of its value;
-//  - a flushed FP32 residual (|r| < 2^-126) changes t by less than
-//    2^-126 / (3 x) <= 2^-86 y.
-// s = y + t is then the correctly-rounded result unless it lies within
-// 2^-62 s of a rounding midpoint (about one call in 500), where cr_pow13_dd
-// decides.
-__device__ __forceinline__ double cr_pow13(double x) {
-  if (!(x >= 0x1p-40 && x <= 0x1p40)) return cr_pow13_dd(x);
-  const float xf = d2f_int(x);
-  double y = f2d_int(f_cbrt(xf));
-#pragma unroll
-  for (int it = 0; it < 2; ++it) {
-    const float yf = d2f_int(y);
-    const double r0 = x - (y * y) * y;
-    y = y + f2d_int(d2f_int(r0) * f_rcp(3.0f * yf * yf));
-  }
-  const lacmo_dd y2 = lacmo_two_prod(y, y);
-  const lacmo_dd y3 = lacmo_dd_mul_d(y2, y);
-  const double r = (x - y3.hi) - y3.lo;
-  const float yf = d2f_int(y);
-  const float tf = d2f_int(r) * f_rcp(3.0f * yf * yf) -
-                   yf * (0x1.555556p-56f * (f_lg2(xf) * 0.693147181f));
-  const double t = f2d_int(tf);
-  const double s = y + t;
-  const double e = (y - s) + t;
-  const uint64_t b = lacmo_as_u64(s);
-  const int64_t ex = (int64_t)((b >> 52) & 0x7ff);
-  double half_ulp = lacmo_as_f64((uint64_t)(ex - 53) << 52);
-  if (e < 0.0 && (b & 0x000fffffffffffffULL) == 0) half_ulp *= 0.5;
-  if (fabs(fabs(e) - half_ulp) <= 0x1p-62 * s) return cr_pow13_dd(x);
-  return s;
-}
-
-__device__ __forceinline__ double col_radius(double m, double rho) {
-  return cr_pow13(LC_FOUR_PI_OVER_THREE_INV * m / rho);
-}
-// collision/all_or_nothing.py:35-67; float -> int as x86-64 compiled code
-// does it (NaN / out of range -> INT64_MIN -> bin 0).  The bin of the
-// correctly-rounded log: with the hardware log the index value is within
-// 1e-12 of it, so unless it lies within 1e-9 of an integer the truncation is
-// the same; near a bin edge the correctly-rounded log decides.
-__device__ __forceinline__ int32_t col_bin(double R, double lo, double bl, int64_t nb) {
-  double v = (log(R) - lo) / bl + 0.5;
-  const double fl = floor(v);
-  if (!(v - fl > 1e-9 && (fl + 1.0) - v > 1e-9 && fabs(v) < 1e15))
-    v = (lacmo_cr_log(R) - lo) / bl + 0.5;
-  int64_t ind = (v > -9.2233720368547758e18 && v < 9.2233720368547758e18) ? (int64_t)v : INT64_MIN;
-  if (ind < 0) ind = 0;
-  else if (ind > nb - 1) ind = nb - 1;
-  return (int32_t)ind;
-}
-// The same bin from an FP32 bin position first: lo_f, inv_bl_f are lo and 1/bl
-// rounded to FP32 and margin bounds the error of the FP32 position (it is
-// derived for radii within 1e-6; R is rounded to within 2^-24 here).  A
-// position farther than margin from every bin edge gives the bin of the exact
-// position; closer ones take col_bin.
-__device__ __forceinline__ int32_t col_bin_f(double R, double lo, double bl, int64_t nb,
-                                             float lo_f, float inv_bl_f, float margin) {
-  const float Rf = d2f_int(R);
-  const float v = (f_lg2(Rf) * 0.693147181f - lo_f) * inv_bl_f + 0.5f;
-  const float fl = floorf(v);
-  if (v - fl > margin && (fl + 1.0f) - v > margin && v > -1e6f && v < 1e6f && Rf > 1e-30f &&
-      Rf < 1e30f) {
-    int32_t kb = __float2int_rz(fl);
-    return kb < 0 ? 0 : (kb > nb - 1 ? (int32_t)nb - 1 : kb);
-  }
-  return col_bin(R, lo, bl, nb);
-}
-__device__ __forceinline__ int64_t pair_rank(int64_t i, int64_t j, int64_t n) {
-  return i * n - i * (i + 1) / 2 + (j - i - 1);
-}
 
 // ---------------------------------------------------------------------------
 // 2-D cells: one warp per cell (collision/all_or_nothing.py:498-635, 637-751,
@@ -226,42 +114,6 @@ __device__ __forceinline__ void make_cellargs(CellArgs& a, const Member& mb, con
   a.gstats = (float4*)mb.w.gstats;
   a.erow = cc.erow;
   a.thin = cc.thin;
-}
-
-// integer-unit conversions (GB300 runs FP64 conversions on its narrow FP64
-// pipe): round to nearest even, and truncation toward zero for r >= 0
-__device__ __noinline__ float d2f_rn_slow(double x) { return (float)x; }
-__device__ __forceinline__ float d2f_rn(double x) {
-  const uint64_t b = (uint64_t)__double_as_longlong(x);
-  const uint32_t e = (uint32_t)(b >> 52) & 0x7ffu;
-  if (e - 897u > 253u) return d2f_rn_slow(x);
-  const uint32_t sign = (uint32_t)(b >> 32) & 0x80000000u;
-  const uint64_t m = b & 0x000fffffffffffffull;
-  const uint32_t fm = (uint32_t)(m >> 29), rem = (uint32_t)m & 0x1fffffffu;
-  uint32_t fb = sign | ((e - 896u) << 23) | fm;
-  fb += (rem > 0x10000000u) || (rem == 0x10000000u && (fm & 1u));
-  return __int_as_float((int)fb);
-}
-// round to nearest even with zero/subnormal results flushed to zero and
-// overflow (and NaN) to infinity: integer instructions only (screen inputs,
-// where a flushed value makes the pair undecided or stays inside the bounds)
-__device__ __forceinline__ float d2f_flush(double x) {
-  const uint64_t b = (uint64_t)__double_as_longlong(x);
-  const uint32_t e = (uint32_t)(b >> 52) & 0x7ffu;
-  const uint32_t sign = (uint32_t)(b >> 32) & 0x80000000u;
-  if (e < 897u) return __int_as_float((int)sign);
-  if (e > 1150u) return __int_as_float((int)(sign | 0x7f800000u));
-  const uint64_t m = b & 0x000fffffffffffffull;
-  const uint32_t fm = (uint32_t)(m >> 29), rem = (uint32_t)m & 0x1fffffffu;
-  uint32_t fb = sign | ((e - 896u) << 23) | fm;
-  fb += (rem > 0x10000000u) || (rem == 0x10000000u && (fm & 1u));
-  return __int_as_float((int)fb);
-}
-__device__ __forceinline__ float d2f_down_pos(double r) {  // r in [0, 1)
-  const uint64_t b = (uint64_t)__double_as_longlong(r);
-  const uint32_t e = (uint32_t)(b >> 52) & 0x7ffu;
-  if (e < 897u) return 0.0f;
-  return __int_as_float((int)(((e - 896u) << 23) | (uint32_t)((b >> 29) & 0x7fffffu)));
 }
 
 // Exact per-SIP collision data (collision/all_or_nothing.py:812-826), kept
@@ -650,16 +502,6 @@ __device__ __forceinline__ bool surely_skips(float4 vi, float4 vj, float cmax, f
   const float p = ((fmaxf(vi.x, vj.x) * cmax) * (rs * rs)) * (dv + 0x1p-21f * sl) + 1e-36f;
   return p < r && vi.x > 0.0f && vj.x > 0.0f;
 }
-// the lower bound of a draw surely_skips takes: from the top word of a Philox
-// draw (23 bits), or of an injected one
-__device__ __forceinline__ float low_of_word(uint32_t x) {
-  return __uint_as_float(0x3f800000u | (x >> 9)) - 1.0f;
-}
-__device__ __forceinline__ float low_of_double(double r) {
-  const uint64_t b = (uint64_t)__double_as_longlong(r);
-  return b < 0x3ff0000000000000ull && b >= 0x3e70000000000000ull ? d2f_down_pos(r) : 0.0f;
-}
-
 // the exact data of a cell's SIPs, computed lazily from the step-start masses
 __device__ __forceinline__ void init_exact_scratch(const CellArgs& a, const CellSmem& S, int n,
                                                    int lane) {
@@ -1186,264 +1028,6 @@ __global__ void k_col_advance(const __grid_constant__ MRef mr, int draws) {
 }
 
 // ---------------------------------------------------------------------------
-// Box models: one CTA runs the whole single-cell step, SIP state in shared
-// memory, one __syncthreads per anti-diagonal.
-constexpr int BOX_THREADS = 1024;
-
-// collision/all_or_nothing.py:109-185 (Golovin kernel, kernel.py:461-480)
-__global__ void __launch_bounds__(BOX_THREADS) k_golovin(double* xis, double* masses, int n,
-                                                         double dtdv, int64_t* no_cols,
-                                                         const double* rnd, uint64_t seed,
-                                                         uint64_t step) {
-  extern __shared__ double sm[];
-  double* X = sm;
-  double* M = sm + n;
-  for (int q = threadIdx.x; q < n; q += blockDim.x) { X[q] = xis[q]; M[q] = masses[q]; }
-  __syncthreads();
-  int64_t c0 = 0, c1 = 0;
-  for (int s = 1; s <= 2 * n - 3; ++s) {
-    const int ilo = s - (n - 1) > 0 ? s - (n - 1) : 0;
-    const int ihi = (s - 1) >> 1;
-    for (int i = ilo + threadIdx.x; i <= ihi; i += blockDim.x) {
-      const int j = s - i;
-      int imin, imax;
-      if (X[i] <= X[j]) { imin = i; imax = j; } else { imin = j; imax = i; }
-      const double xi_min = X[imin], xi_max = X[imax];
-      const double m_min = M[imin], m_max = M[imax];
-      const double p_crit = xi_max * ((m_min + m_max) * 1.5E-18) * dtdv;
-      if (p_crit > 1.0) {
-        c1 += 1;
-        const double xi_col = p_crit * xi_min;
-        M[imin] = (xi_min * m_min + xi_col * m_max) / xi_min;
-        X[imax] -= xi_col;
-      } else {
-        const int64_t rk = pair_rank(i, j, n);
-        const double r = rnd ? rnd[rk] : philox_uniform(seed, (uint64_t)rk, step);
-        if (p_crit > r) {
-          c0 += 1;
-          const double xi_rel_dev = (xi_max - xi_min) / xi_max;
-          if (xi_rel_dev < 1.0E-5) {
-            const double xi_ges = xi_min + xi_max;
-            M[imin] = 2.0 * (xi_min * m_min + xi_max * m_max) / xi_ges;
-            M[imax] = M[imin];
-            X[imax] = 0.5 * 0.7 * xi_ges;
-            X[imin] = 0.5 * xi_ges - X[imax];
-          } else {
-            M[imin] += m_max;
-            X[imax] -= xi_min;
-          }
-        }
-      }
-    }
-    __syncthreads();
-  }
-  for (int q = threadIdx.x; q < n; q += blockDim.x) { xis[q] = X[q]; masses[q] = M[q]; }
-  for (int off = 16; off > 0; off >>= 1) {
-    c0 += __shfl_down_sync(0xffffffffu, c0, off);
-    c1 += __shfl_down_sync(0xffffffffu, c1, off);
-  }
-  if ((threadIdx.x & 31) == 0 && (c0 | c1)) {
-    atomicAdd((unsigned long long*)no_cols, (unsigned long long)c0);
-    atomicAdd((unsigned long long*)(no_cols + 1), (unsigned long long)c1);
-  }
-}
-
-// collision/all_or_nothing.py:392-491 (kernel K(m1, m2) tabulated on a
-// logarithmic mass grid): p_crit = xi_max K[k_i][k_j] dt/dV, the bins of
-// the collected SIP recomputed from its new mass
-__global__ void __launch_bounds__(BOX_THREADS) k_kgrid_box(double* xis, double* masses, int n,
-                                                           double dtdv, const double* K,
-                                                           int64_t nb, double lo, double bl,
-                                                           int64_t* no_cols, const double* rnd,
-                                                           uint64_t seed, uint64_t step) {
-  extern __shared__ double sm[];
-  double* X = sm;
-  double* M = sm + n;
-  int32_t* B = (int32_t*)(sm + 2 * n);
-  for (int q = threadIdx.x; q < n; q += blockDim.x) {
-    X[q] = xis[q]; M[q] = masses[q];
-    B[q] = col_bin(M[q], lo, bl, nb);
-  }
-  __syncthreads();
-  int64_t c0 = 0, c1 = 0;
-  for (int s = 1; s <= 2 * n - 3; ++s) {
-    const int ilo = s - (n - 1) > 0 ? s - (n - 1) : 0;
-    const int ihi = (s - 1) >> 1;
-    for (int i = ilo + threadIdx.x; i <= ihi; i += blockDim.x) {
-      const int j = s - i;
-      int imin, imax;
-      if (X[i] <= X[j]) { imin = i; imax = j; } else { imin = j; imax = i; }
-      const double xi_min = X[imin], xi_max = X[imax];
-      const double m_min = M[imin], m_max = M[imax];
-      const double p_crit = xi_max * K[(int64_t)B[i] * nb + B[j]] * dtdv;
-      if (p_crit > 1.0) {
-        c1 += 1;
-        const double xi_col = p_crit * xi_min;
-        M[imin] = (xi_min * m_min + xi_col * m_max) / xi_min;
-        X[imax] -= xi_col;
-        B[imin] = col_bin(M[imin], lo, bl, nb);
-      } else {
-        const int64_t rk = pair_rank(i, j, n);
-        const double r = rnd ? rnd[rk] : philox_uniform(seed, (uint64_t)rk, step);
-        if (p_crit > r) {
-          c0 += 1;
-          const double xi_rel_dev = (xi_max - xi_min) / xi_max;
-          if (xi_rel_dev < 1.0E-5) {
-            const double xi_ges = xi_min + xi_max;
-            M[imin] = 2.0 * (xi_min * m_min + xi_max * m_max) / xi_ges;
-            M[imax] = M[imin];
-            X[imax] = 0.5 * 0.7 * xi_ges;
-            X[imin] = 0.5 * xi_ges - X[imax];
-            B[imin] = col_bin(M[imin], lo, bl, nb);
-            B[imax] = B[imin];
-          } else {
-            M[imin] += m_max;
-            X[imax] -= xi_min;
-            B[imin] = col_bin(M[imin], lo, bl, nb);
-          }
-        }
-      }
-    }
-    __syncthreads();
-  }
-  for (int q = threadIdx.x; q < n; q += blockDim.x) { xis[q] = X[q]; masses[q] = M[q]; }
-  for (int off = 16; off > 0; off >>= 1) {
-    c0 += __shfl_down_sync(0xffffffffu, c0, off);
-    c1 += __shfl_down_sync(0xffffffffu, c1, off);
-  }
-  if ((threadIdx.x & 31) == 0 && (c0 | c1)) {
-    atomicAdd((unsigned long long*)no_cols, (unsigned long long)c0);
-    atomicAdd((unsigned long long*)(no_cols + 1), (unsigned long long)c1);
-  }
-}
-
-// collision/all_or_nothing.py:269-390 (E_col(R1, R2) table, 1-D velocities)
-__global__ void __launch_bounds__(BOX_THREADS) k_ecol_box(double* xis, double* masses,
-                                                          double* radii, const double* vel,
-                                                          const double* rho, int n, double dtdv,
-                                                          const double* E, int64_t nb, double lo,
-                                                          double bl, int64_t* no_cols,
-                                                          const double* rnd, uint64_t seed,
-                                                          uint64_t step) {
-  extern __shared__ double sm[];
-  double* X = sm;
-  double* M = sm + n;
-  double* R = sm + 2 * n;
-  double* Vv = sm + 3 * n;
-  double* Rh = sm + 4 * n;
-  int32_t* K = (int32_t*)(sm + 5 * n);
-  for (int q = threadIdx.x; q < n; q += blockDim.x) {
-    X[q] = xis[q]; M[q] = masses[q]; R[q] = radii[q]; Vv[q] = vel[q]; Rh[q] = rho[q];
-    K[q] = col_bin(R[q], lo, bl, nb);
-  }
-  __syncthreads();
-  int64_t c0 = 0, c1 = 0;
-  for (int s = 1; s <= 2 * n - 3; ++s) {
-    const int ilo = s - (n - 1) > 0 ? s - (n - 1) : 0;
-    const int ihi = (s - 1) >> 1;
-    for (int i = ilo + threadIdx.x; i <= ihi; i += blockDim.x) {
-      const int j = s - i;
-      int imin, imax;
-      if (X[i] <= X[j]) { imin = i; imax = j; } else { imin = j; imax = i; }
-      const double xi_min = X[imin], xi_max = X[imax];
-      const double m_min = M[imin], m_max = M[imax];
-      const double Rs = R[i] + R[j];
-      const double p_crit = xi_max * dtdv *
-                            (LC_PI * Rs * Rs * __ldg(E + (int64_t)K[i] * nb + K[j]) *
-                             fabs(Vv[i] - Vv[j]) * 1.0E-12);
-      if (p_crit > 1.0) {
-        const double xi_col = p_crit * xi_min;
-        M[imin] = (xi_min * m_min + xi_col * m_max) / xi_min;
-        R[imin] = col_radius(M[imin], Rh[imin]);
-        X[imax] -= xi_col;
-        K[imin] = col_bin(R[imin], lo, bl, nb);
-        c1 += 1;
-      } else {
-        const int64_t rk = pair_rank(i, j, n);
-        const double r = rnd ? rnd[rk] : philox_uniform(seed, (uint64_t)rk, step);
-        if (p_crit > r) {
-          c0 += 1;
-          const double xi_rel_dev = (xi_max - xi_min) / xi_max;
-          if (xi_rel_dev < 1.0E-5) {
-            const double xi_ges = xi_min + xi_max;
-            M[imin] = 2.0 * (xi_min * m_min + xi_max * m_max) / xi_ges;
-            M[imax] = M[imin];
-            R[imin] = col_radius(M[imin], Rh[imin]);
-            R[imax] = R[imin];
-            X[imax] = 0.5 * 0.7 * xi_ges;
-            X[imin] = 0.5 * xi_ges - X[imax];
-            K[imin] = col_bin(R[imin], lo, bl, nb);
-            K[imax] = K[imin];
-          } else {
-            M[imin] += m_max;
-            R[imin] = col_radius(M[imin], Rh[imin]);
-            X[imax] -= xi_min;
-            K[imin] = col_bin(R[imin], lo, bl, nb);
-          }
-        }
-      }
-    }
-    __syncthreads();
-  }
-  for (int q = threadIdx.x; q < n; q += blockDim.x) { xis[q] = X[q]; masses[q] = M[q]; radii[q] = R[q]; }
-  for (int off = 16; off > 0; off >>= 1) {
-    c0 += __shfl_down_sync(0xffffffffu, c0, off);
-    c1 += __shfl_down_sync(0xffffffffu, c1, off);
-  }
-  if ((threadIdx.x & 31) == 0 && (c0 | c1)) {
-    atomicAdd((unsigned long long*)no_cols, (unsigned long long)c0);
-    atomicAdd((unsigned long long*)(no_cols + 1), (unsigned long long)c1);
-  }
-}
-
-// collision/kernel.py:107-167 Beard (1976) terminal velocity (R in um)
-__device__ double beard_velocity(double R) {
-  const double rho_w = 1.0E3, rho_a = 1.225, visc = 1.818E-5, sigma = 73.0E-3;
-  const double g = 9.80665, drho = rho_w - rho_a;
-  if (R < 10.0) {
-    const double l0 = 6.62E-2;
-    const double C1 = drho * g / (4.5 * visc);
-    const double C_sc = 1.0 + 1.257 * l0 / R;
-    return C1 * C_sc * R * R * 1.0E-12;
-  } else if (R < 535.0) {
-    const double N_Da = 32.0E-18 * R * R * R * rho_a * drho * g / (3.0 * visc * visc);
-    double Y = log(N_Da);
-    const double p1[7] = {-0.327815e-5, 0.855176e-4, -0.578878e-3, -0.987059e-3,
-                          -0.153193e-2, 0.992696, -0.318657e1};
-    double r = p1[0] * Y + p1[1];
-    for (int k = 2; k < 7; ++k) r = r * Y + p1[k];
-    const double l0 = 6.62E-2;
-    const double C_sc = 1.0 + 1.257 * l0 / R;
-    return visc * C_sc * exp(r) / (rho_a * R * 2.0E-6);
-  } else if (R < 3500.0) {
-    const double N_Bo = 16.0E-12 * R * R * drho * g / (3.0 * sigma);
-    const double v4 = (visc * visc) * (visc * visc);
-    const double N_P16 = pow(sigma * sigma * sigma * rho_a * rho_a / (v4 * drho * g), 1.0 / 6.0);
-    const double Y = log(N_Bo * N_P16);
-    const double p2[6] = {0.238449e-2, -0.542819e-1, 0.475294, -0.204914e1, 0.523778e1,
-                          -0.500015e1};
-    double r = p2[0] * Y + p2[1];
-    for (int k = 2; k < 6; ++k) r = r * Y + p2[k];
-    return visc * N_P16 * exp(r) / (rho_a * R * 2.0E-6);
-  }
-  return 9.04929248;
-}
-__global__ void k_beard(double* vel, const double* R, int64_t n) {
-  for (int64_t k = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; k < n;
-       k += (int64_t)gridDim.x * blockDim.x)
-    vel[k] = beard_velocity(R[k]);
-}
-__global__ void k_radius_bin(const double* m, const double* rho, int64_t n, double lo, double bl,
-                             int64_t nb, double* R, int64_t* k) {
-  for (int64_t q = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; q < n;
-       q += (int64_t)gridDim.x * blockDim.x) {
-    const double r = col_radius(m[q], rho[q]);
-    R[q] = r;
-    if (k) k[q] = col_bin(r, lo, bl, nb);
-  }
-}
-
-// ---------------------------------------------------------------------------
 static inline int nblk(int64_t n, int t) {
   int64_t b = (n + t - 1) / t;
   if (b < 1) b = 1;
@@ -1483,24 +1067,6 @@ __global__ void k_table_float(const double* __restrict__ E, float* __restrict__ 
       }
     }
   }
-}
-
-// Bound on the error of the FP32 bin position v = (__logf(Rf) - lo_f) *
-// inv_bl_f + 0.5 against the exact (log R - lo) / bl + 0.5, doubled: Rf is
-// within 1e-6 of R (relative), so log Rf within 1e-6; __logf within 2^-21.41
-// absolute on [0.5, 2] and 3 ulp elsewhere (taken as 4 ulp of the largest
-// |log R| a bin edge can have); lo_f and the subtraction round within one ulp
-// of that value together; inv_bl_f, the product and the + 0.5 each within
-// 2^-24 of v <= nb + 1.  Bins closer than this to an edge are taken from the
-// exact FP64 path.
-static float fp32_bin_margin(double lo, double bl, int64_t nb) {
-  if (!(bl > 0.0) || nb <= 0) return 0.5f;
-  const double lmax = fmax(fabs(lo), fabs(lo + (double)(nb + 1) * bl)) + 1.0;
-  const double ulp = ldexp(1.0, (int)floor(log2(lmax)) - 23);
-  const double log_err = fmax(ldexp(1.0, -21) , 4.0 * ulp);
-  const double v_err = (1e-6 + log_err + ulp) / bl + 3.0 * (double)(nb + 1) * ldexp(1.0, -24);
-  const double m = 2.0 * v_err;
-  return (float)(m < 0.5 ? m : 0.5);
 }
 
 // persistent blocks: as many as are resident at once, split over members
@@ -1582,48 +1148,6 @@ cudaError_t launch_collide_cells(const Bt& B, const lacmo_params_t& p, const lac
   k_col_advance<<<dim3(1, B.M), 1, 0, s>>>(B.ref(), d.draws ? 1 : 0); note_launches(1);
   return cudaGetLastError();
 }
-cudaError_t launch_golovin(double* xis, double* m, int64_t n, double dtdv, int64_t* no_cols,
-                           const double* rnd, uint64_t seed, uint64_t step, cudaStream_t s) {
-  size_t sh = (size_t)n * 16;
-  cudaError_t e = cudaFuncSetAttribute(k_golovin, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                       (int)(LACMO_BOX_MAX_SIPS * 16));
-  if (e != cudaSuccess) return e;
-  k_golovin<<<1, BOX_THREADS, sh, s>>>(xis, m, (int)n, dtdv, no_cols, rnd, seed, step); note_launches(1);
-  return cudaGetLastError();
-}
-cudaError_t launch_ecol_box(double* xis, double* m, double* R, const double* vel,
-                            const double* rho, int64_t n, double dtdv, const double* E, int64_t nb,
-                            double lo, double bl, int64_t* no_cols, const double* rnd,
-                            uint64_t seed, uint64_t step, cudaStream_t s) {
-  size_t sh = (size_t)n * 44;
-  cudaError_t e = cudaFuncSetAttribute(k_ecol_box, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                       (int)(LACMO_ECOL_BOX_MAX_SIPS * 44));
-  if (e != cudaSuccess) return e;
-  k_ecol_box<<<1, BOX_THREADS, sh, s>>>(xis, m, R, vel, rho, (int)n, dtdv, E, nb, lo, bl, no_cols,
-                                        rnd, seed, step); note_launches(1);
-  return cudaGetLastError();
-}
-cudaError_t launch_kgrid_box(double* xis, double* m, int64_t n, double dtdv, const double* K,
-                             int64_t nb, double lo, double bl, int64_t* no_cols, const double* rnd,
-                             uint64_t seed, uint64_t step, cudaStream_t s) {
-  size_t sh = (size_t)n * 20;
-  cudaError_t e = cudaFuncSetAttribute(k_kgrid_box, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                       (int)(LACMO_BOX_MAX_SIPS * 20));
-  if (e != cudaSuccess) return e;
-  k_kgrid_box<<<1, BOX_THREADS, sh, s>>>(xis, m, (int)n, dtdv, K, nb, lo, bl, no_cols, rnd, seed,
-                                         step); note_launches(1);
-  return cudaGetLastError();
-}
-cudaError_t launch_beard(double* vel, const double* R, int64_t n, cudaStream_t s) {
-  k_beard<<<nblk(n, 128), 128, 0, s>>>(vel, R, n); note_launches(1);
-  return cudaGetLastError();
-}
-cudaError_t launch_radius_bin(const double* m, const double* rho, int64_t n, double lo, double bl,
-                              int64_t nb, double* R, int64_t* k, cudaStream_t s) {
-  k_radius_bin<<<nblk(n, 128), 128, 0, s>>>(m, rho, n, lo, bl, nb, R, k); note_launches(1);
-  return cudaGetLastError();
-}
-
 }  // namespace lacmo
 
 extern "C" int lacmo_collision_event_log(void* events, int64_t capacity,
