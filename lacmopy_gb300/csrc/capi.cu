@@ -4,6 +4,7 @@
 #include <string.h>
 
 #include <atomic>
+#include <mutex>
 #include <vector>
 
 #include "lacmo_internal.cuh"
@@ -23,6 +24,40 @@ static const int k_tune_options[TUNE_KNOBS][4] = {
 static std::atomic<int> g_tune[TUNE_KNOBS] = {{6}, {3}, {16}};
 int tune_value(int knob) { return g_tune[knob].load(std::memory_order_relaxed); }
 
+static cudaMemPool_t scratch_pool() {
+  static std::mutex mu;
+  static cudaMemPool_t pools[64];
+  int dev = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return nullptr;
+  std::lock_guard<std::mutex> lock(mu);
+  if (!pools[dev]) {
+    cudaMemPoolProps props = {};
+    props.allocType = cudaMemAllocationTypePinned;
+    props.location.type = cudaMemLocationTypeDevice;
+    props.location.id = dev;
+    cudaMemPool_t p = nullptr;
+    if (cudaMemPoolCreate(&p, &props) != cudaSuccess) {
+      cudaGetLastError();
+      return nullptr;
+    }
+    uint64_t keep = 16ull << 20;
+    int off = 0;
+    cudaMemPoolSetAttribute(p, cudaMemPoolAttrReleaseThreshold, &keep);
+    cudaMemPoolSetAttribute(p, cudaMemPoolReuseAllowInternalDependencies, &off);
+    pools[dev] = p;
+  }
+  return pools[dev];
+}
+void* Scratch::get(size_t bytes) {
+  const cudaMemPool_t pool = p_ ? nullptr : scratch_pool();
+  if (!pool) return nullptr;
+  if (cudaMallocFromPoolAsync(&p_, bytes, pool, s_) != cudaSuccess) {
+    cudaGetLastError();
+    p_ = nullptr;
+  }
+  return p_;
+}
+
 static inline size_t al(size_t x) { return (x + 255) & ~(size_t)255; }
 
 struct WsPlan {
@@ -38,10 +73,11 @@ static WsPlan ws_plan(int64_t n, int64_t nx, int64_t nz) {
       8 * (C + 1),     // draw_off
       4 * N,           // perm
       4 * N,           // rank
-      8 * N,           // dmxi
+      16 * C,          // acc64
       4 * N,           // rm_id
       8 * N,           // rm_val
-      8 * cell_records_offset((int64_t)C) + 16 * CELL_REC * C,  // aux: 6 doubles, records
+      8 * cell_records_offset((int64_t)C) +
+          (16 * CELL_REC + CELL_REC64_BYTES) * C,  // aux: 6 doubles, records
       8 * C,           // dTh
       8 * C,           // drv
       8 * C,           // div
@@ -49,8 +85,8 @@ static WsPlan ws_plan(int64_t n, int64_t nx, int64_t nz) {
       8 * N,           // colR
       8 * N,           // colrho
       4 * N,           // colk
-      64,              // scalars
-      0,               // (unused)
+      128,             // scalars
+      8 * C,           // accx
       4 * (size_t)LACMO_MAX_KERNEL_BINS * (LACMO_MAX_KERNEL_BINS + 1),  // Ef, row maxima
       4 * C,           // cell_order
       24 * N,          // gcopy
@@ -77,7 +113,7 @@ bool ws_carve(void* base, size_t bytes, int64_t n, int64_t nx, int64_t nz, Ws* w
   w->draw_off = (int64_t*)(b + p.off[2]);
   w->perm = (int32_t*)(b + p.off[3]);
   w->rank = (int32_t*)(b + p.off[4]);
-  w->dmxi = (double*)(b + p.off[5]);
+  w->acc64 = (long long*)(b + p.off[5]);
   w->rm_id = (int32_t*)(b + p.off[6]);
   w->rm_val = (double*)(b + p.off[7]);
   w->aux = (double*)(b + p.off[8]);
@@ -90,11 +126,12 @@ bool ws_carve(void* base, size_t bytes, int64_t n, int64_t nx, int64_t nz, Ws* w
   w->colk = (int32_t*)(b + p.off[15]);
   char* sc = b + p.off[16];
   w->flags = (uint32_t*)sc;
-  w->rm_count = (int32_t*)(sc + 4);
+  w->wr64 = (long long*)(sc + 64);
   w->cursor = (int64_t*)(sc + 8);
   w->col_step = (int64_t*)(sc + 16);
   w->total_pairs = (int64_t*)(sc + 24);
   w->nfb = (unsigned long long*)(sc + 32);
+  w->accx = (double*)(b + p.off[17]);
   w->Ef = (float*)(b + p.off[18]);
   w->cell_order = (int32_t*)(b + p.off[19]);
   w->cell_ctr = (int32_t*)(sc + 40);
@@ -144,16 +181,19 @@ Bt single(const lacmo_sips_t& sp, const lacmo_grid_t& g, const Ws& w, uint64_t s
   return B;
 }
 
-// integration.py:1095-1294
+// integration.py:1095-1294.  The SIPs are binned by cell only where a collision
+// step follows before the next position update (bin_at_end: after the loop).
 static int subloop(const Bt& B, const lacmo_params_t& p, const lacmo_draws_t& d, int no_cond,
-                   int no_col, cudaStream_t s) {
+                   int no_col, bool bin_at_end, cudaStream_t s) {
   const bool col = p.act_collisions != 0;
   if (col && no_col == 1) LCHK(launch_collide_cells(B, p, d, s));
   for (int k = 0; k < no_cond; ++k) {
     if (col && no_col > 1) LCHK(launch_collide_cells(B, p, d, s));
-    LCHK(launch_particles(B, p, p.dt_sub, p.dt_sub, false, s));
+    const bool last = k == no_cond - 1;
+    const bool bin = col && ((no_col > 1 && !last) || (last && (no_col > no_cond || bin_at_end)));
+    LCHK(launch_particles(B, p, p.dt_sub, p.dt_sub, false, bin, s));
     LCHK(launch_cell_update(B, true, s));
-    LCHK(launch_bin(B, s));
+    if (bin) LCHK(launch_bin(B, s));
   }
   if (col && no_col > no_cond) LCHK(launch_collide_cells(B, p, d, s));
   return LACMO_OK;
@@ -178,7 +218,7 @@ static int subloop_mixed(const Bt& B, const lacmo_params_t& p, const lacmo_draws
 
 // keep_binning: bin the SIPs after the step's last sub-step (single states,
 // whose entry points between steps read the binning); otherwise (mixed
-// batches) the binning is left empty (launch_fold_removals: the scan over
+// batches) the binning is left empty (launch_empty_bin: the scan over
 // zero counts): the next step bins after its half-step move anyway, and the
 // batch's between-step entry points rebin first (lacmo_batch_rebin)
 static int adv_step_mixed(const Bt& B, const lacmo_params_t& p, const lacmo_draws_t& d,
@@ -198,30 +238,34 @@ static int adv_step_mixed(const Bt& B, const lacmo_params_t& p, const lacmo_draw
   // that use it between advection steps
   LCHK(launch_particles_mixed(B, p, p.dt_sub, p.dt_sub_half, true, keep_binning, s));
   LCHK(launch_grid_acc(B, s));
-  LCHK(keep_binning ? launch_bin(B, s) : launch_fold_removals(B, s));
+  LCHK(keep_binning ? launch_bin(B, s) : launch_empty_bin(B, s));
   return LACMO_OK;
 }
 
 static int adv_step(const Bt& B, const lacmo_params_t& p, const lacmo_draws_t& d, cudaStream_t s,
                     bool keep_binning = true) {
   if (p.precision == LACMO_PRECISION_MIXED) return adv_step_mixed(B, p, d, s, keep_binning);
-  // b) x_{n+1/2} (integration.py:1474-1481)
-  LCHK(launch_move(B, p.dt_sub_half, s));
-  LCHK(launch_bin(B, s));
+  LCHK(launch_records64(B, s));
+  const bool col = p.act_collisions != 0;
+  const int nc1 = p.no_col_per_adv == 1 ? 0 : (p.no_col_per_adv == 2 ? 1 : p.scale_dt_cond);
+  const int nc2 = (p.no_col_per_adv == 1 || p.no_col_per_adv == 2) ? 1 : p.scale_dt_cond;
+  // b) x_{n+1/2} (integration.py:1474-1481); collisions before the next move
+  // need the binning
+  const bool bin = col && nc1 >= 1;
+  LCHK(launch_move(B, p.dt_sub_half, bin, s));
+  if (bin) LCHK(launch_bin(B, s));
   // c) advective increments (+ relaxation)
   LCHK(launch_advection(B, p, false, s));
-  int no_col = p.no_col_per_adv == 1 ? 0 : (p.no_col_per_adv == 2 ? 1 : p.scale_dt_cond);
-  int rc = subloop(B, p, d, p.scale_dt_cond, no_col, s);
+  int rc = subloop(B, p, d, p.scale_dt_cond, nc1, true, s);
   if (rc) return rc;
   // e) second-half increments
   LCHK(launch_advection(B, p, true, s));
-  no_col = (p.no_col_per_adv == 1 || p.no_col_per_adv == 2) ? 1 : p.scale_dt_cond;
-  rc = subloop(B, p, d, p.scale_dt_cond - 1, no_col, s);
+  rc = subloop(B, p, d, p.scale_dt_cond - 1, nc2, false, s);
   if (rc) return rc;
   // last sub-step: positions move by dt_sub/2 (integration.py:1593-1610)
-  LCHK(launch_particles(B, p, p.dt_sub, p.dt_sub_half, true, s));
+  LCHK(launch_particles(B, p, p.dt_sub, p.dt_sub_half, true, keep_binning, s));
   LCHK(launch_cell_update(B, true, s));
-  LCHK(launch_bin(B, s));   // the FP64 path counts cells in every sub-step
+  LCHK(keep_binning ? launch_bin(B, s) : launch_empty_bin(B, s));
   return LACMO_OK;
 }
 
@@ -289,8 +333,10 @@ int lacmo_particles_only(const lacmo_sips_t* sp, const lacmo_grid_t* g, const la
   if (!sips_ok(sp) || !grid_ok(g) || !prm_ok(p)) return LACMO_ERR_ARG;
   Ws w;
   if (!ws_carve(ws, bytes, sp->n, g->nx, g->nz, &w)) return LACMO_ERR_WORKSPACE;
-  LCHK(launch_particles(single(*sp, *g, w, 0), *p, dt_sub, dt_sub_pos, true,
-                        (cudaStream_t)stream));
+  const Bt B = single(*sp, *g, w, 0);
+  if (p->precision == LACMO_PRECISION_MIXED) LCHK(launch_records64(B, (cudaStream_t)stream));
+  LCHK(launch_particles(B, *p, dt_sub, dt_sub_pos, true, true, (cudaStream_t)stream));
+  LCHK(launch_clear_acc64(B, (cudaStream_t)stream));   // no cell update takes the sums
   return LACMO_OK;
 }
 
@@ -408,7 +454,8 @@ int lacmo_adv_step_begin(const lacmo_sips_t* sp, const lacmo_grid_t* g, const la
   if (!ws_carve(ws, bytes, sp->n, g->nx, g->nz, &w)) return LACMO_ERR_WORKSPACE;
   cudaStream_t s = (cudaStream_t)stream;
   const Bt B = single(*sp, *g, w, 0);
-  LCHK(launch_move(B, p->dt_sub_half, s));
+  LCHK(launch_records64(B, s));
+  LCHK(launch_move(B, p->dt_sub_half, true, s));
   LCHK(launch_bin(B, s));
   LCHK(launch_advection(B, *p, false, s));
   return LACMO_OK;
@@ -430,7 +477,8 @@ int lacmo_adv_substep(const lacmo_sips_t* sp, const lacmo_grid_t* g, const lacmo
   if (!ws_carve(ws, bytes, sp->n, g->nx, g->nz, &w)) return LACMO_ERR_WORKSPACE;
   cudaStream_t s = (cudaStream_t)stream;
   const Bt B = single(*sp, *g, w, 0);
-  LCHK(launch_particles(B, *p, p->dt_sub, dt_sub_pos, write_T_p != 0, s));
+  if (p->precision == LACMO_PRECISION_MIXED) LCHK(launch_records64(B, s));
+  LCHK(launch_particles(B, *p, p->dt_sub, dt_sub_pos, write_T_p != 0, true, s));
   LCHK(launch_cell_update(B, true, s));
   LCHK(launch_bin(B, s));
   return LACMO_OK;
@@ -748,7 +796,9 @@ int lacmo_batch_particles_only(lacmo_batch* b, const lacmo_params_t* p, void* st
   if (p->precision == LACMO_PRECISION_MIXED)
     LCHK(launch_particles_mixed(b->B, *p, p->dt_sub, p->dt_sub, false, false, (cudaStream_t)stream));
   else
-    LCHK(launch_particles(b->B, *p, p->dt_sub, p->dt_sub, false, (cudaStream_t)stream));
+    LCHK(launch_particles(b->B, *p, p->dt_sub, p->dt_sub, false, false, (cudaStream_t)stream));
+  if (p->precision != LACMO_PRECISION_MIXED)
+    LCHK(launch_clear_acc64(b->B, (cudaStream_t)stream));
   return LACMO_OK;
 }
 
@@ -774,7 +824,7 @@ int lacmo_propagate_particles_subloop_step(const lacmo_sips_t* sp, const lacmo_g
   cudaStream_t s = (cudaStream_t)stream;
   const Bt B = single(*sp, *g, w, 0);
   LCHK(launch_cell_aux(B, s));
-  LCHK(launch_particles(B, *p, dt_sub, dt_sub_pos, true, s));
+  LCHK(launch_particles(B, *p, dt_sub, dt_sub_pos, true, true, s));
   LCHK(launch_cell_update(B, false, s));
   LCHK(launch_bin(B, s));
   return LACMO_OK;

@@ -22,12 +22,17 @@
 // properties.py:429-436) becomes 1 + (kappa / 0.6) (a_w(w_s) - 1), so kappa =
 // 0.6 reproduces the reference.
 //
-// Reverse sweep per sub-step: the local partials come from forward-mode dual
-// numbers through the same formulas; the cell update's Jacobian likewise; the
-// increments' Jacobian from duals through the limited face fluxes.  Sums over
-// a cell's SIPs use atomics (FP64).
+// Reverse sweep per sub-step: the time step's map is differentiated backwards
+// through its evaluations (mass_rate_rev below), in the two-float arithmetic the
+// time step runs in (lacmo_ff.cuh); the converged step, and SIPs outside that
+// arithmetic's range, take forward-mode dual numbers in FP64.  A cell's ambient
+// terms and their derivatives by Theta and r_v are formed once per cell and
+// sub-step; the cell update's Jacobian comes from duals, the increments' from
+// duals through the limited face fluxes.  Sums over a cell's SIPs use atomics
+// (FP64).
 #include <cuda_runtime.h>
 
+#include "lacmo_ff.cuh"
 #include "lacmo_internal.cuh"
 #include "lacmo_physics.cuh"
 
@@ -278,6 +283,157 @@ __device__ __forceinline__ void cell_update(const S& Th, const S& r_v, const S& 
   *rv_out = rv1;
 }
 
+// The derivatives of a cell's terms (CellFF) by Theta (T) and r_v (r), cx and
+// ce by their logarithms
+struct CellGrad {
+  ff S_T, lcx_T, lce_T, la_T, lb_T, c1_T, c2_T;
+  ff S_r, la_r, lb_r, c2_r;
+  double pad[5];
+};
+static_assert(sizeof(CellGrad) == 128, "one line");
+
+// dt gamma and dt dgamma/dm of mass_rate_ff (ammonium sulfate, a_w - 1 scaled by
+// ks) and the reverse of its evaluation: with the adjoints gb of dt gamma and xb
+// of x = dt dgamma/dm, the adjoints of the mass (returned), of m_s, ks and of the
+// cell's terms (added to acc).  The reverse follows the forward's lines upwards;
+// with b(.) the adjoint, the products that recur are
+//   e = b(eps) eps, X = b(x_r) x_r = (b(R) R - e) / 3 (x_r = 3 m_p / (4 pi rho)),
+// and 1 / rho, 1 / m_p enter through u, e, X, x and w alone.
+struct RevAcc {
+  ff ms, ks, S, lcx, lce, la, lb, c1, c2;
+};
+__device__ __forceinline__ ff two(ff a) { return ff{2.0f * a.h, 2.0f * a.l}; }
+struct MassRate {
+  // the forward values the reverse reads
+  ff imp, im, wf, q, ipr, isg, z, R, eps, kel, am1, f2, Seq, pd, da, u, t, v, A, B, y, z3, D, iden,
+      N, E, G, k1, k2, gd, x, P;
+};
+__device__ __forceinline__ bool mass_rate_fwd(double m, double ms, ff msf, const CellFF& c, ff gdt,
+                                              double ks, ff ksf, MassRate& r) {
+  const double mp = m + ms;
+  const ff mpf = d2ff(mp);
+  r.imp = ff_rcp(mpf);
+  r.wf = ff_mul(msf, r.imp);
+  double w = ff2d(r.wf);
+  w = fma(fma(-w, mp, ms), f2d_int(r.imp.h), w);
+  r.im = ff_rcp(d2ff(m));
+  r.q = ff_mul(msf, r.im);
+  const double P = w * (((LC_PAR_WAT_ACT_AS_0 * w + LC_PAR_WAT_ACT_AS_1) * w +
+                         LC_PAR_WAT_ACT_AS_2) * w + LC_PAR_WAT_ACT_AS_3);
+  r.P = d2ff(P);
+  const double aw_m1 = ks * P;
+  r.am1 = ff_add(d2ff(aw_m1), 1.0f);   // a_w
+  ff da = ff_add(FFC(LC_PAR_WAT_ACT_DERIV_AS_1), ff_mul(FFC(LC_PAR_WAT_ACT_DERIV_AS_0), r.wf));
+  da = ff_add(FFC(LC_PAR_WAT_ACT_DERIV_AS_2), ff_mul(da, r.wf));
+  r.da = ff_add(FFC(LC_PAR_WAT_ACT_DERIV_AS_3), ff_mul(da, r.wf));
+  ff pd = ff_horner(FFC(LC_PAR_RHO_DERIV_AS_1), FFC(LC_PAR_RHO_DERIV_AS_0), r.wf);
+  r.pd = ff_horner(FFC(LC_PAR_RHO_DERIV_AS_2), pd, r.wf);
+  ff pr = ff_horner(FFC(LC_PAR_RHO_AS_1), FFC(LC_PAR_RHO_AS_0), r.wf);
+  pr = ff_horner(FFC(LC_PAR_RHO_AS_2), pr, r.wf);
+  r.ipr = ff_rcp(ff_one_plus(ff_mul(pr, r.wf)));
+  const ff sq = ff_mul(FFC(LC_PAR_SIGMA_AS), r.q);
+  const ff sg = ff_add(sq, 1.0f);
+  r.isg = ff_rcp(sg);
+  const ff xr = ff_mul(ff_mul(c.cx, mpf), r.ipr);
+  r.z = ff_icbrt(xr);
+  r.R = ff_mul(ff_mul(xr, r.z), r.z);
+  r.eps = ff_mul(ff_mul(c.ce, sg), ff_mul(r.ipr, r.z));
+  const ff em1 = ff_expm1(r.eps);
+  r.kel = ff_one_plus(em1);
+  const double sm1 = fma(1.0 + aw_m1, ff2d(em1), aw_m1);
+  r.f2 = d2ff(c.S_m1 - sm1);
+  r.Seq = ff_add(d2ff(sm1), 1.0f);
+  r.u = ff_mul(ff_mul(r.wf, r.pd), r.ipr);
+  r.t = ff_mul(ff_add(r.u, 1.0f), FFC(1.0 / 3.0));
+  r.v = ff_mul(r.R, r.t);
+  r.A = ff_add(c.la, r.R);
+  r.B = ff_add(c.lb, r.R);
+  r.y = ff_mul(ff_mul(sq, ff_add(r.q, 1.0f)), r.isg);
+  r.z3 = ff_sub(ff_add(two(r.t), -1.0f), r.y);
+  r.D = ff_sub(ff_mul(ff_mul(r.Seq, r.eps), r.z3),
+               ff_mul(ff_mul(ff_mul(r.wf, r.da), ksf), r.kel));
+  r.E = ff_mul(r.A, r.Seq);
+  r.iden = ff_rcp(ff_add(ff_mul(r.E, c.c1), ff_mul(r.B, c.c2)));
+  r.N = ff_add(ff_mul(ff_add(ff_mul(r.D, r.A), ff_mul(r.Seq, r.v)), c.c1), ff_mul(r.v, c.c2));
+  r.G = ff_mul(ff_mul(gdt, ff_mul(r.R, r.R)), r.iden);
+  r.k1 = ff_sub(two(r.t), ff_mul(r.N, r.iden));
+  r.k2 = ff_sub(ff_mul(r.f2, r.k1), r.D);
+  r.gd = ff_mul(r.G, r.f2);
+  r.x = ff_mul(ff_mul(r.G, r.imp), r.k2);
+  return r.eps.h < 0.25f;
+}
+__device__ __forceinline__ ff mass_rate_rev(const MassRate& r, const CellFF& c, ff msf, ff ksf,
+                                            ff gb, ff xb, RevAcc& acc) {
+  const ff Gi = ff_mul(r.G, r.imp);
+  const ff kb2 = ff_mul(xb, Gi);
+  // b(G) G and b(1/den) / den follow from gd, x, G and H = N / den
+  const ff xx = ff_mul(xb, r.x);                        // xb x
+  const ff GbG = ff_add(ff_mul(gb, r.gd), xx);          // b(G) G
+  ff fb2 = ff_add(ff_mul(gb, r.G), ff_mul(kb2, r.k1));
+  const ff kb1 = ff_mul(kb2, r.f2);
+  ff Db = ff_neg(kb2);
+  ff tb = two(kb1);
+  const ff Nb = ff_neg(ff_mul(kb1, r.iden));
+  // den: b(den) = -(b(G) G + b(H) H) / den, b(H) = -kb1
+  const ff H = ff_mul(r.N, r.iden);
+  const ff db = ff_neg(ff_mul(ff_sub(GbG, ff_mul(kb1, H)), r.iden));
+  ff RbR = two(GbG);                                    // b(R) R
+  const ff Q = ff_add(ff_mul(r.D, r.A), ff_mul(r.Seq, r.v));
+  const ff Qb = ff_mul(Nb, c.c1);
+  acc.c1 = ff_add(acc.c1, ff_add(ff_mul(Nb, Q), ff_mul(db, r.E)));
+  acc.c2 = ff_add(acc.c2, ff_add(ff_mul(Nb, r.v), ff_mul(db, r.B)));
+  const ff vb = ff_add(ff_mul(Nb, c.c2), ff_mul(Qb, r.Seq));
+  Db = ff_add(Db, ff_mul(Qb, r.A));
+  const ff Eb = ff_mul(db, c.c1);
+  const ff Ab = ff_add(ff_mul(Qb, r.D), ff_mul(Eb, r.Seq));
+  const ff Bb = ff_mul(db, c.c2);
+  ff Sb = ff_add(ff_mul(Qb, r.v), ff_mul(Eb, r.A));     // b(S_eq)
+  const ff DSe = ff_mul(Db, r.eps);
+  Sb = ff_add(Sb, ff_mul(DSe, r.z3));
+  const ff zb3 = ff_mul(DSe, r.Seq);
+  ff e = ff_mul(zb3, r.z3);                             // b(eps) eps
+  const ff wda = ff_mul(r.wf, r.da);
+  const ff Wb = ff_neg(ff_mul(Db, r.kel));              // b(ks w a_w')
+  ff mb1 = ff_neg(ff_mul(Db, ff_mul(wda, ksf)));        // b(expm1) through e^eps
+  tb = ff_add(tb, two(zb3));
+  // y = s q (1 + q) / (1 + s q): dy/dq = s (1 + 2q - y) / (1 + s q)
+  ff qb = ff_neg(ff_mul(ff_mul(zb3, FFC(LC_PAR_SIGMA_AS)),
+                        ff_mul(ff_sub(ff_add(two(r.q), 1.0f), r.y), r.isg)));
+  acc.la = ff_add(acc.la, Ab);
+  acc.lb = ff_add(acc.lb, Bb);
+  RbR = ff_add(RbR, ff_mul(ff_add(ff_add(Ab, Bb), ff_mul(vb, r.t)), r.R));
+  tb = ff_add(tb, ff_mul(vb, r.R));
+  const ff ub = ff_mul(tb, FFC(1.0 / 3.0));
+  const ff uw = ff_mul(ub, r.ipr);
+  ff wb = ff_mul(uw, r.pd);
+  const ff pdb = ff_mul(uw, r.wf);
+  acc.S = ff_add(acc.S, fb2);
+  const ff Sq = ff_sub(Sb, fb2);
+  const ff ab = ff_mul(Sq, r.kel);                      // b(a_w)
+  mb1 = ff_add(mb1, ff_mul(Sq, r.am1));
+  e = ff_add(e, ff_mul(ff_mul(mb1, r.kel), r.eps));
+  acc.ks = ff_add(acc.ks, ff_add(ff_mul(ab, r.P), ff_mul(Wb, wda)));
+  // a_w' and its derivative
+  ff dd = ff_add(FFC(2.0 * LC_PAR_WAT_ACT_DERIV_AS_1),
+                 ff_mul(FFC(3.0 * LC_PAR_WAT_ACT_DERIV_AS_0), r.wf));
+  dd = ff_add(FFC(LC_PAR_WAT_ACT_DERIV_AS_2), ff_mul(dd, r.wf));
+  wb = ff_add(wb, ff_mul(ksf, ff_add(ff_mul(ab, r.da),
+                                     ff_mul(Wb, ff_add(r.da, ff_mul(r.wf, dd))))));
+  acc.lce = ff_add(acc.lce, e);
+  qb = ff_add(qb, ff_mul(ff_mul(e, r.isg), FFC(LC_PAR_SIGMA_AS)));
+  const ff X = ff_mul(ff_sub(RbR, e), FFC(1.0 / 3.0));
+  acc.lcx = ff_add(acc.lcx, X);
+  // rho / rho_w: b = -(b(u) u + e + X) / (rho / rho_w)
+  const ff pb = ff_neg(ff_mul(ff_add(ff_add(ff_mul(ub, r.u), e), X), r.ipr));
+  const ff pdd = ff_add(FFC(LC_PAR_RHO_DERIV_AS_1),
+                        ff_mul(FFC(2.0 * LC_PAR_RHO_DERIV_AS_0), r.wf));
+  wb = ff_add(wb, ff_add(ff_mul(pb, r.pd), ff_mul(pdb, pdd)));
+  const ff mpb = ff_mul(r.imp, ff_sub(ff_sub(X, xx), ff_mul(wb, r.wf)));
+  const ff qm = ff_mul(qb, r.im);
+  acc.ms = ff_add(acc.ms, ff_add(ff_add(qm, ff_mul(wb, r.imp)), mpb));
+  return ff_sub(mpb, ff_mul(qm, r.q));
+}
+
 struct Args {
   int64_t n, C;
   double* m_w;          // [n] in/out
@@ -294,18 +450,85 @@ struct Args {
   double dt, ks;
   GridConst g;
   int no_iter;          // 0: implicit step to convergence, else the step's map
+  CellFF* rec;          // [C] the map's cell terms (no_iter > 0), else null
+  CellGrad* grad;       // [C] their derivatives (reverse sweep)
 };
 
-__global__ void k_fwd_sips(Args a, double* tape_m) {
+// a cell's terms for the sub-step that starts from Theta and r_v, as the time
+// step forms them, and (GRAD) their derivatives
+template <bool GRAD>
+__device__ __forceinline__ void write_cell(const Args& a, int64_t c, double Th, double rv) {
+  const double rho_d = a.rho_d[c];
+  const CellState s = cell_state64(Th, rv, rho_d, a.g.p_ref, a.g.p_ref_inv);
+  write_rec64(a.rec + c, s.T, s.S, s.L_v, s.mu, s.rho_f,
+              cell_terms64(s.T, s.p, s.e_s, s.L_v, s.K, s.D_v));
+  if (GRAD) {
+    const Amb<Dual<2>> m = ambient<Dual<2>>(var<2>(Th, 0), var<2>(rv, 1), rho_d, a.g);
+    CellGrad* const g = a.grad + c;
+    const double lr = m.rhow.d[0] / m.rhow.v;
+    g->S_T = d2ff(m.Sat.d[0]);
+    g->S_r = d2ff(m.Sat.d[1]);
+    g->lcx_T = d2ff(-lr);
+    g->lce_T = d2ff(m.sigw.d[0] / m.sigw.v - lr - m.T.d[0] / m.T.v);
+    g->la_T = d2ff(m.lap0.d[0]); g->la_r = d2ff(m.lap0.d[1]);
+    g->lb_T = d2ff(m.lbp0.d[0]); g->lb_r = d2ff(m.lbp0.d[1]);
+    g->c1_T = d2ff(m.c1.d[0]);
+    g->c2_T = d2ff(m.c2.d[0]); g->c2_r = d2ff(m.c2.d[1]);
+  }
+}
+__global__ void k_cell_terms(Args a) {
+  for (int64_t c = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; c < a.C;
+       c += (int64_t)gridDim.x * blockDim.x)
+    write_cell<false>(a, c, a.Th[c], a.r_v[c]);
+}
+__device__ __forceinline__ CellFF load_cell(const CellFF* rec) {
+  CellFF cf;
+  const float4* src = (const float4*)rec;
+  float4* dst = (float4*)&cf;
+#pragma unroll
+  for (int q = 0; q < 6; ++q) dst[q] = __ldg(src + q);
+  return cf;
+}
+
+// one condensation step in FP64: to convergence (no_iter = 0), or of a SIP
+// outside the two-float range
+__device__ __noinline__ double fwd_step64(const Args& a, int32_t c, double mw, double ms) {
+  if (a.no_iter > 0 && ff_mass_ok(mw) && ff_mass_ok(ms)) {
+    const CellState s = cell_state64(a.Th[c], a.r_v[c], a.rho_d[c], a.g.p_ref, a.g.p_ref_inv);
+    const CellTerms t = cell_terms64(s.T, s.p, s.e_s, s.L_v, s.K, s.D_v);
+    CellAmb m;
+    m.T = s.T; m.S = s.S; m.sigw = t.sigw; m.rhow = t.rhow; m.lap0 = t.lap0; m.lbp0 = t.lbp0;
+    m.c1 = t.c1; m.c2 = t.c2;
+    return newton_fast(SOL_AS, a.dt, a.no_iter, mw, ms, cell_fast(SOL_AS, m), a.ks);
+  }
+  const Amb<double> am = ambient<double>(a.Th[c], a.r_v[c], a.rho_d[c], a.g);
+  bool fl;
+  return solve_step(mw, ms, a.ks, am, a.dt, a.no_iter, &fl);
+}
+
+// The SIPs of a forward sub-step.  MAP: the time step's map as the time step runs
+// it (newton_ff), else the converged step.  Bound by FP32 issue (the two-float
+// Newton); 720,000 SIPs took 1326 us a launch with the cell's ambient terms and
+// the Newton per SIP in FP64, 190 us now (110 us once no step exceeds an eighth of
+// the mass).
+template <bool MAP>
+__global__ void __launch_bounds__(128) k_fwd_sips(const __grid_constant__ Args a, double* tape_m) {
+  const ff gdt = d2ff(LC_FOUR_PI * 1.0E12 * a.dt);
   for (int64_t k = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; k < a.n;
        k += (int64_t)gridDim.x * blockDim.x) {
     const double mw = a.m_w[k];
     if (tape_m) tape_m[k] = mw;
     const int32_t c = a.cell[k];
     if (c < 0) continue;
-    const Amb<double> am = ambient<double>(a.Th[c], a.r_v[c], a.rho_d[c], a.g);
-    bool fl;
-    const double m = solve_step(mw, a.m_s[k], a.ks, am, a.dt, a.no_iter, &fl);
+    const double ms = a.m_s[k];
+    double m;
+    if (MAP) {
+      bool ok;
+      m = newton_ff<true>(SOL_AS, a.no_iter, mw, ms, load_cell(a.rec + c), gdt, a.ks, &ok);
+      if (!ok) m = fwd_step64(a, c, mw, ms);
+    } else {
+      m = fwd_step64(a, c, mw, ms);
+    }
     a.m_w[k] = m;
     atomicAdd(a.dml + c, (m - mw) * a.xi[k]);
   }
@@ -318,11 +541,16 @@ __global__ void k_fwd_cells(Args a, double* tape_c) {
     if (tape_c) { tape_c[c] = Th; tape_c[a.C + c] = rv; }
     const double dml = a.dml[c] * 1.0E-18;
     a.dml[c] = 0.0;
-    double Th2, rv2;
-    cell_update<double, double>(Th, rv, dml, a.rho_d[c], a.mdi[c], a.dTh ? a.dTh[c] : 0.0,
-                                a.drv ? a.drv[c] : 0.0, a.g, &Th2, &rv2);
+    const double fT = a.dTh ? a.dTh[c] : 0.0, fr = a.drv ? a.drv[c] : 0.0;
+    double Th2 = Th, rv2 = rv;
+    if (a.rec)
+      cell_step64(&Th2, &rv2, a.rho_d[c], a.mdi[c], a.rec[c].L_v, fT, fr, dml, a.g.V,
+                  a.g.p_ref_inv);
+    else
+      cell_update<double, double>(Th, rv, dml, a.rho_d[c], a.mdi[c], fT, fr, a.g, &Th2, &rv2);
     a.Th[c] = Th2;
     a.r_v[c] = rv2;
+    if (a.rec) write_cell<false>(a, c, Th2, rv2);
   }
 }
 
@@ -338,6 +566,7 @@ __global__ void k_bwd_cells(Args a, const double* tape_c, const double* m_before
   for (int64_t c = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; c < a.C;
        c += (int64_t)gridDim.x * blockDim.x) {
     const double Th = tape_c[c], rv = tape_c[a.C + c];
+    if (a.rec) write_cell<true>(a, c, Th, rv);
     const double dml = a.dml[c] * 1.0E-18;   // recomputed forward sum of this sub-step
     const double fT = a.dTh ? a.dTh[c] : 0.0, fr = a.drv ? a.drv[c] : 0.0;
     Dual<5> Th2, rv2;
@@ -363,55 +592,135 @@ __global__ void k_bwd_sum_dml(Args a, const double* m_before, const double* m_af
   }
 }
 
-__global__ void k_bwd_sips(Args a, const double* tape_c, const double* m_before,
-                           const double* m_after, double* lam_m, const double* lam_dml,
-                           double* lam_Th_pre, double* lam_rv_pre, double* grad_ms,
-                           double* grad_ks) {
+// the partial derivatives of a SIP's new mass by m_w, m_s, ks, Theta and r_v
+struct SipGrad {
+  double m, ms, ks, Th, rv;
+};
+// in FP64 by duals: the time step's map (no_iter > 0), differentiated exactly
+__device__ __noinline__ SipGrad map_grad64(const Args& a, double Th, double rv, double rho_d,
+                                           double mw, double ms) {
+  const Amb<Dual<5>> am = ambient<Dual<5>>(var<5>(Th, 3), var<5>(rv, 4), rho_d, a.g);
+  const Dual<5> mn = newton_map<Dual<5>>(var<5>(mw, 0), var<5>(ms, 1), var<5>(a.ks, 2), am, a.dt,
+                                         a.no_iter);
+  return SipGrad{mn.d[0], mn.d[1], mn.d[2], mn.d[3], mn.d[4]};
+}
+// the converged step: implicit-function theorem
+__device__ __noinline__ SipGrad root_grad64(const Args& a, double Th, double rv, double rho_d,
+                                            double m, double ms) {
+  const double m_eff = ms * (LC_W_S_MAX_AS_INV - 1.0);
+  if (!(m > m_eff)) return SipGrad{0.0, LC_W_S_MAX_AS_INV - 1.0, 0.0, 0.0, 0.0};
+  const Amb<Dual<4>> am = ambient<Dual<4>>(var<4>(Th, 2), var<4>(rv, 3), rho_d, a.g);
+  double dg;
+  {
+    const Amb<double> a0 = ambient<double>(Th, rv, rho_d, a.g);
+    mass_rate<double>(m, ms, a.ks, a0, &dg);
+  }
+  const Dual<4> gam = mass_rate<Dual<4>>(m, var<4>(ms, 0), var<4>(a.ks, 1), am, nullptr);
+  const double inv = 1.0 / (1.0 - a.dt * dg), t = a.dt * inv;
+  return SipGrad{inv, t * gam.d[0], t * gam.d[1], t * gam.d[2], t * gam.d[3]};
+}
+
+// The time step's map backwards: the masses m_1 .. m_{no_iter - 1} forwards
+// (newton_ff's), then from the last evaluation to the first.  An evaluation is
+//   m_{i+1} = max(m_eff, m_i + (dt gamma_i + m_w - m_i) / (1 - x_i)), m_0 = m_w.
+constexpr int REV_MAX = 8;   // evaluations held; more take map_grad64
+__device__ __forceinline__ bool map_grad(const Args& a, const CellFF& cf, const CellGrad* gr, ff gdt,
+                                         double mw, double ms, SipGrad* out) {
+  const double floor_m = ms * (LC_W_S_MAX_AS_INV - 1.0);
+  const ff msf = d2ff(ms), ksf = d2ff(a.ks);
+  double mi[REV_MAX];
+  bool good = ff_mass_ok(mw) && ff_mass_ok(ms);
+  {
+    double m = mw;
+#pragma unroll 1
+    for (int it = 0; it < a.no_iter - 1; ++it) {
+      mi[it] = m;
+      ff gd, x;
+      good = mass_rate_ff<true>(SOL_AS, false, m, ms, msf, cf, gdt, a.ks, gd, x) && good;
+      const ff res = it == 0 ? gd : ff_sub(gd, d2ff(m - mw));
+      m = np_max(floor_m, m + ff2d(ff_mul(res, damp_ff(x))));
+    }
+    mi[a.no_iter - 1] = m;
+    good = good && m < 1e29;
+  }
+  const ff zero = {0.0f, 0.0f};
+  RevAcc acc = {zero, zero, zero, zero, zero, zero, zero, zero, zero};
+  ff mu = {1.0f, 0.0f};       // adjoint of m_{i+1}
+  ff m0b = zero;              // of m_w, beyond m_0's
+#pragma unroll 1
+  for (int it = a.no_iter - 1; it >= 0; --it) {
+    const double m = mi[it];
+    MassRate r;
+    good = mass_rate_fwd(m, ms, msf, cf, gdt, a.ks, ksf, r) && good;
+    const ff dn = damp_ff(r.x);
+    const ff res = it == 0 ? r.gd : ff_sub(r.gd, d2ff(m - mw));
+    const double mn = m + ff2d(ff_mul(res, dn));
+    if (!(mn >= floor_m)) {   // floored: only m_s is left
+      acc.ms = ff_add(acc.ms, ff_mul(mu, FFC(LC_W_S_MAX_AS_INV - 1.0)));
+      mu = zero;
+      break;
+    }
+    const ff gb = ff_mul(mu, dn);
+    ff xb = ff_mul(ff_mul(gb, dn), res);
+    if (!(r.x.h < 0.9f)) xb = zero;
+    const ff mb = mass_rate_rev(r, cf, msf, ksf, gb, xb, acc);
+    if (it > 0) {
+      m0b = ff_add(m0b, gb);
+      mu = ff_add(ff_sub(mu, gb), mb);
+    } else {
+      mu = ff_add(mu, mb);
+    }
+  }
+  auto ld = [&](int q) { const float2 v = __ldg((const float2*)gr + q); return ff{v.x, v.y}; };
+  ff T = ff_add(ff_mul(acc.S, ld(0)), ff_mul(acc.lcx, ld(1)));
+  T = ff_add(T, ff_add(ff_mul(acc.lce, ld(2)), ff_mul(acc.la, ld(3))));
+  T = ff_add(T, ff_add(ff_mul(acc.lb, ld(4)), ff_mul(acc.c1, ld(5))));
+  T = ff_add(T, ff_mul(acc.c2, ld(6)));
+  ff V = ff_add(ff_mul(acc.S, ld(7)), ff_mul(acc.la, ld(8)));
+  V = ff_add(V, ff_add(ff_mul(acc.lb, ld(9)), ff_mul(acc.c2, ld(10))));
+  *out = SipGrad{ff2d(ff_add(mu, m0b)), ff2d(acc.ms), ff2d(acc.ks), ff2d(T), ff2d(V)};
+  return good;
+}
+
+// The SIPs of a reverse sub-step.  Bound by FP32 issue at 8 warps an SM (255
+// registers hold an evaluation's forward values); 720,000 SIPs took 4330 us a
+// launch with duals of five directions through the ambient terms and the
+// evaluations in FP64, 276 us now.
+template <bool MAP>
+__global__ void __launch_bounds__(128) k_bwd_sips(const __grid_constant__ Args a,
+                                                  const double* tape_c, const double* m_before,
+                                                  const double* m_after, double* lam_m,
+                                                  const double* lam_dml, double* lam_Th_pre,
+                                                  double* lam_rv_pre, double* grad_ms,
+                                                  double* grad_ks) {
   double gk = 0.0;
+  const ff gdt = d2ff(LC_FOUR_PI * 1.0E12 * a.dt);
   for (int64_t k = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; k < a.n;
        k += (int64_t)gridDim.x * blockDim.x) {
     const int32_t c = a.cell[k];
     if (c < 0) continue;   // not condensing: m_w passes through
-    const double xi = a.xi[k];
-    const double m = m_after[k];
     const double ms = a.m_s[k];
+    SipGrad g;
+    if (MAP) {
+      const double mw = m_before[k];
+      if (a.no_iter > REV_MAX ||
+          !map_grad(a, load_cell(a.rec + c), a.grad + c, gdt, mw, ms, &g))
+        g = map_grad64(a, tape_c[c], tape_c[a.C + c], a.rho_d[c], mw, ms);
+    } else {
+      g = root_grad64(a, tape_c[c], tape_c[a.C + c], a.rho_d[c], m_after[k], ms);
+    }
     // total adjoint of the new mass: the state after, and the cell sum
-    const double lm = lam_m[k] + lam_dml[c] * xi;
-    if (a.no_iter > 0) {   // the time step's map, differentiated exactly
-      const double Th = tape_c[c], rv = tape_c[a.C + c];
-      const Amb<Dual<5>> am = ambient<Dual<5>>(var<5>(Th, 3), var<5>(rv, 4), a.rho_d[c], a.g);
-      const Dual<5> mn = newton_map<Dual<5>>(var<5>(m_before[k], 0), var<5>(ms, 1),
-                                             var<5>(a.ks, 2), am, a.dt, a.no_iter);
-      grad_ms[k] += lm * mn.d[1];
-      gk += lm * mn.d[2] * (1.0 / 0.6);
-      atomicAdd(lam_Th_pre + c, lm * mn.d[3]);
-      atomicAdd(lam_rv_pre + c, lm * mn.d[4]);
-      lam_m[k] = lm * mn.d[0] - lam_dml[c] * xi;
-      continue;
-    }
-    const double m_eff = ms * (LC_W_S_MAX_AS_INV - 1.0);
-    if (!(m > m_eff)) {
-      grad_ms[k] += lm * (LC_W_S_MAX_AS_INV - 1.0);
-      lam_m[k] = -lam_dml[c] * xi;
-      continue;
-    }
-    const double Th = tape_c[c], rv = tape_c[a.C + c];
-    const Amb<Dual<4>> am = ambient<Dual<4>>(var<4>(Th, 2), var<4>(rv, 3), a.rho_d[c], a.g);
-    double dg;
-    {
-      const Amb<double> a0 = ambient<double>(Th, rv, a.rho_d[c], a.g);
-      mass_rate<double>(m, ms, a.ks, a0, &dg);
-    }
-    const Dual<4> gam = mass_rate<Dual<4>>(m, var<4>(ms, 0), var<4>(a.ks, 1), am, nullptr);
-    const double inv = 1.0 / (1.0 - a.dt * dg);
-    const double t = lm * a.dt * inv;
-    grad_ms[k] += t * gam.d[0];
-    gk += t * gam.d[1] * (1.0 / 0.6);   // ks = kappa / 0.6
-    atomicAdd(lam_Th_pre + c, t * gam.d[2]);
-    atomicAdd(lam_rv_pre + c, t * gam.d[3]);
-    lam_m[k] = lm * inv - lam_dml[c] * xi;
+    const double ld = lam_dml[c] * a.xi[k];
+    const double lm = lam_m[k] + ld;
+    grad_ms[k] += lm * g.ms;
+    gk += lm * g.ks * (1.0 / 0.6);   // ks = kappa / 0.6
+    atomicAdd(lam_Th_pre + c, lm * g.Th);
+    atomicAdd(lam_rv_pre + c, lm * g.rv);
+    lam_m[k] = lm * g.m - ld;
   }
-  if (gk != 0.0) atomicAdd(grad_ks, gk);
+#pragma unroll
+  for (int off = 16; off > 0; off >>= 1) gk += __shfl_down_sync(0xffffffffu, gk, off);
+  if ((threadIdx.x & 31) == 0 && gk != 0.0) atomicAdd(grad_ks, gk);
 }
 
 // ---- advective increments of Theta and r_v (integration.py:80-287 with the
@@ -640,6 +949,7 @@ static Args make_args(int64_t n, int64_t C, double* m_w, const double* m_s, cons
   a.rho_d = rho_d; a.mdi = mdi; a.dTh = dTh; a.drv = drv; a.dml = dml; a.dt = dt;
   a.ks = kappa / 0.6;
   a.g.p_ref = p_ref; a.g.p_ref_inv = 1.0 / p_ref; a.g.V = V;
+  a.rec = nullptr; a.grad = nullptr;
   return a;
 }
 
@@ -658,10 +968,19 @@ int lacmo_adj_forward(int64_t n, int64_t C, double* m_w, const double* m_s, cons
   Args a = make_args(n, C, m_w, m_s, xi, cell, Th, r_v, rho_d, mdi, dTh, drv, dml, dt_sub, kappa,
                      p_ref, V, no_iter);
   if (cudaMemsetAsync(dml, 0, 8 * C, s) != cudaSuccess) return LACMO_ERR_CUDA;
+  Scratch scratch(s);
+  if (no_iter > 0 && n_sub > 0) {
+    a.rec = (CellFF*)scratch.get(sizeof(CellFF) * (size_t)C);
+    if (!a.rec) return LACMO_ERR_CUDA;
+    k_cell_terms<<<nb(C, 32), 32, 0, s>>>(a);
+    note_launches(1);
+  }
   for (int k = 0; k < n_sub; ++k) {
     a.cell = cell + (size_t)k * cell_stride;
-    k_fwd_sips<<<nb(n, 128), 128, 0, s>>>(a, tape_m ? tape_m + (size_t)k * n : nullptr);
-    k_fwd_cells<<<nb(C, 64), 64, 0, s>>>(a, tape_c ? tape_c + (size_t)k * 2 * C : nullptr);
+    double* const tm = tape_m ? tape_m + (size_t)k * n : nullptr;
+    if (a.rec) k_fwd_sips<true><<<nb(n, 128), 128, 0, s>>>(a, tm);
+    else k_fwd_sips<false><<<nb(n, 128), 128, 0, s>>>(a, tm);
+    k_fwd_cells<<<nb(C, 32), 32, 0, s>>>(a, tape_c ? tape_c + (size_t)k * 2 * C : nullptr);
     note_launches(2);
   }
   if (tape_m) {   // the state after the last sub-step closes the tape
@@ -687,15 +1006,25 @@ int lacmo_adj_backward(int64_t n, int64_t C, const double* m_s, const double* xi
   Args a = make_args(n, C, nullptr, m_s, xi, cell, nullptr, nullptr, rho_d, mdi, dTh, drv, dml,
                      dt_sub, kappa, p_ref, V, no_iter);
   if (cudaMemsetAsync(dml, 0, 8 * C, s) != cudaSuccess) return LACMO_ERR_CUDA;
+  Scratch scratch(s);
+  if (no_iter > 0 && n_sub > 0) {
+    a.rec = (CellFF*)scratch.get((sizeof(CellFF) + sizeof(CellGrad)) * (size_t)C);
+    if (!a.rec) return LACMO_ERR_CUDA;
+    a.grad = (CellGrad*)(a.rec + C);
+  }
   for (int k = n_sub - 1; k >= 0; --k) {
     a.cell = cell + (size_t)k * cell_stride;
     const double* mb = tape_m + (size_t)k * n;
     const double* ma = tape_m + (size_t)(k + 1) * n;
     const double* tc = tape_c + (size_t)k * 2 * C;
     k_bwd_sum_dml<<<nb(n, 128), 128, 0, s>>>(a, mb, ma);
-    k_bwd_cells<<<nb(C, 64), 64, 0, s>>>(a, tc, mb, ma, lam_Th, lam_rv, lam_dml, lam_inc);
-    k_bwd_sips<<<nb(n, 128), 128, 0, s>>>(a, tc, mb, ma, lam_m, lam_dml, lam_Th, lam_rv, grad_ms,
-                                          grad_kappa);
+    k_bwd_cells<<<nb(C, 32), 32, 0, s>>>(a, tc, mb, ma, lam_Th, lam_rv, lam_dml, lam_inc);
+    if (a.rec)
+      k_bwd_sips<true><<<nb(n, 128), 128, 0, s>>>(a, tc, mb, ma, lam_m, lam_dml, lam_Th, lam_rv,
+                                                  grad_ms, grad_kappa);
+    else
+      k_bwd_sips<false><<<nb(n, 128), 128, 0, s>>>(a, tc, mb, ma, lam_m, lam_dml, lam_Th, lam_rv,
+                                                   grad_ms, grad_kappa);
     note_launches(3);
   }
   return cudaGetLastError() == cudaSuccess ? LACMO_OK : LACMO_ERR_CUDA;

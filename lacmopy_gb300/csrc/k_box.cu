@@ -38,7 +38,6 @@
 #include <cuda_runtime.h>
 
 #include <atomic>
-#include <mutex>
 
 #include "lacmo_colmath.cuh"
 
@@ -436,34 +435,6 @@ __global__ void __launch_bounds__(BOX_THREADS) k_box_step(const BoxArgs a) {
   }
 }
 
-// Scratch of the screened steps: a few hundred kilobytes, stream-ordered, from
-// a pool of this library's own on each device (at most 16 MB of it stay with the
-// pool at a synchronisation; the rest goes back).  Calls on different streams
-// get different memory and wait for nothing of each other.
-cudaMemPool_t box_pool(int dev) {
-  static std::mutex mu;
-  static cudaMemPool_t pools[64];
-  if (dev < 0 || dev >= 64) return nullptr;
-  std::lock_guard<std::mutex> lock(mu);
-  if (!pools[dev]) {
-    cudaMemPoolProps props = {};
-    props.allocType = cudaMemAllocationTypePinned;
-    props.location.type = cudaMemLocationTypeDevice;
-    props.location.id = dev;
-    cudaMemPool_t p = nullptr;
-    if (cudaMemPoolCreate(&p, &props) != cudaSuccess) {
-      cudaGetLastError();
-      return nullptr;
-    }
-    uint64_t keep = 16ull << 20;
-    int off = 0;
-    cudaMemPoolSetAttribute(p, cudaMemPoolAttrReleaseThreshold, &keep);
-    cudaMemPoolSetAttribute(p, cudaMemPoolReuseAllowInternalDependencies, &off);
-    pools[dev] = p;
-  }
-  return pools[dev];
-}
-
 template <int KIND>
 cudaError_t launch_box(BoxArgs a, cudaStream_t s) {
   constexpr size_t step_sip = KIND == BOX_GOLOVIN ? 16 : (KIND == BOX_KGRID ? 20 : 44);
@@ -490,15 +461,13 @@ cudaError_t launch_box(BoxArgs a, cudaStream_t s) {
   a.screened = 0;
   a.count = nullptr; a.cand = nullptr; a.f = nullptr; a.bin = nullptr; a.erow = nullptr;
   a.dtdv_f = (float)a.dtdv;
-  char* scratch = nullptr;
+  Scratch mem(s);
   if (P > BOX_SELF) {
     const size_t rows = KIND == BOX_GOLOVIN ? 0 : (size_t)a.nb;
     const size_t per = KIND == BOX_GOLOVIN ? 0 : 20;
     const size_t bytes = 256 + 4 * BOX_CAND + per * (size_t)a.n + 4 * rows;
-    cudaMemPool_t pool = box_pool(dev);
-    void* p = nullptr;
-    if (pool && cudaMallocFromPoolAsync(&p, bytes, pool, s) == cudaSuccess) {
-      scratch = (char*)p;
+    char* const scratch = (char*)mem.get(bytes);
+    if (scratch) {   // without, the one CTA runs the diagonals
       a.count = (uint32_t*)scratch;
       a.cand = (uint32_t*)(scratch + 256);
       if (KIND != BOX_GOLOVIN) {
@@ -507,8 +476,6 @@ cudaError_t launch_box(BoxArgs a, cudaStream_t s) {
         a.erow = (float*)(a.bin + a.n);
       }
       a.screened = 1;
-    } else {
-      cudaGetLastError();   // without scratch the one CTA runs the diagonals
     }
   }
   if (a.screened) {
@@ -534,10 +501,6 @@ cudaError_t launch_box(BoxArgs a, cudaStream_t s) {
     k_box_step<KIND><<<1, BOX_THREADS, step_sip * (size_t)a.n + 4 * BOX_CAND, s>>>(a);
     note_launches(1);
     e = cudaGetLastError();
-  }
-  if (scratch) {
-    const cudaError_t f = cudaFreeAsync(scratch, s);
-    if (e == cudaSuccess) e = f;
   }
   return e;
 }

@@ -91,9 +91,7 @@ static int diag_run(DiagArgs d, void* ws, size_t bytes, cudaStream_t s) {
   Ws w;
   if (!ws_carve(ws, bytes, d.n, d.nx, d.nz, &w)) return LACMO_ERR_WORKSPACE;
   const int64_t C = d.nx * d.nz;
-  if (cudaMemsetAsync(w.counts, 0, 4 * (size_t)C, s) != cudaSuccess ||
-      cudaMemsetAsync(w.rm_count, 0, 4, s) != cudaSuccess)
-    return LACMO_ERR_CUDA;
+  if (cudaMemsetAsync(w.counts, 0, 4 * (size_t)C, s) != cudaSuccess) return LACMO_ERR_CUDA;
   lacmo_sips_t sp = {};
   sp.n = d.n; sp.cell = (int32_t*)d.cell;
   lacmo_grid_t g = {};

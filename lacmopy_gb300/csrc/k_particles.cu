@@ -9,16 +9,17 @@
 // cell re-index (integration.py:509-550).  It reads each SIP attribute once
 // and writes it once; grid data come from small L2-resident arrays.
 //
-// Order-dependent sums the reference accumulates in ascending SIP ID (the
-// per-cell condensed mass delta_m_l, integration.py:916-936, and
-// water_removed, integration.py:620-628) are formed here in the same order:
-// k_cell_update folds each cell's dm*xi over the cell's SIPs sorted by ID, and
-// the removal list is sorted by ID before it is folded.  Results are therefore
-// deterministic and, given identical per-SIP values, equal to the reference's.
+// Sums the reference accumulates in ascending SIP ID (the per-cell condensed
+// mass delta_m_l, integration.py:916-936, and water_removed, :620-628) are exact
+// 128-bit integer sums here (acc_add64), rounded to FP64 once: independent of
+// the order, so a step gives the same bits run to run and batched or not, within
+// the rounding of the reference's sequential sums, and no sub-step needs its
+// SIPs sorted.
 #include <cuda_runtime.h>
 
 #include <atomic>
 
+#include "lacmo_ff.cuh"
 #include "lacmo_internal.cuh"
 #include "lacmo_physics.cuh"
 
@@ -61,16 +62,19 @@ __global__ void k_cells_export(const int32_t* __restrict__ cell, const double* _
 // per-cell terms of the mass rate for the next sub-step; their FP32 copies in
 // the cell records (cell_records) feed the mixed-precision kernel without
 // double->float conversions there
-__device__ __forceinline__ void write_aux(const double* gsf, const double* gmp, double* aux,
-                                          int64_t c, int64_t C) {
-  CellAmb a = make_cell_amb(gsf[c], gsf[C + c], gsf[6 * C + c], gsf[7 * C + c], gmp[2 * C + c],
-                            gmp[c], gmp[C + c]);
-  aux[c] = a.sigw; aux[C + c] = a.rhow; aux[2 * C + c] = a.lap0; aux[3 * C + c] = a.lbp0;
-  aux[4 * C + c] = a.c1; aux[5 * C + c] = a.c2;
+// a cell's terms and records from its fields; returns its surface tension of water
+__device__ __forceinline__ double write_terms(double* aux, int64_t c, int64_t C, double T,
+                                              double p, double S, double e_s, double L_v,
+                                              double K, double D_v, double mu, double rho_f) {
+  const CellTerms t = cell_terms64(T, p, e_s, L_v, K, D_v);
+  aux[c] = t.sigw; aux[C + c] = t.rhow; aux[2 * C + c] = t.lap0; aux[3 * C + c] = t.lbp0;
+  aux[4 * C + c] = t.c1; aux[5 * C + c] = t.c2;
   float4* af = cell_records(aux, C) + CELL_REC * c;
-  af[0] = make_float4((float)a.T, (float)(a.S - 1.0), (float)a.sigw, (float)a.rhow);
-  af[1] = make_float4((float)a.lap0, (float)a.lbp0, (float)a.c1, (float)a.c2);
-  af[2] = make_float4((float)gmp[5 * C + c], (float)gmp[6 * C + c], 0.0f, 0.0f);
+  af[0] = make_float4((float)T, (float)(S - 1.0), (float)t.sigw, (float)t.rhow);
+  af[1] = make_float4((float)t.lap0, (float)t.lbp0, (float)t.c1, (float)t.c2);
+  af[2] = make_float4((float)mu, (float)rho_f, 0.0f, 0.0f);
+  write_rec64(cell_rec64(aux, C) + 2 * c, T, S, L_v, mu, rho_f, t);
+  return t.sigw;
 }
 
 __global__ void k_cell_aux(const __grid_constant__ MRef mr) {
@@ -80,7 +84,8 @@ __global__ void k_cell_aux(const __grid_constant__ MRef mr) {
   double* aux = mb.w.aux;
   for (int64_t c = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; c < C;
        c += (int64_t)gridDim.x * blockDim.x)
-    write_aux(gsf, gmp, aux, c, C);
+    write_terms(aux, c, C, gsf[c], gsf[C + c], gsf[6 * C + c], gsf[7 * C + c], gmp[2 * C + c],
+                gmp[c], gmp[C + c], gmp[5 * C + c], gmp[6 * C + c]);
 }
 
 // ---------------------------------------------------------------------------
@@ -100,70 +105,16 @@ __global__ void k_histogram(const __grid_constant__ MRef mr) {
   }
 }
 
-// Single block: folds the sorted ground-removal list into water_removed, then
-// the exclusive scans of the SIP counts (slots) and pair counts (draws).
+// Single block: the exclusive scans of the SIP counts (slots) and pair counts
+// (draws), and the collision work order.
 __global__ void __launch_bounds__(1024) k_scan(const __grid_constant__ MRef mr) {
   const Member& mb = mr.get();
-  int32_t *counts = mb.w.counts, *start = mb.w.start, *rm_count = mb.w.rm_count,
-          *rm_id = mb.w.rm_id;
+  int32_t *counts = mb.w.counts, *start = mb.w.start;
   int64_t *draw_off = mb.w.draw_off, *total_pairs = mb.w.total_pairs;
-  double *rm_val = mb.w.rm_val, *water_removed = mb.sp.water_removed;
   const int64_t C = mb.g.nx * mb.g.nz;
   __shared__ int64_t s_slot[1024];
   __shared__ int64_t s_pair[1024];
-  __shared__ int32_t s_id[2048];
-  __shared__ double s_val[2048];
   const int t = threadIdx.x;
-  // ---- ground removals, ascending ID (integration.py:620-628) ----
-  int nrm = *rm_count;
-  if (nrm > 0 && nrm <= 2048) {
-    int P = 1;
-    while (P < nrm) P <<= 1;
-    for (int q = t; q < P; q += blockDim.x) {
-      s_id[q] = q < nrm ? rm_id[q] : 0x7fffffff;
-      s_val[q] = q < nrm ? rm_val[q] : 0.0;
-    }
-    __syncthreads();
-    for (int kk = 2; kk <= P; kk <<= 1) {
-      for (int jj = kk >> 1; jj > 0; jj >>= 1) {
-        for (int q = t; q < P; q += blockDim.x) {
-          int p2 = q ^ jj;
-          if (p2 > q) {
-            bool up = ((q & kk) == 0);
-            int a = s_id[q], b = s_id[p2];
-            if ((a > b) == up) {
-              s_id[q] = b; s_id[p2] = a;
-              double v = s_val[q]; s_val[q] = s_val[p2]; s_val[p2] = v;
-            }
-          }
-        }
-        __syncthreads();
-      }
-    }
-    if (t == 0) {
-      double wr = water_removed[0];
-      for (int q = 0; q < nrm; ++q) wr += s_val[q];
-      water_removed[0] = wr;
-    }
-    __syncthreads();
-  } else if (nrm > 2048) {
-    // rare: repeated extraction of the smallest remaining ID
-    if (t == 0) {
-      double wr = water_removed[0];
-      int32_t last = -1;
-      for (int r = 0; r < nrm; ++r) {
-        int32_t best = 0x7fffffff; int bq = -1;
-        for (int q = 0; q < nrm; ++q)
-          if (rm_id[q] > last && rm_id[q] < best) { best = rm_id[q]; bq = q; }
-        wr += rm_val[bq];
-        last = best;
-      }
-      water_removed[0] = wr;
-    }
-    __syncthreads();
-  }
-  if (t == 0) *rm_count = 0;
-  // ---- scans ----
   int64_t chunk = (C + blockDim.x - 1) / blockDim.x;
   int64_t b0 = t * chunk, b1 = b0 + chunk < C ? b0 + chunk : C;
   int64_t ss = 0, sp = 0;
@@ -345,9 +296,9 @@ struct PArgs {
   double x_min, x_max, z_min, z_cap, dx, dz;
   double dt_sub, dt_pos, g_set;
   int no_iter, sol, write_Tp;
-  double* dmxi;
-  int32_t *counts, *rank, *rm_count, *rm_id;
-  double* rm_val;
+  int32_t *counts, *rank;
+  long long *acc64, *wr64;      // FP64: per-cell and water sums (acc_add64)
+  double* accx;                 // FP64: values beyond their range
   // mixed precision: SIPs whose Newton repeats in FP64 (k_newton_fallback),
   // queued in scratch that mixed sub-steps leave unused
   int32_t *fb_count, *fb_done, *fb_id, *fb_c;
@@ -388,8 +339,8 @@ __device__ __forceinline__ PArgs make_pargs(const Member& mb, const PCall& c) {
   a.dx = g.dx; a.dz = g.dz;
   a.dt_sub = c.dt_sub; a.dt_pos = c.dt_pos; a.g_set = c.g_set;
   a.no_iter = c.no_iter; a.sol = c.sol; a.write_Tp = c.write_Tp;
-  a.dmxi = w.dmxi; a.counts = w.counts; a.rank = w.rank; a.rm_count = w.rm_count;
-  a.rm_id = w.rm_id; a.rm_val = w.rm_val; a.flags = w.flags;
+  a.counts = w.counts; a.rank = w.rank; a.flags = w.flags;
+  a.acc64 = w.acc64; a.wr64 = w.wr64; a.accx = w.accx;
   a.fb_count = w.fb_count; a.fb_done = w.fb_done; a.fb_id = w.rm_id; a.fb_c = w.colk;
   a.fb_mw = w.rm_val;
   a.acc = w.div; a.hist = c.hist; a.nfb = w.nfb;
@@ -455,171 +406,382 @@ __device__ __forceinline__ void interp_wind(const float4 w0, const float4 w1, co
   }
 }
 
+// The records of the FP64 kernel at the start of a step: the thermodynamic terms
+// from the cell's fields and per-cell terms (the cell update rewrites them every
+// sub-step), and its wind (grid.py:257-323): the values the bilinear interpolation starts from and the differences between its corners
+// (indices below zero wrap as in k_wind_table).
+__global__ void k_records64(const __grid_constant__ MRef mr) {
+  const Member& mb = mr.get();
+  const double *gsf = mb.g.scalar_fields, *gmp = mb.g.mat_prop, *aux = mb.w.aux;
+  const double* in = mb.g.velocity;
+  const int64_t nx = mb.g.nx, nz = mb.g.nz, C = nx * nz;
+  WindFF* rec = (WindFF*)cell_rec64(mb.w.aux, C);
+  for (int64_t c = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; c < C;
+       c += (int64_t)gridDim.x * blockDim.x) {
+    const int64_t i = c / nz, j = c - i * nz;
+    auto at = [&](int comp, int64_t ii, int64_t jj) {
+      if (ii < 0) ii += nx + 1;
+      if (jj < 0) jj += nz + 1;
+      return in[((int64_t)comp * (nx + 1) + ii) * (nz + 1) + jj];
+    };
+    WindFF w;
+    w.U0[0] = at(0, i, j - 1); w.U0[1] = at(0, i, j);
+    for (int b = 0; b < 3; ++b) w.dxU[b] = at(0, i + 1, j - 1 + b) - at(0, i, j - 1 + b);
+    for (int b = 0; b < 2; ++b) w.dyU[b] = at(0, i, j + b) - at(0, i, j - 1 + b);
+    w.V0[0] = at(1, i - 1, j); w.V0[1] = at(1, i, j);
+    for (int a = 0; a < 3; ++a) w.dyV[a] = at(1, i - 1 + a, j + 1) - at(1, i - 1 + a, j);
+    for (int a = 0; a < 2; ++a) w.dxV[a] = at(1, i + a, j) - at(1, i - 1 + a, j);
+    w.i = (int32_t)i; w.j = (int32_t)j;
+    w.edge = (j == 0 ? 1 : 0) | (j == nz - 1 ? 2 : 0);
+    w.pad = 0;
+    rec[2 * c + 1] = w;
+    write_rec64(cell_rec64(mb.w.aux, C) + 2 * c, gsf[c], gsf[6 * C + c], gmp[2 * C + c],
+                gmp[5 * C + c], gmp[6 * C + c],
+                CellTerms{aux[c], aux[C + c], aux[2 * C + c], aux[3 * C + c], aux[4 * C + c],
+                          aux[5 * C + c]});
+  }
+}
+__global__ void k_clear_acc64(const __grid_constant__ MRef mr) {
+  const Member& mb = mr.get();
+  const int64_t C = mb.g.nx * mb.g.nz;
+  for (int64_t c = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; c < C;
+       c += (int64_t)gridDim.x * blockDim.x) {
+    mb.w.acc64[2 * c] = 0;
+    mb.w.acc64[2 * c + 1] = 0;
+    mb.w.accx[c] = 0.0;
+  }
+}
+
+// ---- exact sums of FP64 values as 128-bit integers in units of 2^-40 (fg):
+// v = hi 2^2 + lo 2^-40 with 0 <= |lo| < 2^42, each part summed by a 64-bit
+// integer atomic (executed by L2, in any order).  A sum holds 2^21 values of
+// magnitude below 2^60; what lies beyond, infinities and NaN go to a plain FP64
+// sum (over).
+constexpr int ACC64_LO = 42;
+__device__ __forceinline__ void acc_add64(long long* acc, double* over, double v) {
+  const uint64_t b = (uint64_t)__double_as_longlong(v);
+  const int e = (int)((b >> 52) & 0x7ffu);
+  if (e >= 1023 + 60) {
+    atomicAdd(over, v);
+    return;
+  }
+  const int sh = e - 1075 + 40;   // v 2^40 = m 2^sh
+  if (sh <= -54 || e == 0) return;   // rounds to zero
+  const uint64_t m = (b & 0x000fffffffffffffull) | 0x0010000000000000ull;
+  uint64_t lo, hi;
+  if (sh < 0) {
+    const uint64_t r = (m + (1ull << (-sh - 1))) >> (-sh);
+    lo = r & ((1ull << ACC64_LO) - 1);
+    hi = r >> ACC64_LO;
+  } else {
+    lo = sh < ACC64_LO ? (m << sh) & ((1ull << ACC64_LO) - 1) : 0;
+    hi = sh <= ACC64_LO ? m >> (ACC64_LO - sh) : m << (sh - ACC64_LO);
+  }
+  if (b >> 63) { lo = 0 - lo; hi = 0 - hi; }
+  if (lo) atomicAdd((unsigned long long*)acc + 1, (unsigned long long)lo);
+  if (hi) atomicAdd((unsigned long long*)acc, (unsigned long long)hi);
+}
+__device__ __forceinline__ double acc_value64(long long hi, long long lo) {
+  return fma((double)hi, 4.0, (double)lo * 0x1p-40);
+}
+
+// Rare paths of the FP64 kernel, out of line.
+// near or past a boundary: periodic x (integration.py:577-583), capped z
+// (:585-589), and whether the SIP reached the ground (:606)
+struct Edges {
+  double x_max, z_cap, z_min;
+};
+__device__ __noinline__ int particle_edges(Edges e, double x, double z, double* xo, double* zo) {
+  x = py_mod(x, e.x_max);
+  z = np_min(z, e.z_cap);
+  *xo = x; *zo = z;
+  return z <= e.z_min ? 1 : 0;
+}
+__device__ __noinline__ int floor_div(double x, double d) {
+  const double q = floor(x / d);
+  return q > 2.0e9 ? 2000000000 : (q < -2.0e9 ? -2000000000 : (q == q ? (int)q : -1));
+}
+// the Newton of SIPs outside the two-float form's bounds: newton_fast, for
+// masses beyond FP32 and NaN newton_full
+__device__ __noinline__ double particle_newton64(const PArgs& a, int32_t c, double mw, double ms) {
+  const int64_t C = a.nx * a.nz;
+  CellAmb amb;
+  amb.T = a.gsf[c]; amb.p = a.gsf[C + c]; amb.S = a.gsf[6 * C + c]; amb.e_s = a.gsf[7 * C + c];
+  amb.K = a.gmp[c]; amb.D_v = a.gmp[C + c]; amb.L_v = a.gmp[2 * C + c];
+  amb.sigw = a.aux[c]; amb.rhow = a.aux[C + c]; amb.lap0 = a.aux[2 * C + c];
+  amb.lbp0 = a.aux[3 * C + c]; amb.c1 = a.aux[4 * C + c]; amb.c2 = a.aux[5 * C + c];
+  if (ff_mass_ok(mw) && ff_mass_ok(ms))
+    return newton_fast(a.sol, a.dt_sub, a.no_iter, mw, ms, cell_fast(a.sol, amb), 1.0) - mw;
+  const double m_p = mw + ms;
+  const double w_s = ms / m_p;
+  const double rho = (a.sol == SOL_AS) ? density_AS_solution_rw(w_s, amb.rhow)
+                                       : density_NaCl_solution(w_s, amb.T);
+  const double R = radius_from_mass(m_p, rho);
+  const double sig = (a.sol == SOL_AS) ? surface_tension_AS_sw(w_s, amb.sigw)
+                                       : surface_tension_NaCl_sw(w_s, amb.sigw);
+  return newton_full(a.sol, a.dt_sub, a.no_iter, mw, ms, w_s, R, amb.T, rho, sig, amb, nullptr);
+}
+// the drag update of integration.py:699-718 in FP64 throughout, for drops
+// whose velocity does not follow the air (k dt below 8, radii above some 30 um)
+// or with a Reynolds correction
+__device__ __noinline__ void particle_drag64(const PArgs& a, int32_t c, double mw, double ms,
+                                             double uf, double wf, double* u, double* w) {
+  const int64_t C = a.nx * a.nz;
+  const double m_p = mw + ms;
+  const double rho = density_AS_solution_rw(ms / m_p, a.aux[C + c]);
+  const double R = radius_from_mass(m_p, rho);
+  const double mu_f = a.gmp[5 * C + c], rho_f = a.gmp[6 * C + c];
+  const double d0 = uf - *u, d1 = wf - *w;
+  const double vel_dev = sqrt(d0 * d0 + d1 * d1);
+  const double Re_p = 2.0E-6 * rho_f * R * vel_dev / mu_f;
+  double k_dt = 4.5E12 * a.dt_sub * mu_f / (rho * R * R);
+  if (Re_p > 0.5) {
+    if (Re_p < 1000.0) k_dt *= (1 + 0.15 * pow(Re_p, 0.687));
+    else k_dt *= 0.0183333333333 * Re_p;
+  }
+  *u = (*u + k_dt * uf) / (1.0 + k_dt);
+  *w = (*w + k_dt * wf - a.dt_sub * a.g_set) / (1.0 + k_dt);
+}
+// a SIP removed earlier: its position moves on, its relative position keeps
+// the per-call division of integration.py:548-549
+__device__ __noinline__ void particle_inactive(const PArgs& a, int64_t k, int32_t c) {
+  const int64_t i = -1 - (int64_t)c;
+  const double x = a.pos[k] + a.dt_pos * a.vel[k];
+  const double z = a.pos[a.n + k] + a.dt_pos * a.vel[a.n + k];
+  a.pos[k] = py_mod(x, a.x_max);
+  a.pos[a.n + k] = np_min(z, a.z_cap);
+  a.rel[k] = a.rel[k] / a.dx - (double)i;
+  a.rel[a.n + k] = a.rel[a.n + k] / a.dz - (-1.0);
+}
+// a SIP reaching the ground (integration.py:606-630); returns its new z
+__device__ __noinline__ double particle_removed(const PArgs& a, int64_t k, int32_t c, double x,
+                                                double z, double mw) {
+  const int64_t i = (int64_t)c / a.nz, j = (int64_t)c - i * a.nz;
+  acc_add64(a.wr64, a.water_removed, a.xi[k] * mw);
+  const double rel_x = (x - a.x_min) / a.dx - (double)i;
+  const double rel_z = (z - a.z_min) / a.dz - (double)j;
+  // the re-index of this call leaves the old relative position divided by the
+  // cell size (integration.py:548-549)
+  a.rel[k] = rel_x / a.dx - (double)i;
+  a.rel[a.n + k] = rel_z / a.dz - (-1.0);
+  return a.z_min - 0.01 * a.dz;
+}
+
+// The FP64 sub-step.  In plain FP64 this kernel was bound by the FP64 pipe: some
+// 670 FP64 instructions per SIP at 2 lanes an SM and clock, 478 us per launch
+// over 360,000 SIPs.  The Newton and the drag now run in two-float arithmetic
+// around the FP64 operations that decide the result's rounding (lacmo_ff.cuh;
+// about 60 a SIP are left, and some 3500 FP32 and integer instructions): 87 us.
+// New cell indices come from the FP32 position where it is clear of the cell's
+// edges, boundaries likewise.
+// SIPs that need plain FP64 for the Newton (a step of more than an eighth of
+// the mass, a radius below 5 nm) or the drag (drops above some 30 um) wait in
+// the block's queue until its other SIPs are done: a few of them in every warp
+// would hold all warps on the FP64 pipe, gathered they fill a few warps (a
+// raining state of 545,000 SIPs, 1.3% of them large drops, averaged over 20
+// sub-steps from a state out of equilibrium: 291 us in place, 217 us gathered,
+// 203 us with newton_fast; 732 us in plain FP64).
+constexpr int PQ = 1024;   // queue slots; a SIP beyond them is done in place
 template <bool PHYS>
 __global__ void __launch_bounds__(128) k_particles(const __grid_constant__ PK x) {
   __shared__ PArgs s_a;
-  if (threadIdx.x == 0) s_a = make_pargs(x.m.get(), x.c);
+  __shared__ int32_t s_q[PHYS ? PQ : 1];
+  __shared__ int s_n;
+  if (threadIdx.x == 0) {
+    s_a = make_pargs(x.m.get(), x.c);
+    s_n = 0;
+  }
   __syncthreads();
   const PArgs& a = s_a;
   const int64_t C = a.nx * a.nz;
-  const GridVel gv{a.gv, a.nx, a.nz};
-  for (int64_t k = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; k < a.n;
-       k += (int64_t)gridDim.x * blockDim.x) {
-    const int32_t c = a.cell[k];
-    const bool active = c >= 0;
-    const int64_t i = active ? (int64_t)c / a.nz : (int64_t)(-1 - c);
-    const int64_t j = active ? (int64_t)c - i * a.nz : -1;
-    double x = a.pos[k], z = a.pos[a.n + k];
-    double u = a.vel[k], w = a.vel[a.n + k];
-    double mw = a.m_w[k];
-    double xik = 0.0;
-    double rel_x = 0.0, rel_z = 0.0;
-    if (PHYS) {
-      const double T_p = __ldg(a.gsf + i * a.nz + (active ? j : a.nz - 1));
-      if (a.write_Tp) a.T_p[k] = T_p;
-      if (active) {
-        CellAmb amb;
-        amb.T = T_p; amb.p = __ldg(a.gsf + C + c); amb.S = __ldg(a.gsf + 6 * C + c);
-        amb.e_s = __ldg(a.gsf + 7 * C + c); amb.K = __ldg(a.gmp + c); amb.D_v = __ldg(a.gmp + C + c);
-        amb.L_v = __ldg(a.gmp + 2 * C + c);
-        amb.sigw = __ldg(a.aux + c); amb.rhow = __ldg(a.aux + C + c);
-        amb.lap0 = __ldg(a.aux + 2 * C + c); amb.lbp0 = __ldg(a.aux + 3 * C + c);
-        amb.c1 = __ldg(a.aux + 4 * C + c); amb.c2 = __ldg(a.aux + 5 * C + c);
+  const int nx = (int)a.nx, nz = (int)a.nz;
+  const CellFF* const rec = cell_rec64((double*)a.aux, C);
+  // FP32 positions are within 2^-23 of the domain: margins around boundaries
+  // (m) and cell edges (cells) inside which FP64 decides
+  const float ext = fmaxf(fmaxf(fabsf(a.x_maxf), fabsf(a.z_capf)), fabsf(a.z_minf));
+  const float mpos = fmaxf(1e-3f, ext * 0x1p-20f);
+  const float mcell = fmaxf(1e-4f, fmaxf((float)nx, (float)nz) * 0x1p-20f);
+  // pass 0: the block's SIPs; pass 1: its queue
+#pragma unroll 1
+  for (int pass = 0; pass < (PHYS ? 2 : 1); ++pass) {
+    if (pass) __syncthreads();
+    const int64_t stride = pass ? blockDim.x : (int64_t)gridDim.x * blockDim.x;
+    const int64_t end = pass ? min(s_n, PQ) : a.n;
+#pragma unroll 1
+    for (int64_t q = pass ? threadIdx.x : blockIdx.x * (int64_t)blockDim.x + threadIdx.x; q < end;
+         q += stride) {
+      const int64_t k = pass ? s_q[q] : q;
+      const int32_t c = a.cell[k];
+      if (c < 0) {
+        if (PHYS && a.write_Tp) a.T_p[k] = __ldg(a.gsf + (int64_t)(-1 - c) * nz + nz - 1);
+        particle_inactive(a, k, c);
+        continue;
+      }
+      const double x0 = a.pos[k], z0 = a.pos[a.n + k];
+      double u = a.vel[k], w = a.vel[a.n + k];
+      double mw = PHYS ? a.m_w[k] : 0.0;
+      if (PHYS) {
         const double ms = a.m_s[k];
-        xik = a.xi[k];
-        // integration.py:1044 compute_R_p_w_s_rho_p, :916-936 Newton
-        double m_p = mw + ms;
-        double w_s = ms / m_p;
-        double rho = (a.sol == SOL_AS) ? density_AS_solution_rw(w_s, amb.rhow)
-                                       : density_NaCl_solution(w_s, T_p);
-        double R = radius_from_mass(m_p, rho);
-        double sig = (a.sol == SOL_AS) ? surface_tension_AS_sw(w_s, amb.sigw)
-                                       : surface_tension_NaCl_sw(w_s, amb.sigw);
-        double dm = newton_full(a.sol, a.dt_sub, a.no_iter, mw, ms, w_s, R, T_p, rho, sig, amb,
-                                nullptr);
-        mw += dm;
-        a.dmxi[k] = dm * xik;
-        // integration.py:1075 radius of ammonium sulfate whatever the solute
-        m_p = mw + ms;
-        w_s = ms / m_p;
-        rho = density_AS_solution_rw(w_s, amb.rhow);
-        R = radius_from_mass(m_p, rho);
-        // integration.py:699-718
-        rel_x = (x - a.x_min) / a.dx - (double)i;
-        rel_z = (z - a.z_min) / a.dz - (double)j;
+        const WindFF* const wr = (const WindFF*)(rec + 2 * (int64_t)c + 1);
+        CellFF cf;
+        {
+          const float4* src = (const float4*)(rec + 2 * (int64_t)c);
+          float4* dst = (float4*)&cf;
+#pragma unroll
+          for (int e = 0; e < 6; ++e) dst[e] = __ldg(src + e);
+        }
+        bool ok;
+        const double m = newton_ff<false>(a.sol, a.no_iter, mw, ms, cf,
+                                          d2ff(LC_FOUR_PI * 1.0E12 * a.dt_sub), 1.0, &ok);
+        double dm = m - mw;
+        bool slow = !ok;
+        // integration.py:699-718 with the radius of ammonium sulfate whatever the
+        // solute (:1075): the wind at the SIP
+        const int4 wi = __ldg((const int4*)&wr->i);
+        const double rx = fma(-(double)wi.x, a.dx, x0 - a.x_min) * a.inv_dx;
+        const double rz = fma(-(double)wi.y, a.dz, z0 - a.z_min) * a.inv_dz;
+        const double* const wd = (const double*)wr;
+        auto ld = [&](int at) { return __ldg(wd + at); };
+        // compared with 0.5 by their bits (an FP32 copy would take the wrong piece
+        // next to it)
+        const long long half = 0x3fe0000000000000ll;
+        const long long bx = __double_as_longlong(rx), bz = __double_as_longlong(rz);
         double uf, wf;
-        gv.interp(i, j, rel_x, rel_z, uf, wf);
-        const double mu_f = __ldg(a.gmp + 5 * C + c), rho_f = __ldg(a.gmp + 6 * C + c);
-        const double d0 = uf - u, d1 = wf - w;
-        const double vel_dev = sqrt(d0 * d0 + d1 * d1);
-        const double Re_p = 2.0E-6 * rho_f * R * vel_dev / mu_f;
-        double k_dt = 4.5E12 * a.dt_sub * mu_f / (rho * R * R);
-        if (Re_p > 0.5) {
-          if (Re_p < 1000.0) k_dt *= (1 + 0.15 * pow(Re_p, 0.687));
-          else k_dt *= 0.0183333333333 * Re_p;
+        {
+          // rows of u: b0 = 0 below the cell's middle (row j - 1), 1 above; the
+          // bottom and top rows are linear in x at their outer half
+          const bool lin = ((wi.z & 1) && bz <= half) || ((wi.z & 2) && bz >= half);
+          const int b0 = (lin || bz > half) ? 1 : 0;
+          const double dx0 = ld(2 + b0);
+          uf = fma(rx, dx0, ld(b0));
+          if (!lin)
+            uf = fma(rz + (b0 ? -0.5 : 0.5), fma(rx, ld(3 + b0) - dx0, ld(5 + b0)), uf);
+          const int a0 = bx > half ? 1 : 0;
+          const double dy0 = ld(9 + a0);
+          wf = fma(rx + (a0 ? -0.5 : 0.5), fma(rz, ld(10 + a0) - dy0, ld(12 + a0)),
+                   fma(rz, dy0, ld(7 + a0)));
         }
-        u = (u + k_dt * uf) / (1.0 + k_dt);
-        w = (w + k_dt * wf - a.dt_sub * a.g_set) / (1.0 + k_dt);
+        const double du = uf - u, dw = wf - w;
+        const ff mpf = d2ff((mw + dm) + ms);
+        const ff wfr = ff_mul(d2ff(ms), ff_rcp(mpf));
+        ff pr = ff_horner(FFC(LC_PAR_RHO_AS_1), FFC(LC_PAR_RHO_AS_0), wfr);
+        pr = ff_horner(FFC(LC_PAR_RHO_AS_2), pr, wfr);
+        const ff ipr = ff_rcp(ff_one_plus(ff_mul(pr, wfr)));
+        const ff xr = ff_mul(ff_mul(cf.cx, mpf), ipr);
+        const ff z = ff_icbrt(xr);   // 1 / R
+        const ff kd = ff_mul(ff_mul(ff_mul(d2ff(4.5E12 * a.dt_sub), cf.mr), ipr), ff_mul(z, z));
+        const ff duf = d2ff(du), dwf = d2ff(dw + a.dt_sub * a.g_set);
+        const float dwh = d2f_int(dw);
+        const float Re = 2.0E-6f * cf.rm * f_sqrt(duf.h * duf.h + dwh * dwh) * f_rcp(z.h);
+        slow = slow || !(Re < 0.499f && kd.h > 8.0f);
+        if (slow && pass == 0) {
+          const int at = atomicAdd(&s_n, 1);
+          if (at < PQ) {
+            s_q[at] = (int32_t)k;
+            continue;
+          }
+        }
+        if (!ok) dm = particle_newton64(a, c, mw, ms);
+        mw += dm;
+        if (!slow) {
+          // (u + k uf) / (1 + k) = uf - (uf - u) / (1 + k)
+          const ff inv = ff_rcp(ff_add(kd, 1.0f));
+          u = uf - ff2d(ff_mul(duf, inv));
+          w = wf - ff2d(ff_mul(dwf, inv));
+        } else {
+          particle_drag64(a, c, mw, ms, uf, wf, &u, &w);
+        }
+        if (a.write_Tp) a.T_p[k] = __ldg(a.gsf + c);
+        acc_add64(a.acc64 + 2 * (int64_t)c, a.accx + c, dm * a.xi[k]);
       }
-    } else if (active) {
-      xik = a.xi[k];
-      rel_x = (x - a.x_min) / a.dx - (double)i;
-      rel_z = (z - a.z_min) / a.dz - (double)j;
-    }
-    // integration.py:552-630
-    x += a.dt_pos * u;
-    z += a.dt_pos * w;
-    x = py_mod(x, a.x_max);
-    z = np_min(z, a.z_cap);
-    int32_t newc = c;
-    if (active) {
-      if (z <= a.z_min) {
-        z = a.z_min - 0.01 * a.dz;
+      // integration.py:552-630
+      double xn = x0 + a.dt_pos * u, zn = z0 + a.dt_pos * w;
+      float px = d2f_int(xn), pz = d2f_int(zn);
+      bool removed = false;
+      if (!(px > mpos && px < a.x_maxf - mpos && pz < a.z_capf - mpos && pz > a.z_minf + mpos)) {
+        removed = particle_edges(Edges{a.x_max, a.z_cap, a.z_min}, xn, zn, &xn, &zn) != 0;
+        px = d2f_int(xn); pz = d2f_int(zn);
+      }
+      int32_t newc;
+      if (removed) {
+        zn = particle_removed(a, k, c, x0, z0, PHYS ? mw : a.m_w[k]);
         u = 0.0; w = 0.0;
-        const int slot = atomicAdd(a.rm_count, 1);
-        a.rm_id[slot] = (int32_t)k;
-        a.rm_val[slot] = xik * mw;
-        // the re-index of this call leaves the old relative position divided
-        // by the cell size (integration.py:548-549)
-        a.rel[k] = rel_x / a.dx - (double)i;
-        a.rel[a.n + k] = rel_z / a.dz - (-1.0);
-        newc = (int32_t)(-1 - i);
+        newc = -1 - (int32_t)(c / nz);
       } else {
-        int64_t ci = (int64_t)floor(x / a.dx), cj = (int64_t)floor(z / a.dz);
-        if (ci >= a.nx || ci < 0 || cj >= a.nz || cj < 0) {
+        const float qx = px * a.inv_dxf, qz = pz * a.inv_dzf;
+        int ci = __float2int_rd(qx), cj = __float2int_rd(qz);
+        const float fx = qx - floorf(qx), fz = qz - floorf(qz);
+        if (!(fx > mcell && fx < 1.0f - mcell)) ci = floor_div(xn, a.dx);
+        if (!(fz > mcell && fz < 1.0f - mcell)) cj = floor_div(zn, a.dz);
+        if (ci >= nx || ci < 0 || cj >= nz || cj < 0) {
           atomicOr(a.flags, LACMO_FLAG_CELL_CLAMPED);
-          ci = ci < 0 ? 0 : (ci >= a.nx ? a.nx - 1 : ci);
-          cj = cj < 0 ? 0 : (cj >= a.nz ? a.nz - 1 : cj);
+          ci = ci < 0 ? 0 : (ci >= nx ? nx - 1 : ci);
+          cj = cj < 0 ? 0 : (cj >= nz ? nz - 1 : cj);
         }
-        newc = (int32_t)(ci * a.nz + cj);
-        a.rank[k] = atomicAdd(a.counts + newc, 1);
+        newc = ci * nz + cj;
+        if (a.hist) a.rank[k] = atomicAdd(a.counts + newc, 1);
       }
-    } else {
-      a.rel[k] = a.rel[k] / a.dx - (double)i;
-      a.rel[a.n + k] = a.rel[a.n + k] / a.dz - (-1.0);
+      a.pos[k] = xn; a.pos[a.n + k] = zn;
+      if (PHYS || removed) { a.vel[k] = u; a.vel[a.n + k] = w; }
+      if (PHYS) a.m_w[k] = mw;
+      a.cell[k] = newc;
     }
-    a.pos[k] = x; a.pos[a.n + k] = z;
-    a.vel[k] = u; a.vel[a.n + k] = w;
-    if (PHYS && active) a.m_w[k] = mw;
-    a.cell[k] = newc;
   }
 }
 
 // ---------------------------------------------------------------------------
-// integration.py:402-484 for one cell (and update_material_properties :359)
-__device__ __forceinline__ void grid_cell_update(double* gsf, double* gmp, int64_t c, int64_t C,
-                                                 double p_ref, double p_ref_inv, double dTh,
-                                                 double drv, double dml, double V) {
-  double Th = gsf[2 * C + c];
+// integration.py:402-484 for one cell (and update_material_properties :359),
+// and the cell's terms and records for the next sub-step (aux may be null)
+__device__ __forceinline__ void grid_cell_update(double* gsf, double* gmp, double* aux, int64_t c,
+                                                 int64_t C, double p_ref, double p_ref_inv,
+                                                 double dTh, double drv, double dml, double V) {
+  double Th = gsf[2 * C + c], r_v = gsf[4 * C + c];
   const double rho_d = gsf[3 * C + c];
-  double r_v = gsf[4 * C + c];
-  const double mdi = gsf[8 * C + c];
-  const double L_v = gmp[2 * C + c];
-  Th += dTh;
-  r_v += drv - dml * mdi;
-  const double ToT = pow(p_ref_inv * LC_R_D * rho_d * Th, LC_KAPPA_FACTOR2);
-  Th += ToT * (L_v * dml) / (LC_C_PD * rho_d * V * (1.0 + r_v * LC_HEAT_FACTOR_R_V));
-  const double pdr = pow(rho_d * Th * LC_R_D * p_ref_inv, LC_KAPPA_FACTOR);
-  const double T = Th * pow(pdr, LC_KAPPA_AIR_DRY);
-  const double p = pdr * p_ref * (1 + r_v / LC_EPSILON_GC);
-  const double e_s = 2.53E11 * exp(-5420.0 / T);
-  const double S = rho_d * r_v * T * LC_R_V / e_s;
-  gsf[c] = T; gsf[C + c] = p; gsf[2 * C + c] = Th; gsf[4 * C + c] = r_v;
-  gsf[6 * C + c] = S; gsf[7 * C + c] = e_s;
-  gmp[c] = 4.1868E-3 * (5.69 + 0.017 * (T - 273.15));
-  gmp[C + c] = 4.01218E-5 * pow(T, 1.94) / p;
-  gmp[2 * C + c] = 1.0E3 * (2500.82 - 2.358 * (T - 273.0));
-  gmp[3 * C + c] = surface_tension_water(T);
-  gmp[4 * C + c] = LC_C_PD * (1 + 0.897 * r_v);
-  gmp[5 * C + c] = 1.458E-6 * pow(T, 1.5) / (T + 110.4);
-  gmp[6 * C + c] = rho_d * (1.0 + r_v);
+  cell_step64(&Th, &r_v, rho_d, gsf[8 * C + c], gmp[2 * C + c], dTh, drv, dml, V, p_ref_inv);
+  const CellState a = cell_state64(Th, r_v, rho_d, p_ref, p_ref_inv);
+  gsf[c] = a.T; gsf[C + c] = a.p; gsf[2 * C + c] = Th; gsf[4 * C + c] = r_v;
+  gsf[6 * C + c] = a.S; gsf[7 * C + c] = a.e_s;
+  gmp[c] = a.K; gmp[C + c] = a.D_v; gmp[2 * C + c] = a.L_v;
+  gmp[4 * C + c] = LC_C_PD * (1 + 0.897 * r_v); gmp[5 * C + c] = a.mu; gmp[6 * C + c] = a.rho_f;
+  gmp[3 * C + c] = aux ? write_terms(aux, c, C, a.T, a.p, a.S, a.e_s, a.L_v, a.K, a.D_v, a.mu,
+                                     a.rho_f)
+                       : surface_tension_water(a.T);
 }
 
-// one thread per cell: delta_m_l as the ascending-ID fold of dm*xi over the
-// cell's SIPs (integration.py:916-936), then the grid update of the cell and
-// its mass-rate terms for the next sub-step; all lanes carry FP64 work
+// one thread per cell: delta_m_l from the cell's exact sum of dm*xi
+// (integration.py:916-936; then zeroed), the grid update of the cell and its
+// terms for the next sub-step; the first thread adds the water removed at the
+// ground
 __global__ void __launch_bounds__(32) k_cell_update(const __grid_constant__ MRef mr,
                                                      int grid_update) {
   const Member& mb = mr.get();
-  const int32_t* __restrict__ start = mb.w.start;
-  const int32_t* __restrict__ perm = mb.w.perm;
-  const double* __restrict__ dmxi = mb.w.dmxi;
   double *delta_m_l = mb.g.delta_m_l, *gsf = mb.g.scalar_fields, *gmp = mb.g.mat_prop,
          *aux = mb.w.aux;
   const double *dTh = mb.w.dTh, *drv = mb.w.drv;
   const int64_t C = mb.g.nx * mb.g.nz;
   const double p_ref = mb.g.p_ref, p_ref_inv = mb.g.p_ref_inv, V = mb.g.volume_cell;
+  if (blockIdx.x == 0 && threadIdx.x == 0) {
+    long long* wr = mb.w.wr64;
+    if (wr[0] | wr[1]) {
+      mb.sp.water_removed[0] += acc_value64(wr[0], wr[1]);
+      wr[0] = wr[1] = 0;
+    }
+  }
   for (int64_t c = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; c < C;
        c += (int64_t)gridDim.x * blockDim.x) {
-    const int32_t b = start[c], e = start[c + 1];
-    double acc = 0.0;
-#pragma unroll 8
-    for (int32_t k = b; k < e; ++k) acc += __ldg(dmxi + __ldg(perm + k));
-    const double dml = acc * 1.0E-18;
+    long long* acc = mb.w.acc64 + 2 * c;
+    double sum = acc_value64(acc[0], acc[1]);
+    acc[0] = 0;
+    acc[1] = 0;
+    const double x = mb.w.accx[c];
+    if (x != 0.0) {   // NaN too
+      sum += x;
+      mb.w.accx[c] = 0.0;
+    }
+    const double dml = sum * 1.0E-18;
     delta_m_l[c] = dml;
     if (grid_update) {
-      grid_cell_update(gsf, gmp, c, C, p_ref, p_ref_inv, dTh[c], drv[c], dml, V);
-      write_aux(gsf, gmp, aux, c, C);
+      grid_cell_update(gsf, gmp, aux, c, C, p_ref, p_ref_inv, dTh[c], drv[c], dml, V);
     }
   }
 }
@@ -639,8 +801,7 @@ __global__ void __launch_bounds__(32) k_cell_update(const __grid_constant__ MRef
 //    executes, independent of their order.
 // The Newton condensation and the drag update run in FP32 (lacmo_physics.cuh)
 // with the FP64 Newton for SIPs near the critical radius.  water_removed takes
-// the SIPs reaching the ground with FP64 atomics, in arbitrary order (the
-// removal list of the FP64 path holds the FP64 Newton queue here).
+// the SIPs reaching the ground with FP64 atomics, in arbitrary order.
 // Rare FP64 paths stay out of line (__noinline__) so that the common path
 // issues no FP64 instruction, not even predicated off.
 // removed SIP: only the relative position keeps its per-call division
@@ -667,6 +828,9 @@ __device__ __noinline__ double mixed_newton_fp64(NewtonFP64 a, int32_t c, double
   amb.sigw = __ldg(a.aux + c); amb.rhow = __ldg(a.aux + C + c);
   amb.lap0 = __ldg(a.aux + 2 * C + c); amb.lbp0 = __ldg(a.aux + 3 * C + c);
   amb.c1 = __ldg(a.aux + 4 * C + c); amb.c2 = __ldg(a.aux + 5 * C + c);
+  atomicAdd(a.nfb, 1ull);
+  if (ff_mass_ok(mw) && ff_mass_ok(ms))
+    return newton_fast(a.sol, a.dt_sub, a.no_iter, mw, ms, cell_fast(a.sol, amb), 1.0) - mw;
   const double m_p = mw + ms;
   const double w_s = ms / m_p;
   const double rho64 = (a.sol == SOL_AS) ? density_AS_solution_rw(w_s, amb.rhow)
@@ -674,7 +838,6 @@ __device__ __noinline__ double mixed_newton_fp64(NewtonFP64 a, int32_t c, double
   const double R64 = radius_from_mass(m_p, rho64);
   const double sig64 = (a.sol == SOL_AS) ? surface_tension_AS_sw(w_s, amb.sigw)
                                          : surface_tension_NaCl_sw(w_s, amb.sigw);
-  atomicAdd(a.nfb, 1ull);
   return newton_full(a.sol, a.dt_sub, a.no_iter, mw, ms, w_s, R64, T_p, rho64, sig64, amb,
                      nullptr);
 }
@@ -1196,8 +1359,7 @@ __global__ void k_grid_only(double* gsf, double* gmp, double* aux, const double*
                             double p_ref_inv, double V) {
   for (int64_t c = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; c < C;
        c += (int64_t)gridDim.x * blockDim.x) {
-    grid_cell_update(gsf, gmp, c, C, p_ref, p_ref_inv, dTh[c], drv[c], dml[c], V);
-    if (aux) write_aux(gsf, gmp, aux, c, C);
+    grid_cell_update(gsf, gmp, aux, c, C, p_ref, p_ref_inv, dTh[c], drv[c], dml[c], V);
   }
 }
 
@@ -1405,8 +1567,16 @@ static PCall pcall(const lacmo_params_t& p, double dt_sub, double dt_pos, bool w
 }
 cudaError_t launch_cell_aux(const Bt& B, cudaStream_t s) {
   k_cell_aux<<<grid2(B.nx * B.nz, 32, B.M), 32, 0, s>>>(B.ref()); note_launches(1);
-  // the wind part of the cell records too, for sub-steps run before a full step
+  // the wind parts of the cell records too, for sub-steps run before a full step
   k_wind_table<<<grid2(B.nx * B.nz, 256, B.M), 256, 0, s>>>(B.ref()); note_launches(1);
+  return launch_records64(B, s);
+}
+cudaError_t launch_records64(const Bt& B, cudaStream_t s) {
+  k_records64<<<grid2(B.nx * B.nz, 32, B.M), 32, 0, s>>>(B.ref()); note_launches(1);
+  return cudaGetLastError();
+}
+cudaError_t launch_clear_acc64(const Bt& B, cudaStream_t s) {
+  k_clear_acc64<<<grid2(B.nx * B.nz, 128, B.M), 128, 0, s>>>(B.ref()); note_launches(1);
   return cudaGetLastError();
 }
 __global__ void k_set_i64(int64_t* p, int64_t v) { *p = v; }
@@ -1419,9 +1589,8 @@ cudaError_t launch_histogram(const Bt& B, cudaStream_t s) {
   k_histogram<<<grid2(B.n_max, 256, B.M), 256, 0, s>>>(B.ref()); note_launches(1);
   return cudaGetLastError();
 }
-// the ground removals folded into water_removed without binning (k_scan over
-// counts left at zero: the binning it writes is empty until the next one)
-cudaError_t launch_fold_removals(const Bt& B, cudaStream_t s) {
+// the binning left empty (k_scan over counts left at zero) until the next one
+cudaError_t launch_empty_bin(const Bt& B, cudaStream_t s) {
   k_scan<<<dim3(1, B.M), 1024, 0, s>>>(B.ref()); note_launches(1);
   return cudaGetLastError();
 }
@@ -1434,14 +1603,14 @@ cudaError_t launch_bin(const Bt& B, cudaStream_t s) {
   return cudaGetLastError();
 }
 cudaError_t launch_particles(const Bt& B, const lacmo_params_t& p, double dt_sub,
-                             double dt_sub_pos, bool write_Tp, cudaStream_t s) {
-  PK x{B.ref(), pcall(p, dt_sub, dt_sub_pos, write_Tp, true)};
+                             double dt_sub_pos, bool write_Tp, bool hist, cudaStream_t s) {
+  PK x{B.ref(), pcall(p, dt_sub, dt_sub_pos, write_Tp, hist)};
   k_particles<true><<<grid2(B.n_max, 128, B.M, 152 * 16), 128, 0, s>>>(x); note_launches(1);
   return cudaGetLastError();
 }
-cudaError_t launch_move(const Bt& B, double dt_pos, cudaStream_t s) {
+cudaError_t launch_move(const Bt& B, double dt_pos, bool hist, cudaStream_t s) {
   lacmo_params_t p = {};
-  PK x{B.ref(), pcall(p, 0.0, dt_pos, false, true)};
+  PK x{B.ref(), pcall(p, 0.0, dt_pos, false, hist)};
   k_particles<false><<<grid2(B.n_max, 128, B.M, 152 * 16), 128, 0, s>>>(x); note_launches(1);
   return cudaGetLastError();
 }

@@ -54,14 +54,14 @@ static cudaError_t scratch_address(void** out) {
 }
 
 // zero the cell counters and the scalars; set the collision-step counter
-__global__ void k_static_clear(int32_t* counts, int64_t C, uint32_t* flags, int32_t* rm_count,
+__global__ void k_static_clear(int32_t* counts, int64_t C, uint32_t* flags,
                                int64_t* cursor, int64_t* col_step, int64_t* total,
                                int32_t* cell_ctr, int64_t step) {
   for (int64_t c = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; c < C;
        c += (int64_t)gridDim.x * blockDim.x)
     counts[c] = 0;
   if (blockIdx.x == 0 && threadIdx.x == 0) {
-    *flags = 0; *rm_count = 0; *cursor = 0; *col_step = step; *total = 0; *cell_ctr = 0;
+    *flags = 0; *cursor = 0; *col_step = step; *total = 0; *cell_ctr = 0;
   }
 }
 
@@ -102,7 +102,6 @@ extern "C" int lacmo_collision_step_cells_noalloc(double* xi, double* m_w, doubl
   w.Ef = (float*)(b + st_off_Ef);
   char* sc = b + st_off_scalars;
   w.flags = (uint32_t*)sc;
-  w.rm_count = (int32_t*)(sc + 4);
   w.cursor = (int64_t*)(sc + 8);
   w.col_step = (int64_t*)(sc + 16);
   w.total_pairs = (int64_t*)(sc + 24);
@@ -116,7 +115,7 @@ extern "C" int lacmo_collision_step_cells_noalloc(double* xi, double* m_w, doubl
   lacmo_grid_t g = {};
   g.nx = nx; g.nz = nz; g.scalar_fields = (double*)grid_T;
   int blocks = (int)((C + 255) / 256 < 1024 ? (C + 255) / 256 : 1024);
-  k_static_clear<<<blocks > 0 ? blocks : 1, 256, 0, s>>>(w.counts, C, w.flags, w.rm_count,
+  k_static_clear<<<blocks > 0 ? blocks : 1, 256, 0, s>>>(w.counts, C, w.flags,
                                                          w.cursor, w.col_step, w.total_pairs,
                                                          w.cell_ctr, (int64_t)step);
   note_launches(1);

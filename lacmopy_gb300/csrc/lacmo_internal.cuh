@@ -15,21 +15,22 @@ struct Ws {
   int64_t* draw_off;   // [C+1] first pair draw of each cell, relative to the cursor
   int32_t* perm;       // [n]   SIP IDs sorted by (cell, ID)
   int32_t* rank;       // [n]   arrival slot of each SIP inside its cell
-  double* dmxi;        // [n]   dm * xi of the last condensation sub-step
-  int32_t* rm_id;      // [n]   SIPs removed at the ground in the last sub-step
-  double* rm_val;      // [n]   their xi * m_w
+  int32_t* rm_id;      // [n]   mixed precision: SIPs queued for the FP64 Newton
+  double* rm_val;      // [n]   their masses before the sub-step
   double* aux;         // [6][C] per-cell terms: sigma_w, rho_w, l_alpha, l_beta, c1, c2,
-                       // then the mixed path's FP32 table [C][12]
+                       // then the cell records of the mixed and of the FP64 path
   double* dTh;         // [C]   Delta Theta (advection + relaxation) per sub-step
   double* drv;         // [C]   Delta r_v per sub-step
-  double* div;         // [C]   divergence scratch
+  double* div;         // [C]   mixed precision: exact sums of dm * xi
+  long long* acc64;    // [C][2] FP64: exact sums of dm * xi (acc_add64)
+  double* accx;        // [C]   FP64: dm * xi beyond their range
   double* relax;       // [2][nz] relaxation terms (r_v, Theta)
   double* colR;        // [n]   collision scratch for cells above the shared-memory size
   double* colrho;      // [n]
   int32_t* colk;       // [n]
   // scalars
   uint32_t* flags;
-  int32_t* rm_count;
+  long long* wr64;     // [2] FP64: exact sum of the water removed (acc_add64)
   int64_t* cursor;     // injected-draw cursor
   int64_t* col_step;   // collision-step counter (Philox)
   int64_t* total_pairs;
@@ -54,6 +55,13 @@ __host__ __device__ inline float4* cell_records(double* aux, int64_t C) {
   return (float4*)(aux + cell_records_offset(C));
 }
 constexpr int CELL_REC = 8;   // float4 per cell record
+// The records of the FP64 particle kernel after those: two 128-byte lines per
+// cell (CellFF, WindFF of lacmo_ff.cuh)
+struct CellFF;
+__host__ __device__ inline CellFF* cell_rec64(double* aux, int64_t C) {
+  return (CellFF*)(cell_records(aux, C) + CELL_REC * C);
+}
+constexpr int CELL_REC64_BYTES = 256;
 
 
 // launch-shape knobs of lacmo_tune_* (process-wide; read at launch, so a
@@ -65,6 +73,24 @@ size_t ws_bytes(int64_t n, int64_t nx, int64_t nz);
 bool ws_carve(void* base, size_t bytes, int64_t n, int64_t nx, int64_t nz, Ws* ws);
 // process-wide count of kernels this library has launched (lacmo_kernel_launches)
 void note_launches(int k);
+
+// Stream-ordered scratch for entry points without a workspace, from a pool of
+// this library's own on each device: at most 16 MB of it stay with the pool at a
+// synchronisation, the rest goes back.  Calls on different streams get different
+// memory and wait for nothing of each other.  Freed (stream-ordered) with the
+// object.
+class Scratch {
+ public:
+  explicit Scratch(cudaStream_t s) : s_(s), p_(nullptr) {}
+  ~Scratch() { if (p_) cudaFreeAsync(p_, s_); }
+  Scratch(const Scratch&) = delete;
+  Scratch& operator=(const Scratch&) = delete;
+  void* get(size_t bytes);   // null when there is none
+
+ private:
+  cudaStream_t s_;
+  void* p_;
+};
 
 // Philox4x32-10 (Salmon, Moraes, Dror, Shaw, SC'11): one block of 128 random
 // bits per (key, counter).  A collision pair of rank k draws from block
@@ -141,10 +167,14 @@ cudaError_t launch_cell_aux(const Bt& B, cudaStream_t s);
 cudaError_t launch_set_i64(int64_t* p, int64_t v, cudaStream_t s);
 cudaError_t launch_histogram(const Bt& B, cudaStream_t s);
 cudaError_t launch_bin(const Bt& B, cudaStream_t s);
-cudaError_t launch_fold_removals(const Bt& B, cudaStream_t s);
+cudaError_t launch_empty_bin(const Bt& B, cudaStream_t s);
+// hist: count the SIPs per new cell for a binning that follows
 cudaError_t launch_particles(const Bt& B, const lacmo_params_t& p, double dt_sub,
-                             double dt_sub_pos, bool write_Tp, cudaStream_t s);
-cudaError_t launch_move(const Bt& B, double dt_pos, cudaStream_t s);
+                             double dt_sub_pos, bool write_Tp, bool hist, cudaStream_t s);
+cudaError_t launch_move(const Bt& B, double dt_pos, bool hist, cudaStream_t s);
+cudaError_t launch_records64(const Bt& B, cudaStream_t s);
+// empty the FP64 sums of a particle launch that no cell update follows
+cudaError_t launch_clear_acc64(const Bt& B, cudaStream_t s);
 cudaError_t launch_particles_mixed(const Bt& B, const lacmo_params_t& p, double dt_sub,
                                    double dt_sub_pos, bool write_Tp, bool hist, cudaStream_t s);
 cudaError_t launch_move_mixed(const Bt& B, double dt_pos, cudaStream_t s);
