@@ -514,6 +514,100 @@ __device__ __forceinline__ void init_exact_scratch(const CellArgs& a, const Cell
   __syncwarp();
 }
 
+// The events of one window of the per-pair draws (k_collide_cells), taken in
+// their order: screen_pair places the pairs the first screen left (bits of ev.m),
+// the first one it does not skip is the next event, and after a collection the
+// window's later pairs are screened again with the draws they already have; an
+// event that changes nothing leaves the later screens valid.  Out of line: the
+// window loop around it then reloads nothing (a step of 5625 cells of 64 SIPs,
+// fresh: 124 us with the events in the loop, 74 us without, and with the load
+// below).  An event costs one more screen of its window, where letting every lane run
+// on to its own first hit cost a screen of the whole rest of the cell: a step
+// of a raining 75 x 75 x 128 state (14 collections per cell on average, 190 in the
+// heaviest) took 10.6 ms, 0.94 ms now.
+// Returns false when the event limit is passed (ev.pos: the first rank left).
+struct PairEvents {
+  int pos, events, c0, c1;
+  uint32_t m;
+};
+__device__ __noinline__ PhiloxBlock injected_couple(const double* rnd, int p, int P) {
+  PhiloxBlock x = {0, 0, 0, 0};
+  if (p < P) {
+    const uint64_t q = (uint64_t)__double_as_longlong(rnd[p]);
+    x.x0 = (uint32_t)(q >> 32); x.x1 = (uint32_t)q;
+  }
+  if (p + 1 < P) {
+    const uint64_t q = (uint64_t)__double_as_longlong(rnd[p + 1]);
+    x.x2 = (uint32_t)(q >> 32); x.x3 = (uint32_t)q;
+  }
+  return x;
+}
+__device__ __noinline__ bool window_events(const CellArgs& a, CellSmem S, int n, int P, int w0,
+                                           int i, int j, PhiloxBlock x, float cmax, double Tc,
+                                           bool use_E, bool injected, int event_limit,
+                                           PairEvents& ev) {
+  constexpr unsigned FULL = 0xffffffffu;
+  const int lane = threadIdx.x & 31;
+  const bool same = j < n - 1;
+  const int i2 = same ? i : i + 1, j2 = same ? j + 1 : i + 2;
+  const int p = w0 + 2 * lane;
+  uint32_t m = ev.m;
+  ev.c0 = ev.c1 = 0;
+  for (;;) {
+    uint32_t sc = 0;   // screen_pair's answers, two bits per pair
+    float r_lo, r_hi;
+    if (m & 1u) {
+      if (injected) injected_interval(__hiloint2double((int)x.x0, (int)x.x1), r_lo, r_hi);
+      else philox_interval(philox_half53(x, false), r_lo, r_hi);
+      sc = (uint32_t)screen_pair(a, use_E, S.v[i], S.sk[i], S.v[j], S.sk[j], r_lo, r_hi);
+    }
+    if (m & 2u) {
+      if (injected) injected_interval(__hiloint2double((int)x.x2, (int)x.x3), r_lo, r_hi);
+      else philox_interval(philox_half53(x, true), r_lo, r_hi);
+      sc |= (uint32_t)screen_pair(a, use_E, S.v[i2], S.sk[i2], S.v[j2], S.sk[j2], r_lo, r_hi) << 2;
+    }
+    int done = w0;
+    bool changed = false;
+    unsigned hits;
+    while (!changed && (hits = __ballot_sync(FULL, sc != 0)) != 0) {
+      if (ev.events == 0) {
+        // exact data of the cell's SIPs, computed lazily from the step-start masses
+        init_exact_scratch(a, S, n, lane);
+        ev.events = 1;
+      }
+      const int L = __ffs(hits) - 1;
+      const uint32_t scL = __shfl_sync(FULL, sc, L);
+      const bool sec = (scL & 3u) == 0;
+      const uint64_t dr = ((uint64_t)(sec ? x.x2 : x.x0) << 32) | (sec ? x.x3 : x.x1);
+      const int o = warp_event(a, S, __shfl_sync(FULL, sec ? i2 : i, L),
+                               __shfl_sync(FULL, sec ? j2 : j, L), Tc, use_E,
+                               draw_of(injected, __shfl_sync(FULL, dr, L)),
+                               (sec ? scL >> 2 : scL & 3u) == 1u);
+      if (lane == L) {
+        ev.c0 += o == 1;
+        ev.c1 += o == 2;
+        sc &= sec ? 3u : 12u;
+      }
+      done = w0 + 2 * L + (sec ? 2 : 1);
+      changed = o != 0;
+      if (changed && ++ev.events > event_limit) {
+        ev.pos = done;
+        return false;
+      }
+    }
+    if (!changed) break;
+    const float r0 = injected ? low_of_double(__hiloint2double((int)x.x0, (int)x.x1))
+                              : low_of_word(x.x0);
+    const float r1 = injected ? low_of_double(__hiloint2double((int)x.x2, (int)x.x3))
+                              : low_of_word(x.x2);
+    m = 0;
+    if (p < P && p >= done && !surely_skips(S.v[i], S.v[j], cmax, r0)) m = 1;
+    if (p + 1 < P && p + 1 >= done && !surely_skips(S.v[i2], S.v[j2], cmax, r1)) m |= 2;
+  }
+  ev.pos = w0 + 64;
+  return true;
+}
+
 // order-preserving keys of non-NaN floats (for warp min/max reductions)
 __device__ __forceinline__ uint32_t ord_key(float f) {
   const uint32_t b = __float_as_uint(f);
@@ -566,7 +660,7 @@ __device__ __forceinline__ void advance_seg(int n, int B, int& i, int& b, int ad
 // one lane.  The statistics of the blocks it may have changed are refreshed,
 // and the next round starts after it.
 __device__ __forceinline__ int2 thin_cell(const CellArgs& a, const CellSmem S, int n, double Tc,
-                                       bool use_E, uint64_t pc1, int lane) {
+                                       bool use_E, uint64_t pc1, float cmax, int lane) {
   static_assert(LACMO_THIN_L == 32, "one block of slots per warp");
   int c0 = 0, c1 = 0;   // this lane's outcome counts
   constexpr unsigned FULL = 0xffffffffu;
@@ -665,8 +759,10 @@ __device__ __forceinline__ int2 thin_cell(const CellArgs& a, const CellSmem S, i
         unsigned todo = __ballot_sync(FULL, mine);   // pairs not processed yet
         while (todo) {
           int sc = 0;
-          if ((todo >> lane) & 1u)
-            sc = screen_pair(a, use_E, S.v[ei], S.sk[ei], S.v[q], S.sk[q], r_lo, r_hi);
+          const float4 ve = S.v[ei];
+          const bool left = ((todo >> lane) & 1u) && !surely_skips(ve, S.v[q], cmax, r_lo);
+          if (!__any_sync(FULL, left)) break;
+          if (left) sc = screen_pair(a, use_E, ve, S.sk[ei], S.v[q], S.sk[q], r_lo, r_hi);
           unsigned cand = __ballot_sync(FULL, sc != 0);
           bool col_now = false;
           while (cand) {
@@ -782,7 +878,7 @@ __global__ void __launch_bounds__(CELL_WARPS * 32, MINB)
   const bool use_E = a.E != nullptr;
   const float c43 = (float)LC_FOUR_PI_OVER_THREE_INV;
   float cmax = 0.0f;   // surely_skips' factor
-  if constexpr (!THIN) {
+  {
     float em = a.E_const_f;
     if (use_E) {
       // the largest of the row maxima (infinity without them: every pair is screened)
@@ -832,9 +928,24 @@ __global__ void __launch_bounds__(CELL_WARPS * 32, MINB)
                          (float)LC_PAR_WATER_DENS_1 * ((Tf - (float)LC_PAR_WATER_DENS_2) *
                                                         (Tf - (float)LC_PAR_WATER_DENS_2));
     // load: FP32 copies, FP32 radius and bin (exact when near a bin edge)
+    // The next slot's data are fetched while this one is worked on: the gathers
+    // by SIP ID waited for memory slot after slot (a step of the 64-member
+    // ensemble, 51.9 million SIPs: 5.00 ms before, 4.31 ms with them in flight).
+    int32_t id_n = lane < n ? ids[lane] : 0;
+    double mw_n = 0.0, ms_n = 0.0, xi_n = 0.0, u_n = 0.0, w_n = 0.0;
+    if (lane < n) {
+      mw_n = a.m_w[id_n]; ms_n = a.m_s[id_n]; xi_n = a.xi[id_n];
+      u_n = a.vel[id_n]; w_n = a.vel[a.n + id_n];
+    }
     for (int q = lane; q < n; q += 32) {
-      const int32_t id = ids[q];
-      const float mwf = d2f_rn(a.m_w[id]), msf = d2f_rn(a.m_s[id]);
+      const int32_t id = id_n;
+      const double mw_q = mw_n, ms_q = ms_n, xi_q = xi_n, u_q = u_n, w_q = w_n;
+      if (q + 32 < n) {
+        id_n = ids[q + 32];
+        mw_n = a.m_w[id_n]; ms_n = a.m_s[id_n]; xi_n = a.xi[id_n];
+        u_n = a.vel[id_n]; w_n = a.vel[a.n + id_n];
+      }
+      const float mwf = d2f_rn(mw_q), msf = d2f_rn(ms_q);
       const float mpf = mwf + msf;
       const float wsf = msf / mpf;
       const float rho = (a.sol == SOL_AS)
@@ -859,14 +970,14 @@ __global__ void __launch_bounds__(CELL_WARPS * 32, MINB)
           kb = exact_bin_of(a, id, Tc);
         }
       }
-      S.v[q] = make_float4(d2f_rn(a.xi[id]), Rf, d2f_rn(a.vel[id]), d2f_rn(a.vel[a.n + id]));
+      S.v[q] = make_float4(d2f_rn(xi_q), Rf, d2f_rn(u_q), d2f_rn(w_q));
       S.sk[q] = kb;
       S.sid[q] = id;
     }
     __syncwarp();
     const int P = (int)((int64_t)n * (n - 1) / 2);
     if constexpr (THIN) {
-      const int2 tc = thin_cell(a, S, n, Tc, use_E, pc1, lane);
+      const int2 tc = thin_cell(a, S, n, Tc, use_E, pc1, cmax, lane);
       c0 += tc.x;
       c1 += tc.y;
       __syncwarp();
@@ -875,104 +986,50 @@ __global__ void __launch_bounds__(CELL_WARPS * 32, MINB)
     // Speculative sequential order, one window of 64 pairs (lexicographic
     // order) at a time: lane l draws the couple of ranks (w0 + 2l, w0 + 2l + 1),
     // one Philox block per couple, and screens both pairs with the current
-    // state (surely_skips, then screen_pair for the few left).  The first pair
-    // the screens do not skip is the next event of the sequential order (every
-    // pair before it is skipped with the very state it would see), processed by
-    // the warp.  An event that changes nothing leaves the later screens valid;
-    // after a collection the window's later pairs are screened again with the
-    // draws they already have.  So an event costs one more screen of its
-    // window, where letting every lane run on to its own first hit cost a screen
-    // of the whole rest of the cell: a step of a raining 75 x 75 x 128 state (14
-    // collections per cell on average, 190 in the heaviest) went from 10.6 ms to
-    // 1.1 ms; a fresh 75 x 75 x 64 state stays at 125 us (the Philox blocks).
-    // A cell with many events finishes with the anti-diagonal schedule from its
-    // current position: the sequence costs a chain of some 4 us per event, the
-    // 2n - 3 diagonals about as much each.
+    // state (surely_skips).  The few left go to window_events, which takes the
+    // window's events in their order.  A cell with many events finishes with the
+    // anti-diagonal schedule from its current position: the sequence costs a
+    // chain of some 4 us per event, the 2n - 3 diagonals about as much each.
     const int event_limit = 64 + 2 * n;
-    int pos = 0;           // first rank not processed yet
-    int events = 0;
-    bool diagonal = false;
+    PairEvents ev;
+    ev.pos = 0;            // first rank not processed yet
+    ev.events = 0;
     int i = 0, j = 1 + 2 * lane;   // the pair of rank w0 + 2 lane
     float4 vi = S.v[0];
-    for (int w0 = 0; w0 < P && !diagonal; w0 += 64, j += 64) {
+    for (int w0 = 0; w0 < P; w0 += 64, j += 64) {
       if (j > n - 1) {
         while (j > n - 1 && i < n - 2) { j += i + 2 - n; ++i; }
         vi = S.v[i];
       }
       const int p = w0 + 2 * lane;
-      const bool has0 = p < P, has1 = p + 1 < P;
       // the next pair in lexicographic order: the same row, or the next one's first
       const bool same = j < n - 1;
       const int i2 = same ? i : i + 1, j2 = same ? j + 1 : i + 2;
-      PhiloxBlock x = {0, 0, 0, 0};   // the couple's draws (injected ones as their bits)
+      PhiloxBlock x;   // the couple's draws (injected ones as their bits)
+      float r0, r1;
       if (rnd) {
-        if (has0) {
-          const uint64_t q = (uint64_t)__double_as_longlong(rnd[p]);
-          x.x0 = (uint32_t)(q >> 32); x.x1 = (uint32_t)q;
-        }
-        if (has1) {
-          const uint64_t q = (uint64_t)__double_as_longlong(rnd[p + 1]);
-          x.x2 = (uint32_t)(q >> 32); x.x3 = (uint32_t)q;
-        }
+        x = injected_couple(rnd, p, P);
+        r0 = low_of_double(__hiloint2double((int)x.x0, (int)x.x1));
+        r1 = low_of_double(__hiloint2double((int)x.x2, (int)x.x3));
       } else {
         x = philox_block(a.seed, (uint64_t)(p >> 1), pc1);
+        r0 = low_of_word(x.x0);
+        r1 = low_of_word(x.x2);
       }
-      const float r0 = rnd ? low_of_double(__hiloint2double((int)x.x0, (int)x.x1))
-                           : low_of_word(x.x0);
-      const float r1 = rnd ? low_of_double(__hiloint2double((int)x.x2, (int)x.x3))
-                           : low_of_word(x.x2);
-      int done = w0;   // ranks below it are done
-      for (;;) {       // screen the window's pairs from rank `done` on
-        bool m0 = false, m1 = false;
-        if (has0) m0 = p >= done && !surely_skips(vi, S.v[j], cmax, r0);
-        if (has1)
-          m1 = p + 1 >= done && !surely_skips(same ? vi : S.v[i2], S.v[j2], cmax, r1);
-        if (!__any_sync(0xffffffffu, m0 | m1)) break;
-        uint32_t sc = 0;   // screen_pair's answers, two bits per pair
-        float r_lo, r_hi;
-        if (m0) {
-          if (rnd) injected_interval(__hiloint2double((int)x.x0, (int)x.x1), r_lo, r_hi);
-          else philox_interval(philox_half53(x, false), r_lo, r_hi);
-          sc = (uint32_t)screen_pair(a, use_E, vi, S.sk[i], S.v[j], S.sk[j], r_lo, r_hi);
-        }
-        if (m1) {
-          if (rnd) injected_interval(__hiloint2double((int)x.x2, (int)x.x3), r_lo, r_hi);
-          else philox_interval(philox_half53(x, true), r_lo, r_hi);
-          sc |= (uint32_t)screen_pair(a, use_E, S.v[i2], S.sk[i2], S.v[j2], S.sk[j2], r_lo, r_hi)
-                << 2;
-        }
-        bool changed = false;
-        unsigned hits;
-        while (!changed && (hits = __ballot_sync(0xffffffffu, sc != 0)) != 0) {
-          if (events == 0) {
-            // exact data of the cell's SIPs, computed lazily from the step-start masses
-            init_exact_scratch(a, S, n, lane);
-            events = 1;
-          }
-          const int L = __ffs(hits) - 1;
-          const uint32_t scL = __shfl_sync(0xffffffffu, sc, L);
-          const bool sec = (scL & 3u) == 0;
-          const uint64_t dr = ((uint64_t)(sec ? x.x2 : x.x0) << 32) | (sec ? x.x3 : x.x1);
-          const int o = warp_event(
-              a, S, __shfl_sync(0xffffffffu, sec ? i2 : i, L),
-              __shfl_sync(0xffffffffu, sec ? j2 : j, L), Tc, use_E,
-              draw_of(rnd != nullptr, __shfl_sync(0xffffffffu, dr, L)),
-              (sec ? scL >> 2 : scL & 3u) == 1u);
-          if (lane == L) {
-            c0 += o == 1;
-            c1 += o == 2;
-            sc &= sec ? 3u : 12u;
-          }
-          done = w0 + 2 * L + (sec ? 2 : 1);
-          changed = o != 0;
-          if (changed && ++events > event_limit) diagonal = true;
-        }
-        if (!changed) break;
-        vi = S.v[i];   // SIP i may have changed
-        if (diagonal) break;
-      }
-      pos = diagonal ? done : w0 + 64;
+      bool m0 = false, m1 = false;
+      if (p < P) m0 = !surely_skips(vi, S.v[j], cmax, r0);
+      if (p + 1 < P) m1 = !surely_skips(same ? vi : S.v[i2], S.v[j2], cmax, r1);
+      if (!__any_sync(0xffffffffu, m0 | m1)) continue;
+      ev.m = (m0 ? 1 : 0) | (m1 ? 2 : 0);
+      const bool go_on = window_events(a, S, n, P, w0, i, j, x, cmax, Tc, use_E, rnd != nullptr,
+                                       event_limit, ev);
+      c0 += ev.c0;
+      c1 += ev.c1;
+      if (!go_on) break;
+      vi = S.v[i];   // SIP i may have changed
     }
+    const int pos = ev.pos;
+    const bool diagonal = ev.events > event_limit;
     if (diagonal) {
       // anti-diagonal schedule of the pairs from rank pos on
       for (int s = 1; s <= 2 * n - 3; ++s) {
