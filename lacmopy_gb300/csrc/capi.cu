@@ -77,7 +77,7 @@ static WsPlan ws_plan(int64_t n, int64_t nx, int64_t nz) {
       4 * N,           // rm_id
       8 * N,           // rm_val
       8 * cell_records_offset((int64_t)C) +
-          (16 * CELL_REC + CELL_REC64_BYTES) * C,  // aux: 6 doubles, records
+          (16 * CELL_REC + CELL_REC64_BYTES + 48) * C,  // aux: 6 doubles, records, mixed's 6
       8 * C,           // dTh
       8 * C,           // drv
       8 * C,           // div

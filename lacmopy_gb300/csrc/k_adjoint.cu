@@ -34,6 +34,7 @@
 
 #include "lacmo_ff.cuh"
 #include "lacmo_internal.cuh"
+#include "lacmo_math64.cuh"
 #include "lacmo_physics.cuh"
 
 namespace lacmo {
@@ -460,20 +461,36 @@ template <bool GRAD>
 __device__ __forceinline__ void write_cell(const Args& a, int64_t c, double Th, double rv) {
   const double rho_d = a.rho_d[c];
   const CellState s = cell_state64(Th, rv, rho_d, a.g.p_ref, a.g.p_ref_inv);
-  write_rec64(a.rec + c, s.T, s.S, s.L_v, s.mu, s.rho_f,
-              cell_terms64(s.T, s.p, s.e_s, s.L_v, s.K, s.D_v));
+  write_rec64(a.rec + c, s.T, s.S, s.L_v, s.mu, s.rho_f, s.t);
   if (GRAD) {
-    const Amb<Dual<2>> m = ambient<Dual<2>>(var<2>(Th, 0), var<2>(rv, 1), rho_d, a.g);
+    // logarithmic derivatives: T ~ Theta^kf (kf = 1 / (1 - kappa)), p the same
+    // and 1 + r_v / eps, e_s' / e_s = 5420 / T^2
     CellGrad* const g = a.grad + c;
-    const double lr = m.rhow.d[0] / m.rhow.v;
-    g->S_T = d2ff(m.Sat.d[0]);
-    g->S_r = d2ff(m.Sat.d[1]);
-    g->lcx_T = d2ff(-lr);
-    g->lce_T = d2ff(m.sigw.d[0] / m.sigw.v - lr - m.T.d[0] / m.T.v);
-    g->la_T = d2ff(m.lap0.d[0]); g->la_r = d2ff(m.lap0.d[1]);
-    g->lb_T = d2ff(m.lbp0.d[0]); g->lb_r = d2ff(m.lbp0.d[1]);
-    g->c1_T = d2ff(m.c1.d[0]);
-    g->c2_T = d2ff(m.c2.d[0]); g->c2_r = d2ff(m.c2.d[1]);
+    const double iTh = rcp64(Th), iT = rcp64(s.T);
+    const double lT = LC_KAPPA_FACTOR * iTh, T_T = lT * s.T;
+    const double lp_r = rcp64(LC_EPSILON_GC + rv);
+    const double les = 5420.0 * iT * iT * T_T;
+    const double lK = 4.1868E-3 * 0.017 * T_T * rcp64(s.K);
+    const double lD = 1.94 * lT - lT;              // D_v ~ T^1.94 / p
+    const double lL = -2358.0 * T_T * rcp64(s.L_v);
+    const double tau = 1.0 - s.T * (1.0 / 647.096);
+    const double lsig = (1.256 * rcp64(tau) - 0.625 * rcp64(1.0 - 0.625 * tau)) *
+                        (-1.0 / 647.096) * T_T;
+    const double lrho = 2.0 * LC_PAR_WATER_DENS_1 * (s.T - LC_PAR_WATER_DENS_2) * T_T *
+                        rcp64(s.t.rhow);
+    const double dT = s.T - LC_T_ALPHA_0;
+    g->S_T = d2ff(s.S * (lT - les));
+    g->S_r = d2ff(s.S * rcp64(rv));
+    g->lcx_T = d2ff(-lrho);
+    g->lce_T = d2ff(lsig - lrho - lT);
+    g->la_T = d2ff(s.t.lap0 * (LC_C_ALPHA_2 * T_T * rcp64(LC_C_ALPHA_1 + LC_C_ALPHA_2 * dT) + lK -
+                               lT));
+    g->la_r = d2ff(-s.t.lap0 * lp_r);
+    g->lb_T = d2ff(s.t.lbp0 * (LC_C_BETA_2 * T_T * rcp64(1.0 + LC_C_BETA_2 * dT) + lD));
+    g->lb_r = d2ff(-s.t.lbp0 * lp_r);
+    g->c1_T = d2ff(s.t.c1 * (2.0 * (lL - lT) - lK));
+    g->c2_T = d2ff(s.t.c2 * (lT - lD - les));
+    g->c2_r = d2ff(s.t.c2 * lp_r);
   }
 }
 __global__ void k_cell_terms(Args a) {
@@ -495,10 +512,9 @@ __device__ __forceinline__ CellFF load_cell(const CellFF* rec) {
 __device__ __noinline__ double fwd_step64(const Args& a, int32_t c, double mw, double ms) {
   if (a.no_iter > 0 && ff_mass_ok(mw) && ff_mass_ok(ms)) {
     const CellState s = cell_state64(a.Th[c], a.r_v[c], a.rho_d[c], a.g.p_ref, a.g.p_ref_inv);
-    const CellTerms t = cell_terms64(s.T, s.p, s.e_s, s.L_v, s.K, s.D_v);
     CellAmb m;
-    m.T = s.T; m.S = s.S; m.sigw = t.sigw; m.rhow = t.rhow; m.lap0 = t.lap0; m.lbp0 = t.lbp0;
-    m.c1 = t.c1; m.c2 = t.c2;
+    m.T = s.T; m.S = s.S; m.sigw = s.t.sigw; m.rhow = s.t.rhow; m.lap0 = s.t.lap0;
+    m.lbp0 = s.t.lbp0; m.c1 = s.t.c1; m.c2 = s.t.c2;
     return newton_fast(SOL_AS, a.dt, a.no_iter, mw, ms, cell_fast(SOL_AS, m), a.ks);
   }
   const Amb<double> am = ambient<double>(a.Th[c], a.r_v[c], a.rho_d[c], a.g);
@@ -566,19 +582,40 @@ __global__ void k_bwd_cells(Args a, const double* tape_c, const double* m_before
   for (int64_t c = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; c < a.C;
        c += (int64_t)gridDim.x * blockDim.x) {
     const double Th = tape_c[c], rv = tape_c[a.C + c];
-    if (a.rec) write_cell<true>(a, c, Th, rv);
     const double dml = a.dml[c] * 1.0E-18;   // recomputed forward sum of this sub-step
     const double fT = a.dTh ? a.dTh[c] : 0.0, fr = a.drv ? a.drv[c] : 0.0;
-    Dual<5> Th2, rv2;
-    cell_update<Dual<5>, Dual<5>>(var<5>(Th, 0), var<5>(rv, 1), var<5>(dml, 2), a.rho_d[c],
-                                  a.mdi[c], var<5>(fT, 3), var<5>(fr, 4), a.g, &Th2, &rv2);
     const double lT = lam_Th[c], lr = lam_rv[c];
-    lam_Th[c] = lT * Th2.d[0] + lr * rv2.d[0];
-    lam_rv[c] = lT * Th2.d[1] + lr * rv2.d[1];
-    lam_dml[c] = (lT * Th2.d[2] + lr * rv2.d[2]) * 1.0E-18;   // per fg of dm*xi
+    double Tv[5], rvv[5];   // partials of the new Theta and r_v by Theta, r_v, dml, dTh, drv
+    if (a.rec) {
+      write_cell<true>(a, c, Th, rv);
+      // cell_step64: Theta' = Th1 + A, A = (c Th1)^kf2 L_v dml / (C (1 + h r_v'))
+      const double L_v = a.rec[c].L_v;
+      const double Th1 = Th + fT, rv1 = rv + (fr - dml * a.mdi[c]);
+      const double ToT = exp64(LC_KAPPA_FACTOR2 * log64(a.g.p_ref_inv * LC_R_D * a.rho_d[c] * Th1));
+      const double ih = rcp64(1.0 + rv1 * LC_HEAT_FACTOR_R_V);
+      const double B = ToT * ih * rcp64(LC_C_PD * a.rho_d[c] * a.g.V);   // A = B L_v dml
+      const double A = B * L_v * dml;
+      const double T = 273.0 + (2500.82 - L_v * 1.0E-3) * (1.0 / 2.358);
+      const double Ar = -A * LC_HEAT_FACTOR_R_V * ih;
+      Tv[3] = 1.0 + A * LC_KAPPA_FACTOR2 * rcp64(Th1);
+      Tv[0] = Tv[3] - B * dml * 2358.0 * LC_KAPPA_FACTOR * T * rcp64(Th);
+      Tv[1] = Tv[4] = Ar;
+      Tv[2] = B * L_v - Ar * a.mdi[c];
+      rvv[0] = rvv[3] = 0.0;
+      rvv[1] = rvv[4] = 1.0;
+      rvv[2] = -a.mdi[c];
+    } else {
+      Dual<5> Th2, rv2;
+      cell_update<Dual<5>, Dual<5>>(var<5>(Th, 0), var<5>(rv, 1), var<5>(dml, 2), a.rho_d[c],
+                                    a.mdi[c], var<5>(fT, 3), var<5>(fr, 4), a.g, &Th2, &rv2);
+      for (int q = 0; q < 5; ++q) { Tv[q] = Th2.d[q]; rvv[q] = rv2.d[q]; }
+    }
+    lam_Th[c] = lT * Tv[0] + lr * rvv[0];
+    lam_rv[c] = lT * Tv[1] + lr * rvv[1];
+    lam_dml[c] = (lT * Tv[2] + lr * rvv[2]) * 1.0E-18;   // per fg of dm*xi
     if (lam_inc) {
-      lam_inc[c] += lT * Th2.d[3] + lr * rv2.d[3];
-      lam_inc[a.C + c] += lT * Th2.d[4] + lr * rv2.d[4];
+      lam_inc[c] += lT * Tv[3] + lr * rvv[3];
+      lam_inc[a.C + c] += lT * Tv[4] + lr * rvv[4];
     }
     a.dml[c] = 0.0;
   }

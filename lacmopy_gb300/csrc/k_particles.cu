@@ -21,6 +21,7 @@
 
 #include "lacmo_ff.cuh"
 #include "lacmo_internal.cuh"
+#include "lacmo_math64.cuh"
 #include "lacmo_physics.cuh"
 
 namespace lacmo {
@@ -62,19 +63,25 @@ __global__ void k_cells_export(const int32_t* __restrict__ cell, const double* _
 // per-cell terms of the mass rate for the next sub-step; their FP32 copies in
 // the cell records (cell_records) feed the mixed-precision kernel without
 // double->float conversions there
-// a cell's terms and records from its fields; returns its surface tension of water
-__device__ __forceinline__ double write_terms(double* aux, int64_t c, int64_t C, double T,
-                                              double p, double S, double e_s, double L_v,
-                                              double K, double D_v, double mu, double rho_f) {
-  const CellTerms t = cell_terms64(T, p, e_s, L_v, K, D_v);
+// the mixed path's terms and record of a cell
+__device__ __forceinline__ void write_mixed(double* aux, int64_t c, int64_t C, double T, double S,
+                                            double sigw, double rhow, double lap0, double lbp0,
+                                            double c1, double c2, double mu, double rho_f) {
+  double* const am = mixed_aux(aux, C);
+  am[c] = sigw; am[C + c] = rhow; am[2 * C + c] = lap0; am[3 * C + c] = lbp0;
+  am[4 * C + c] = c1; am[5 * C + c] = c2;
+  float4* af = cell_records(aux, C) + CELL_REC * c;
+  af[0] = make_float4((float)T, (float)(S - 1.0), (float)sigw, (float)rhow);
+  af[1] = make_float4((float)lap0, (float)lbp0, (float)c1, (float)c2);
+  af[2] = make_float4((float)mu, (float)rho_f, 0.0f, 0.0f);
+}
+// the FP64 path's
+__device__ __forceinline__ void write_fp64(double* aux, int64_t c, int64_t C, double T, double S,
+                                           double L_v, double mu, double rho_f,
+                                           const CellTerms& t) {
   aux[c] = t.sigw; aux[C + c] = t.rhow; aux[2 * C + c] = t.lap0; aux[3 * C + c] = t.lbp0;
   aux[4 * C + c] = t.c1; aux[5 * C + c] = t.c2;
-  float4* af = cell_records(aux, C) + CELL_REC * c;
-  af[0] = make_float4((float)T, (float)(S - 1.0), (float)t.sigw, (float)t.rhow);
-  af[1] = make_float4((float)t.lap0, (float)t.lbp0, (float)t.c1, (float)t.c2);
-  af[2] = make_float4((float)mu, (float)rho_f, 0.0f, 0.0f);
   write_rec64(cell_rec64(aux, C) + 2 * c, T, S, L_v, mu, rho_f, t);
-  return t.sigw;
 }
 
 __global__ void k_cell_aux(const __grid_constant__ MRef mr) {
@@ -84,8 +91,14 @@ __global__ void k_cell_aux(const __grid_constant__ MRef mr) {
   double* aux = mb.w.aux;
   for (int64_t c = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; c < C;
        c += (int64_t)gridDim.x * blockDim.x)
-    write_terms(aux, c, C, gsf[c], gsf[C + c], gsf[6 * C + c], gsf[7 * C + c], gmp[2 * C + c],
-                gmp[c], gmp[C + c], gmp[5 * C + c], gmp[6 * C + c]);
+  {
+    const double T = gsf[c], p = gsf[C + c], S = gsf[6 * C + c], e_s = gsf[7 * C + c],
+                 K = gmp[c], D_v = gmp[C + c], L_v = gmp[2 * C + c], mu = gmp[5 * C + c],
+                 rho_f = gmp[6 * C + c];
+    const CellAmb a = make_cell_amb(T, p, S, e_s, L_v, K, D_v);
+    write_mixed(aux, c, C, a.T, a.S, a.sigw, a.rhow, a.lap0, a.lbp0, a.c1, a.c2, mu, rho_f);
+    write_fp64(aux, c, C, T, S, L_v, mu, rho_f, cell_terms64(T, p, e_s, L_v, K, D_v));
+  }
 }
 
 // ---------------------------------------------------------------------------
@@ -412,7 +425,7 @@ __device__ __forceinline__ void interp_wind(const float4 w0, const float4 w1, co
 // (indices below zero wrap as in k_wind_table).
 __global__ void k_records64(const __grid_constant__ MRef mr) {
   const Member& mb = mr.get();
-  const double *gsf = mb.g.scalar_fields, *gmp = mb.g.mat_prop, *aux = mb.w.aux;
+  const double *gsf = mb.g.scalar_fields, *gmp = mb.g.mat_prop;
   const double* in = mb.g.velocity;
   const int64_t nx = mb.g.nx, nz = mb.g.nz, C = nx * nz;
   WindFF* rec = (WindFF*)cell_rec64(mb.w.aux, C);
@@ -435,10 +448,9 @@ __global__ void k_records64(const __grid_constant__ MRef mr) {
     w.edge = (j == 0 ? 1 : 0) | (j == nz - 1 ? 2 : 0);
     w.pad = 0;
     rec[2 * c + 1] = w;
-    write_rec64(cell_rec64(mb.w.aux, C) + 2 * c, gsf[c], gsf[6 * C + c], gmp[2 * C + c],
-                gmp[5 * C + c], gmp[6 * C + c],
-                CellTerms{aux[c], aux[C + c], aux[2 * C + c], aux[3 * C + c], aux[4 * C + c],
-                          aux[5 * C + c]});
+    write_fp64(mb.w.aux, c, C, gsf[c], gsf[6 * C + c], gmp[2 * C + c], gmp[5 * C + c],
+               gmp[6 * C + c], cell_terms64(gsf[c], gsf[C + c], gsf[7 * C + c], gmp[2 * C + c],
+                                            gmp[c], gmp[C + c]));
   }
 }
 __global__ void k_clear_acc64(const __grid_constant__ MRef mr) {
@@ -743,9 +755,12 @@ __device__ __forceinline__ void grid_cell_update(double* gsf, double* gmp, doubl
   gsf[6 * C + c] = a.S; gsf[7 * C + c] = a.e_s;
   gmp[c] = a.K; gmp[C + c] = a.D_v; gmp[2 * C + c] = a.L_v;
   gmp[4 * C + c] = LC_C_PD * (1 + 0.897 * r_v); gmp[5 * C + c] = a.mu; gmp[6 * C + c] = a.rho_f;
-  gmp[3 * C + c] = aux ? write_terms(aux, c, C, a.T, a.p, a.S, a.e_s, a.L_v, a.K, a.D_v, a.mu,
-                                     a.rho_f)
-                       : surface_tension_water(a.T);
+  gmp[3 * C + c] = a.t.sigw;
+  if (aux) {
+    write_mixed(aux, c, C, a.T, a.S, a.t.sigw, a.t.rhow, a.t.lap0, a.t.lbp0, a.t.c1, a.t.c2, a.mu,
+                a.rho_f);
+    write_fp64(aux, c, C, a.T, a.S, a.L_v, a.mu, a.rho_f, a.t);
+  }
 }
 
 // one thread per cell: delta_m_l from the cell's exact sum of dm*xi
@@ -818,6 +833,10 @@ struct NewtonFP64 {
   int sol, no_iter;
   unsigned long long* nfb;
 };
+// FAST: newton_fast (k_newton_fallback: 24 -> 16 us a launch, its latency); the
+// particle kernel, which calls it for a rare SIP leaving the domain, keeps
+// newton_full: the larger callee cost its main path 8% through the registers
+template <bool FAST>
 __device__ __noinline__ double mixed_newton_fp64(NewtonFP64 a, int32_t c, double mw, double ms) {
   const int64_t C = a.C;
   const double T_p = __ldg(a.gsf + c);   // the cell temperature
@@ -829,7 +848,7 @@ __device__ __noinline__ double mixed_newton_fp64(NewtonFP64 a, int32_t c, double
   amb.lap0 = __ldg(a.aux + 2 * C + c); amb.lbp0 = __ldg(a.aux + 3 * C + c);
   amb.c1 = __ldg(a.aux + 4 * C + c); amb.c2 = __ldg(a.aux + 5 * C + c);
   atomicAdd(a.nfb, 1ull);
-  if (ff_mass_ok(mw) && ff_mass_ok(ms))
+  if (FAST && ff_mass_ok(mw) && ff_mass_ok(ms))
     return newton_fast(a.sol, a.dt_sub, a.no_iter, mw, ms, cell_fast(a.sol, amb), 1.0) - mw;
   const double m_p = mw + ms;
   const double w_s = ms / m_p;
@@ -1206,7 +1225,7 @@ __global__ void __launch_bounds__(PM_THREADS, MINB) k_particles_mixed(const __gr
         // a queued SIP leaving the domain: its FP64 Newton here, for the
         // water it takes along
         const double mw0 = tl.get(S, PF_MW, t);
-        const double dm = mixed_newton_fp64(NewtonFP64{a.gsf, a.gmp, a.aux, (int64_t)C, a.dt_sub,
+        const double dm = mixed_newton_fp64<false>(NewtonFP64{a.gsf, a.gmp, mixed_aux((double*)a.aux, C), (int64_t)C, a.dt_sub,
                                                        a.sol, a.no_iter, a.nfb},
                                             c, mw0, tl.get(S, PF_MS, t));
         mw = mw0 + dm;
@@ -1271,7 +1290,9 @@ __global__ void __launch_bounds__(128) k_newton_fallback(const __grid_constant__
     if (k < 0) continue;   // handled where it left the domain
     const int32_t c = a.fb_c[q];
     const double mw0 = a.fb_mw[q];
-    const double dm = mixed_newton_fp64(NewtonFP64{a.gsf, a.gmp, a.aux, a.nx * a.nz, a.dt_sub,
+    const double dm = mixed_newton_fp64<true>(NewtonFP64{a.gsf, a.gmp,
+                                                         mixed_aux((double*)a.aux, a.nx * a.nz),
+                                                         a.nx * a.nz, a.dt_sub,
                                                    a.sol, a.no_iter, a.nfb},
                                         c, mw0, a.m_s[k]);
     a.m_w[k] = mw0 + dm;
@@ -1328,8 +1349,9 @@ __device__ __forceinline__ void grid_cell_update_mixed(double* gsf, double* gmp,
   const double lbp0 = LC_C_BETA_1 * (1.0 + LC_C_BETA_2 * (T - LC_T_ALPHA_0)) * D_v;
   const double c1 = L_v * L_v / (LC_R_V * K * T * T);
   const double c2 = LC_R_V * T / (D_v * e_s);
-  aux[c] = sigw; aux[C + c] = rhow; aux[2 * C + c] = lap0; aux[3 * C + c] = lbp0;
-  aux[4 * C + c] = c1; aux[5 * C + c] = c2;
+  double* const am = mixed_aux(aux, C);
+  am[c] = sigw; am[C + c] = rhow; am[2 * C + c] = lap0; am[3 * C + c] = lbp0;
+  am[4 * C + c] = c1; am[5 * C + c] = c2;
   float4* af = cell_records(aux, C) + CELL_REC * c;
   af[0] = make_float4((float)T, (float)(S - 1.0), (float)sigw, (float)rhow);
   af[1] = make_float4((float)lap0, (float)lbp0, (float)c1, (float)c2);

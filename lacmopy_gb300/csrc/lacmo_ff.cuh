@@ -128,26 +128,6 @@ struct CellFF {
   double L_v;       // heat of vaporisation
   double pad[3];
 };
-// the record from a cell's fields and terms (out of line, like those)
-static __device__ __noinline__ void write_rec64(CellFF* out, double T, double S, double L_v,
-                                                double mu, double rho_f, CellTerms t) {
-  const double irho = 1.0 / t.rhow;
-  CellFF r;
-  r.S_m1 = S - 1.0;
-  r.cx = d2ff(LC_FOUR_PI_OVER_THREE_INV * irho);
-  r.ce = d2ff(2.0E6 * t.sigw * irho / (LC_R_V * T));
-  r.la = d2ff(t.lap0); r.lb = d2ff(t.lbp0); r.c1 = d2ff(t.c1); r.c2 = d2ff(t.c2);
-  r.n0 = d2ff((LC_PAR_SOL_DENS_NACL_0 + LC_PAR_SOL_DENS_NACL_2 * T +
-               LC_PAR_SOL_DENS_NACL_5 * T * T) * irho);
-  r.n1 = d2ff((LC_PAR_SOL_DENS_NACL_1 + LC_PAR_SOL_DENS_NACL_4 * T) * irho);
-  r.n3 = d2ff(LC_PAR_SOL_DENS_NACL_3 * irho);
-  r.mr = d2ff(mu * irho);
-  r.rm = (float)(rho_f / mu);
-  r.T = (float)T;
-  r.L_v = L_v;
-  r.pad[0] = r.pad[1] = r.pad[2] = 0.0;
-  *out = r;
-}
 struct WindFF {
   double U0[2];     // u at (i, j - 1), (i, j)
   double dxU[3];    // u(i + 1, j - 1 + b) - u(i, j - 1 + b)

@@ -62,6 +62,11 @@ __host__ __device__ inline CellFF* cell_rec64(double* aux, int64_t C) {
   return (CellFF*)(cell_records(aux, C) + CELL_REC * C);
 }
 constexpr int CELL_REC64_BYTES = 256;
+// and the mixed path's own copy of the six FP64 per-cell terms: each path forms
+// them its own way, and keeps its bits
+__host__ __device__ inline double* mixed_aux(double* aux, int64_t C) {
+  return (double*)((char*)cell_rec64(aux, C) + CELL_REC64_BYTES * C);
+}
 
 
 // launch-shape knobs of lacmo_tune_* (process-wide; read at launch, so a

@@ -81,58 +81,6 @@ LACMO_DEV double radius_from_mass(double m, double rho) {
   return cbrt(LC_FOUR_PI_OVER_THREE_INV * m / rho);
 }
 
-// The cell update of integration.py:402-438 (Theta, r_v) and the fields that
-// follow from it (atmosphere.py, update_material_properties :359), in FP64.  The
-// powers go through one logarithm each, pow(x, y) = exp(y log x), with |y log x|
-// below 1 (the Exner powers share log x; T^1.94 = T^2 T^-0.06, T^1.5 = T
-// sqrt(T)), so that exp's argument carries no more than half an ulp of 1.  Out of
-// line: the time step, its start and the adjoint's replay run the same code and
-// get the same bits.
-static __device__ __noinline__ void cell_step64(double* Th_io, double* rv_io, double rho_d,
-                                                double mdi, double L_v0, double dTh, double drv,
-                                                double dml, double V, double p_ref_inv) {
-  const double Th = *Th_io + dTh;
-  const double r_v = *rv_io + (drv - dml * mdi);
-  const double ToT = exp(LC_KAPPA_FACTOR2 * log(p_ref_inv * LC_R_D * rho_d * Th));
-  *Th_io = Th + ToT * (L_v0 * dml) / (LC_C_PD * rho_d * V * (1.0 + r_v * LC_HEAT_FACTOR_R_V));
-  *rv_io = r_v;
-}
-struct CellState {
-  double T, p, e_s, S, K, D_v, L_v, mu, rho_f;
-};
-static __device__ __noinline__ CellState cell_state64(double Th, double r_v, double rho_d,
-                                                      double p_ref, double p_ref_inv) {
-  CellState a;
-  const double L2 = log(rho_d * Th * LC_R_D * p_ref_inv);
-  const double pdr = exp(LC_KAPPA_FACTOR * L2);
-  a.T = Th * exp((LC_KAPPA_FACTOR * LC_KAPPA_AIR_DRY) * L2);
-  a.p = pdr * p_ref * (1 + r_v / LC_EPSILON_GC);
-  a.e_s = 2.53E11 * exp(-5420.0 / a.T);
-  a.S = rho_d * r_v * a.T * LC_R_V / a.e_s;
-  a.K = 4.1868E-3 * (5.69 + 0.017 * (a.T - 273.15));
-  a.D_v = 4.01218E-5 * (a.T * a.T * exp(-0.06 * log(a.T))) / a.p;
-  a.L_v = 1.0E3 * (2500.82 - 2.358 * (a.T - 273.0));
-  a.mu = 1.458E-6 * (a.T * sqrt(a.T)) / (a.T + 110.4);
-  a.rho_f = rho_d * (1.0 + r_v);
-  return a;
-}
-// the terms of make_cell_amb from the cell's fields
-struct CellTerms {
-  double sigw, rhow, lap0, lbp0, c1, c2;
-};
-static __device__ __noinline__ CellTerms cell_terms64(double T, double p, double e_s, double L_v,
-                                                      double K, double D_v) {
-  CellTerms t;
-  const double tau = 1 - T / 647.096;
-  t.sigw = 0.2358 * exp(1.256 * log(tau)) * (1 - 0.625 * tau);
-  t.rhow = density_water(T);
-  t.lap0 = (LC_C_ALPHA_1 + LC_C_ALPHA_2 * (T - LC_T_ALPHA_0)) * K / p;
-  t.lbp0 = LC_C_BETA_1 * (1.0 + LC_C_BETA_2 * (T - LC_T_ALPHA_0)) * D_v;
-  t.c1 = L_v * L_v / (LC_R_V * K * T * T);
-  t.c2 = LC_R_V * T / (D_v * e_s);
-  return t;
-}
-
 // Cell-constant terms, microphysics.py:989-1017, 1026-1051, 1454-1455
 LACMO_DEV CellAmb make_cell_amb(double T, double p, double S, double e_s, double L_v, double K,
                                 double D_v) {
