@@ -87,7 +87,7 @@ static WsPlan ws_plan(int64_t n, int64_t nx, int64_t nz) {
       4 * N,           // colk
       128,             // scalars
       8 * C,           // accx
-      4 * (size_t)LACMO_MAX_KERNEL_BINS * (LACMO_MAX_KERNEL_BINS + 1),  // Ef, row maxima
+      4 * (size_t)LACMO_MAX_KERNEL_BINS * (LACMO_MAX_KERNEL_BINS + 2),  // Ef, row maxima and bounds
       4 * C,           // cell_order
       24 * N,          // gcopy
       32 * (N / 32 + C + 1),  // gstats

@@ -60,8 +60,8 @@ struct CellArgs {
   const int64_t *cursor, *col_step, *total_pairs;
   int64_t* no_cols;
   uint32_t* flags;
-  double *gR, *grho;   // per SIP: exact radius and density, or the step-start m_p, m_s
-  int32_t* gk;         // per SIP: exact kernel bin, or -1 while gR/grho hold m_p, m_s
+  double *gR, *grho;   // per slot: exact radius and density
+  int32_t* gk;         // per slot: exact kernel bin, GK_NONE or GK_STALE
   float dtdv_f, lo_f, inv_bl_f, E_const_f;   // FP32 copies for the screen
   float bin_margin;    // distance from a bin edge below which the FP32 bin is not trusted
   const float* Ef;     // FP32 efficiency table, or null (then E is read and rounded)
@@ -70,8 +70,21 @@ struct CellArgs {
   float* gcopy;                // [6][n] FP32 copies by slot, for cells above CELL_SMEM
   float4* gstats;              // block statistics of cells above CELL_SMEM (thinned draws)
   const float* erow;           // largest FP32 efficiency of each table row (thinned draws)
+  const float* ecap;           // the same as a bound: infinity for a row with a NaN
   int thin;                    // thinned Philox draws (lacmo_thin.h)
+  float cmax;                  // surely_skips' factor for the whole table
+  int64_t draw_base;           // *cursor
+  uint64_t cstep;              // *col_step
 };
+
+// A block's dynamic shared memory: its arguments (all its warps belong to one
+// member), then a slice per warp.
+constexpr size_t CELL_ARGS_BYTES = (sizeof(CellArgs) + 15) / 16 * 16;
+constexpr size_t CELL_WARP_BYTES = (size_t)CELL_SMEM * (4 * 4 + 4 + 4) + (CELL_SMEM / 32) * 32;
+__device__ __forceinline__ CellArgs& cell_args() {
+  extern __shared__ float4 fsm[];
+  return *(CellArgs*)fsm;
+}
 
 // the parameters a collision step shares across members
 struct CellCommon {
@@ -88,7 +101,7 @@ struct CellCommon {
   int64_t n_draws;
   float dtdv_f, lo_f, inv_bl_f, E_const_f, bin_margin;
   const float* Ef;
-  const float* erow;
+  const float *erow, *ecap;
   int thin;
 };
 struct CK {
@@ -113,17 +126,20 @@ __device__ __forceinline__ void make_cellargs(CellArgs& a, const Member& mb, con
   a.gcopy = mb.w.gcopy;
   a.gstats = (float4*)mb.w.gstats;
   a.erow = cc.erow;
+  a.ecap = cc.ecap;
   a.thin = cc.thin;
 }
 
 // Exact per-SIP collision data (collision/all_or_nothing.py:812-826), kept
-// in gR / grho / gk and computed on first need.  The density belongs to the
-// step-start masses and the cell temperature (the reference keeps it for the
-// whole step); the radius and its kernel bin follow from the current masses
-// and that density, which the reference recomputes after every collection
-// (all_or_nothing.py:596-633).  A radius only matters when an exact
-// evaluation reads it, so after a collection it is recomputed lazily:
-//   gk = GK_NONE:  nothing computed; gR, grho hold the step-start m_p, m_s
+// in gR / grho / gk by slot (a cell's lie side by side) and computed on first
+// need.  The density belongs to the step-start masses and the cell temperature
+// (the reference keeps it for the whole step); the radius and its kernel bin
+// follow from the current masses and that density, which the reference
+// recomputes after every collection (all_or_nothing.py:596-633).  A radius only
+// matters when an exact evaluation reads it, so after a collection it is
+// recomputed lazily:
+//   gk = GK_NONE:  nothing computed; the masses are still those of the step's start
+//                  (whoever changes them computes the density first)
 //   gk = GK_STALE: grho holds the density; gR, gk are out of date
 //   gk >= 0:       gR, gk are the exact radius and bin of the current masses
 constexpr int32_t GK_NONE = -1, GK_STALE = -2;
@@ -132,47 +148,81 @@ __device__ __forceinline__ double density_of(const CellArgs& a, double m_p, doub
   return (a.sol == SOL_AS) ? density_water(Tc) * poly_rho_AS(w_s)
                            : density_NaCl_solution(w_s, Tc);
 }
-__device__ __noinline__ void compute_density(const CellArgs& a, int32_t id, double Tc) {
-  a.grho[id] = density_of(a, a.gR[id], a.grho[id], Tc);
-  a.gk[id] = GK_STALE;
+__device__ __noinline__ void compute_density(int32_t id, int32_t s, double Tc) {
+  const CellArgs& a = cell_args();
+  const double ms = a.m_s[id];
+  a.grho[s] = density_of(a, a.m_w[id] + ms, ms, Tc);
+  a.gk[s] = GK_STALE;
 }
-__device__ __forceinline__ void ensure_density(const CellArgs& a, int32_t id, double Tc) {
-  if (a.gk[id] == GK_NONE) compute_density(a, id, Tc);
+__device__ __forceinline__ void ensure_density(const CellArgs& a, int32_t id, int32_t s, double Tc) {
+  if (a.gk[s] == GK_NONE) compute_density(id, s, Tc);
 }
-__device__ __noinline__ void compute_exact(const CellArgs& a, int32_t id, double Tc, bool use_E) {
-  if (a.gk[id] == GK_NONE) a.grho[id] = density_of(a, a.gR[id], a.grho[id], Tc);
-  const double R = col_radius(a.m_w[id] + a.m_s[id], a.grho[id]);
-  a.gR[id] = R;
-  a.gk[id] = use_E ? col_bin_f(R, a.lo, a.bl, a.nb, a.lo_f, a.inv_bl_f, a.bin_margin) : 0;
+__device__ __noinline__ void compute_exact(int32_t id, int32_t s, double Tc,
+                                           bool use_E) {
+  const CellArgs& a = cell_args();
+  ensure_density(a, id, s, Tc);
+  const double R = col_radius(a.m_w[id] + a.m_s[id], a.grho[s]);
+  a.gR[s] = R;
+  a.gk[s] = use_E ? col_bin_f(R, a.lo, a.bl, a.nb, a.lo_f, a.inv_bl_f, a.bin_margin) : 0;
 }
 // the exact kernel bin of SIP id from its current masses, stored nowhere
-__device__ __noinline__ int32_t exact_bin_of(const CellArgs& a, int32_t id, double Tc) {
+__device__ __noinline__ int32_t exact_bin_of(int32_t id, double Tc) {
+  const CellArgs& a = cell_args();
   const double m_p = a.m_w[id] + a.m_s[id];
   return col_bin(col_radius(m_p, density_of(a, m_p, a.m_s[id], Tc)), a.lo, a.bl, a.nb);
 }
-__device__ __forceinline__ void ensure_exact(const CellArgs& a, int32_t id, double Tc, bool use_E) {
-  if (a.gk[id] < 0) compute_exact(a, id, Tc, use_E);
+__device__ __forceinline__ void ensure_exact(const CellArgs& a, int32_t id, int32_t s, double Tc,
+                                             bool use_E) {
+  if (a.gk[s] < 0) compute_exact(id, s, Tc, use_E);
 }
 
 // FP32 copies of a cell's SIPs: v = (xi, R, u, w) per SIP, the kernel bin
-// and the SIP ID; in a warp's shared-memory slice, or in the cell's slots of
-// the global scratch for cells above the shared-memory size
-struct CellSmem {
-  float4* v;
-  int32_t *sk, *sid;
-  float4* st;   // thinned draws: statistics of block b at st[2b], st[2b + 1]
+// and the SIP ID, and for thinned draws the statistics of block b at st[2b],
+// st[2b + 1]; base is the cell's first slot.  They lie in a warp's shared-memory
+// slice or, for cells above its size (BIG), in the cell's slots of the global
+// scratch.  The slice is known by the warp's index and the arguments by their
+// place in shared memory: pointers to either held some ten registers of every
+// thread, and what they pushed out to local memory did not fit into L1 beside the
+// slices (a step of the 64-member ensemble 4.10 ms with pointers, 3.91 ms without;
+// of 12 raining members, thinned, 3.28 and 3.08 ms).
+template <bool BIG>
+struct Cell;
+template <>
+struct Cell<false> {
+  int w;
+  int32_t base;
+  __device__ __forceinline__ float4* v() const {
+    extern __shared__ float4 fsm[];
+    return (float4*)((char*)fsm + CELL_ARGS_BYTES + (size_t)w * CELL_WARP_BYTES);
+  }
+  __device__ __forceinline__ int32_t* sk() const { return (int32_t*)(v() + CELL_SMEM); }
+  __device__ __forceinline__ int32_t* sid() const { return sk() + CELL_SMEM; }
+  __device__ __forceinline__ float4* st() const { return (float4*)(sid() + CELL_SMEM); }
+};
+template <>
+struct Cell<true> {
+  float4* v_;
+  int32_t *sk_, *sid_;
+  float4* st_;
+  int32_t base;
+  __device__ __forceinline__ float4* v() const { return v_; }
+  __device__ __forceinline__ int32_t* sk() const { return sk_; }
+  __device__ __forceinline__ int32_t* sid() const { return sid_; }
+  __device__ __forceinline__ float4* st() const { return st_; }
 };
 
 // SIP id's masses changed in a collection: its exact radius and bin become
-// stale, and its FP32 copies at slot l follow now from the FP32 masses and
-// the step-start density (the radius within the screen's 1e-6, as at the
+// stale, and its FP32 copies at slot l of the cell follow now from the FP32 masses
+// and the step-start density (the radius within the screen's 1e-6, as at the
 // cell's load; a bin near an edge is computed exactly, as there).
-__device__ __noinline__ void masses_changed(const CellArgs& a, const CellSmem* S, int32_t id,
+template <bool BIG>
+__device__ __noinline__ void masses_changed(Cell<BIG> S, int32_t id,
                                             int l, double Tc, bool use_E) {
-  a.gk[id] = GK_STALE;
-  if (!S) return;
+  const CellArgs& a = cell_args();
+  const int32_t s = S.base + l;
+  a.gk[s] = GK_STALE;
   const float Rf = lt_cbrtf((float)LC_FOUR_PI_OVER_THREE_INV * d2f_rn(a.m_w[id] + a.m_s[id]) /
-                            d2f_rn(a.grho[id]));
+                            d2f_rn(a.grho[s]));
   int32_t kb = 0;
   if (use_E) {
     const float v = (__logf(Rf) - a.lo_f) * a.inv_bl_f + 0.5f;
@@ -182,19 +232,20 @@ __device__ __noinline__ void masses_changed(const CellArgs& a, const CellSmem* S
       kb = __float2int_rz(fl);
       kb = kb < 0 ? 0 : (kb > a.nb - 1 ? (int32_t)a.nb - 1 : kb);
     } else {
-      compute_exact(a, id, Tc, use_E);
-      kb = a.gk[id];
+      compute_exact(id, s, Tc, use_E);
+      kb = a.gk[s];
     }
   }
-  S->v[l].y = Rf;
-  S->sk[l] = kb;
+  S.v()[l].y = Rf;
+  S.sk()[l] = kb;
 }
 
 // append a collection to the event log; a cell's events come from one warp
 // in its sequential order, one at a time, so their slots increase in that
 // order (slots past the capacity are counted, not written)
-__device__ __noinline__ void log_event(const CellArgs& a, int32_t imin, int32_t imax, int kind,
+__device__ __noinline__ void log_event(int32_t imin, int32_t imax, int kind,
                                        double x, double y) {
+  const CellArgs& a = cell_args();
   const unsigned long long slot = atomicAdd(a.log_count, 1ull);
   if (slot < (unsigned long long)a.log_cap) {
     EvRec r;
@@ -204,79 +255,78 @@ __device__ __noinline__ void log_event(const CellArgs& a, int32_t imin, int32_t 
 }
 
 // One ordinary collection (p_crit <= 1 and p_crit > r) of the pair imin/imax
-// (collision/all_or_nothing.py:607-633) on the global arrays; the density of
-// imin must be known.  S (may be null) receives the FP32 copies at local
-// slots lmin/lmax.
-__device__ __forceinline__ void collect_once(const CellArgs& a, const CellSmem* S, int32_t imin,
+// (collision/all_or_nothing.py:607-633), at the cell's slots lmin/lmax; the
+// density of imin must be known.
+template <bool BIG>
+__device__ __forceinline__ void collect_once(const CellArgs& a, Cell<BIG> S, int32_t imin,
                                              int32_t imax, int lmin, int lmax, double Tc,
                                              bool use_E) {
-  double *XI = a.xi, *MW = a.m_w, *MS = a.m_s, *RR = a.gR;
-  const double* RHO = a.grho;
+  double *XI = a.xi, *MW = a.m_w, *MS = a.m_s;
+  const int32_t smin = S.base + lmin, smax = S.base + lmax;
   const double xi_min = XI[imin], xi_max = XI[imax];
   const double m_w_min = MW[imin], m_w_max = MW[imax];
   const double m_s_min = MS[imin], m_s_max = MS[imax];
   const double xi_rel_dev = (xi_max - xi_min) / xi_max;
   if (xi_rel_dev < 1.0E-5) {
-    if (a.log) log_event(a, imin, imax, 1, xi_min, xi_max);
+    if (a.log) log_event(imin, imax, 1, xi_min, xi_max);
     // both radii follow from imin's density (all_or_nothing.py:615-624):
     // computed now, not left stale
-    ensure_density(a, imax, Tc);
+    ensure_density(a, imax, smax, Tc);
     const double xi_ges = xi_min + xi_max;
     MW[imin] = 2.0 * (xi_min * m_w_min + xi_max * m_w_max) / xi_ges;
     MS[imin] = 2.0 * (xi_min * m_s_min + xi_max * m_s_max) / xi_ges;
     MW[imax] = MW[imin];
     MS[imax] = MS[imin];
-    RR[imin] = col_radius((MW[imin] + MS[imin]), RHO[imin]);
-    RR[imax] = RR[imin];
+    const double R = col_radius((MW[imin] + MS[imin]), a.grho[smin]);
     XI[imax] = 0.5 * 0.7 * xi_ges;
     XI[imin] = 0.5 * xi_ges - XI[imax];
-    a.gk[imin] = use_E ? col_bin_f(RR[imin], a.lo, a.bl, a.nb, a.lo_f, a.inv_bl_f, a.bin_margin)
-                       : 0;
-    a.gk[imax] = a.gk[imin];
-    if (S) {
-      S->v[lmin].x = d2f_rn(XI[imin]); S->v[lmax].x = d2f_rn(XI[imax]);
-      S->v[lmin].y = d2f_rn(RR[imin]); S->v[lmax].y = S->v[lmin].y;
-      S->sk[lmin] = a.gk[imin]; S->sk[lmax] = a.gk[imax];
-    }
+    const int32_t gk =
+        use_E ? col_bin_f(R, a.lo, a.bl, a.nb, a.lo_f, a.inv_bl_f, a.bin_margin) : 0;
+    a.gR[smin] = a.gR[smax] = R;
+    a.gk[smin] = a.gk[smax] = gk;
+    S.v()[lmin].x = d2f_rn(XI[imin]); S.v()[lmax].x = d2f_rn(XI[imax]);
+    S.v()[lmin].y = S.v()[lmax].y = d2f_rn(R);
+    S.sk()[lmin] = S.sk()[lmax] = gk;
   } else {
-    if (a.log) log_event(a, imin, imax, 0, 0.0, 0.0);
+    if (a.log) log_event(imin, imax, 0, 0.0, 0.0);
     MW[imin] += m_w_max;
     MS[imin] += m_s_max;
     XI[imax] -= xi_min;
-    masses_changed(a, S, imin, lmin, Tc, use_E);
-    if (S) S->v[lmax].x = d2f_rn(XI[imax]);
+    masses_changed(S, imin, lmin, Tc, use_E);
+    S.v()[lmax].x = d2f_rn(XI[imax]);
   }
 }
 
 // Exact FP64 evaluation of the pair ii/jj (collision/all_or_nothing.py:
-// 553-633) in the reference's operation order, on the global arrays.  Returns
-// 0 (no collision), 1 (one collection) or 2 (multiple collection).  Sm holds
-// the warp's shared-memory slice, or null (cells above its size).
-__device__ __noinline__ int exact_pair(const CellArgs& a, CellSmem Sm, int32_t ii, int32_t jj,
+// 553-633) in the reference's operation order, at the cell's slots li/lj.
+// Returns 0 (no collision), 1 (one collection) or 2 (multiple collection).
+template <bool BIG>
+__device__ __noinline__ int exact_pair(Cell<BIG> S, int32_t ii, int32_t jj,
                                        int li, int lj, double Tc, bool use_E, double r) {
-  const CellSmem* S = &Sm;
-  ensure_exact(a, ii, Tc, use_E);
-  ensure_exact(a, jj, Tc, use_E);
-  double *XI = a.xi, *MW = a.m_w, *MS = a.m_s, *RR = a.gR;
+  const CellArgs& a = cell_args();
+  const int32_t si = S.base + li, sj = S.base + lj;
+  ensure_exact(a, ii, si, Tc, use_E);
+  ensure_exact(a, jj, sj, Tc, use_E);
+  double *XI = a.xi, *MW = a.m_w, *MS = a.m_s;
   const double *U = a.vel, *W = a.vel + a.n;
   int32_t imin, imax;
   int lmin, lmax;
   if (XI[ii] <= XI[jj]) { imin = ii; imax = jj; lmin = li; lmax = lj; }
   else { imin = jj; imax = ii; lmin = lj; lmax = li; }
   const double xi_min = XI[imin], xi_max = XI[imax];
-  const double Rs = RR[ii] + RR[jj];
-  const double e = use_E ? __ldg(a.E + (int64_t)a.gk[ii] * a.nb + a.gk[jj]) : a.E_const;
+  const double Rs = a.gR[si] + a.gR[sj];
+  const double e = use_E ? __ldg(a.E + (int64_t)a.gk[si] * a.nb + a.gk[sj]) : a.E_const;
   const double du = U[ii] - U[jj], dw = W[ii] - W[jj];
   const double dv = sqrt(du * du + dw * dw);
   const double p_crit = xi_max * a.dtdv * (LC_PI * Rs * Rs * e * dv * 1.0E-12);
   if (p_crit > 1.0) {
-    if (a.log) log_event(a, imin, imax, 2, p_crit, 0.0);
+    if (a.log) log_event(imin, imax, 2, p_crit, 0.0);
     const double xi_col = p_crit * xi_min;
     MW[imin] = MW[imin] + p_crit * MW[imax];
     MS[imin] = MS[imin] + p_crit * MS[imax];
     XI[imax] -= xi_col;
-    masses_changed(a, S, imin, lmin, Tc, use_E);
-    if (S) S->v[lmax].x = d2f_rn(XI[imax]);
+    masses_changed(S, imin, lmin, Tc, use_E);
+    S.v()[lmax].x = d2f_rn(XI[imax]);
     return 2;
   }
   if (!(p_crit > r)) return 0;
@@ -285,15 +335,23 @@ __device__ __noinline__ int exact_pair(const CellArgs& a, CellSmem Sm, int32_t i
 }
 
 // A pair the FP32 bounds place certainly in an ordinary collection.
-__device__ __noinline__ void certain_collection(const CellArgs& a, CellSmem S, int i, int j,
+template <bool BIG>
+__device__ __noinline__ void certain_collection(Cell<BIG> S, int i, int j,
                                                 double Tc, bool use_E) {
-  const int32_t ii = S.sid[i], jj = S.sid[j];
+  const CellArgs& a = cell_args();
+  const int32_t ii = S.sid()[i], jj = S.sid()[j];
   const bool lo_i = a.xi[ii] <= a.xi[jj];
   const int32_t imin = lo_i ? ii : jj, imax = lo_i ? jj : ii;
-  ensure_density(a, imin, Tc);
-  collect_once(a, &S, imin, imax, lo_i ? i : j, lo_i ? j : i, Tc, use_E);
+  const int lmin = lo_i ? i : j, lmax = lo_i ? j : i;
+  ensure_density(a, imin, S.base + lmin, Tc);
+  collect_once(a, S, imin, imax, lmin, lmax, Tc, use_E);
 }
 
+// all_or_nothing.py:609-610 (out of line: the compiler would run the quotient's
+// chain of FP64 operations in every event)
+__device__ __noinline__ bool equal_multiplicities(double xi_min, double xi_max) {
+  return (xi_max - xi_min) / xi_max < 1.0E-5;
+}
 // One event of a cell's sequential order, taken by a whole warp: the pair of
 // slots (l0, l1) with draw r, either placed certainly in an ordinary collection
 // by the FP32 bounds (certain) or evaluated exactly.  Even lanes hold SIP l0,
@@ -301,21 +359,28 @@ __device__ __noinline__ void certain_collection(const CellArgs& a, CellSmem S, i
 // radii run side by side, and the updated masses stay in registers for the
 // FP32 copies instead of being read back, so an event costs one round of
 // loads and one chain of FP64 operations (its latency is what a raining cell
-// waits for).  Same decisions and operation order as exact_pair and
+// waits for; some 100 cycles an operation, so the test for equal multiplicities
+// runs in FP32 and the density of imax is left out where nothing reads it).
+// Keeping SIP l0 in registers over all events of its row, its partners' data
+// formed in all lanes at once, was slower (a step of the raining 75 x 75 x 128
+// state 1.20 ms against 0.94 ms): most rows hold one event.  Same decisions and operation order as exact_pair and
 // collect_once.  Returns 0 (no collision), 1 (one collection) or 2 (multiple
 // collection), the same in all lanes.
-__device__ __noinline__ int warp_event(const CellArgs& a, CellSmem S, int l0, int l1, double Tc,
+template <bool BIG>
+__device__ __forceinline__ int warp_event(Cell<BIG> S, int l0, int l1, double Tc,
                                        bool use_E, double r, bool certain) {
+  const CellArgs& a = cell_args();
   constexpr unsigned FULL = 0xffffffffu;
   const int lane = threadIdx.x & 31, me = lane & 1;
   const bool writes = lane < 2;
   const int l = me ? l1 : l0;
-  const int32_t id = S.sid[l];
+  const int32_t id = S.sid()[l];
   // one round of independent loads
   double xi = a.xi[id];
   double mw = a.m_w[id], ms = a.m_s[id];
-  int32_t gk = a.gk[id];
-  double R = a.gR[id], rho = a.grho[id];
+  const int32_t s = S.base + l;
+  int32_t gk = a.gk[s];
+  double R = a.gR[s], rho = a.grho[s];
   const double u = certain ? 0.0 : a.vel[id], w = certain ? 0.0 : a.vel[a.n + id];
   const double xo = __shfl_xor_sync(FULL, xi, 1);
   // imin is l0's SIP when XI[ii] <= XI[jj], else l1's
@@ -323,16 +388,16 @@ __device__ __noinline__ int warp_event(const CellArgs& a, CellSmem S, int l0, in
   const bool lo0 = x0 <= x1;
   const bool is_min = (me == 0) == lo0;
   if (gk == GK_NONE && (!certain || is_min)) {
-    rho = density_of(a, R, rho, Tc);   // R, rho held the step-start m_p, m_s
+    rho = density_of(a, mw + ms, ms, Tc);
     gk = GK_STALE;
-    if (writes) { a.grho[id] = rho; a.gk[id] = gk; }
+    if (writes) { a.grho[s] = rho; a.gk[s] = gk; }
   }
   double p_crit = 0.0;
   if (!certain) {
     if (gk < 0) {
       R = col_radius(mw + ms, rho);
       gk = use_E ? col_bin_f(R, a.lo, a.bl, a.nb, a.lo_f, a.inv_bl_f, a.bin_margin) : 0;
-      if (writes) { a.gR[id] = R; a.gk[id] = gk; }
+      if (writes) { a.gR[s] = R; a.gk[s] = gk; }
     }
     const int32_t go = __shfl_xor_sync(FULL, gk, 1);
     const double Ro = __shfl_xor_sync(FULL, R, 1);
@@ -356,7 +421,7 @@ __device__ __noinline__ int warp_event(const CellArgs& a, CellSmem S, int l0, in
   bool split = false;
   if (p_crit > 1.0) {
     out = 2;
-    if (a.log && lane == 0) log_event(a, imin, imax, 2, p_crit, 0.0);
+    if (a.log && lane == 0) log_event(imin, imax, 2, p_crit, 0.0);
     if (is_min) {
       mw = mw + p_crit * mwo;
       ms = ms + p_crit * mso;
@@ -364,11 +429,13 @@ __device__ __noinline__ int warp_event(const CellArgs& a, CellSmem S, int l0, in
       xi -= p_crit * xi_min;
     }
   } else {
-    // xi_rel_dev < 1e-5; clear of the limit, a product decides
-    const double d = xi_max - xi_min;
-    split = !(xi_max > 0.0 && d > 2.0E-5 * xi_max) && d / xi_max < 1.0E-5;
+    // xi_rel_dev < 1e-5: the FP32 copies decide where they are clear of the limit
+    const float xf = d2f_flush(xi), xof = __shfl_xor_sync(FULL, xf, 1);
+    const float xmaxf = fmaxf(xf, xof);
+    if (!(xmaxf - fminf(xf, xof) > 2.0E-5f * xmaxf && xmaxf < 3.0E38f && fminf(xf, xof) > 0.0f))
+      split = equal_multiplicities(xi_min, xi_max);
     if (!split) {
-      if (a.log && lane == 0) log_event(a, imin, imax, 0, 0.0, 0.0);
+      if (a.log && lane == 0) log_event(imin, imax, 0, 0.0, 0.0);
       if (is_min) {
         mw += mwo;
         ms += mso;
@@ -376,11 +443,11 @@ __device__ __noinline__ int warp_event(const CellArgs& a, CellSmem S, int l0, in
         xi -= xi_min;
       }
     } else {
-      if (a.log && lane == 0) log_event(a, imin, imax, 1, xi_min, xi_max);
+      if (a.log && lane == 0) log_event(imin, imax, 1, xi_min, xi_max);
       if (gk == GK_NONE) {
         // imax's density belongs to its step-start masses
-        rho = density_of(a, R, rho, Tc);
-        if (writes) a.grho[id] = rho;
+        rho = density_of(a, mw + ms, ms, Tc);
+        if (writes) a.grho[s] = rho;
       }
       const double rhoo = __shfl_xor_sync(FULL, rho, 1);
       const double xi_ges = xi_min + xi_max;
@@ -395,40 +462,48 @@ __device__ __noinline__ int warp_event(const CellArgs& a, CellSmem S, int l0, in
       gk = use_E ? col_bin_f(R, a.lo, a.bl, a.nb, a.lo_f, a.inv_bl_f, a.bin_margin) : 0;
     }
   }
-  if (writes) {
-    if (is_min || split) { a.m_w[id] = mw; a.m_s[id] = ms; }
-    if (!is_min || split) { a.xi[id] = xi; S.v[l].x = d2f_rn(xi); }
-    if (split) {
-      a.gR[id] = R;
-      a.gk[id] = gk;
-      S.v[l].y = d2f_rn(R);
-      S.sk[l] = gk;
-    } else if (is_min) {
-      // the exact radius and bin become stale; the FP32 copies follow now
-      // (masses_changed)
-      const float Rf = lt_cbrtf((float)LC_FOUR_PI_OVER_THREE_INV * d2f_rn(mw + ms) / d2f_rn(rho));
-      int32_t kb = 0;
-      gk = GK_STALE;
-      if (use_E) {
-        const float v = (__logf(Rf) - a.lo_f) * a.inv_bl_f + 0.5f;
-        const float fl = floorf(v);
-        if (v - fl > a.bin_margin && (fl + 1.0f) - v > a.bin_margin && v > -1e6f && v < 1e6f &&
-            Rf > 0.f) {
-          kb = __float2int_rz(fl);
-          kb = kb < 0 ? 0 : (kb > a.nb - 1 ? (int32_t)a.nb - 1 : kb);
-        } else {
-          R = col_radius(mw + ms, rho);
-          a.gR[id] = R;
-          kb = gk = col_bin_f(R, a.lo, a.bl, a.nb, a.lo_f, a.inv_bl_f, a.bin_margin);
-        }
+  // the FP32 copies.  imin's exact radius and bin become stale (masses_changed);
+  // everything is formed before the first store, after which the compiler reads
+  // a's and S's members again
+  float Rf = 0.0f;
+  int32_t kb = 0;
+  const float xif = d2f_rn(xi);
+  bool exact = split;   // R and gk are new
+  if (split) {
+    Rf = d2f_rn(R);
+    kb = gk;
+  } else {
+    Rf = lt_cbrtf((float)LC_FOUR_PI_OVER_THREE_INV * d2f_rn(mw + ms) / d2f_rn(rho));
+    gk = GK_STALE;
+    if (use_E) {
+      const float v = (__logf(Rf) - a.lo_f) * a.inv_bl_f + 0.5f;
+      const float fl = floorf(v);
+      if (v - fl > a.bin_margin && (fl + 1.0f) - v > a.bin_margin && v > -1e6f && v < 1e6f &&
+          Rf > 0.f) {
+        kb = __float2int_rz(fl);
+        kb = kb < 0 ? 0 : (kb > a.nb - 1 ? (int32_t)a.nb - 1 : kb);
+      } else if (is_min) {
+        R = col_radius(mw + ms, rho);
+        kb = gk = col_bin_f(R, a.lo, a.bl, a.nb, a.lo_f, a.inv_bl_f, a.bin_margin);
+        exact = true;
       }
-      a.gk[id] = gk;
-      S.v[l].y = Rf;
-      S.sk[l] = kb;
     }
   }
-  __threadfence_block();
-  __syncwarp();
+  if (writes) {
+    if (is_min || split) {
+      a.m_w[id] = mw;
+      a.m_s[id] = ms;
+      if (exact) a.gR[s] = R;
+      a.gk[s] = gk;
+      S.v()[l].y = Rf;
+      S.sk()[l] = kb;
+    }
+    if (!is_min || split) {
+      a.xi[id] = xi;
+      S.v()[l].x = xif;
+    }
+  }
+  __syncwarp();   // orders the stores before the next event's loads
   return out;
 }
 
@@ -502,15 +577,11 @@ __device__ __forceinline__ bool surely_skips(float4 vi, float4 vj, float cmax, f
   const float p = ((fmaxf(vi.x, vj.x) * cmax) * (rs * rs)) * (dv + 0x1p-21f * sl) + 1e-36f;
   return p < r && vi.x > 0.0f && vj.x > 0.0f;
 }
-// the exact data of a cell's SIPs, computed lazily from the step-start masses
-__device__ __forceinline__ void init_exact_scratch(const CellArgs& a, const CellSmem& S, int n,
+// no exact data yet for the cell's n SIPs
+template <bool BIG>
+__device__ __forceinline__ void init_exact_scratch(const CellArgs& a, Cell<BIG> S, int n,
                                                    int lane) {
-  for (int q = lane; q < n; q += 32) {
-    const int32_t id = S.sid[q];
-    a.gR[id] = a.m_w[id] + a.m_s[id];
-    a.grho[id] = a.m_s[id];
-    a.gk[id] = -1;
-  }
+  for (int q = lane; q < n; q += 32) a.gk[S.base + q] = GK_NONE;
   __syncwarp();
 }
 
@@ -520,11 +591,11 @@ __device__ __forceinline__ void init_exact_scratch(const CellArgs& a, const Cell
 // window's later pairs are screened again with the draws they already have; an
 // event that changes nothing leaves the later screens valid.  Out of line: the
 // window loop around it then reloads nothing (a step of 5625 cells of 64 SIPs,
-// fresh: 124 us with the events in the loop, 74 us without, and with the load
-// below).  An event costs one more screen of its window, where letting every lane run
+// fresh: 124 us with the events in the loop, 74 us without).  An event costs one more screen of its window, where letting every lane run
 // on to its own first hit cost a screen of the whole rest of the cell: a step
 // of a raining 75 x 75 x 128 state (14 collections per cell on average, 190 in the
-// heaviest) took 10.6 ms, 0.94 ms now.
+// heaviest, whose chain of events of some 5 us each is what the step waits for) took
+// 10.6 ms, 0.83 ms now.
 // Returns false when the event limit is passed (ev.pos: the first rank left).
 struct PairEvents {
   int pos, events, c0, c1;
@@ -542,10 +613,12 @@ __device__ __noinline__ PhiloxBlock injected_couple(const double* rnd, int p, in
   }
   return x;
 }
-__device__ __noinline__ bool window_events(const CellArgs& a, CellSmem S, int n, int P, int w0,
+template <bool BIG>
+__device__ __noinline__ bool window_events(Cell<BIG> S, int n, int P, int w0,
                                            int i, int j, PhiloxBlock x, float cmax, double Tc,
                                            bool use_E, bool injected, int event_limit,
                                            PairEvents& ev) {
+  const CellArgs& a = cell_args();
   constexpr unsigned FULL = 0xffffffffu;
   const int lane = threadIdx.x & 31;
   const bool same = j < n - 1;
@@ -559,19 +632,18 @@ __device__ __noinline__ bool window_events(const CellArgs& a, CellSmem S, int n,
     if (m & 1u) {
       if (injected) injected_interval(__hiloint2double((int)x.x0, (int)x.x1), r_lo, r_hi);
       else philox_interval(philox_half53(x, false), r_lo, r_hi);
-      sc = (uint32_t)screen_pair(a, use_E, S.v[i], S.sk[i], S.v[j], S.sk[j], r_lo, r_hi);
+      sc = (uint32_t)screen_pair(a, use_E, S.v()[i], S.sk()[i], S.v()[j], S.sk()[j], r_lo, r_hi);
     }
     if (m & 2u) {
       if (injected) injected_interval(__hiloint2double((int)x.x2, (int)x.x3), r_lo, r_hi);
       else philox_interval(philox_half53(x, true), r_lo, r_hi);
-      sc |= (uint32_t)screen_pair(a, use_E, S.v[i2], S.sk[i2], S.v[j2], S.sk[j2], r_lo, r_hi) << 2;
+      sc |= (uint32_t)screen_pair(a, use_E, S.v()[i2], S.sk()[i2], S.v()[j2], S.sk()[j2], r_lo, r_hi) << 2;
     }
     int done = w0;
     bool changed = false;
     unsigned hits;
     while (!changed && (hits = __ballot_sync(FULL, sc != 0)) != 0) {
       if (ev.events == 0) {
-        // exact data of the cell's SIPs, computed lazily from the step-start masses
         init_exact_scratch(a, S, n, lane);
         ev.events = 1;
       }
@@ -579,7 +651,7 @@ __device__ __noinline__ bool window_events(const CellArgs& a, CellSmem S, int n,
       const uint32_t scL = __shfl_sync(FULL, sc, L);
       const bool sec = (scL & 3u) == 0;
       const uint64_t dr = ((uint64_t)(sec ? x.x2 : x.x0) << 32) | (sec ? x.x3 : x.x1);
-      const int o = warp_event(a, S, __shfl_sync(FULL, sec ? i2 : i, L),
+      const int o = warp_event(S, __shfl_sync(FULL, sec ? i2 : i, L),
                                __shfl_sync(FULL, sec ? j2 : j, L), Tc, use_E,
                                draw_of(injected, __shfl_sync(FULL, dr, L)),
                                (sec ? scL >> 2 : scL & 3u) == 1u);
@@ -601,8 +673,8 @@ __device__ __noinline__ bool window_events(const CellArgs& a, CellSmem S, int n,
     const float r1 = injected ? low_of_double(__hiloint2double((int)x.x2, (int)x.x3))
                               : low_of_word(x.x2);
     m = 0;
-    if (p < P && p >= done && !surely_skips(S.v[i], S.v[j], cmax, r0)) m = 1;
-    if (p + 1 < P && p + 1 >= done && !surely_skips(S.v[i2], S.v[j2], cmax, r1)) m |= 2;
+    if (p < P && p >= done && !surely_skips(S.v()[i], S.v()[j], cmax, r0)) m = 1;
+    if (p + 1 < P && p + 1 >= done && !surely_skips(S.v()[i2], S.v()[j2], cmax, r1)) m |= 2;
   }
   ev.pos = w0 + 64;
   return true;
@@ -620,11 +692,12 @@ __device__ __forceinline__ float ord_val(uint32_t k) {
 // statistics (lt_block_stats) of block b, slots [32 b, min(32 b + 32, n)),
 // from the FP32 copies, warp-cooperative: st[2b] = (xmax, Rmax, umin, umax),
 // st[2b + 1] = (wmin, wmax, ok, 0)
-__device__ __forceinline__ void block_stats(const CellSmem& S, int n, int b, int lane) {
+template <bool BIG>
+__device__ __forceinline__ void block_stats(Cell<BIG> S, int n, int b, int lane) {
   constexpr unsigned FULL = 0xffffffffu;
   const int q = (b << 5) + lane;
   const bool in = q < n;
-  const float4 v = in ? S.v[q] : make_float4(1.0f, 0.0f, 0.0f, 0.0f);
+  const float4 v = in ? S.v()[q] : make_float4(1.0f, 0.0f, 0.0f, 0.0f);
   const bool bad = in && !(v.x > 0.0f && v.y == v.y && v.z == v.z && v.w == v.w);
   const int ok = __ballot_sync(FULL, bad) == 0u;
   const uint32_t xk = __reduce_max_sync(FULL, in ? ord_key(v.x) : 0u);
@@ -634,8 +707,8 @@ __device__ __forceinline__ void block_stats(const CellSmem& S, int n, int b, int
   const uint32_t wlo = __reduce_min_sync(FULL, in ? ord_key(v.w) : 0xffffffffu);
   const uint32_t whi = __reduce_max_sync(FULL, in ? ord_key(v.w) : 0u);
   if (lane == 0) {
-    S.st[2 * b] = make_float4(ord_val(xk), ord_val(Rk), ord_val(ulo), ord_val(uhi));
-    S.st[2 * b + 1] = make_float4(ord_val(wlo), ord_val(whi), __int_as_float(ok), 0.0f);
+    S.st()[2 * b] = make_float4(ord_val(xk), ord_val(Rk), ord_val(ulo), ord_val(uhi));
+    S.st()[2 * b + 1] = make_float4(ord_val(wlo), ord_val(whi), __int_as_float(ok), 0.0f);
   }
 }
 
@@ -649,6 +722,17 @@ __device__ __forceinline__ void advance_seg(int n, int B, int& i, int& b, int ad
   }
 }
 
+// surely_skips' factor for an efficiency of at most em
+__device__ __forceinline__ float skip_factor(const CellArgs& a, float em) {
+  return ((a.dtdv_f * (float)(LC_PI * 1.0E-12)) * fmaxf(em, 0.0f)) * (1.0f + 0x1p-13f);
+}
+// warp_event out of line, for thin_cell's two kinds of events
+template <bool BIG>
+__device__ __noinline__ int event_call(Cell<BIG> S, int l0, int l1, double Tc, bool use_E, double r,
+                                       bool certain) {
+  return warp_event(S, l0, l1, Tc, use_E, r, certain);
+}
+
 // The thinned draws of lacmo_thin.h for one cell, warp-cooperative.  A round
 // takes 32 consecutive segments, one per lane (lane 0 the current part of the
 // current segment): each lane bounds its segment from SIP i and the block
@@ -659,8 +743,10 @@ __device__ __forceinline__ void advance_seg(int n, int B, int& i, int& b, int ad
 // hit's first-hit draws evaluated by all lanes at once and the hit pair by
 // one lane.  The statistics of the blocks it may have changed are refreshed,
 // and the next round starts after it.
-__device__ __forceinline__ int2 thin_cell(const CellArgs& a, const CellSmem S, int n, double Tc,
-                                       bool use_E, uint64_t pc1, float cmax, int lane) {
+template <bool BIG>
+__device__ __forceinline__ int2 thin_cell(Cell<BIG> S, int n, double Tc,
+                                       bool use_E, uint64_t pc1, int lane) {
+  const CellArgs& a = cell_args();
   static_assert(LACMO_THIN_L == 32, "one block of slots per warp");
   int c0 = 0, c1 = 0;   // this lane's outcome counts
   constexpr unsigned FULL = 0xffffffffu;
@@ -702,10 +788,10 @@ __device__ __forceinline__ int2 thin_cell(const CellArgs& a, const CellSmem S, i
     bool indiv = false, hit = false;
     int e = 0;
     if (valid) {
-      const float4 vi = S.v[i];
-      const float4 s0 = S.st[2 * b], s1 = S.st[2 * b + 1];
+      const float4 vi = S.v()[i];
+      const float4 s0 = S.st()[2 * b], s1 = S.st()[2 * b + 1];
       const lt_block_t st{s0.x, s0.y, s0.z, s0.w, s1.x, s1.y, __float_as_int(s1.z)};
-      const float er = use_E ? __ldg(a.erow + S.sk[i]) : a.E_const_f;
+      const float er = use_E ? __ldg(a.erow + S.sk()[i]) : a.E_const_f;
       const float Q = lt_segment_bound(vi.x, vi.y, vi.z, vi.w, &st, er, a.dtdv_f);
       indiv = !(Q >= 0.0f && Q < LACMO_THIN_TAU);
       if (!indiv) {
@@ -740,7 +826,6 @@ __device__ __forceinline__ int2 thin_cell(const CellArgs& a, const CellSmem S, i
       const int eb = (int)(qb & 0x7ffu), ee = (int)((qb >> 11) & 0x7fu);
       const bool eind = ((qb >> 18) & 1u) != 0;
       const uint32_t esub = qb >> 19;
-      if (!scratch) { init_exact_scratch(a, S, n, lane); scratch = true; }
       int next_j = eend;
       bool changed = false;
       if (eind) {
@@ -758,16 +843,19 @@ __device__ __forceinline__ int2 thin_cell(const CellArgs& a, const CellSmem S, i
         }
         unsigned todo = __ballot_sync(FULL, mine);   // pairs not processed yet
         while (todo) {
+          // SIP ei's row bounds the efficiency
+          const float cmax = skip_factor(a, use_E ? __ldg(a.ecap + S.sk()[ei]) : a.E_const_f);
           int sc = 0;
-          const float4 ve = S.v[ei];
-          const bool left = ((todo >> lane) & 1u) && !surely_skips(ve, S.v[q], cmax, r_lo);
+          const float4 ve = S.v()[ei];
+          const bool left = ((todo >> lane) & 1u) && !surely_skips(ve, S.v()[q], cmax, r_lo);
           if (!__any_sync(FULL, left)) break;
-          if (left) sc = screen_pair(a, use_E, ve, S.sk[ei], S.v[q], S.sk[q], r_lo, r_hi);
+          if (left) sc = screen_pair(a, use_E, ve, S.sk()[ei], S.v()[q], S.sk()[q], r_lo, r_hi);
           unsigned cand = __ballot_sync(FULL, sc != 0);
           bool col_now = false;
           while (cand) {
+            if (!scratch) { init_exact_scratch(a, S, n, lane); scratch = true; }
             const int t = __ffs(cand) - 1;
-            const int o = warp_event(a, S, ei, ej + t, Tc, use_E,
+            const int o = event_call(S, ei, ej + t, Tc, use_E,
                                      philox_from_bits(__shfl_sync(FULL, k53, t)),
                                      __shfl_sync(FULL, sc, t) == 1);
             if (lane == t) {
@@ -800,9 +888,10 @@ __device__ __forceinline__ int2 thin_cell(const CellArgs& a, const CellSmem S, i
         const float r_lo = normal ? d2f_down_pos(r) : 0.0f;
         const float r_hi = normal ? __uint_as_float(__float_as_uint(r_lo) + 1u) : 0x1p-126f;
         const int hj = ej + g;
-        const int sc = screen_pair(a, use_E, S.v[ei], S.sk[ei], S.v[hj], S.sk[hj], r_lo, r_hi);
+        const int sc = screen_pair(a, use_E, S.v()[ei], S.sk()[ei], S.v()[hj], S.sk()[hj], r_lo, r_hi);
         if (sc != 0) {
-          const int o = warp_event(a, S, ei, hj, Tc, use_E, r, sc == 1);
+          if (!scratch) { init_exact_scratch(a, S, n, lane); scratch = true; }
+          const int o = event_call(S, ei, hj, Tc, use_E, r, sc == 1);
           if (lane == 0) {
             c0 += o == 1;
             c1 += o == 2;
@@ -846,143 +935,75 @@ __device__ __forceinline__ int2 thin_cell(const CellArgs& a, const CellSmem S, i
   return make_int2((int)c0, (int)c1);
 }
 
-// One warp per cell.  Shared memory holds FP32 copies of xi, R, u, w and the
-// kernel bin (24 B per SIP with the SIP ID); the pairs are screened in
-// parallel in lexicographic order and only the events of the sequential
-// order (collections and undecided pairs) are processed one at a time.
-constexpr size_t CELL_WARP_BYTES = (size_t)CELL_SMEM * (4 * 4 + 4 + 4) + (CELL_SMEM / 32) * 32;
-
-// THIN: the thinned draws, else per-pair draws.  MINB: resident blocks per
-// SM the register budget is set for (the TUNE_COLLISION_BLOCKS knob picks the
-// instance; 3 by default: the thinned rounds gain more from the warps than
-// they lose to spills)
-template <bool THIN, int MINB>
-__global__ void __launch_bounds__(CELL_WARPS * 32, MINB)
-    k_collide_cells(const __grid_constant__ CK x) {
-  // the member's arguments, once per block (all warps of a block belong to
-  // the same member); shared memory keeps them addressable without a copy
-  // per thread
-  __shared__ CellArgs s_args;
-  if (threadIdx.x == 0) make_cellargs(s_args, x.m.get(), x.cc);
-  __syncthreads();
-  const CellArgs& a = s_args;
-  extern __shared__ float4 fsm[];   // 16-byte aligned warp slices
-  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-  float* const wslice = (float*)((char*)fsm + (size_t)wid * CELL_WARP_BYTES);
-  const int64_t cursor = a.draws ? *a.cursor : 0;
-  if (a.draws && cursor + *a.total_pairs > a.n_draws) {
-    if (blockIdx.x == 0 && threadIdx.x == 0) atomicOr(a.flags, LACMO_FLAG_DRAWS_SHORT);
-    return;
-  }
-  const uint64_t cstep = (uint64_t)*a.col_step;
+// One cell by one warp: the pairs are screened in parallel in lexicographic
+// order and only the events of the sequential order (collections and undecided
+// pairs) are processed one at a time.  Returns this lane's outcome counts.
+template <bool THIN, bool BIG>
+__device__ __forceinline__ int2 collide_cell(const Cell<BIG> S, int64_t c, int n, int lane) {
+  const CellArgs& a = cell_args();
   const bool use_E = a.E != nullptr;
-  const float c43 = (float)LC_FOUR_PI_OVER_THREE_INV;
-  float cmax = 0.0f;   // surely_skips' factor
-  {
-    float em = a.E_const_f;
-    if (use_E) {
-      // the largest of the row maxima (infinity without them: every pair is screened)
-      em = a.erow ? 0.0f : __uint_as_float(0x7f800000u);
-      if (a.erow) {
-        for (int64_t q = lane; q < a.nb; q += 32) em = fmaxf(em, __ldg(a.erow + q));
-        em = __uint_as_float(__reduce_max_sync(0xffffffffu, __float_as_uint(em)));
-      }
-    }
-    cmax = ((a.dtdv_f * (float)(LC_PI * 1.0E-12)) * fmaxf(em, 0.0f)) * (1.0f + 0x1p-13f);
+  const double Tc = a.T[c];
+  const uint64_t pc1 = (a.cstep << 32) | (uint64_t)c;
+  const int32_t* ids = a.perm + S.base;
+  // FP32 copies, FP32 radius and bin (exact when near a bin edge)
+  const float Tf = d2f_rn(Tc);
+  const float rhow_f = (float)LC_PAR_WATER_DENS_0 +
+                       (float)LC_PAR_WATER_DENS_1 * ((Tf - (float)LC_PAR_WATER_DENS_2) *
+                                                      (Tf - (float)LC_PAR_WATER_DENS_2));
+  // The next slot's data are fetched while this one is worked on: the gathers
+  // by SIP ID waited for memory slot after slot (a step of the 64-member
+  // ensemble, 51.9 million SIPs: 5.00 ms before, 4.31 ms with them in flight).
+  int32_t id_n = lane < n ? ids[lane] : 0;
+  double mw_n = 0.0, ms_n = 0.0, xi_n = 0.0, u_n = 0.0, w_n = 0.0;
+  if (lane < n) {
+    mw_n = a.m_w[id_n]; ms_n = a.m_s[id_n]; xi_n = a.xi[id_n];
+    u_n = a.vel[id_n]; w_n = a.vel[a.n + id_n];
   }
-  int64_t c0 = 0, c1 = 0;
-  // persistent warps take the member's cells, largest first, from a counter
-  for (;;) {
-    int idx = 0;
-    if (lane == 0) idx = atomicAdd(a.cell_ctr, 1);
-    idx = __shfl_sync(0xffffffffu, idx, 0);
-    if (idx >= a.C) break;
-    const int64_t c = a.cell_order[idx];
-    const int32_t b = a.start[c];
-    const int n = a.start[c + 1] - b;
-    if (n < 2) break;   // the remaining cells hold fewer than two SIPs
-    if (n > 65535) {    // pair ranks would leave 32 bits
-      if (lane == 0) atomicOr(a.flags, LACMO_FLAG_CELL_TOO_BIG);
-      continue;
-    }
-    const double Tc = a.T[c];
-    const double* rnd = a.draws ? a.draws + cursor + a.draw_off[c] : nullptr;
-    const uint64_t pc1 = (cstep << 32) | (uint64_t)c;
-    const int32_t* ids = a.perm + b;
-    // cells above the shared-memory size keep their copies in global scratch
-    const bool big = n > CELL_SMEM;
-    CellSmem S;
-    if (big) {
-      S.v = (float4*)a.gcopy + b;
-      S.sk = (int32_t*)((float4*)a.gcopy + a.n) + b;
-      S.sid = S.sk + a.n;
-      S.st = a.gstats + 2 * ((int64_t)(b >> 5) + c);
-    } else {
-      S.v = (float4*)wslice;
-      S.sk = (int32_t*)(S.v + CELL_SMEM);
-      S.sid = S.sk + CELL_SMEM;
-      S.st = (float4*)(S.sid + CELL_SMEM);
-    }
-    const float Tf = d2f_rn(Tc);
-    const float rhow_f = (float)LC_PAR_WATER_DENS_0 +
-                         (float)LC_PAR_WATER_DENS_1 * ((Tf - (float)LC_PAR_WATER_DENS_2) *
-                                                        (Tf - (float)LC_PAR_WATER_DENS_2));
-    // load: FP32 copies, FP32 radius and bin (exact when near a bin edge)
-    // The next slot's data are fetched while this one is worked on: the gathers
-    // by SIP ID waited for memory slot after slot (a step of the 64-member
-    // ensemble, 51.9 million SIPs: 5.00 ms before, 4.31 ms with them in flight).
-    int32_t id_n = lane < n ? ids[lane] : 0;
-    double mw_n = 0.0, ms_n = 0.0, xi_n = 0.0, u_n = 0.0, w_n = 0.0;
-    if (lane < n) {
+  for (int q = lane; q < n; q += 32) {
+    const int32_t id = id_n;
+    const double mw_q = mw_n, ms_q = ms_n, xi_q = xi_n, u_q = u_n, w_q = w_n;
+    if (q + 32 < n) {
+      id_n = ids[q + 32];
       mw_n = a.m_w[id_n]; ms_n = a.m_s[id_n]; xi_n = a.xi[id_n];
       u_n = a.vel[id_n]; w_n = a.vel[a.n + id_n];
     }
-    for (int q = lane; q < n; q += 32) {
-      const int32_t id = id_n;
-      const double mw_q = mw_n, ms_q = ms_n, xi_q = xi_n, u_q = u_n, w_q = w_n;
-      if (q + 32 < n) {
-        id_n = ids[q + 32];
-        mw_n = a.m_w[id_n]; ms_n = a.m_s[id_n]; xi_n = a.xi[id_n];
-        u_n = a.vel[id_n]; w_n = a.vel[a.n + id_n];
+    const float mwf = d2f_rn(mw_q), msf = d2f_rn(ms_q);
+    const float mpf = mwf + msf;
+    const float wsf = msf / mpf;
+    const float rho = (a.sol == SOL_AS)
+                          ? rhow_f * ((((float)LC_PAR_RHO_AS_0 * wsf + (float)LC_PAR_RHO_AS_1) *
+                                           wsf + (float)LC_PAR_RHO_AS_2) * wsf +
+                                      (float)LC_PAR_RHO_AS_3)
+                          : (float)LC_PAR_SOL_DENS_NACL_0 + (float)LC_PAR_SOL_DENS_NACL_1 * wsf +
+                                (float)LC_PAR_SOL_DENS_NACL_2 * Tf +
+                                (float)LC_PAR_SOL_DENS_NACL_3 * wsf * wsf +
+                                (float)LC_PAR_SOL_DENS_NACL_4 * wsf * Tf +
+                                (float)LC_PAR_SOL_DENS_NACL_5 * Tf * Tf;
+    const float Rf = lt_cbrtf((float)LC_FOUR_PI_OVER_THREE_INV * mpf / rho);
+    int32_t kb = 0;
+    if (use_E) {
+      const float v = (__logf(Rf) - a.lo_f) * a.inv_bl_f + 0.5f;
+      const float fl = floorf(v);
+      if (v - fl > a.bin_margin && (fl + 1.0f) - v > a.bin_margin && v > -1e6f && v < 1e6f &&
+          Rf > 0.f) {
+        kb = __float2int_rz(fl);
+        kb = kb < 0 ? 0 : (kb > a.nb - 1 ? (int32_t)a.nb - 1 : kb);
+      } else {
+        kb = exact_bin_of(id, Tc);
       }
-      const float mwf = d2f_rn(mw_q), msf = d2f_rn(ms_q);
-      const float mpf = mwf + msf;
-      const float wsf = msf / mpf;
-      const float rho = (a.sol == SOL_AS)
-                            ? rhow_f * ((((float)LC_PAR_RHO_AS_0 * wsf + (float)LC_PAR_RHO_AS_1) *
-                                             wsf + (float)LC_PAR_RHO_AS_2) * wsf +
-                                        (float)LC_PAR_RHO_AS_3)
-                            : (float)LC_PAR_SOL_DENS_NACL_0 + (float)LC_PAR_SOL_DENS_NACL_1 * wsf +
-                                  (float)LC_PAR_SOL_DENS_NACL_2 * Tf +
-                                  (float)LC_PAR_SOL_DENS_NACL_3 * wsf * wsf +
-                                  (float)LC_PAR_SOL_DENS_NACL_4 * wsf * Tf +
-                                  (float)LC_PAR_SOL_DENS_NACL_5 * Tf * Tf;
-      const float Rf = lt_cbrtf(c43 * mpf / rho);
-      int32_t kb = 0;
-      if (use_E) {
-        const float v = (__logf(Rf) - a.lo_f) * a.inv_bl_f + 0.5f;
-        const float fl = floorf(v);
-        if (v - fl > a.bin_margin && (fl + 1.0f) - v > a.bin_margin && v > -1e6f && v < 1e6f &&
-            Rf > 0.f) {
-          kb = __float2int_rz(fl);
-          kb = kb < 0 ? 0 : (kb > a.nb - 1 ? (int32_t)a.nb - 1 : kb);
-        } else {
-          kb = exact_bin_of(a, id, Tc);
-        }
-      }
-      S.v[q] = make_float4(d2f_rn(xi_q), Rf, d2f_rn(u_q), d2f_rn(w_q));
-      S.sk[q] = kb;
-      S.sid[q] = id;
     }
-    __syncwarp();
+    S.v()[q] = make_float4(d2f_rn(xi_q), Rf, d2f_rn(u_q), d2f_rn(w_q));
+    S.sk()[q] = kb;
+    S.sid()[q] = id;
+  }
+  __syncwarp();
+  if constexpr (THIN) {
+    return thin_cell(S, n, Tc, use_E, pc1, lane);
+  } else {
+    int c0 = 0, c1 = 0;
+    const float cmax = a.cmax;
+    const double* rnd = a.draws ? a.draws + a.draw_base + a.draw_off[c] : nullptr;
     const int P = (int)((int64_t)n * (n - 1) / 2);
-    if constexpr (THIN) {
-      const int2 tc = thin_cell(a, S, n, Tc, use_E, pc1, cmax, lane);
-      c0 += tc.x;
-      c1 += tc.y;
-      __syncwarp();
-      continue;
-    }
     // Speculative sequential order, one window of 64 pairs (lexicographic
     // order) at a time: lane l draws the couple of ranks (w0 + 2l, w0 + 2l + 1),
     // one Philox block per couple, and screens both pairs with the current
@@ -995,11 +1016,11 @@ __global__ void __launch_bounds__(CELL_WARPS * 32, MINB)
     ev.pos = 0;            // first rank not processed yet
     ev.events = 0;
     int i = 0, j = 1 + 2 * lane;   // the pair of rank w0 + 2 lane
-    float4 vi = S.v[0];
+    float4 vi = S.v()[0];
     for (int w0 = 0; w0 < P; w0 += 64, j += 64) {
       if (j > n - 1) {
         while (j > n - 1 && i < n - 2) { j += i + 2 - n; ++i; }
-        vi = S.v[i];
+        vi = S.v()[i];
       }
       const int p = w0 + 2 * lane;
       // the next pair in lexicographic order: the same row, or the next one's first
@@ -1017,16 +1038,16 @@ __global__ void __launch_bounds__(CELL_WARPS * 32, MINB)
         r1 = low_of_word(x.x2);
       }
       bool m0 = false, m1 = false;
-      if (p < P) m0 = !surely_skips(vi, S.v[j], cmax, r0);
-      if (p + 1 < P) m1 = !surely_skips(same ? vi : S.v[i2], S.v[j2], cmax, r1);
+      if (p < P) m0 = !surely_skips(vi, S.v()[j], cmax, r0);
+      if (p + 1 < P) m1 = !surely_skips(same ? vi : S.v()[i2], S.v()[j2], cmax, r1);
       if (!__any_sync(0xffffffffu, m0 | m1)) continue;
       ev.m = (m0 ? 1 : 0) | (m1 ? 2 : 0);
-      const bool go_on = window_events(a, S, n, P, w0, i, j, x, cmax, Tc, use_E, rnd != nullptr,
+      const bool go_on = window_events(S, n, P, w0, i, j, x, cmax, Tc, use_E, rnd != nullptr,
                                        event_limit, ev);
       c0 += ev.c0;
       c1 += ev.c1;
       if (!go_on) break;
-      vi = S.v[i];   // SIP i may have changed
+      vi = S.v()[i];   // SIP i may have changed
     }
     const int pos = ev.pos;
     const bool diagonal = ev.events > event_limit;
@@ -1047,14 +1068,14 @@ __global__ void __launch_bounds__(CELL_WARPS * 32, MINB)
             k53 = philox_bits53(a.seed, (uint64_t)rk, pc1);
             philox_interval(k53, r_lo, r_hi);
           }
-          const int sc = screen_pair(a, use_E, S.v[i], S.sk[i], S.v[j], S.sk[j], r_lo, r_hi);
+          const int sc = screen_pair(a, use_E, S.v()[i], S.sk()[i], S.v()[j], S.sk()[j], r_lo, r_hi);
           if (sc == 0) continue;
           if (sc == 1) {
-            certain_collection(a, S, i, j, Tc, use_E);
+            certain_collection(S, i, j, Tc, use_E);
             c0 += 1;
             continue;
           }
-          const int o = exact_pair(a, S, S.sid[i], S.sid[j], i, j, Tc, use_E,
+          const int o = exact_pair(S, S.sid()[i], S.sid()[j], i, j, Tc, use_E,
                                    rnd ? rnd[rk] : philox_from_bits(k53));
           c0 += o == 1;
           c1 += o == 2;
@@ -1063,17 +1084,81 @@ __global__ void __launch_bounds__(CELL_WARPS * 32, MINB)
         __syncwarp();
       }
     }
+    return make_int2(c0, c1);
+  }
+}
+// cells above the shared-memory size, out of line
+template <bool THIN>
+__device__ __noinline__ int2 collide_big(int64_t c, int32_t b, int n) {
+  const CellArgs& a = cell_args();
+  Cell<true> S;
+  S.base = b;
+  S.v_ = (float4*)a.gcopy + b;
+  S.sk_ = (int32_t*)((float4*)a.gcopy + a.n) + b;
+  S.sid_ = S.sk_ + a.n;
+  S.st_ = a.gstats + 2 * ((int64_t)(b >> 5) + c);
+  return collide_cell<THIN>(S, c, n, threadIdx.x & 31);
+}
+
+// THIN: the thinned draws, else per-pair draws.  MINB: resident blocks per
+// SM the register budget is set for (the TUNE_COLLISION_BLOCKS knob picks the
+// instance; 3 by default)
+template <bool THIN, int MINB>
+__global__ void __launch_bounds__(CELL_WARPS * 32, MINB)
+    k_collide_cells(const __grid_constant__ CK x) {
+  CellArgs& a = cell_args();
+  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+  if (threadIdx.x == 0) {
+    make_cellargs(a, x.m.get(), x.cc);
+    a.draw_base = a.draws ? *a.cursor : 0;
+    a.cstep = (uint64_t)*a.col_step;
+  }
+  __syncthreads();
+  if (a.draws && a.draw_base + *a.total_pairs > a.n_draws) {
+    if (blockIdx.x == 0 && threadIdx.x == 0) atomicOr(a.flags, LACMO_FLAG_DRAWS_SHORT);
+    return;
+  }
+  if constexpr (!THIN) {   // surely_skips' factor
+    if (wid == 0) {
+      float em = a.E_const_f;
+      if (a.E) {
+        // the largest of the row bounds (infinity without them: every pair is screened)
+        em = a.ecap ? 0.0f : __uint_as_float(0x7f800000u);
+        if (a.ecap) {
+          for (int64_t q = lane; q < a.nb; q += 32) em = fmaxf(em, __ldg(a.ecap + q));
+          em = __uint_as_float(__reduce_max_sync(0xffffffffu, __float_as_uint(em)));
+        }
+      }
+      if (lane == 0) a.cmax = skip_factor(a, em);
+    }
+    __syncthreads();
+  }
+  // persistent warps take the member's cells, largest first, from a counter
+  for (;;) {
+    int idx = 0;
+    if (lane == 0) idx = atomicAdd(a.cell_ctr, 1);
+    idx = __shfl_sync(0xffffffffu, idx, 0);
+    if (idx >= a.C) break;
+    const int64_t c = a.cell_order[idx];
+    const int32_t b = a.start[c];
+    const int n = a.start[c + 1] - b;
+    if (n < 2) break;   // the remaining cells hold fewer than two SIPs
+    if (n > 65535) {    // pair ranks would leave 32 bits
+      if (lane == 0) atomicOr(a.flags, LACMO_FLAG_CELL_TOO_BIG);
+      continue;
+    }
+    const int2 k = n > CELL_SMEM ? collide_big<THIN>(c, b, n)
+                                 : collide_cell<THIN>(Cell<false>{wid, b}, c, n, lane);
     __syncwarp();
-  }
-  // counters (integer sums commute)
-#pragma unroll
-  for (int off = 16; off > 0; off >>= 1) {
-    c0 += __shfl_down_sync(0xffffffffu, c0, off);
-    c1 += __shfl_down_sync(0xffffffffu, c1, off);
-  }
-  if (lane == 0 && (c0 | c1)) {
-    atomicAdd((unsigned long long*)a.no_cols, (unsigned long long)c0);
-    atomicAdd((unsigned long long*)(a.no_cols + 1), (unsigned long long)c1);
+    // counters (integer sums commute)
+    if (__any_sync(0xffffffffu, k.x | k.y)) {
+      const unsigned k0 = __reduce_add_sync(0xffffffffu, (unsigned)k.x);
+      const unsigned k1 = __reduce_add_sync(0xffffffffu, (unsigned)k.y);
+      if (lane == 0) {
+        atomicAdd((unsigned long long*)a.no_cols, (unsigned long long)k0);
+        atomicAdd((unsigned long long*)(a.no_cols + 1), (unsigned long long)k1);
+      }
+    }
   }
 }
 
@@ -1090,37 +1175,40 @@ static inline int nblk(int64_t n, int t) {
   if (b < 1) b = 1;
   return (int)(b < 152 * 32 ? b : 152 * 32);
 }
-static const size_t CELL_SMEM_BYTES = (size_t)CELL_WARPS * CELL_WARP_BYTES;
+static const size_t CELL_SMEM_BYTES = CELL_ARGS_BYTES + (size_t)CELL_WARPS * CELL_WARP_BYTES;
 
 // The FP32 copy of the efficiency table and the largest FP32 efficiency of
 // each row, one warp per row: the maximum of the row's positive values by a
 // warp reduction; a row with a NaN, or whose largest value is not positive
 // (where the sign of a zero or the place of a NaN decides), is taken in column
-// order by one lane, as the oracle does
+// order by one lane, as the oracle does.  ecap bounds the row from above whatever
+// it holds: a row with a NaN gets infinity (in column order a NaN hides the values
+// before it)
 __global__ void k_table_float(const double* __restrict__ E, float* __restrict__ Ef,
-                              float* __restrict__ erow, int64_t nb) {
+                              float* __restrict__ erow, float* __restrict__ ecap, int64_t nb) {
   const int lane = threadIdx.x & 31;
   const int64_t warps = (int64_t)gridDim.x * (blockDim.x >> 5);
   for (int64_t k = blockIdx.x * (int64_t)(blockDim.x >> 5) + (threadIdx.x >> 5); k < nb;
        k += warps) {
     const double* row = E + k * nb;
     uint32_t mk = 0;
-    bool odd = false;
+    bool nan = false;
     for (int64_t q = lane; q < nb; q += 32) {
       const float v = (float)__ldg(row + q);
       Ef[k * nb + q] = v;
-      odd |= v != v;
+      nan |= v != v;
       if (v > 0.0f) mk = max(mk, __float_as_uint(v));   // positive floats order as integers
     }
     mk = __reduce_max_sync(0xffffffffu, mk);
-    odd = __any_sync(0xffffffffu, odd) || mk == 0;
+    nan = __any_sync(0xffffffffu, nan);
     if (lane == 0) {
-      if (odd) {
+      if (nan || mk == 0) {
         float mx = (float)row[0];
         for (int64_t q = 1; q < nb; ++q) mx = lt_max(mx, (float)row[q]);
         erow[k] = mx;
+        ecap[k] = nan ? __uint_as_float(0x7f800000u) : mx;
       } else {
-        erow[k] = __uint_as_float(mk);
+        erow[k] = ecap[k] = __uint_as_float(mk);
       }
     }
   }
@@ -1178,15 +1266,16 @@ cudaError_t launch_collide_cells(const Bt& B, const lacmo_params_t& p, const lac
   cc.bin_margin = fp32_bin_margin(cc.lo, cc.bl, cc.nb);
   cc.E_const_f = (float)cc.E_const;
   cc.Ef = nullptr;
-  cc.erow = nullptr;
+  cc.erow = cc.ecap = nullptr;
   float* Ef = B.one.w.Ef;   // member 0's slot serves the whole batch
   if (p.E_col_grid && Ef && p.no_kernel_bins <= LACMO_MAX_KERNEL_BINS) {
     float* erow = Ef + (int64_t)LACMO_MAX_KERNEL_BINS * LACMO_MAX_KERNEL_BINS;
-    k_table_float<<<nblk(p.no_kernel_bins * 32, 128), 128, 0, s>>>(p.E_col_grid, Ef, erow,
-                                                                   p.no_kernel_bins);
+    k_table_float<<<nblk(p.no_kernel_bins * 32, 128), 128, 0, s>>>(
+        p.E_col_grid, Ef, erow, erow + LACMO_MAX_KERNEL_BINS, p.no_kernel_bins);
     note_launches(1);
     cc.Ef = Ef;
     cc.erow = erow;
+    cc.ecap = erow + LACMO_MAX_KERNEL_BINS;
   }
   // thinned draws need the row maxima of a tabulated efficiency
   cc.thin = (p.thin_draws != 0 && d.draws == nullptr && (!p.E_col_grid || cc.erow)) ? 1 : 0;

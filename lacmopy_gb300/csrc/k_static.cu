@@ -37,7 +37,7 @@ constexpr size_t st_off_gcopy = a256(st_off_order + 4 * STATIC_MAX_CELLS);
 constexpr size_t st_off_gstats = a256(st_off_gcopy + 24 * STATIC_MAX_SIPS);
 constexpr size_t st_off_Ef = a256(st_off_gstats + 32 * (STATIC_MAX_SIPS / 32 + STATIC_MAX_CELLS + 1));
 constexpr size_t st_off_scalars =
-    a256(st_off_Ef + 4 * (size_t)LACMO_MAX_KERNEL_BINS * (LACMO_MAX_KERNEL_BINS + 1));
+    a256(st_off_Ef + 4 * (size_t)LACMO_MAX_KERNEL_BINS * (LACMO_MAX_KERNEL_BINS + 2));
 constexpr size_t STATIC_BYTES = st_off_scalars + 256;
 
 static __device__ __align__(256) unsigned char g_noalloc_scratch[STATIC_BYTES];

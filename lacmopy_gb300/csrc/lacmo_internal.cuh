@@ -25,7 +25,7 @@ struct Ws {
   long long* acc64;    // [C][2] FP64: exact sums of dm * xi (acc_add64)
   double* accx;        // [C]   FP64: dm * xi beyond their range
   double* relax;       // [2][nz] relaxation terms (r_v, Theta)
-  double* colR;        // [n]   collision scratch for cells above the shared-memory size
+  double* colR;        // [n]   exact collision data by slot
   double* colrho;      // [n]
   int32_t* colk;       // [n]
   // scalars
@@ -36,7 +36,7 @@ struct Ws {
   int64_t* total_pairs;
   unsigned long long* nfb;   // mixed precision: Newton repeats in FP64
   float* Ef;                 // [LACMO_MAX_KERNEL_BINS^2] FP32 copy of the efficiency table,
-                             // then [LACMO_MAX_KERNEL_BINS] row maxima
+                             // then [LACMO_MAX_KERNEL_BINS] row maxima and as many bounds
   int32_t* cell_order;       // [C]   cells by descending SIP count (collision work order)
   int32_t* cell_ctr;         // next entry of cell_order a collision warp takes
   int32_t *fb_count, *fb_done;   // mixed precision: FP64 Newton queue length, blocks done

@@ -64,3 +64,23 @@ def test_windows_match_oracle(oracle_cr, draws, boost, rain):
             xi, mw, ms, st["vel"], T, st["cells"], st["grid_no_cells"], *args, u)
     assert boost * (1 + rain) == 1.0 or nc.sum() > 0
     _compare(ds, st, xi, mw, ms, nc)
+
+
+def test_efficiency_table_with_nan(oracle_cr):
+    """A NaN in a row of the efficiency table hides the values before it from a
+    maximum taken in column order; the first screen must not rely on that one."""
+    from lacmopy_gb300 import DeviceState
+    st = _state(2)
+    E = st["E_col_grid"] = st["E_col_grid"].copy()
+    E[:, -1] = np.nan
+    E[::2, 3] = np.nan
+    xi, mw, ms = st["xi"].copy(), st["m_w"].copy(), st["m_s"].copy()
+    nc, cs = np.zeros(2, np.int64), np.zeros(1, np.int64)
+    ds = DeviceState(st, draws="philox", seed=17)
+    ds.collision_step()
+    oracle_cr.collision_step_all_cells_philox(
+        xi, mw, ms, st["vel"], st["grid_scalar_fields"][0], st["cells"], st["grid_no_cells"],
+        st["dt_col_over_dV"], E, st["no_kernel_bins"], st["R_kernel_low_log"],
+        st["bin_factor_R_log"], nc, "AS", 17, cs)
+    assert nc.sum() > 0
+    _compare(ds, st, xi, mw, ms, nc)
