@@ -540,7 +540,7 @@ __global__ void __launch_bounds__(128) k_fwd_sips(const __grid_constant__ Args a
     double m;
     if (MAP) {
       bool ok;
-      m = newton_ff<true>(SOL_AS, a.no_iter, mw, ms, load_cell(a.rec + c), gdt, a.ks, &ok);
+      m = newton_ff<true, false>(SOL_AS, a.no_iter, mw, ms, load_cell(a.rec + c), gdt, a.ks, &ok);
       if (!ok) m = fwd_step64(a, c, mw, ms);
     } else {
       m = fwd_step64(a, c, mw, ms);
@@ -673,7 +673,7 @@ __device__ __forceinline__ bool map_grad(const Args& a, const CellFF& cf, const 
     for (int it = 0; it < a.no_iter - 1; ++it) {
       mi[it] = m;
       ff gd, x;
-      good = mass_rate_ff<true>(SOL_AS, false, m, ms, msf, cf, gdt, a.ks, gd, x) && good;
+      good = mass_rate_ff<true, false>(SOL_AS, false, m, ms, msf, cf, gdt, a.ks, gd, x) && good;
       const ff res = it == 0 ? gd : ff_sub(gd, d2ff(m - mw));
       m = np_max(floor_m, m + ff2d(ff_mul(res, damp_ff(x))));
     }

@@ -583,7 +583,7 @@ __device__ __noinline__ double particle_removed(const PArgs& a, int64_t k, int32
 // 670 FP64 instructions per SIP at 2 lanes an SM and clock, 478 us per launch
 // over 360,000 SIPs.  The Newton and the drag now run in two-float arithmetic
 // around the FP64 operations that decide the result's rounding (lacmo_ff.cuh;
-// about 60 a SIP are left, and some 3500 FP32 and integer instructions): 87 us.
+// about 65 a SIP are left, and some 3700 FP32 and integer instructions): 94 us.
 // New cell indices come from the FP32 position where it is clear of the cell's
 // edges, boundaries likewise.
 // SIPs that need plain FP64 for the Newton (a step of more than an eighth of
@@ -592,9 +592,13 @@ __device__ __noinline__ double particle_removed(const PArgs& a, int64_t k, int32
 // would hold all warps on the FP64 pipe, gathered they fill a few warps (a
 // raining state of 545,000 SIPs, 1.3% of them large drops, averaged over 20
 // sub-steps from a state out of equilibrium: 291 us in place, 217 us gathered,
-// 203 us with newton_fast; 732 us in plain FP64).
+// 144 us with newton_fast and no more blocks than are resident; 732 us in plain
+// FP64).
+__device__ __forceinline__ double i2d_int(int i) {   // i >= 0
+  return i < (1 << 24) ? f2d_int((float)i) : (double)i;
+}
 constexpr int PQ = 1024;   // queue slots; a SIP beyond them is done in place
-template <bool PHYS>
+template <bool PHYS, bool FULL>
 __global__ void __launch_bounds__(128) k_particles(const __grid_constant__ PK x) {
   __shared__ PArgs s_a;
   __shared__ int32_t s_q[PHYS ? PQ : 1];
@@ -643,15 +647,19 @@ __global__ void __launch_bounds__(128) k_particles(const __grid_constant__ PK x)
           for (int e = 0; e < 6; ++e) dst[e] = __ldg(src + e);
         }
         bool ok;
-        const double m = newton_ff<false>(a.sol, a.no_iter, mw, ms, cf,
+        const double m = newton_ff<false, FULL>(a.sol, a.no_iter, mw, ms, cf,
                                           d2ff(LC_FOUR_PI * 1.0E12 * a.dt_sub), 1.0, &ok);
         double dm = m - mw;
         bool slow = !ok;
         // integration.py:699-718 with the radius of ammonium sulfate whatever the
         // solute (:1075): the wind at the SIP
         const int4 wi = __ldg((const int4*)&wr->i);
-        const double rx = fma(-(double)wi.x, a.dx, x0 - a.x_min) * a.inv_dx;
-        const double rz = fma(-(double)wi.y, a.dz, z0 - a.z_min) * a.inv_dz;
+        // (no FP64 instruction for an origin at 0 or for an index)
+        double xo = x0, zo = z0;
+        if (__double_as_longlong(a.x_min) << 1) xo = x0 - a.x_min;
+        if (__double_as_longlong(a.z_min) << 1) zo = z0 - a.z_min;
+        const double rx = fma(-i2d_int(wi.x), a.dx, xo) * a.inv_dx;
+        const double rz = fma(-i2d_int(wi.y), a.dz, zo) * a.inv_dz;
         const double* const wd = (const double*)wr;
         auto ld = [&](int at) { return __ldg(wd + at); };
         // compared with 0.5 by their bits (an FP32 copy would take the wrong piece
@@ -674,7 +682,7 @@ __global__ void __launch_bounds__(128) k_particles(const __grid_constant__ PK x)
                    fma(rz, dy0, ld(7 + a0)));
         }
         const double du = uf - u, dw = wf - w;
-        const ff mpf = d2ff((mw + dm) + ms);
+        const ff mpf = d2ff(m + ms);   // (ok) a step below m / 8: mw + dm is m
         const ff wfr = ff_mul(d2ff(ms), ff_rcp(mpf));
         ff pr = ff_horner(FFC(LC_PAR_RHO_AS_1), FFC(LC_PAR_RHO_AS_0), wfr);
         pr = ff_horner(FFC(LC_PAR_RHO_AS_2), pr, wfr);
@@ -693,13 +701,17 @@ __global__ void __launch_bounds__(128) k_particles(const __grid_constant__ PK x)
             continue;
           }
         }
-        if (!ok) dm = particle_newton64(a, c, mw, ms);
-        mw += dm;
+        if (ok) {
+          mw = m;
+        } else {
+          dm = particle_newton64(a, c, mw, ms);
+          mw += dm;
+        }
         if (!slow) {
           // (u + k uf) / (1 + k) = uf - (uf - u) / (1 + k)
           const ff inv = ff_rcp(ff_add(kd, 1.0f));
-          u = uf - ff2d(ff_mul(duf, inv));
-          w = wf - ff2d(ff_mul(dwf, inv));
+          u = uf - ff2d_of<FULL>(ff_mul(duf, inv));
+          w = wf - ff2d_of<FULL>(ff_mul(dwf, inv));
         } else {
           particle_drag64(a, c, mw, ms, uf, wf, &u, &w);
         }
@@ -1624,16 +1636,48 @@ cudaError_t launch_bin(const Bt& B, cudaStream_t s) {
   note_launches(1);
   return cudaGetLastError();
 }
-cudaError_t launch_particles(const Bt& B, const lacmo_params_t& p, double dt_sub,
-                             double dt_sub_pos, bool write_Tp, bool hist, cudaStream_t s) {
-  PK x{B.ref(), pcall(p, dt_sub, dt_sub_pos, write_Tp, hist)};
-  k_particles<true><<<grid2(B.n_max, 128, B.M, 152 * 16), 128, 0, s>>>(x); note_launches(1);
-  return cudaGetLastError();
-}
 cudaError_t launch_move(const Bt& B, double dt_pos, bool hist, cudaStream_t s) {
   lacmo_params_t p = {};
   PK x{B.ref(), pcall(p, 0.0, dt_pos, false, hist)};
-  k_particles<false><<<grid2(B.n_max, 128, B.M, 152 * 16), 128, 0, s>>>(x); note_launches(1);
+  k_particles<false, false><<<grid2(B.n_max, 128, B.M, 152 * 16), 128, 0, s>>>(x); note_launches(1);
+  return cudaGetLastError();
+}
+// blocks of a kernel resident on the GPU at once, by device
+static cudaError_t resident_blocks(const void* f, int threads, size_t smem,
+                                   std::atomic<int>* cached, int* res) {
+  int dev = 0;
+  cudaError_t e = cudaGetDevice(&dev);
+  if (e != cudaSuccess) return e;
+  *res = dev < 64 ? cached[dev].load() : 0;
+  if (*res > 0) return cudaSuccess;
+  int per_sm = 0, sms = 0;
+  e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, f, threads, smem);
+  if (e != cudaSuccess) return e;
+  e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+  if (e != cudaSuccess) return e;
+  *res = per_sm * sms > 0 ? per_sm * sms : 1;
+  if (dev < 64) cached[dev].store(*res);
+  return cudaSuccess;
+}
+// No more blocks than are resident at once: a block's queue holds its place until
+// the few SIPs in it are done, some 15 us (360,000 SIPs: 128 us a launch with up to
+// 2432 blocks, 114 us with the 608 that are resident; 545,000 SIPs, 1.3% of them
+// large drops: 198 and 153 us).  States that fill the GPU more than once over
+// are bound by the FP64 pipe and take FULL (the two above: 107 and 144 us); smaller
+// ones wait for one SIP's chain, which FULL lengthens (1920 SIPs: 23.6 us without,
+// 23.9 us with it).
+cudaError_t launch_particles(const Bt& B, const lacmo_params_t& p, double dt_sub,
+                             double dt_sub_pos, bool write_Tp, bool hist, cudaStream_t s) {
+  PK x{B.ref(), pcall(p, dt_sub, dt_sub_pos, write_Tp, hist)};
+  static std::atomic<int> cached[64];
+  int res = 0;
+  cudaError_t e = resident_blocks((const void*)k_particles<true, true>, 128, 0, cached, &res);
+  if (e != cudaSuccess) return e;
+  const int cap = res / B.M > 0 ? res / B.M : 1;
+  const dim3 grid = grid2(B.n_max, 128, B.M, cap);
+  if (B.n_max > 128 * (int64_t)cap) k_particles<true, true><<<grid, 128, 0, s>>>(x);
+  else k_particles<true, false><<<grid, 128, 0, s>>>(x);
+  note_launches(1);
   return cudaGetLastError();
 }
 // Resident-sized grid for the pipelined mixed kernel: each thread walks many
@@ -1641,20 +1685,10 @@ cudaError_t launch_move(const Bt& B, double dt_pos, bool hist, cudaStream_t s) {
 template <bool PHYS, int MINB>
 static cudaError_t mixed_launch(const Bt& B, const PK& x, cudaStream_t s) {
   static std::atomic<int> cached[64];
-  int dev = 0;
-  cudaError_t e = cudaGetDevice(&dev);
+  int res = 0;
+  cudaError_t e = resident_blocks((const void*)k_particles_mixed<PHYS, MINB>, PM_THREADS, PM_SMEM,
+                                  cached, &res);
   if (e != cudaSuccess) return e;
-  int res = dev < 64 ? cached[dev].load() : 0;
-  if (res <= 0) {
-    int per_sm = 0, sms = 0;
-    e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_particles_mixed<PHYS, MINB>,
-                                                      PM_THREADS, PM_SMEM);
-    if (e != cudaSuccess) return e;
-    e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-    if (e != cudaSuccess) return e;
-    res = per_sm * sms > 0 ? per_sm * sms : 1;
-    if (dev < 64) cached[dev].store(res);
-  }
   // resident-sized grid: each warp walks many tiles through the staging
   // pipeline; small states take one block per tile (more blocks in flight
   // hide the latency better)

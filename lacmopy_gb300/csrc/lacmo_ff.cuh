@@ -112,6 +112,19 @@ LACMO_DEV ff d2ff(double x) {
   return r;
 }
 LACMO_DEV double ff2d(ff a) { return f2d_int(a.h) + f2d_int(a.l); }
+// The same bits without an FP64 instruction, |l| <= ulp(h) / 2: l in units of h's 53-bit ulp (half
+// of it below a power of two), rounded by the conversion to integer, added to h's
+// bits.  Some 18 integer instructions where one FP64 addition takes the SM's FP64
+// pipe for as long as 64 of them; for kernels that fill that pipe (its chain is some
+// tens of cycles longer than the addition's).
+LACMO_DEV double ff2d_int(ff a) {
+  const uint32_t hb = __float_as_uint(a.h), eh = (hb >> 23) & 0xffu;
+  if (eh - 53u >= 202u) return ff2d(a);   // 0, below 2^-74, not finite
+  const uint32_t lb = __float_as_uint(a.l) ^ (hb & 0x80000000u);   // l away from zero
+  const uint32_t below = (hb & 0x007fffffu) == 0u ? lb >> 31 : 0u;
+  const int k = __float2int_rn(fm(__uint_as_float(lb), __uint_as_float((306u + below - eh) << 23)));
+  return __longlong_as_double(__double_as_longlong(f2d_int(a.h)) + (long long)k);
+}
 
 // ---------------------------------------------------------------------------
 // A cell's terms for the FP64 particle sub-step: one record of 128 bytes
@@ -155,13 +168,16 @@ static_assert(sizeof(CellFF) == 128 && sizeof(WindFF) == 128, "one line each");
 // evaluation; the reference's iterations use those of ammonium sulfate).
 // ks scales a_w - 1 (KS; the adjoint's hygroscopicity).
 // Returns false when eps leaves the series' range (0.25; R below some 5 nm).
-template <bool KS>
+// FULL: for a full FP64 pipe (ff2d_int).
+template <bool FULL>
+LACMO_DEV double ff2d_of(ff a) { return FULL ? ff2d_int(a) : ff2d(a); }
+template <bool KS, bool FULL>
 LACMO_DEV bool mass_rate_ff(int sol, bool nacl_rho, double m, double ms, ff msf, const CellFF& c,
                             ff gdt, double ks, ff& gd, ff& x) {
   const double mp = m + ms;
   const ff imp = ff_rcp(d2ff(mp));
   const ff wf = ff_mul(msf, imp);
-  double w = ff2d(wf);
+  double w = ff2d_of<FULL>(wf);
   w = fma(fma(-w, mp, ms), f2d_int(imp.h), w);   // m_s / m_p, one correction
   const ff q = ff_mul(msf, ff_rcp(d2ff(m)));
   ff pr, pd, da;
@@ -205,7 +221,7 @@ LACMO_DEV bool mass_rate_ff(int sol, bool nacl_rho, double m, double ms, ff msf,
   const ff R = ff_mul(ff_mul(xr, z), z);
   const ff eps = ff_mul(ff_mul(c.ce, sg), ff_mul(ipr, z));
   const ff em1 = ff_expm1(eps);
-  const double sm1 = fma(1.0 + aw_m1, ff2d(em1), aw_m1);   // S_eq - 1
+  const double sm1 = fma(1.0 + aw_m1, ff2d_of<FULL>(em1), aw_m1);   // S_eq - 1
   const double f2d_ = c.S_m1 - sm1;
   const ff f2 = d2ff(f2d_);
   const ff Seq = ff_add(d2ff(sm1), 1.0f);
@@ -242,20 +258,25 @@ LACMO_DEV bool ff_mass_ok(double m) {
 // map in 64-bit mantissas (80,000 SIPs of fresh and raining states, AS and NaCl)
 // the masses are off by 0.3 to 0.9 of newton_full's error in every range of
 // step sizes below an eighth, and by 1.3 to 10 of it above.
-template <bool KS>
+template <bool KS, bool FULL>
 LACMO_DEV double newton_ff(int sol, int no_iter, double m_w, double m_s, const CellFF& c, ff gdt,
                            double ks, bool* ok) {
   const double floor_m = m_s * (LC_W_S_MAX_AS_INV - 1.0);
   const ff msf = d2ff(m_s);
   ff gd, x;
-  bool good = mass_rate_ff<KS>(sol, sol != SOL_AS, m_w, m_s, msf, c, gdt, ks, gd, x);
-  double m = np_max(floor_m, m_w + ff2d(ff_mul(gd, damp_ff(x))));
+  bool good = mass_rate_ff<KS, FULL>(sol, sol != SOL_AS, m_w, m_s, msf, c, gdt, ks, gd, x);
+  // np_max for a positive floor by the bits; NaN and infinity clear good
+  auto floored = [&](double m) {
+    good = good && (uint32_t)((__double2hiint(m) >> 20) & 0x7ff) != 0x7ffu;
+    return __double_as_longlong(m) > __double_as_longlong(floor_m) ? m : floor_m;
+  };
+  double m = floored(m_w + ff2d_of<FULL>(ff_mul(gd, damp_ff(x))));
   for (int it = 0;;) {
     const ff d = d2ff(m - m_w);
     good = good && fabsf(d.h) <= 0.125f * d2f_int(m);
     if (++it >= no_iter) break;
-    good = mass_rate_ff<KS>(sol, false, m, m_s, msf, c, gdt, ks, gd, x) && good;
-    m = np_max(floor_m, m + ff2d(ff_mul(ff_sub(gd, d), damp_ff(x))));
+    good = mass_rate_ff<KS, FULL>(sol, false, m, m_s, msf, c, gdt, ks, gd, x) && good;
+    m = floored(m + ff2d_of<FULL>(ff_mul(ff_sub(gd, d), damp_ff(x))));
   }
   *ok = good && ff_mass_ok(m_w) && ff_mass_ok(m_s) && m < 1e29;
   return m;

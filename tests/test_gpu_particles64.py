@@ -216,3 +216,26 @@ def test_map_gradient_vs_torch(no_iter):
     assert abs(float(J.detach()) - float(J_r.detach())) <= 1e-11 * abs(float(J_r.detach()))
     for x, y in zip(g, r):
         assert float((x.cpu() - y).abs().max()) <= 1e-9 * float(y.abs().max())
+
+
+@pytest.mark.parametrize("solute", ["AS", "NaCl"])
+def test_full_and_sparse_grids_agree(solute):
+    """The conversions without FP64 instructions (states of more SIPs than are
+    resident) give the bits of the plain ones: a state too small for them, and
+    the same state twice in a batch that is large enough."""
+    import copy
+    from lacmopy_gb300 import BatchState, DeviceState, synthetic
+    st = synthetic.make_icmw_state(Nx=25, Nz=25, no_spcm=(32, 40), seed=8, kernel_type="Long_Bott",
+                                   drizzle_fraction=0.05, r_tot=11E-3)
+    st["solute_type"] = solute
+    assert 39000 < st["xi"].size < 77000   # between two and four blocks of 128 an SM
+    one = DeviceState(copy.deepcopy(st), draws="philox", seed=5)
+    one.adv_step(2)
+    two = BatchState([copy.deepcopy(st), copy.deepcopy(st)], [5, 5], precision="fp64",
+                     draws="philox")
+    two.adv_step(2)
+    a = one.snapshot()
+    for m in range(2):
+        b = two.snapshot(m)
+        for k in ("m_w", "vel", "pos", "xi", "grid_scalar_fields", "water_removed"):
+            assert np.array_equal(a[k], b[k]), k
