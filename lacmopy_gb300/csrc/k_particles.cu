@@ -118,64 +118,99 @@ __global__ void k_histogram(const __grid_constant__ MRef mr) {
   }
 }
 
+// Exclusive sums of a and b over the block's 1024 threads; the block's sums come
+// back in ta, tb.  w: shared memory, free again after the caller's next barrier.
+__device__ __forceinline__ void block_exclusive(int32_t& a, int64_t& b, int32_t& ta, int64_t& tb,
+                                                int32_t (*wa)[33], int64_t (*wb)[33]) {
+  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+  int32_t x = a;
+  int64_t y = b;
+#pragma unroll
+  for (int off = 1; off < 32; off <<= 1) {
+    const int32_t u = __shfl_up_sync(0xffffffffu, x, off);
+    const int64_t v = __shfl_up_sync(0xffffffffu, y, off);
+    if (lane >= off) { x += u; y += v; }
+  }
+  if (lane == 31) { (*wa)[wid] = x; (*wb)[wid] = y; }
+  __syncthreads();
+  // every warp sums the warps' totals up
+  int32_t p = (*wa)[lane];
+  int64_t q = (*wb)[lane];
+#pragma unroll
+  for (int off = 1; off < 32; off <<= 1) {
+    const int32_t u = __shfl_up_sync(0xffffffffu, p, off);
+    const int64_t v = __shfl_up_sync(0xffffffffu, q, off);
+    if (lane >= off) { p += u; q += v; }
+  }
+  ta = __shfl_sync(0xffffffffu, p, 31);
+  tb = __shfl_sync(0xffffffffu, q, 31);
+  const int32_t p0 = __shfl_sync(0xffffffffu, p, wid > 0 ? wid - 1 : 0);
+  const int64_t q0 = __shfl_sync(0xffffffffu, q, wid > 0 ? wid - 1 : 0);
+  a = x - a + (wid ? p0 : 0);
+  b = y - b + (wid ? q0 : 0);
+}
 // Single block: the exclusive scans of the SIP counts (slots) and pair counts
-// (draws), and the collision work order.
+// (draws), and the collision work order: cells by descending SIP count (a counting
+// sort on min(count, 1023); the order inside a size class is arbitrary).  Waits
+// for barriers, loads and atomics, so a tile of 1024 cells takes one barrier, its
+// counts are there before, and a warp whose cells are of one class takes their
+// places with one atomic (120 cells: 5.7 us with scans through shared memory and
+// strided chunks, 3.3 us now; 5625 cells: 15.6 and 9.8 us).
 __global__ void __launch_bounds__(1024) k_scan(const __grid_constant__ MRef mr) {
   const Member& mb = mr.get();
-  int32_t *counts = mb.w.counts, *start = mb.w.start;
+  int32_t *counts = mb.w.counts, *start = mb.w.start, *order = mb.w.cell_order;
   int64_t *draw_off = mb.w.draw_off, *total_pairs = mb.w.total_pairs;
   const int64_t C = mb.g.nx * mb.g.nz;
-  __shared__ int64_t s_slot[1024];
-  __shared__ int64_t s_pair[1024];
-  const int t = threadIdx.x;
-  int64_t chunk = (C + blockDim.x - 1) / blockDim.x;
-  int64_t b0 = t * chunk, b1 = b0 + chunk < C ? b0 + chunk : C;
-  int64_t ss = 0, sp = 0;
-  for (int64_t c = b0; c < b1; ++c) {
-    int64_t m = counts[c];
-    ss += m; sp += m * (m - 1) / 2;
-  }
-  s_slot[t] = ss; s_pair[t] = sp;
-  __syncthreads();
-  for (int off = 1; off < (int)blockDim.x; off <<= 1) {
-    int64_t a = t >= off ? s_slot[t - off] : 0, b = t >= off ? s_pair[t - off] : 0;
-    __syncthreads();
-    s_slot[t] += a; s_pair[t] += b;
-    __syncthreads();
-  }
-  int64_t os = s_slot[t] - ss, op = s_pair[t] - sp;
-  for (int64_t c = b0; c < b1; ++c) {
-    int64_t m = counts[c];
-    start[c] = (int32_t)os; draw_off[c] = op;
-    os += m; op += m * (m - 1) / 2;
-    counts[c] = 0;
-  }
-  if (t == blockDim.x - 1) { start[C] = (int32_t)os; draw_off[C] = op; *total_pairs = op; }
-  // ---- collision work order: cells by descending SIP count (a counting
-  // sort on min(count, 1023); the order inside a size class is arbitrary) ----
   __shared__ int32_t s_hist[1024];
-  int32_t* order = mb.w.cell_order;
+  __shared__ int32_t s_a[2][33];
+  __shared__ int64_t s_b[2][33];
+  const int t = threadIdx.x, lane = t & 31;
   s_hist[t] = 0;
   __syncthreads();
-  for (int64_t c = b0; c < b1; ++c) {
-    const int32_t m = start[c + 1] - start[c];
-    atomicAdd(&s_hist[1023 - (m < 1023 ? m : 1023)], 1);
+  auto size_class = [](int32_t m) { return 1023 - (m < 1023 ? m : 1023); };
+  int32_t os = 0;
+  int64_t op = 0;
+  int32_t next = t < C ? counts[t] : 0;
+  for (int64_t base = 0, tile = 0; base < C; base += 1024, ++tile) {
+    const int64_t c = base + t;
+    const int32_t m = next;
+    next = c + 1024 < C ? counts[c + 1024] : 0;
+    // one atomic for a warp of one class (fresh states), else one per cell
+    const int key = c < C ? size_class(m) : -1;
+    if (__all_sync(0xffffffffu, key == __shfl_sync(0xffffffffu, key, 0))) {
+      if (lane == 0 && key >= 0) atomicAdd(&s_hist[key], 32);
+    } else if (key >= 0) {
+      atomicAdd(&s_hist[key], 1);
+    }
+    int32_t a = m, ta;
+    int64_t b = (int64_t)m * (m - 1) / 2, tb;
+    block_exclusive(a, b, ta, tb, &s_a[tile & 1], &s_b[tile & 1]);
+    if (c < C) {
+      start[c] = os + a;
+      draw_off[c] = op + b;
+    }
+    os += ta;
+    op += tb;
   }
+  if (t == 0) { start[C] = os; draw_off[C] = op; *total_pairs = op; }
   __syncthreads();
-  const int32_t hv = s_hist[t];
-  s_slot[t] = hv;
+  int32_t first = s_hist[t], ta;
+  int64_t z = 0, tb;
+  block_exclusive(first, z, ta, tb, &s_a[0], &s_b[0]);
+  s_hist[t] = first;
   __syncthreads();
-  for (int off = 1; off < 1024; off <<= 1) {
-    const int64_t add = t >= off ? s_slot[t - off] : 0;
-    __syncthreads();
-    s_slot[t] += add;
-    __syncthreads();
-  }
-  s_hist[t] = (int32_t)(s_slot[t] - hv);
-  __syncthreads();
-  for (int64_t c = b0; c < b1; ++c) {
-    const int32_t m = start[c + 1] - start[c];
-    order[atomicAdd(&s_hist[1023 - (m < 1023 ? m : 1023)], 1)] = (int32_t)c;
+  for (int64_t base = 0; base < C; base += 1024) {
+    const int64_t c = base + t;
+    const int key = c < C ? size_class(counts[c]) : -1;
+    if (c < C) counts[c] = 0;
+    if (__all_sync(0xffffffffu, key == __shfl_sync(0xffffffffu, key, 0))) {
+      int at = 0;
+      if (lane == 0 && key >= 0) at = atomicAdd(&s_hist[key], 32);
+      at = __shfl_sync(0xffffffffu, at, 0);
+      if (key >= 0) order[at + lane] = (int32_t)c;
+    } else if (key >= 0) {
+      order[atomicAdd(&s_hist[key], 1)] = (int32_t)c;
+    }
   }
 }
 
@@ -1427,38 +1462,43 @@ __global__ void __launch_bounds__(256) k_r_l(const __grid_constant__ MRef mr) {
 __device__ __forceinline__ double limiter_arg(double a0, double a1, double a2) {
   const double r = (fabs(a1 - a2) > 1.0E-8 * fabs(a0 - a1)) ? (a0 - a1) / (a1 - a2)
                                                              : (a0 - a1) * 1.0E8 * np_sign(a1 - a2);
-  const double K = (1.0 + 2.0 * r) * LC_ONE_THIRD;
+  const double K = __dmul_rn(1.0 + 2.0 * r, LC_ONE_THIRD);
   return np_max(0.0, fmin(2.0 * r, fmin(K, 2.0)));
 }
-__device__ __forceinline__ double face_flux(double u, double am2, double am1, double a0,
-                                            double ap1) {
-  const double lp = limiter_arg(a0, am1, am2);
-  const double f_pos = am1 + 0.5 * lp * (am1 - am2);
-  const double ln = limiter_arg(am1, a0, ap1);
-  const double f_neg = a0 + 0.5 * ln * (a0 - ap1);
-  return (u >= 0.0) ? u * f_pos : u * f_neg;
+// the field at a face, from the limiter of the upwind side only
+__device__ __forceinline__ double face_value(double u, double am2, double am1, double a0,
+                                             double ap1) {
+  const bool pos = u >= 0.0;
+  const double o = pos ? a0 : am1, p = pos ? am1 : a0, q = pos ? am2 : ap1;
+  return __fma_rn(0.5 * limiter_arg(o, p, q), p - q, p);
 }
-__device__ __forceinline__ int64_t bc_idx(int64_t i, int64_t N, int bc) {
-  if (bc == 0) { i %= N; return i < 0 ? i + N : i; }
+// i in [-2, N + 1], wrapped (bc 0) or clamped
+__device__ __forceinline__ int bc_idx(int i, int N, int bc) {
+  if (bc == 0) return N == 1 ? 0 : (i < 0 ? i + N : (i >= N ? i - N : i));
   return i < 0 ? 0 : (i > N - 1 ? N - 1 : i);
 }
-// integration.py:150-287, divergence of field * flux in cell (i, j)
-__device__ double divergence_cell(const double* f, const double* flux, int64_t nx, int64_t nz,
-                                  int64_t i, int64_t j, double dx, double dz, int bcx, int bcz) {
-  double Fx[2], Fz[2];
-  for (int s = 0; s < 2; ++s) {
-    const int64_t fi = i + s;  // face index
-    double u = flux[fi * (nz + 1) + j];
-    Fx[s] = face_flux(u, f[bc_idx(fi - 2, nx, bcx) * nz + j], f[bc_idx(fi - 1, nx, bcx) * nz + j],
-                      f[bc_idx(fi, nx, bcx) * nz + j], f[bc_idx(fi + 1, nx, bcx) * nz + j]);
-    if (bcx == 1 && (fi == 0 || fi == nx)) Fx[s] = 0.0;
-    const int64_t fj = j + s;
-    double w = flux[(nx + 1) * (nz + 1) + i * (nz + 1) + fj];
-    Fz[s] = face_flux(w, f[i * nz + bc_idx(fj - 2, nz, bcz)], f[i * nz + bc_idx(fj - 1, nz, bcz)],
-                      f[i * nz + bc_idx(fj, nz, bcz)], f[i * nz + bc_idx(fj + 1, nz, bcz)]);
-    if (bcz == 1 && (fj == 0 || fj == nz)) Fz[s] = 0.0;
-  }
-  return (Fx[1] - Fx[0]) / dx + (Fz[1] - Fz[0]) / dz;
+// integration.py:150-287, divergence of field * flux in cell (i, j): the part of
+// the faces across x (dir 0) or z (dir 1).  Roundings are written out, and fuse
+// forms the difference of the two fluxes with one (r_v across x): the mixed path
+// rounds cell terms to FP32, where an increment's last bit shows.
+__device__ __forceinline__ double divergence_part(const double* f, const double* flux, int nx,
+                                                  int nz, int i, int j, int dir, double d, int bc,
+                                                  bool fuse) {
+  const int N = dir ? nz : nx, at = dir ? j : i;
+  const int64_t step = dir ? 1 : nz, fstep = dir ? 1 : nz + 1;
+  const double* const g = f + (dir ? (int64_t)i * nz : j);
+  const double* const u = flux + (dir ? (int64_t)(nx + 1) * (nz + 1) : 0) + (int64_t)i * (nz + 1) + j;
+  double v[5];
+#pragma unroll
+  for (int e = 0; e < 5; ++e) v[e] = g[bc_idx(at + e - 2, N, bc) * step];
+  const double u0 = u[0], u1 = u[fstep];
+  const double f0 = face_value(u0, v[0], v[1], v[2], v[3]);
+  const double f1 = face_value(u1, v[1], v[2], v[3], v[4]);
+  double F0 = __dmul_rn(u0, f0), F1 = __dmul_rn(u1, f1);
+  if (bc == 1 && at == 0) F0 = 0.0;
+  if (bc == 1 && at + 1 == N) F1 = 0.0;
+  if (fuse) return __fma_rn(u1, f1, -F0) / d;
+  return __dsub_rn(F1, F0) / d;
 }
 
 __global__ void k_divergence(const double* f, const double* flux, int64_t nx, int64_t nz, double dx,
@@ -1466,7 +1506,8 @@ __global__ void k_divergence(const double* f, const double* flux, int64_t nx, in
   for (int64_t c = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; c < nx * nz;
        c += (int64_t)gridDim.x * blockDim.x) {
     const int64_t i = c / nz, j = c - i * nz;
-    out[c] = divergence_cell(f, flux, nx, nz, i, j, dx, dz, bcx, bcz);
+    out[c] = divergence_part(f, flux, (int)nx, (int)nz, (int)i, (int)j, 0, dx, bcx, false) +
+             divergence_part(f, flux, (int)nx, (int)nz, (int)i, (int)j, 1, dz, bcz, false);
   }
 }
 
@@ -1505,32 +1546,41 @@ __global__ void k_relaxation2(const __grid_constant__ MRef mr, const double* pro
 }
 
 // integration.py:1483-1508 (factor 1) and 1536-1561 (factor 2, minus the
-// previous increment): advective + relaxation increments per sub-step
+// previous increment): advective + relaxation increments per sub-step.  Bound
+// by the chain of FP64 operations of a face (and, with many members, by the FP64
+// pipe): four lanes per cell, r_v and Theta across x and across z, two faces each
+// (5625 cells: 21.0 us with one thread per cell and both limiters of every
+// face, 5.9 us now; 64 members of 5625 cells: 303 and 163 us).
 __global__ void k_advection(const __grid_constant__ MRef mr, double dt_sub, int relax_on,
                             int second) {
   const Member& mb = mr.get();
   const double *gsf = mb.g.scalar_fields, *flux = mb.g.mass_flux_air_dry, *relax = mb.w.relax;
-  const int64_t nx = mb.g.nx, nz = mb.g.nz;
+  const int nx = (int)mb.g.nx, nz = (int)mb.g.nz;
   const double dx = mb.g.dx, dz = mb.g.dz;
-  double *dTh = mb.w.dTh, *drv = mb.w.drv;
-  const int64_t C = nx * nz;
-  for (int64_t c = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; c < C;
-       c += (int64_t)gridDim.x * blockDim.x) {
-    const int64_t i = c / nz, j = c - i * nz;
+  const int64_t C = (int64_t)nx * nz;
+  const int role = threadIdx.x & 3, th = role & 1, dir = role >> 1;
+  double* const out = th ? mb.w.dTh : mb.w.drv;
+  const int64_t cells = (int64_t)gridDim.x * blockDim.x >> 2;
+  for (int64_t c0 = (int64_t)blockIdx.x * blockDim.x >> 2; c0 < C; c0 += cells) {
+    int64_t c = c0 + (threadIdx.x >> 2);
+    const bool in = c < C;
+    if (!in) c = C - 1;
+    const int i = (int)(c / nz), j = (int)(c - (int64_t)i * nz);
+    const double part = divergence_part(gsf + (th ? 2 : 4) * C, flux, nx, nz, i, j, dir,
+                                        dir ? dz : dx, dir, !dir && !th);
+    const double div = part + __shfl_xor_sync(0xffffffffu, part, 2);
+    if (dir || !in) continue;
     const double rdi = gsf[9 * C + c];
-    const double drv_div = divergence_cell(gsf + 4 * C, flux, nx, nz, i, j, dx, dz, 0, 1);
-    const double dth_div = divergence_cell(gsf + 2 * C, flux, nx, nz, i, j, dx, dz, 0, 1);
-    double a, b;
+    double a;
+    const double w = -dt_sub * div, w2 = -2.0 * dt_sub * div;
     if (!second) {
-      a = -dt_sub * drv_div * rdi;
-      b = -dt_sub * dth_div * rdi;
-      if (relax_on) { a += relax[j]; b += relax[nz + j]; }
+      a = __dmul_rn(w, rdi);
+      if (relax_on) a = __dadd_rn(a, relax[th * nz + j]);
     } else {
-      a = -2.0 * dt_sub * drv_div * rdi - drv[c];
-      b = -2.0 * dt_sub * dth_div * rdi - dTh[c];
-      if (relax_on) { a += 2. * relax[j]; b += 2. * relax[nz + j]; }
+      a = __fma_rn(w2, rdi, -out[c]);
+      if (relax_on) a = __fma_rn(2., relax[th * nz + j], a);
     }
-    drv[c] = a; dTh[c] = b;
+    out[c] = a;
   }
 }
 
@@ -1749,7 +1799,7 @@ cudaError_t launch_advection(const Bt& B, const lacmo_params_t& p, bool second, 
                                                            p.init_profile_Theta,
                                                            p.relaxation_time_profile, p.dt_sub); note_launches(1);
   }
-  k_advection<<<grid2(B.nx * B.nz, 32, B.M), 32, 0, s>>>(B.ref(), p.dt_sub, relax_on ? 1 : 0,
+  k_advection<<<grid2(4 * B.nx * B.nz, 32, B.M), 32, 0, s>>>(B.ref(), p.dt_sub, relax_on ? 1 : 0,
                                                           second ? 1 : 0); note_launches(1);
   return cudaGetLastError();
 }
