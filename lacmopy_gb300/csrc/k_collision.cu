@@ -366,7 +366,7 @@ __device__ __noinline__ bool equal_multiplicities(double xi_min, double xi_max) 
 // state 1.20 ms against 0.94 ms): most rows hold one event.  Same decisions and operation order as exact_pair and
 // collect_once.  Returns 0 (no collision), 1 (one collection) or 2 (multiple
 // collection), the same in all lanes.
-template <bool BIG>
+template <bool THIN, bool BIG>
 __device__ __forceinline__ int warp_event(Cell<BIG> S, int l0, int l1, double Tc,
                                        bool use_E, double r, bool certain) {
   const CellArgs& a = cell_args();
@@ -473,7 +473,8 @@ __device__ __forceinline__ int warp_event(Cell<BIG> S, int l0, int l1, double Tc
     Rf = d2f_rn(R);
     kb = gk;
   } else {
-    Rf = lt_cbrtf((float)LC_FOUR_PI_OVER_THREE_INV * d2f_rn(mw + ms) / d2f_rn(rho));
+    const float mf = (float)LC_FOUR_PI_OVER_THREE_INV * d2f_rn(mw + ms), rf = d2f_rn(rho);
+    Rf = THIN ? lt_cbrtf(mf / rf) : f_cbrt(mf * f_rcp(rf));
     gk = GK_STALE;
     if (use_E) {
       const float v = (__logf(Rf) - a.lo_f) * a.inv_bl_f + 0.5f;
@@ -595,7 +596,7 @@ __device__ __forceinline__ void init_exact_scratch(const CellArgs& a, Cell<BIG> 
 // on to its own first hit cost a screen of the whole rest of the cell: a step
 // of a raining 75 x 75 x 128 state (14 collections per cell on average, 190 in the
 // heaviest, whose chain of events of some 5 us each is what the step waits for) took
-// 10.6 ms, 0.83 ms now.
+// 10.6 ms, 0.78 ms now.
 // Returns false when the event limit is passed (ev.pos: the first rank left).
 struct PairEvents {
   int pos, events, c0, c1;
@@ -651,7 +652,7 @@ __device__ __noinline__ bool window_events(Cell<BIG> S, int n, int P, int w0,
       const uint32_t scL = __shfl_sync(FULL, sc, L);
       const bool sec = (scL & 3u) == 0;
       const uint64_t dr = ((uint64_t)(sec ? x.x2 : x.x0) << 32) | (sec ? x.x3 : x.x1);
-      const int o = warp_event(S, __shfl_sync(FULL, sec ? i2 : i, L),
+      const int o = warp_event<false>(S, __shfl_sync(FULL, sec ? i2 : i, L),
                                __shfl_sync(FULL, sec ? j2 : j, L), Tc, use_E,
                                draw_of(injected, __shfl_sync(FULL, dr, L)),
                                (sec ? scL >> 2 : scL & 3u) == 1u);
@@ -735,7 +736,7 @@ __device__ __forceinline__ float skip_factor(const CellArgs& a, float em) {
 template <bool BIG>
 __device__ __noinline__ int event_call(Cell<BIG> S, int l0, int l1, double Tc, bool use_E, double r,
                                        bool certain) {
-  return warp_event(S, l0, l1, Tc, use_E, r, certain);
+  return warp_event<true>(S, l0, l1, Tc, use_E, r, certain);
 }
 
 // The thinned draws of lacmo_thin.h for one cell, warp-cooperative.  A round
@@ -948,7 +949,8 @@ __device__ __forceinline__ int2 collide_cell(const Cell<BIG> S, int64_t c, int n
   const double Tc = a.T[c];
   const uint64_t pc1 = (a.cstep << 32) | (uint64_t)c;
   const int32_t* ids = a.perm + S.base;
-  // FP32 copies, FP32 radius and bin (exact when near a bin edge)
+  // FP32 copies, FP32 radius and bin (exact when near a bin edge).  Thinned draws
+  // bound segments with the radius' bits; per-pair screens take it within 1e-6
   const float Tf = d2f_rn(Tc);
   const float rhow_f = (float)LC_PAR_WATER_DENS_0 +
                        (float)LC_PAR_WATER_DENS_1 * ((Tf - (float)LC_PAR_WATER_DENS_2) *
@@ -972,7 +974,7 @@ __device__ __forceinline__ int2 collide_cell(const Cell<BIG> S, int64_t c, int n
     }
     const float mwf = d2f_rn(mw_q), msf = d2f_rn(ms_q);
     const float mpf = mwf + msf;
-    const float wsf = msf / mpf;
+    const float wsf = THIN ? msf / mpf : msf * f_rcp(mpf);
     const float rho = (a.sol == SOL_AS)
                           ? rhow_f * ((((float)LC_PAR_RHO_AS_0 * wsf + (float)LC_PAR_RHO_AS_1) *
                                            wsf + (float)LC_PAR_RHO_AS_2) * wsf +
@@ -982,7 +984,8 @@ __device__ __forceinline__ int2 collide_cell(const Cell<BIG> S, int64_t c, int n
                                 (float)LC_PAR_SOL_DENS_NACL_3 * wsf * wsf +
                                 (float)LC_PAR_SOL_DENS_NACL_4 * wsf * Tf +
                                 (float)LC_PAR_SOL_DENS_NACL_5 * Tf * Tf;
-    const float Rf = lt_cbrtf((float)LC_FOUR_PI_OVER_THREE_INV * mpf / rho);
+    const float V = (float)LC_FOUR_PI_OVER_THREE_INV * mpf;
+    const float Rf = THIN ? lt_cbrtf(V / rho) : f_cbrt(V * f_rcp(rho));
     int32_t kb = 0;
     if (use_E) {
       const float v = (__logf(Rf) - a.lo_f) * a.inv_bl_f + 0.5f;
