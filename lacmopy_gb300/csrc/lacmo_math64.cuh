@@ -77,6 +77,10 @@ LACMO_DEV double log64(double x) {
   return __fma_rn(ed, LN2_HI, __dadd_rn(f, __fma_rn(ed, LN2_LO, -w)));
 }
 
+// (the aarch64 compiler fails on these inlined into the four-lane update)
+static __device__ __noinline__ double log64_call(double x) { return log64(x); }
+static __device__ __noinline__ double exp64_call(double x) { return exp64(x); }
+
 // ---- the cell update of integration.py:402-438 (Theta, r_v) and the fields that
 // follow from it (atmosphere.py, update_material_properties :359).  The powers
 // go through one logarithm each, pow(x, y) = exp(y log x), with |y log x| below
@@ -135,14 +139,17 @@ static __device__ __noinline__ CellState cell_state64(double Th, double r_v, dou
   a.t = cell_terms64(a.T, a.p, a.e_s, a.L_v, a.K, a.D_v);
   return a;
 }
-// the FP64 path's record of a cell
+// the FP64 path's record of a cell; irho = rcp64(rho_w), kelvin: kelvin_term64
+LACMO_DEV double kelvin_term64(double T, double sigw, double irho) {
+  return div64(__dmul_rn(__dmul_rn(2.0E6, sigw), irho), __dmul_rn(LC_R_V, T));
+}
 static __device__ __noinline__ void write_rec64(CellFF* out, double T, double S, double L_v,
-                                                double mu, double rho_f, CellTerms t) {
-  const double irho = rcp64(t.rhow);
+                                                double mu, double rho_f, CellTerms t, double irho,
+                                                double kelvin) {
   CellFF r;
   r.S_m1 = __dsub_rn(S, 1.0);
   r.cx = d2ff(__dmul_rn(LC_FOUR_PI_OVER_THREE_INV, irho));
-  r.ce = d2ff(div64(__dmul_rn(__dmul_rn(2.0E6, t.sigw), irho), __dmul_rn(LC_R_V, T)));
+  r.ce = d2ff(kelvin);
   r.la = d2ff(t.lap0); r.lb = d2ff(t.lbp0); r.c1 = d2ff(t.c1); r.c2 = d2ff(t.c2);
   const double n0 = __fma_rn(__fma_rn(LC_PAR_SOL_DENS_NACL_5, T, LC_PAR_SOL_DENS_NACL_2), T,
                              LC_PAR_SOL_DENS_NACL_0);
@@ -155,6 +162,11 @@ static __device__ __noinline__ void write_rec64(CellFF* out, double T, double S,
   r.L_v = L_v;
   r.pad[0] = r.pad[1] = r.pad[2] = 0.0;
   *out = r;
+}
+static __device__ __noinline__ void write_rec64(CellFF* out, double T, double S, double L_v,
+                                                double mu, double rho_f, CellTerms t) {
+  const double irho = rcp64(t.rhow);
+  write_rec64(out, T, S, L_v, mu, rho_f, t, irho, kelvin_term64(T, t.sigw, irho));
 }
 
 }  // namespace lacmo
