@@ -618,7 +618,7 @@ __device__ __noinline__ double particle_removed(const PArgs& a, int64_t k, int32
 // 670 FP64 instructions per SIP at 2 lanes an SM and clock, 478 us per launch
 // over 360,000 SIPs.  The Newton and the drag now run in two-float arithmetic
 // around the FP64 operations that decide the result's rounding (lacmo_ff.cuh;
-// about 65 a SIP are left, and some 3700 FP32 and integer instructions): 94 us.
+// about 65 a SIP are left, and some 3700 FP32 and integer instructions): 87 us.
 // New cell indices come from the FP32 position where it is clear of the cell's
 // edges, boundaries likewise.
 // SIPs that need plain FP64 for the Newton (a step of more than an eighth of
@@ -627,8 +627,8 @@ __device__ __noinline__ double particle_removed(const PArgs& a, int64_t k, int32
 // would hold all warps on the FP64 pipe, gathered they fill a few warps (a
 // raining state of 545,000 SIPs, 1.3% of them large drops, averaged over 20
 // sub-steps from a state out of equilibrium: 291 us in place, 217 us gathered,
-// 144 us with newton_fast and no more blocks than are resident; 732 us in plain
-// FP64).
+// 144 us with newton_fast and no more blocks than are resident, 135 us when the
+// queue's second pass does only what is left of a SIP; 732 us in plain FP64).
 __device__ __forceinline__ double i2d_int(int i) {   // i >= 0
   return i < (1 << 24) ? f2d_int((float)i) : (double)i;
 }
@@ -661,7 +661,11 @@ __global__ void __launch_bounds__(128) k_particles(const __grid_constant__ PK x)
 #pragma unroll 1
     for (int64_t q = pass ? threadIdx.x : blockIdx.x * (int64_t)blockDim.x + threadIdx.x; q < end;
          q += stride) {
-      const int64_t k = pass ? s_q[q] : q;
+      // a queue entry: SIP, and in the sign bit whether its Newton is still to do
+      // (else its new mass is stored and only the drag is left)
+      const int32_t e = pass ? s_q[q] : 0;
+      const bool redo = e < 0;
+      const int64_t k = pass ? (int64_t)(e & 0x7fffffff) : q;
       const int32_t c = a.cell[k];
       if (c < 0) {
         if (PHYS && a.write_Tp) a.T_p[k] = __ldg(a.gsf + (int64_t)(-1 - c) * nz + nz - 1);
@@ -681,11 +685,26 @@ __global__ void __launch_bounds__(128) k_particles(const __grid_constant__ PK x)
 #pragma unroll
           for (int e = 0; e < 6; ++e) dst[e] = __ldg(src + e);
         }
-        bool ok;
-        const double m = newton_ff<false, FULL>(a.sol, a.no_iter, mw, ms, cf,
-                                          d2ff(LC_FOUR_PI * 1.0E12 * a.dt_sub), 1.0, &ok);
-        double dm = m - mw;
-        bool slow = !ok;
+        double m = mw, dm = 0.0;
+        if (pass == 0) {
+          bool ok;
+          m = newton_ff<false, FULL>(a.sol, a.no_iter, mw, ms, cf,
+                                     d2ff(LC_FOUR_PI * 1.0E12 * a.dt_sub), 1.0, &ok);
+          dm = m - mw;   // a step below m / 8: mw + dm is m
+          if (!ok) {
+            const int at = atomicAdd(&s_n, 1);
+            if (at < PQ) {
+              s_q[at] = (int32_t)((uint32_t)k | 0x80000000u);
+              continue;
+            }
+            dm = particle_newton64(a, c, mw, ms);
+            m = mw + dm;
+          }
+        } else if (redo) {
+          dm = particle_newton64(a, c, mw, ms);
+          m = mw + dm;
+        }
+        if (pass == 0 || redo) acc_add64(a.acc64 + 2 * (int64_t)c, a.accx + c, dm * a.xi[k]);
         // integration.py:699-718 with the radius of ammonium sulfate whatever the
         // solute (:1075): the wind at the SIP
         const int4 wi = __ldg((const int4*)&wr->i);
@@ -717,7 +736,7 @@ __global__ void __launch_bounds__(128) k_particles(const __grid_constant__ PK x)
                    fma(rz, dy0, ld(7 + a0)));
         }
         const double du = uf - u, dw = wf - w;
-        const ff mpf = d2ff(m + ms);   // (ok) a step below m / 8: mw + dm is m
+        const ff mpf = d2ff(m + ms);
         const ff wfr = ff_mul(d2ff(ms), ff_rcp(mpf));
         ff pr = ff_horner(FFC(LC_PAR_RHO_AS_1), FFC(LC_PAR_RHO_AS_0), wfr);
         pr = ff_horner(FFC(LC_PAR_RHO_AS_2), pr, wfr);
@@ -728,30 +747,24 @@ __global__ void __launch_bounds__(128) k_particles(const __grid_constant__ PK x)
         const ff duf = d2ff(du), dwf = d2ff(dw + a.dt_sub * a.g_set);
         const float dwh = d2f_int(dw);
         const float Re = 2.0E-6f * cf.rm * f_sqrt(duf.h * duf.h + dwh * dwh) * f_rcp(z.h);
-        slow = slow || !(Re < 0.499f && kd.h > 8.0f);
-        if (slow && pass == 0) {
-          const int at = atomicAdd(&s_n, 1);
-          if (at < PQ) {
-            s_q[at] = (int32_t)k;
-            continue;
-          }
-        }
-        if (ok) {
-          mw = m;
-        } else {
-          dm = particle_newton64(a, c, mw, ms);
-          mw += dm;
-        }
-        if (!slow) {
+        if (Re < 0.499f && kd.h > 8.0f && (pass == 0 || (ff_mass_ok(m) && ff_mass_ok(ms)))) {
           // (u + k uf) / (1 + k) = uf - (uf - u) / (1 + k)
           const ff inv = ff_rcp(ff_add(kd, 1.0f));
           u = uf - ff2d_of<FULL>(ff_mul(duf, inv));
           w = wf - ff2d_of<FULL>(ff_mul(dwf, inv));
         } else {
-          particle_drag64(a, c, mw, ms, uf, wf, &u, &w);
+          if (pass == 0) {
+            const int at = atomicAdd(&s_n, 1);
+            if (at < PQ) {
+              a.m_w[k] = m;
+              s_q[at] = (int32_t)k;
+              continue;
+            }
+          }
+          particle_drag64(a, c, m, ms, uf, wf, &u, &w);
         }
+        mw = m;
         if (a.write_Tp) a.T_p[k] = __ldg(a.gsf + c);
-        acc_add64(a.acc64 + 2 * (int64_t)c, a.accx + c, dm * a.xi[k]);
       }
       // integration.py:552-630
       double xn = x0 + a.dt_pos * u, zn = z0 + a.dt_pos * w;
@@ -1786,7 +1799,8 @@ static cudaError_t resident_blocks(const void* f, int threads, size_t smem,
 // large drops: 198 and 153 us).  States that fill the GPU more than once over
 // are bound by the FP64 pipe and take FULL (the two above: 107 and 144 us); smaller
 // ones wait for one SIP's chain, which FULL lengthens (1920 SIPs: 23.6 us without,
-// 23.9 us with it).
+// 23.9 us with it).  The queue's second pass doing only what is left of a SIP
+// took all of these to 97, 135 and 19.0 us.
 cudaError_t launch_particles(const Bt& B, const lacmo_params_t& p, double dt_sub,
                              double dt_sub_pos, bool write_Tp, bool hist, cudaStream_t s) {
   PK x{B.ref(), pcall(p, dt_sub, dt_sub_pos, write_Tp, hist)};
