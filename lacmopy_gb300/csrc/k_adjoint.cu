@@ -523,13 +523,25 @@ __device__ __noinline__ double fwd_step64(const Args& a, int32_t c, double mw, d
 }
 
 // The SIPs of a forward sub-step.  MAP: the time step's map as the time step runs
-// it (newton_ff), else the converged step.  Bound by FP32 issue (the two-float
-// Newton); 720,000 SIPs took 1326 us a launch with the cell's ambient terms and
-// the Newton per SIP in FP64, 190 us now (110 us once no step exceeds an eighth of
-// the mass).
-template <bool MAP>
+// it (newton_ff; FULL as there), else the converged step.  SIPs whose step needs
+// plain FP64 wait in the block's queue, as in the time step.  Bound by FP32 issue
+// and the FP64 pipe; 720,000 SIPs took 1326 us a launch with the cell's ambient
+// terms and the Newton per SIP in FP64, 190 us with plain FP64 in
+// place, 140 us now.
+constexpr int FQ = 1024;
+template <bool MAP, bool FULL>
 __global__ void __launch_bounds__(128) k_fwd_sips(const __grid_constant__ Args a, double* tape_m) {
+  __shared__ int32_t s_q[MAP ? FQ : 1];
+  __shared__ int s_n;
+  if (MAP) {
+    if (threadIdx.x == 0) s_n = 0;
+    __syncthreads();
+  }
   const ff gdt = d2ff(LC_FOUR_PI * 1.0E12 * a.dt);
+  auto put = [&](int64_t k, int32_t c, double mw, double m) {
+    a.m_w[k] = m;
+    atomicAdd(a.dml + c, (m - mw) * a.xi[k]);
+  };
   for (int64_t k = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; k < a.n;
        k += (int64_t)gridDim.x * blockDim.x) {
     const double mw = a.m_w[k];
@@ -540,13 +552,29 @@ __global__ void __launch_bounds__(128) k_fwd_sips(const __grid_constant__ Args a
     double m;
     if (MAP) {
       bool ok;
-      m = newton_ff<true, false>(SOL_AS, a.no_iter, mw, ms, load_cell(a.rec + c), gdt, a.ks, &ok);
-      if (!ok) m = fwd_step64(a, c, mw, ms);
+      m = newton_ff<true, FULL>(SOL_AS, a.no_iter, mw, ms, load_cell(a.rec + c), gdt, a.ks, &ok);
+      if (!ok) {
+        const int at = atomicAdd(&s_n, 1);
+        if (at < FQ) {
+          s_q[at] = (int32_t)k;
+          continue;
+        }
+        m = fwd_step64(a, c, mw, ms);
+      }
     } else {
       m = fwd_step64(a, c, mw, ms);
     }
-    a.m_w[k] = m;
-    atomicAdd(a.dml + c, (m - mw) * a.xi[k]);
+    put(k, c, mw, m);
+  }
+  if (MAP) {
+    __syncthreads();
+    const int end = s_n < FQ ? s_n : FQ;
+    for (int q = threadIdx.x; q < end; q += blockDim.x) {
+      const int64_t k = s_q[q];
+      const int32_t c = a.cell[k];
+      const double mw = a.m_w[k];
+      put(k, c, mw, fwd_step64(a, c, mw, a.m_s[k]));
+    }
   }
 }
 
@@ -1012,11 +1040,16 @@ int lacmo_adj_forward(int64_t n, int64_t C, double* m_w, const double* m_s, cons
     k_cell_terms<<<nb(C, 32), 32, 0, s>>>(a);
     note_launches(1);
   }
+  static std::atomic<int> cached[64];
+  int res = 0;   // blocks of k_fwd_sips resident at once
+  if (resident_blocks((const void*)k_fwd_sips<true, true>, 128, 0, cached, &res) != cudaSuccess)
+    return LACMO_ERR_CUDA;
   for (int k = 0; k < n_sub; ++k) {
     a.cell = cell + (size_t)k * cell_stride;
     double* const tm = tape_m ? tape_m + (size_t)k * n : nullptr;
-    if (a.rec) k_fwd_sips<true><<<nb(n, 128), 128, 0, s>>>(a, tm);
-    else k_fwd_sips<false><<<nb(n, 128), 128, 0, s>>>(a, tm);
+    if (!a.rec) k_fwd_sips<false, false><<<nb(n, 128), 128, 0, s>>>(a, tm);
+    else if (n > 128 * (int64_t)res) k_fwd_sips<true, true><<<res, 128, 0, s>>>(a, tm);
+    else k_fwd_sips<true, false><<<nb(n, 128), 128, 0, s>>>(a, tm);
     k_fwd_cells<<<nb(C, 32), 32, 0, s>>>(a, tape_c ? tape_c + (size_t)k * 2 * C : nullptr);
     note_launches(2);
   }

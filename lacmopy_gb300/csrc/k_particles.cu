@@ -1776,23 +1776,6 @@ cudaError_t launch_move(const Bt& B, double dt_pos, bool hist, cudaStream_t s) {
   k_particles<false, false><<<grid2(B.n_max, 128, B.M, 152 * 16), 128, 0, s>>>(x); note_launches(1);
   return cudaGetLastError();
 }
-// blocks of a kernel resident on the GPU at once, by device
-static cudaError_t resident_blocks(const void* f, int threads, size_t smem,
-                                   std::atomic<int>* cached, int* res) {
-  int dev = 0;
-  cudaError_t e = cudaGetDevice(&dev);
-  if (e != cudaSuccess) return e;
-  *res = dev < 64 ? cached[dev].load() : 0;
-  if (*res > 0) return cudaSuccess;
-  int per_sm = 0, sms = 0;
-  e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, f, threads, smem);
-  if (e != cudaSuccess) return e;
-  e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-  if (e != cudaSuccess) return e;
-  *res = per_sm * sms > 0 ? per_sm * sms : 1;
-  if (dev < 64) cached[dev].store(*res);
-  return cudaSuccess;
-}
 // No more blocks than are resident at once: a block's queue holds its place until
 // the few SIPs in it are done, some 15 us (360,000 SIPs: 128 us a launch with up to
 // 2432 blocks, 114 us with the 608 that are resident; 545,000 SIPs, 1.3% of them

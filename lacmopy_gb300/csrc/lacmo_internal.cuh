@@ -1,6 +1,8 @@
 // Internal definitions shared by the kernels and the C ABI layer.
 #pragma once
 #include <cuda_runtime.h>
+
+#include <atomic>
 #include <stdint.h>
 
 #include "../../include/lacmo_gb300.h"
@@ -221,5 +223,23 @@ cudaError_t launch_ecol_box(double* xis, double* m, double* R, const double* vel
 cudaError_t launch_beard(double* vel, const double* R, int64_t n, cudaStream_t s);
 cudaError_t launch_radius_bin(const double* m, const double* rho, int64_t n, double lo, double bl,
                               int64_t nb, double* R, int64_t* k, cudaStream_t s);
+
+// blocks of a kernel resident on the GPU at once, by device
+static inline cudaError_t resident_blocks(const void* f, int threads, size_t smem,
+                                   std::atomic<int>* cached, int* res) {
+  int dev = 0;
+  cudaError_t e = cudaGetDevice(&dev);
+  if (e != cudaSuccess) return e;
+  *res = dev < 64 ? cached[dev].load() : 0;
+  if (*res > 0) return cudaSuccess;
+  int per_sm = 0, sms = 0;
+  e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, f, threads, smem);
+  if (e != cudaSuccess) return e;
+  e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+  if (e != cudaSuccess) return e;
+  *res = per_sm * sms > 0 ? per_sm * sms : 1;
+  if (dev < 64) cached[dev].store(*res);
+  return cudaSuccess;
+}
 
 }  // namespace lacmo

@@ -239,3 +239,17 @@ def test_full_and_sparse_grids_agree(solute):
         b = two.snapshot(m)
         for k in ("m_w", "vel", "pos", "xi", "grid_scalar_fields", "water_removed"):
             assert np.array_equal(a[k], b[k]), k
+
+
+def test_forward_of_a_full_grid_replays_the_product():
+    """More SIPs than are resident: the replay takes the conversions without FP64
+    instructions and the queue, and still gives the product's masses."""
+    import torch
+    from lacmopy_gb300 import adjoint, synthetic
+    st = synthetic.make_icmw_state(Nx=40, Nz=40, no_spcm=(26, 38), seed=9, kernel_type="Long_Bott",
+                                   drizzle_fraction=0.05, r_tot=11E-3)
+    assert st["xi"].size > 100000
+    model = adjoint.StepModel(st, 1)
+    m_w, m_s, xi, Th, rv = model.run(full=True)
+    torch.testing.assert_close(m_w, model.product.m_w, rtol=1e-11, atol=1e-30)
+    torch.testing.assert_close(Th, model.product.gsf[2].reshape(-1), rtol=1e-13, atol=0)
