@@ -453,6 +453,7 @@ struct Args {
   int no_iter;          // 0: implicit step to convergence, else the step's map
   CellFF* rec;          // [C] the map's cell terms (no_iter > 0), else null
   CellGrad* grad;       // [C] their derivatives (reverse sweep)
+  CellFast* fast;       // [C] the terms in FP64 (forward sweep)
 };
 
 // a cell's terms for the sub-step that starts from Theta and r_v, as the time
@@ -462,6 +463,12 @@ __device__ __forceinline__ void write_cell(const Args& a, int64_t c, double Th, 
   const double rho_d = a.rho_d[c];
   const CellState s = cell_state64(Th, rv, rho_d, a.g.p_ref, a.g.p_ref_inv);
   write_rec64(a.rec + c, s.T, s.S, s.L_v, s.mu, s.rho_f, s.t);
+  if (!GRAD) {
+    CellAmb m;
+    m.T = s.T; m.S = s.S; m.sigw = s.t.sigw; m.rhow = s.t.rhow; m.lap0 = s.t.lap0;
+    m.lbp0 = s.t.lbp0; m.c1 = s.t.c1; m.c2 = s.t.c2;
+    a.fast[c] = cell_fast(SOL_AS, m);
+  }
   if (GRAD) {
     // logarithmic derivatives: T ~ Theta^kf (kf = 1 / (1 - kappa)), p the same
     // and 1 + r_v / eps, e_s' / e_s = 5420 / T^2
@@ -510,13 +517,8 @@ __device__ __forceinline__ CellFF load_cell(const CellFF* rec) {
 // one condensation step in FP64: to convergence (no_iter = 0), or of a SIP
 // outside the two-float range
 __device__ __noinline__ double fwd_step64(const Args& a, int32_t c, double mw, double ms) {
-  if (a.no_iter > 0 && ff_mass_ok(mw) && ff_mass_ok(ms)) {
-    const CellState s = cell_state64(a.Th[c], a.r_v[c], a.rho_d[c], a.g.p_ref, a.g.p_ref_inv);
-    CellAmb m;
-    m.T = s.T; m.S = s.S; m.sigw = s.t.sigw; m.rhow = s.t.rhow; m.lap0 = s.t.lap0;
-    m.lbp0 = s.t.lbp0; m.c1 = s.t.c1; m.c2 = s.t.c2;
-    return newton_fast(SOL_AS, a.dt, a.no_iter, mw, ms, cell_fast(SOL_AS, m), a.ks);
-  }
+  if (a.fast && ff_mass_ok(mw) && ff_mass_ok(ms))
+    return newton_fast(SOL_AS, a.dt, a.no_iter, mw, ms, a.fast[c], a.ks);
   const Amb<double> am = ambient<double>(a.Th[c], a.r_v[c], a.rho_d[c], a.g);
   bool fl;
   return solve_step(mw, ms, a.ks, am, a.dt, a.no_iter, &fl);
@@ -527,7 +529,8 @@ __device__ __noinline__ double fwd_step64(const Args& a, int32_t c, double mw, d
 // plain FP64 wait in the block's queue, as in the time step.  Bound by FP32 issue
 // and the FP64 pipe; 720,000 SIPs took 1326 us a launch with the cell's ambient
 // terms and the Newton per SIP in FP64, 190 us with plain FP64 in
-// place, 140 us now.
+// place, 140 us gathered, 117 us
+// with the cell's FP64 terms stored beside its record.
 constexpr int FQ = 1024;
 template <bool MAP, bool FULL>
 __global__ void __launch_bounds__(128) k_fwd_sips(const __grid_constant__ Args a, double* tape_m) {
@@ -1014,7 +1017,7 @@ static Args make_args(int64_t n, int64_t C, double* m_w, const double* m_s, cons
   a.rho_d = rho_d; a.mdi = mdi; a.dTh = dTh; a.drv = drv; a.dml = dml; a.dt = dt;
   a.ks = kappa / 0.6;
   a.g.p_ref = p_ref; a.g.p_ref_inv = 1.0 / p_ref; a.g.V = V;
-  a.rec = nullptr; a.grad = nullptr;
+  a.rec = nullptr; a.grad = nullptr; a.fast = nullptr;
   return a;
 }
 
@@ -1035,8 +1038,9 @@ int lacmo_adj_forward(int64_t n, int64_t C, double* m_w, const double* m_s, cons
   if (cudaMemsetAsync(dml, 0, 8 * C, s) != cudaSuccess) return LACMO_ERR_CUDA;
   Scratch scratch(s);
   if (no_iter > 0 && n_sub > 0) {
-    a.rec = (CellFF*)scratch.get(sizeof(CellFF) * (size_t)C);
+    a.rec = (CellFF*)scratch.get((sizeof(CellFF) + sizeof(CellFast)) * (size_t)C);
     if (!a.rec) return LACMO_ERR_CUDA;
+    a.fast = (CellFast*)(a.rec + C);
     k_cell_terms<<<nb(C, 32), 32, 0, s>>>(a);
     note_launches(1);
   }
