@@ -103,6 +103,26 @@ __global__ void k_cell_aux(const __grid_constant__ MRef mr) {
 
 // ---------------------------------------------------------------------------
 // binning: histogram (arrival rank) -> scan -> scatter -> order by ID
+// The arrival rank of a SIP in cell c, for the lanes that come here together: one
+// atomic for a run of neighbouring lanes with the same cell (SIPs in memory order
+// start out cell by cell; the half-step move of 64 members, 51.9 million SIPs,
+// 1204 us with an atomic each, 895 us now; k_histogram over 720,000 SIPs 35 and
+// 7 us).
+__device__ __forceinline__ int32_t rank_in(int32_t* counts, int32_t c) {
+  const unsigned here = __activemask();
+  const int lane = threadIdx.x & 31;
+  const unsigned below = here & ((1u << lane) - 1u);
+  const int32_t prev = __shfl_sync(here, c, below ? 31 - __clz(below) : lane);
+  const unsigned heads = __ballot_sync(here, !below || prev != c);
+  if (heads == here) return atomicAdd(counts + c, 1);   // no two alike (raining states)
+  const unsigned upto = (2u << lane) - 1u;
+  const int head = 31 - __clz(heads & upto);
+  const unsigned after = heads & ~upto;
+  const unsigned run = here & ~((1u << head) - 1u) & (after ? (after & -after) - 1u : ~0u);
+  int32_t base = 0;
+  if (lane == head) base = atomicAdd(counts + c, __popc(run));
+  return __shfl_sync(here, base, head) + __popc(run & below);
+}
 __global__ void k_histogram(const __grid_constant__ MRef mr) {
   const Member& mb = mr.get();
   const int32_t* __restrict__ cell = mb.sp.cell;
@@ -113,7 +133,7 @@ __global__ void k_histogram(const __grid_constant__ MRef mr) {
        k += (int64_t)gridDim.x * blockDim.x) {
     int32_t c = cell[k];
     if (c < 0) continue;
-    if (c < C) rank[k] = atomicAdd(counts + c, 1);
+    if (c < C) rank[k] = rank_in(counts, c);
     else atomicOr(mb.w.flags, LACMO_FLAG_CELL_RANGE);   // left out of the binning
   }
 }
@@ -791,7 +811,7 @@ __global__ void __launch_bounds__(128) k_particles(const __grid_constant__ PK x)
           cj = cj < 0 ? 0 : (cj >= nz ? nz - 1 : cj);
         }
         newc = ci * nz + cj;
-        if (a.hist) a.rank[k] = atomicAdd(a.counts + newc, 1);
+        if (a.hist) a.rank[k] = rank_in(a.counts, newc);
       }
       a.pos[k] = xn; a.pos[a.n + k] = zn;
       if (PHYS || removed) { a.vel[k] = u; a.vel[a.n + k] = w; }
@@ -1383,7 +1403,7 @@ __global__ void __launch_bounds__(PM_THREADS, MINB) k_particles_mixed(const __gr
         cj = cj < 0 ? 0 : (cj >= nz ? nz - 1 : cj);
       }
       newc = (int32_t)(ci * nz + cj);
-      if (a.hist) a.rank[k] = atomicAdd(a.counts + newc, 1);
+      if (a.hist) a.rank[k] = rank_in(a.counts, newc);
       if (PHYS) __stcs(a.m_w + k, tl.get(S, PF_MW, t) + f2d_int(d));
     }
     // streaming stores (evict first)
