@@ -844,68 +844,31 @@ __device__ __forceinline__ void grid_cell_update(double* gsf, double* gmp, doubl
 }
 
 // grid_cell_update by four lanes of a warp for each cell (role 0 to 3), bit for
-// bit: logarithms, exponentials and quotients that do not depend on each other run
-// side by side, one in each lane, so the chain of FP64 operations a cell waits for is
-// less than half of one thread's.  in: a cell to be written.
+// bit.  in: a cell to be written.
 __device__ __forceinline__ void grid_cell_update_x4(double* gsf, double* gmp, double* aux,
                                                     int64_t c, int64_t C, double p_ref,
                                                     double p_ref_inv, double dTh, double drv,
                                                     double dml, double V, bool in) {
-  const int lane = threadIdx.x & 31, role = lane & 3;
-  auto from = [&](double v, int r) { return __shfl_sync(0xffffffffu, v, (lane & 28) | r); };
-  auto pick = [&](double a0, double a1, double a2, double a3) {
-    return role < 2 ? (role ? a1 : a0) : (role == 2 ? a2 : a3);
-  };
+  const int role = threadIdx.x & 3;
   double Th = gsf[2 * C + c], r_v = gsf[4 * C + c];
   const double rho_d = gsf[3 * C + c];
   cell_step64(&Th, &r_v, rho_d, gsf[8 * C + c], gmp[2 * C + c], dTh, drv, dml, V, p_ref_inv);
-  // cell_state64 and cell_terms64
-  const double L2 = log64_call(__dmul_rn(__dmul_rn(__dmul_rn(rho_d, Th), LC_R_D), p_ref_inv));
-  const double e0 = exp64_call(__dmul_rn(role ? LC_KAPPA_FACTOR * LC_KAPPA_AIR_DRY : LC_KAPPA_FACTOR, L2));
-  const double T = __dmul_rn(Th, from(e0, 1));
-  const double p = __dmul_rn(__dmul_rn(from(e0, 0), p_ref), __fma_rn(r_v, 1.0 / LC_EPSILON_GC, 1.0));
-  const double K = __dmul_rn(4.1868E-3, __fma_rn(0.017, __dsub_rn(T, 273.15), 5.69));
-  const double L_v = __dmul_rn(1.0E3, __fma_rn(-2.358, __dsub_rn(T, 273.0), 2500.82));
-  const double T2 = __dmul_rn(T, T), RvT = __dmul_rn(LC_R_V, T);
-  const double tau = __dsub_rn(1.0, __dmul_rn(T, 1.0 / 647.096));
-  const double d = __dsub_rn(T, LC_PAR_WATER_DENS_2);
-  const double rhow = __fma_rn(LC_PAR_WATER_DENS_1, __dmul_rn(d, d), LC_PAR_WATER_DENS_0);
-  const double irho = rcp64(rhow);
-  const double dT = __dsub_rn(T, LC_T_ALPHA_0);
-  // -5420 / T, mu, lap0, c1
-  const double q1 = div64(
-      pick(-5420.0, __dmul_rn(1.458E-6, __dmul_rn(T, sqrt64(T))),
-           __dmul_rn(__fma_rn(LC_C_ALPHA_2, dT, LC_C_ALPHA_1), K), __dmul_rn(L_v, L_v)),
-      pick(T, __dadd_rn(T, 110.4), p, __dmul_rn(__dmul_rn(__dmul_rn(LC_R_V, K), T), T)));
-  const double lg = log64_call(role == 2 ? tau : T);
-  const double e1 = exp64_call(pick(q1, __dmul_rn(-0.06, lg), __dmul_rn(1.256, lg), 0.0));
-  const double e_s = __dmul_rn(2.53E11, from(e1, 0));
-  const double sigw = __dmul_rn(__dmul_rn(0.2358, from(e1, 2)), __fma_rn(-0.625, tau, 1.0));
-  // S, D_v, the Kelvin term
-  const double q2 = div64(
-      pick(__dmul_rn(__dmul_rn(__dmul_rn(rho_d, r_v), T), LC_R_V),
-           __dmul_rn(4.01218E-5, __dmul_rn(T2, e1)), __dmul_rn(__dmul_rn(2.0E6, sigw), irho), 1.0),
-      pick(e_s, p, RvT, 1.0));
-  const double S = from(q2, 0), D_v = from(q2, 1);
-  const double c2 = div64(RvT, __dmul_rn(D_v, e_s));
-  const double mu = from(q1, 1), lap0 = from(q1, 2), c1 = from(q1, 3);
-  const double lbp0 = __dmul_rn(__dmul_rn(LC_C_BETA_1, __fma_rn(LC_C_BETA_2, dT, 1.0)), D_v);
-  const double rho_f = __dmul_rn(rho_d, __dadd_rn(1.0, r_v));
-  const double kelvin = from(q2, 2);
+  double irho, kelvin;
+  const CellState a = cell_state64_x4(Th, r_v, rho_d, p_ref, p_ref_inv, &irho, &kelvin);
   if (!in) return;
   if (role == 0) {
-    gsf[c] = T; gsf[C + c] = p; gsf[2 * C + c] = Th; gsf[4 * C + c] = r_v;
-    gsf[6 * C + c] = S; gsf[7 * C + c] = e_s;
-    write_mixed(aux, c, C, T, S, sigw, rhow, lap0, lbp0, c1, c2, mu, rho_f);
+    gsf[c] = a.T; gsf[C + c] = a.p; gsf[2 * C + c] = Th; gsf[4 * C + c] = r_v;
+    gsf[6 * C + c] = a.S; gsf[7 * C + c] = a.e_s;
+    write_mixed(aux, c, C, a.T, a.S, a.t.sigw, a.t.rhow, a.t.lap0, a.t.lbp0, a.t.c1, a.t.c2, a.mu,
+                a.rho_f);
   } else if (role == 1) {
-    gmp[c] = K; gmp[C + c] = D_v; gmp[2 * C + c] = L_v; gmp[3 * C + c] = sigw;
-    gmp[4 * C + c] = LC_C_PD * (1 + 0.897 * r_v); gmp[5 * C + c] = mu; gmp[6 * C + c] = rho_f;
+    gmp[c] = a.K; gmp[C + c] = a.D_v; gmp[2 * C + c] = a.L_v; gmp[3 * C + c] = a.t.sigw;
+    gmp[4 * C + c] = LC_C_PD * (1 + 0.897 * r_v); gmp[5 * C + c] = a.mu; gmp[6 * C + c] = a.rho_f;
   } else if (role == 2) {
-    aux[c] = sigw; aux[C + c] = rhow; aux[2 * C + c] = lap0; aux[3 * C + c] = lbp0;
-    aux[4 * C + c] = c1; aux[5 * C + c] = c2;
+    aux[c] = a.t.sigw; aux[C + c] = a.t.rhow; aux[2 * C + c] = a.t.lap0;
+    aux[3 * C + c] = a.t.lbp0; aux[4 * C + c] = a.t.c1; aux[5 * C + c] = a.t.c2;
   } else {
-    write_rec64(cell_rec64(aux, C) + 2 * c, T, S, L_v, mu, rho_f,
-                CellTerms{sigw, rhow, lap0, lbp0, c1, c2}, irho, kelvin);
+    write_rec64(cell_rec64(aux, C) + 2 * c, a.T, a.S, a.L_v, a.mu, a.rho_f, a.t, irho, kelvin);
   }
 }
 

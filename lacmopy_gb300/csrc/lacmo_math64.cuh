@@ -139,6 +139,58 @@ static __device__ __noinline__ CellState cell_state64(double Th, double r_v, dou
   a.t = cell_terms64(a.T, a.p, a.e_s, a.L_v, a.K, a.D_v);
   return a;
 }
+// cell_state64 by four lanes of a warp for each cell (threadIdx.x & 3: role 0 to 3;
+// all 32 lanes take part), bit for bit: logarithms, exponentials and quotients that
+// do not depend on each other run side by side, one in each lane, so the chain of
+// FP64 operations a cell waits for is less than half of one thread's.  irho and
+// kelvin: see write_rec64.
+LACMO_DEV CellState cell_state64_x4(double Th, double r_v, double rho_d, double p_ref,
+                                    double p_ref_inv, double* irho, double* kelvin) {
+  const int lane = threadIdx.x & 31, role = lane & 3;
+  auto from = [&](double v, int r) { return __shfl_sync(0xffffffffu, v, (lane & 28) | r); };
+  auto pick = [&](double a0, double a1, double a2, double a3) {
+    return role < 2 ? (role ? a1 : a0) : (role == 2 ? a2 : a3);
+  };
+  CellState a;
+  const double L2 = log64_call(__dmul_rn(__dmul_rn(__dmul_rn(rho_d, Th), LC_R_D), p_ref_inv));
+  const double e0 =
+      exp64_call(__dmul_rn(role ? LC_KAPPA_FACTOR * LC_KAPPA_AIR_DRY : LC_KAPPA_FACTOR, L2));
+  const double T = a.T = __dmul_rn(Th, from(e0, 1));
+  a.p = __dmul_rn(__dmul_rn(from(e0, 0), p_ref), __fma_rn(r_v, 1.0 / LC_EPSILON_GC, 1.0));
+  a.K = __dmul_rn(4.1868E-3, __fma_rn(0.017, __dsub_rn(T, 273.15), 5.69));
+  a.L_v = __dmul_rn(1.0E3, __fma_rn(-2.358, __dsub_rn(T, 273.0), 2500.82));
+  const double T2 = __dmul_rn(T, T), RvT = __dmul_rn(LC_R_V, T);
+  const double tau = __dsub_rn(1.0, __dmul_rn(T, 1.0 / 647.096));
+  const double d = __dsub_rn(T, LC_PAR_WATER_DENS_2);
+  a.t.rhow = __fma_rn(LC_PAR_WATER_DENS_1, __dmul_rn(d, d), LC_PAR_WATER_DENS_0);
+  *irho = rcp64(a.t.rhow);
+  const double dT = __dsub_rn(T, LC_T_ALPHA_0);
+  // -5420 / T, mu, lap0, c1
+  const double q1 = div64(
+      pick(-5420.0, __dmul_rn(1.458E-6, __dmul_rn(T, sqrt64(T))),
+           __dmul_rn(__fma_rn(LC_C_ALPHA_2, dT, LC_C_ALPHA_1), a.K), __dmul_rn(a.L_v, a.L_v)),
+      pick(T, __dadd_rn(T, 110.4), a.p, __dmul_rn(__dmul_rn(__dmul_rn(LC_R_V, a.K), T), T)));
+  const double lg = log64_call(role == 2 ? tau : T);
+  const double e1 = exp64_call(pick(q1, __dmul_rn(-0.06, lg), __dmul_rn(1.256, lg), 0.0));
+  a.e_s = __dmul_rn(2.53E11, from(e1, 0));
+  a.t.sigw = __dmul_rn(__dmul_rn(0.2358, from(e1, 2)), __fma_rn(-0.625, tau, 1.0));
+  // S, D_v, the Kelvin term
+  const double q2 = div64(
+      pick(__dmul_rn(__dmul_rn(__dmul_rn(rho_d, r_v), T), LC_R_V),
+           __dmul_rn(4.01218E-5, __dmul_rn(T2, e1)), __dmul_rn(__dmul_rn(2.0E6, a.t.sigw), *irho),
+           1.0),
+      pick(a.e_s, a.p, RvT, 1.0));
+  a.S = from(q2, 0);
+  a.D_v = from(q2, 1);
+  *kelvin = from(q2, 2);
+  a.t.c2 = div64(RvT, __dmul_rn(a.D_v, a.e_s));
+  a.mu = from(q1, 1);
+  a.t.lap0 = from(q1, 2);
+  a.t.c1 = from(q1, 3);
+  a.t.lbp0 = __dmul_rn(__dmul_rn(LC_C_BETA_1, __fma_rn(LC_C_BETA_2, dT, 1.0)), a.D_v);
+  a.rho_f = __dmul_rn(rho_d, __dadd_rn(1.0, r_v));
+  return a;
+}
 // the FP64 path's record of a cell; irho = rcp64(rho_w), kelvin: kelvin_term64
 LACMO_DEV double kelvin_term64(double T, double sigw, double irho) {
   return div64(__dmul_rn(__dmul_rn(2.0E6, sigw), irho), __dmul_rn(LC_R_V, T));
