@@ -99,7 +99,8 @@ typedef struct {
 } lacmo_params_t;
 
 /* Arithmetic of lacmo_integrate_adv_step.  FP64: the reference's FP64 path
- * (per-cell sums in SIP-ID order).  MIXED: the Newton condensation and the
+ * to a few roundings (per-cell sums and water_removed exact integer sums of the
+ * FP64 products, in units of 2^-40 fg, so their order does not matter).  MIXED: the Newton condensation and the
  * drag update in FP32, with the Newton repeated in FP64 for SIPs near the
  * critical radius of activation; state, positions, per-cell condensed-mass
  * sums (into Theta / r_v), multiplicities and the collision step stay FP64;
@@ -308,8 +309,7 @@ int lacmo_adv_substep(const lacmo_sips_t* sips, const lacmo_grid_t* grid,
 /* The two halves of a particle sub-step, for callers that time or schedule
  * them separately: the fused per-SIP kernel (condensation, drag, position,
  * re-index; it also counts SIPs per new cell), and the cell binning that
- * folds the ground-removal list into water_removed and sorts the SIPs by
- * (cell, ID).  lacmo_bin must follow lacmo_particles_only before any other
+ * sorts the SIPs by (cell, ID).  lacmo_bin must follow lacmo_particles_only before any other
  * entry point uses the binning. */
 int lacmo_particles_only(const lacmo_sips_t* sips, const lacmo_grid_t* grid,
                          const lacmo_params_t* prm, double dt_sub, double dt_sub_pos, void* ws,

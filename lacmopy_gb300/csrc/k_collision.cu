@@ -352,20 +352,20 @@ __device__ __noinline__ void certain_collection(Cell<BIG> S, int i, int j,
 __device__ __noinline__ bool equal_multiplicities(double xi_min, double xi_max) {
   return (xi_max - xi_min) / xi_max < 1.0E-5;
 }
-// One event of a cell's sequential order, taken by a whole warp: the pair of
-// slots (l0, l1) with draw r, either placed certainly in an ordinary collection
-// by the FP32 bounds (certain) or evaluated exactly.  Even lanes hold SIP l0,
-// odd lanes SIP l1 (lanes 0 and 1 write): both SIPs' loads, densities and
-// radii run side by side, and the updated masses stay in registers for the
-// FP32 copies instead of being read back, so an event costs one round of
-// loads and one chain of FP64 operations (its latency is what a raining cell
-// waits for; some 100 cycles an operation, so the test for equal multiplicities
-// runs in FP32 and the density of imax is left out where nothing reads it).
-// Keeping SIP l0 in registers over all events of its row, its partners' data
-// formed in all lanes at once, was slower (a step of the raining 75 x 75 x 128
-// state 1.20 ms against 0.94 ms): most rows hold one event.  Same decisions and operation order as exact_pair and
-// collect_once.  Returns 0 (no collision), 1 (one collection) or 2 (multiple
-// collection), the same in all lanes.
+// One event of a cell's sequential order, taken by a whole warp: the pair of slots
+// (l0, l1) with draw r, either placed certainly in an ordinary collection by the
+// FP32 bounds (certain) or evaluated exactly.  Even lanes hold SIP l0, odd lanes
+// SIP l1 (lanes 0 and 1 write): both SIPs' loads, densities and radii run side by
+// side, and the updated masses stay in registers for the FP32 copies instead of
+// being read back, so an event costs one round of loads and one chain of FP64
+// operations (its latency is what a raining cell waits for; some 100 cycles an
+// operation, so the test for equal multiplicities runs in FP32 and the density of
+// imax is left out where nothing reads it). Keeping SIP l0 in registers over all
+// events of its row, its partners' data formed in all lanes at once, was slower (a
+// step of the raining 75 x 75 x 128 state 1.20 ms against 0.94 ms): most rows hold
+// one event.  Same decisions and operation order as exact_pair and collect_once.
+// Returns 0 (no collision), 1 (one collection) or 2 (multiple collection), the same
+// in all lanes.
 template <bool THIN, bool BIG>
 __device__ __forceinline__ int warp_event(Cell<BIG> S, int l0, int l1, double Tc,
                                        bool use_E, double r, bool certain) {
@@ -586,17 +586,17 @@ __device__ __forceinline__ void init_exact_scratch(const CellArgs& a, Cell<BIG> 
   __syncwarp();
 }
 
-// The events of one window of the per-pair draws (k_collide_cells), taken in
-// their order: screen_pair places the pairs the first screen left (bits of ev.m),
-// the first one it does not skip is the next event, and after a collection the
-// window's later pairs are screened again with the draws they already have; an
-// event that changes nothing leaves the later screens valid.  Out of line: the
-// window loop around it then reloads nothing (a step of 5625 cells of 64 SIPs,
-// fresh: 124 us with the events in the loop, 74 us without).  An event costs one more screen of its window, where letting every lane run
-// on to its own first hit cost a screen of the whole rest of the cell: a step
-// of a raining 75 x 75 x 128 state (14 collections per cell on average, 190 in the
-// heaviest, whose chain of events of some 5 us each is what the step waits for) took
-// 10.6 ms, 0.78 ms now.
+// The events of one window of the per-pair draws (k_collide_cells), taken in their
+// order: screen_pair places the pairs the first screen left (bits of ev.m), the
+// first one it does not skip is the next event, and after a collection the window's
+// later pairs are screened again with the draws they already have; an event that
+// changes nothing leaves the later screens valid.  Out of line: the window loop
+// around it then reloads nothing (a step of 5625 cells of 64 SIPs, fresh: 124 us
+// with the events in the loop, 74 us without).  An event costs one more screen of
+// its window, where letting every lane run on to its own first hit cost a screen of
+// the whole rest of the cell: a step of a raining 75 x 75 x 128 state (14
+// collections per cell on average, 190 in the heaviest, whose chain of events of
+// some 5 us each is what the step waits for) took 10.6 ms, 0.78 ms now.
 // Returns false when the event limit is passed (ev.pos: the first rank left).
 struct PairEvents {
   int pos, events, c0, c1;

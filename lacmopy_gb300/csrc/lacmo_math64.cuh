@@ -1,8 +1,8 @@
 // FP64 exp, log, square root, reciprocal and quotient with few FP64
 // instructions, for the per-cell thermodynamics.
 //
-// Those kernels run one thread per cell and wait for one serial chain of FP64
-// operations (some 60 cycles each on GB300).  Here the leading terms stay FP64
+// Those kernels run one to four threads per cell and wait for one serial chain of
+// FP64 operations (some 60 to 100 cycles each on GB300).  Here the leading terms stay FP64
 // and the series' tails, small against them, are two-float (lacmo_ff.cuh): 11 FP64
 // instructions for exp and for log.  Reductions and series are the textbook ones
 // (Muller, Elementary Functions, 3rd ed.): exp(x) = 2^k exp(r), |r| <= ln 2 / 2,
@@ -86,8 +86,8 @@ static __device__ __noinline__ double exp64_call(double x) { return exp64(x); }
 // go through one logarithm each, pow(x, y) = exp(y log x), with |y log x| below
 // 1 (the Exner powers share log x; T^1.94 = T^2 T^-0.06, T^1.5 = T sqrt(T)), so
 // that exp's argument carries no more than half an ulp of 1.  Out of line, and
-// with every rounding written out: the time step, its start, the mixed path and
-// the adjoint's replay run the same code and get the same bits.
+// with every rounding written out: the time step, its start and the adjoint's replay
+// run the same code and get the same bits.
 static __device__ __noinline__ void cell_step64(double* Th_io, double* rv_io, double rho_d,
                                                 double mdi, double L_v0, double dTh, double drv,
                                                 double dml, double V, double p_ref_inv) {
