@@ -99,9 +99,10 @@ typedef struct {
 } lacmo_params_t;
 
 /* Arithmetic of lacmo_integrate_adv_step.  FP64: the reference's FP64 path
- * to a few roundings (per-cell sums and water_removed exact integer sums of the
- * FP64 products, in units of 2^-40 fg, so their order does not matter).  MIXED: the Newton condensation and the
- * drag update in FP32, with the Newton repeated in FP64 for SIPs near the
+ * to a few roundings (per-cell sums and water_removed are integer sums of the
+ * FP64 products, exact from 2^-12 fg up and in units of 2^-64 fg below, so their
+ * order does not matter; products of 2^104 fg and more, or 2^60 fg in a state of
+ * 2^31 SIPs, are added in FP64).  MIXED: the Newton condensation and the drag update in FP32, with the Newton repeated in FP64 for SIPs near the
  * critical radius of activation; state, positions, per-cell condensed-mass
  * sums (into Theta / r_v), multiplicities and the collision step stay FP64;
  * the per-cell sums of dm * xi are exact integer sums (units of 2^-4 fg), so

@@ -73,7 +73,7 @@ static WsPlan ws_plan(int64_t n, int64_t nx, int64_t nz) {
       8 * (C + 1),     // draw_off
       4 * N,           // perm
       4 * N,           // rank
-      16 * C,          // acc64
+      32 * C,          // acc64
       4 * N,           // rm_id
       8 * N,           // rm_val
       8 * cell_records_offset((int64_t)C) +

@@ -10,11 +10,11 @@
 // and writes it once; grid data come from small L2-resident arrays.
 //
 // Sums the reference accumulates in ascending SIP ID (the per-cell condensed
-// mass delta_m_l, integration.py:916-936, and water_removed, :620-628) are exact
-// 128-bit integer sums here (acc_add64), rounded to FP64 once: independent of
-// the order, so a step gives the same bits run to run and batched or not, within
-// the rounding of the reference's sequential sums, and no sub-step needs its
-// SIPs sorted.
+// mass delta_m_l, integration.py:916-936, and water_removed, :620-628) are integer
+// sums of every bit of their terms here (acc_add64, which states the range), brought
+// to FP64 at the end: independent of the order, so a step gives the same bits run to
+// run and batched or not, within the rounding of the reference's sequential sums,
+// and no sub-step needs its SIPs sorted.
 #include <cuda_runtime.h>
 
 #include <atomic>
@@ -354,6 +354,72 @@ __global__ void __launch_bounds__(256) k_order(const __grid_constant__ MRef mr) 
   }
 }
 
+// ---- exact sums of FP64 values as integers in units of 2^-64 (fg): four words
+// of b bits each, each summed by a 64-bit integer atomic (executed by L2, in any
+// order).  b = acc_bits(n) leaves a word room for one value from every SIP of the
+// member, so no word wraps: |sum of n parts below 2^b| < 2^62.  A value keeps all
+// its bits from 2^-12 fg up; below that it is rounded to 2^-64 fg.  What lies
+// beyond the four words (2^104 fg for up to 2^20 SIPs, 2^60 fg for 2^31),
+// infinities and NaN go to a plain FP64 sum (over).
+constexpr int ACC64_WORDS = 4, ACC64_UNIT = 64;
+__device__ __forceinline__ int acc_bits(int64_t n) {
+  const int log_n = n > 1 ? 64 - __clzll(n - 1) : 0;   // n <= 2^log_n
+  return log_n < 20 ? 42 : 62 - log_n;
+}
+__device__ __forceinline__ void acc_add64(long long* acc, int bits, double* over, double v) {
+  const uint64_t u = (uint64_t)__double_as_longlong(v);
+  int s = (int)((u >> 52) & 0x7ffu) - (1075 - ACC64_UNIT);   // v 2^64 = m 2^s
+  if (s > ACC64_WORDS * bits - 53) {
+    atomicAdd(over, v);
+    return;
+  }
+  if (s < -53) return;   // rounds to zero
+  uint64_t m = (u & 0x000fffffffffffffull) | 0x0010000000000000ull;
+  if (s < 0) {
+    m = (m + (1ull << (-s - 1))) >> (-s);
+    s = 0;
+  }
+  // m 2^s from word k on: 53 bits reach into at most three words
+  const int k = (s >= bits) + (s >= 2 * bits) + (s >= 3 * bits);
+  s -= k * bits;
+  const uint64_t mask = (1ull << bits) - 1;
+  uint64_t p0 = (m << s) & mask;
+  m >>= bits - s;
+  uint64_t p1 = m & mask, p2 = m >> bits;
+  if (u >> 63) { p0 = 0 - p0; p1 = 0 - p1; p2 = 0 - p2; }
+  unsigned long long* const w = (unsigned long long*)acc + k;
+  if (p0) atomicAdd(w, (unsigned long long)p0);
+  if (p1) atomicAdd(w + 1, (unsigned long long)p1);
+  if (p2) atomicAdd(w + 2, (unsigned long long)p2);
+}
+// The sum, within 0.8 of its last place: the words' carries taken up so that each
+// holds at most half of 2^b, then from the top down; the sums are exact up to 53
+// bits, and from the first one rounded on a word adds a quarter of a last place
+// at most.
+__device__ __forceinline__ double acc_value64(longlong2 a, longlong2 b, int bits) {
+  const long long half = 1ll << (bits - 1);
+  long long c = (a.x + half) >> bits;
+  const long long w0 = a.x - (c << bits);
+  a.y += c;
+  c = (a.y + half) >> bits;
+  const long long w1 = a.y - (c << bits);
+  b.x += c;
+  c = (b.x + half) >> bits;
+  const long long w2 = b.x - (c << bits), w3 = b.y + c;
+  const double base = __longlong_as_double((long long)(1023 + bits) << 52);
+  double v = (double)w1;
+  if (w2 | w3) v = fma(fma((double)w3, base, (double)w2), base, v);
+  return fma(v, base, (double)w0) * 0x1p-64;
+}
+__device__ __forceinline__ double acc_read64(const long long* acc, int bits) {
+  const longlong2* const p = (const longlong2*)acc;
+  return acc_value64(p[0], p[1], bits);
+}
+__device__ __forceinline__ void acc_clear64(long long* acc) {
+  longlong2* const p = (longlong2*)acc;
+  p[0] = p[1] = make_longlong2(0, 0);
+}
+
 // ---------------------------------------------------------------------------
 struct PArgs {
   double *pos, *vel, *m_w, *rel, *T_p;
@@ -367,6 +433,7 @@ struct PArgs {
   int32_t *counts, *rank;
   long long *acc64, *wr64;      // FP64: per-cell and water sums (acc_add64)
   double* accx;                 // FP64: values beyond their range
+  int acc_bits;                 // FP64: bits of the sums' words
   // mixed precision: SIPs whose Newton repeats in FP64 (k_newton_fallback),
   // queued in scratch that mixed sub-steps leave unused
   int32_t *fb_count, *fb_done, *fb_id, *fb_c;
@@ -408,7 +475,7 @@ __device__ __forceinline__ PArgs make_pargs(const Member& mb, const PCall& c) {
   a.dt_sub = c.dt_sub; a.dt_pos = c.dt_pos; a.g_set = c.g_set;
   a.no_iter = c.no_iter; a.sol = c.sol; a.write_Tp = c.write_Tp;
   a.counts = w.counts; a.rank = w.rank; a.flags = w.flags;
-  a.acc64 = w.acc64; a.wr64 = w.wr64; a.accx = w.accx;
+  a.acc64 = w.acc64; a.wr64 = w.wr64; a.accx = w.accx; a.acc_bits = acc_bits(sp.n);
   a.fb_count = w.fb_count; a.fb_done = w.fb_done; a.fb_id = w.rm_id; a.fb_c = w.colk;
   a.fb_mw = w.rm_val;
   a.acc = w.div; a.hist = c.hist; a.nfb = w.nfb;
@@ -513,43 +580,9 @@ __global__ void k_clear_acc64(const __grid_constant__ MRef mr) {
   const int64_t C = mb.g.nx * mb.g.nz;
   for (int64_t c = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; c < C;
        c += (int64_t)gridDim.x * blockDim.x) {
-    mb.w.acc64[2 * c] = 0;
-    mb.w.acc64[2 * c + 1] = 0;
+    acc_clear64(mb.w.acc64 + ACC64_WORDS * c);
     mb.w.accx[c] = 0.0;
   }
-}
-
-// ---- exact sums of FP64 values as 128-bit integers in units of 2^-40 (fg):
-// v = hi 2^2 + lo 2^-40 with 0 <= |lo| < 2^42, each part summed by a 64-bit
-// integer atomic (executed by L2, in any order).  A sum holds 2^21 values of
-// magnitude below 2^60; what lies beyond, infinities and NaN go to a plain FP64
-// sum (over).
-constexpr int ACC64_LO = 42;
-__device__ __forceinline__ void acc_add64(long long* acc, double* over, double v) {
-  const uint64_t b = (uint64_t)__double_as_longlong(v);
-  const int e = (int)((b >> 52) & 0x7ffu);
-  if (e >= 1023 + 60) {
-    atomicAdd(over, v);
-    return;
-  }
-  const int sh = e - 1075 + 40;   // v 2^40 = m 2^sh
-  if (sh <= -54 || e == 0) return;   // rounds to zero
-  const uint64_t m = (b & 0x000fffffffffffffull) | 0x0010000000000000ull;
-  uint64_t lo, hi;
-  if (sh < 0) {
-    const uint64_t r = (m + (1ull << (-sh - 1))) >> (-sh);
-    lo = r & ((1ull << ACC64_LO) - 1);
-    hi = r >> ACC64_LO;
-  } else {
-    lo = sh < ACC64_LO ? (m << sh) & ((1ull << ACC64_LO) - 1) : 0;
-    hi = sh <= ACC64_LO ? m >> (ACC64_LO - sh) : m << (sh - ACC64_LO);
-  }
-  if (b >> 63) { lo = 0 - lo; hi = 0 - hi; }
-  if (lo) atomicAdd((unsigned long long*)acc + 1, (unsigned long long)lo);
-  if (hi) atomicAdd((unsigned long long*)acc, (unsigned long long)hi);
-}
-__device__ __forceinline__ double acc_value64(long long hi, long long lo) {
-  return fma((double)hi, 4.0, (double)lo * 0x1p-40);
 }
 
 // Rare paths of the FP64 kernel, out of line.
@@ -624,7 +657,7 @@ __device__ __noinline__ void particle_inactive(const PArgs& a, int64_t k, int32_
 __device__ __noinline__ double particle_removed(const PArgs& a, int64_t k, int32_t c, double x,
                                                 double z, double mw) {
   const int64_t i = (int64_t)c / a.nz, j = (int64_t)c - i * a.nz;
-  acc_add64(a.wr64, a.water_removed, a.xi[k] * mw);
+  acc_add64(a.wr64, a.acc_bits, a.water_removed, a.xi[k] * mw);
   const double rel_x = (x - a.x_min) / a.dx - (double)i;
   const double rel_z = (z - a.z_min) / a.dz - (double)j;
   // the re-index of this call leaves the old relative position divided by the
@@ -724,7 +757,8 @@ __global__ void __launch_bounds__(128) k_particles(const __grid_constant__ PK x)
           dm = particle_newton64(a, c, mw, ms);
           m = mw + dm;
         }
-        if (pass == 0 || redo) acc_add64(a.acc64 + 2 * (int64_t)c, a.accx + c, dm * a.xi[k]);
+        if (pass == 0 || redo)
+          acc_add64(a.acc64 + ACC64_WORDS * (int64_t)c, a.acc_bits, a.accx + c, dm * a.xi[k]);
         // integration.py:699-718 with the radius of ammonium sulfate whatever the
         // solute (:1075): the wind at the SIP
         const int4 wi = __ldg((const int4*)&wr->i);
@@ -885,11 +919,12 @@ __global__ void __launch_bounds__(32) k_cell_update(const __grid_constant__ MRef
   const double *dTh = mb.w.dTh, *drv = mb.w.drv;
   const int64_t C = mb.g.nx * mb.g.nz;
   const double p_ref = mb.g.p_ref, p_ref_inv = mb.g.p_ref_inv, V = mb.g.volume_cell;
+  const int bits = acc_bits(mb.sp.n);
   if (blockIdx.x == 0 && threadIdx.x == 0) {
-    long long* wr = mb.w.wr64;
-    if (wr[0] | wr[1]) {
-      mb.sp.water_removed[0] += acc_value64(wr[0], wr[1]);
-      wr[0] = wr[1] = 0;
+    long long* const wr = mb.w.wr64;
+    if (wr[0] | wr[1] | wr[2] | wr[3]) {
+      mb.sp.water_removed[0] += acc_read64(wr, bits);
+      acc_clear64(wr);
     }
   }
   __syncwarp();
@@ -898,15 +933,14 @@ __global__ void __launch_bounds__(32) k_cell_update(const __grid_constant__ MRef
     int64_t c = c0 + (threadIdx.x >> 2);
     const bool in = c < C, first = in && (threadIdx.x & 3) == 0;
     if (!in) c = C - 1;
-    long long* acc = mb.w.acc64 + 2 * c;
-    double sum = acc_value64(acc[0], acc[1]);
+    long long* const acc = mb.w.acc64 + ACC64_WORDS * c;
+    double sum = acc_read64(acc, bits);
     const double x = mb.w.accx[c];
     if (x != 0.0) sum += x;   // NaN too
     const double dml = sum * 1.0E-18;
     __syncwarp();   // all lanes have read the sums
     if (first) {
-      acc[0] = 0;
-      acc[1] = 0;
+      acc_clear64(acc);
       if (x != 0.0) mb.w.accx[c] = 0.0;
       delta_m_l[c] = dml;
     }

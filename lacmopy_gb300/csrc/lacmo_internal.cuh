@@ -24,7 +24,7 @@ struct Ws {
   double* dTh;         // [C]   Delta Theta (advection + relaxation) per sub-step
   double* drv;         // [C]   Delta r_v per sub-step
   double* div;         // [C]   mixed precision: exact sums of dm * xi
-  long long* acc64;    // [C][2] FP64: exact sums of dm * xi (acc_add64)
+  long long* acc64;    // [C][4] FP64: exact sums of dm * xi (acc_add64)
   double* accx;        // [C]   FP64: dm * xi beyond their range
   double* relax;       // [2][nz] relaxation terms (r_v, Theta)
   double* colR;        // [n]   exact collision data by slot
@@ -32,7 +32,7 @@ struct Ws {
   int32_t* colk;       // [n]
   // scalars
   uint32_t* flags;
-  long long* wr64;     // [2] FP64: exact sum of the water removed (acc_add64)
+  long long* wr64;     // [4] FP64: exact sum of the water removed (acc_add64)
   int64_t* cursor;     // injected-draw cursor
   int64_t* col_step;   // collision-step counter (Philox)
   int64_t* total_pairs;
