@@ -309,8 +309,9 @@ int lacmo_adv_substep(const lacmo_sips_t* sips, const lacmo_grid_t* grid,
                       size_t ws_bytes, void* stream);
 /* The two halves of a particle sub-step, for callers that time or schedule
  * them separately: the fused per-SIP kernel (condensation, drag, position,
- * re-index; it also counts SIPs per new cell), and the cell binning that
- * sorts the SIPs by (cell, ID).  lacmo_bin must follow lacmo_particles_only before any other
+ * re-index; it also counts SIPs per new cell and adds the water removed at the
+ * ground to water_removed), and the cell binning that sorts the SIPs by
+ * (cell, ID).  lacmo_bin must follow lacmo_particles_only before any other
  * entry point uses the binning. */
 int lacmo_particles_only(const lacmo_sips_t* sips, const lacmo_grid_t* grid,
                          const lacmo_params_t* prm, double dt_sub, double dt_sub_pos, void* ws,

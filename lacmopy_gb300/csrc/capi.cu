@@ -336,7 +336,7 @@ int lacmo_particles_only(const lacmo_sips_t* sp, const lacmo_grid_t* g, const la
   const Bt B = single(*sp, *g, w, 0);
   if (p->precision == LACMO_PRECISION_MIXED) LCHK(launch_records64(B, (cudaStream_t)stream));
   LCHK(launch_particles(B, *p, dt_sub, dt_sub_pos, true, true, (cudaStream_t)stream));
-  LCHK(launch_clear_acc64(B, (cudaStream_t)stream));   // no cell update takes the sums
+  LCHK(launch_clear_acc64(B, (cudaStream_t)stream));
   return LACMO_OK;
 }
 
@@ -456,6 +456,7 @@ int lacmo_adv_step_begin(const lacmo_sips_t* sp, const lacmo_grid_t* g, const la
   const Bt B = single(*sp, *g, w, 0);
   LCHK(launch_records64(B, s));
   LCHK(launch_move(B, p->dt_sub_half, true, s));
+  LCHK(launch_clear_acc64(B, s));   // the water this move took to the ground
   LCHK(launch_bin(B, s));
   LCHK(launch_advection(B, *p, false, s));
   return LACMO_OK;

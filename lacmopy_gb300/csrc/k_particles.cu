@@ -575,9 +575,20 @@ __global__ void k_records64(const __grid_constant__ MRef mr) {
                                             gmp[c], gmp[C + c]));
   }
 }
+// the sum of the water removed at the ground into water_removed; one thread
+__device__ __forceinline__ void take_water(const Member& mb) {
+  long long* const wr = mb.w.wr64;
+  if (wr[0] | wr[1] | wr[2] | wr[3]) {
+    mb.sp.water_removed[0] += acc_read64(wr, acc_bits(mb.sp.n));
+    acc_clear64(wr);
+  }
+}
+// where no cell update follows: the water removed is taken, the cells' sums are
+// dropped
 __global__ void k_clear_acc64(const __grid_constant__ MRef mr) {
   const Member& mb = mr.get();
   const int64_t C = mb.g.nx * mb.g.nz;
+  if (blockIdx.x == 0 && threadIdx.x == 0) take_water(mb);
   for (int64_t c = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; c < C;
        c += (int64_t)gridDim.x * blockDim.x) {
     acc_clear64(mb.w.acc64 + ACC64_WORDS * c);
@@ -920,13 +931,7 @@ __global__ void __launch_bounds__(32) k_cell_update(const __grid_constant__ MRef
   const int64_t C = mb.g.nx * mb.g.nz;
   const double p_ref = mb.g.p_ref, p_ref_inv = mb.g.p_ref_inv, V = mb.g.volume_cell;
   const int bits = acc_bits(mb.sp.n);
-  if (blockIdx.x == 0 && threadIdx.x == 0) {
-    long long* const wr = mb.w.wr64;
-    if (wr[0] | wr[1] | wr[2] | wr[3]) {
-      mb.sp.water_removed[0] += acc_read64(wr, bits);
-      acc_clear64(wr);
-    }
-  }
+  if (blockIdx.x == 0 && threadIdx.x == 0) take_water(mb);
   __syncwarp();
   const int64_t cells = (int64_t)gridDim.x * 8;
   for (int64_t c0 = (int64_t)blockIdx.x * 8; c0 < C; c0 += cells) {

@@ -180,7 +180,8 @@ cudaError_t launch_particles(const Bt& B, const lacmo_params_t& p, double dt_sub
                              double dt_sub_pos, bool write_Tp, bool hist, cudaStream_t s);
 cudaError_t launch_move(const Bt& B, double dt_pos, bool hist, cudaStream_t s);
 cudaError_t launch_records64(const Bt& B, cudaStream_t s);
-// empty the FP64 sums of a particle launch that no cell update follows
+// after a particle launch that no cell update follows: the water removed into
+// water_removed, the cells' sums emptied
 cudaError_t launch_clear_acc64(const Bt& B, cudaStream_t s);
 cudaError_t launch_particles_mixed(const Bt& B, const lacmo_params_t& p, double dt_sub,
                                    double dt_sub_pos, bool write_Tp, bool hist, cudaStream_t s);

@@ -1,0 +1,102 @@
+"""The entry points between and inside advection steps: the water removed at the
+ground arrives with the call that removed it.
+
+Tolerance: water removed is a sum of positive products, 1e-12 (the product's and
+the reference's sums differ by their roundings only, some 1e-13 for the 300 SIPs
+here)."""
+import copy
+import ctypes
+import math
+
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+
+def _falling(seed=4, n_low=300):
+    """A small state with SIPs just above the ground, falling."""
+    from lacmopy_gb300 import synthetic
+    st = synthetic.make_icmw_state(Nx=6, Nz=5, no_spcm=(6, 8), seed=seed, kernel_type="Long_Bott",
+                                   r_tot=11E-3)
+    rng = np.random.default_rng(seed)
+    dx, dz = st["grid_steps"]
+    sel = rng.permutation(st["xi"].size)[:n_low]
+    st["pos"][1, sel] = rng.uniform(0.0, 1.5, n_low)
+    st["cells"][1, sel] = np.floor(st["pos"][1, sel] / dz).astype(np.int64)
+    st["rel_pos"][1, sel] = st["pos"][1, sel] / dz - st["cells"][1, sel]
+    R = rng.uniform(100.0, 400.0, n_low)
+    st["m_w"][sel] = 4.18879e3 * R ** 3
+    st["xi"][sel] = rng.uniform(1e2, 1e4, n_low)
+    st["vel"][1, sel] = -5.0
+    return st
+
+
+class Ledger:
+    """water_removed against the SIPs that left since the last look."""
+
+    def __init__(self, ds):
+        self.ds = ds
+        self.act = ds.cell.cpu().numpy() >= 0
+        self.total = float(ds.water_removed.cpu()[0])
+
+    def check(self, least):
+        act = self.ds.cell.cpu().numpy() >= 0
+        left = self.act & ~act
+        self.act = act
+        m_w, xi = self.ds.m_w.cpu().numpy(), self.ds.xi.cpu().numpy()
+        self.total += math.fsum(m_w[left] * xi[left])
+        assert np.count_nonzero(left) >= least
+        np.testing.assert_allclose(self.ds.water_removed.cpu().numpy()[0], self.total, rtol=1e-12)
+
+
+def _call(ds, name, *args):
+    from lacmopy_gb300 import _lib
+    from lacmopy_gb300.device import _ptr, _stream
+    _lib.check(getattr(ds.lib, name)(ctypes.byref(ds.sips), ctypes.byref(ds.grid), *args,
+                                     _ptr(ds.ws), ds.ws_bytes, _stream()), name)
+
+
+@pytest.mark.parametrize("precision", ["fp64", "mixed"])
+def test_water_removed_by_the_particle_pass_alone(precision):
+    from lacmopy_gb300 import DeviceState, _lib
+    st = _falling()
+    st["act_collisions"] = False
+    ds = DeviceState(st, draws="philox", seed=3, precision=precision)
+    water = Ledger(ds)
+    prm = ctypes.byref(ds.params)
+    for _ in range(2):
+        _call(ds, "lacmo_particles_only", prm, 0.1, 0.1)
+        _call(ds, "lacmo_bin")
+        water.check(10)
+    # whole steps of either precision afterwards neither lose nor repeat it
+    for p in (_lib.PRECISION_MIXED, _lib.PRECISION_FP64):
+        ds.params.precision = p
+        ds.adv_step(1)
+        water.check(0)
+
+
+def test_water_removed_by_the_half_step_move():
+    from lacmopy_gb300 import DeviceState
+    ds = DeviceState(_falling(), draws="philox", seed=3)
+    water = Ledger(ds)
+    prm = ctypes.byref(ds.params)
+    _call(ds, "lacmo_adv_step_begin", prm)
+    water.check(10)
+    _call(ds, "lacmo_adv_substep", prm, ds.params.dt_sub, 0)
+    water.check(1)
+
+
+def test_water_removed_by_a_batch_particle_pass():
+    from lacmopy_gb300 import BatchState, _lib
+    from lacmopy_gb300.device import _stream
+    b = BatchState([_falling(4), _falling(5)], [3, 4], precision="fp64", draws="philox")
+    water = [Ledger(m) for m in b.members]
+    for _ in range(2):
+        _lib.check(b.lib.lacmo_batch_particles_only(b.handle, ctypes.byref(b.params), _stream()),
+                   "batch_particles_only")
+        for w in water:
+            w.check(10)
+    b.adv_step(1)
+    for w in water:
+        w.check(0)
