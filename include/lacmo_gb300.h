@@ -277,9 +277,10 @@ int lacmo_batch_prepare(lacmo_batch* batch, const lacmo_params_t* prm, void* str
 int lacmo_batch_adv_step(lacmo_batch* batch, const lacmo_params_t* prm, void* stream);
 /* A mixed-precision batch step does not bin its SIPs after its last sub-step
  * (the next step bins after its half-step move; water_removed is complete
- * all the same), so between steps a member's binning is empty; lacmo_batch_rebin bins every member's SIPs by their
- * current cells, for entry points that read a member's binning between steps
- * (lacmo_update_grid_r_l with lacmo_batch_member_workspace). */
+ * all the same), so between steps a member's binning is empty; lacmo_batch_rebin
+ * bins every member's SIPs by their current cells, for entry points that read a
+ * member's binning between steps (lacmo_update_grid_r_l with
+ * lacmo_batch_member_workspace).  An FP64 batch step bins, like a single state's. */
 int lacmo_batch_rebin(lacmo_batch* batch, void* stream);
 /* a CUDA graph of n_steps batch advection steps (see lacmo_plan_create) */
 int lacmo_batch_plan_create(lacmo_batch* batch, const lacmo_params_t* prm, int n_steps,

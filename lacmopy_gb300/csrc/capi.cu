@@ -262,10 +262,11 @@ static int adv_step(const Bt& B, const lacmo_params_t& p, const lacmo_draws_t& d
   LCHK(launch_advection(B, p, true, s));
   rc = subloop(B, p, d, p.scale_dt_cond - 1, nc2, false, s);
   if (rc) return rc;
-  // last sub-step: positions move by dt_sub/2 (integration.py:1593-1610)
-  LCHK(launch_particles(B, p, p.dt_sub, p.dt_sub_half, true, keep_binning, s));
+  // last sub-step: positions move by dt_sub/2 (integration.py:1593-1610); the
+  // binning afterwards is there for the entry points between steps, in batches too
+  LCHK(launch_particles(B, p, p.dt_sub, p.dt_sub_half, true, true, s));
   LCHK(launch_cell_update(B, true, s));
-  LCHK(keep_binning ? launch_bin(B, s) : launch_empty_bin(B, s));
+  LCHK(launch_bin(B, s));
   return LACMO_OK;
 }
 

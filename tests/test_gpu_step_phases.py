@@ -1,10 +1,10 @@
 """The entry points between and inside advection steps: the water removed at the
-ground arrives with the call that removed it.
+ground arrives with the call that removed it, and a member of an FP64 batch is
+binned after its step.
 
 Tolerance: water removed is a sum of positive products, 1e-12 (the product's and
 the reference's sums differ by their roundings only, some 1e-13 for the 300 SIPs
 here)."""
-import copy
 import ctypes
 import math
 
@@ -100,3 +100,24 @@ def test_water_removed_by_a_batch_particle_pass():
     b.adv_step(1)
     for w in water:
         w.check(0)
+
+
+@pytest.mark.parametrize("graph", [False, True])
+def test_members_of_an_fp64_batch_are_binned_after_a_step(graph):
+    from lacmopy_gb300 import BatchState, DeviceState, _lib
+    from lacmopy_gb300.device import _stream
+    b = BatchState([_falling(4), _falling(5)], [3, 4], precision="fp64", draws="philox")
+    b.adv_step(2, graph=graph)
+    for m, seed in ((0, 4), (1, 5)):
+        mb = b.members[m]
+        ws, size = ctypes.c_void_p(), ctypes.c_size_t()
+        _lib.check(b.lib.lacmo_batch_member_workspace(b.handle, m, ctypes.byref(ws),
+                                                      ctypes.byref(size)), "member_workspace")
+        _lib.check(b.lib.lacmo_update_grid_r_l(ctypes.byref(mb.sips), ctypes.byref(mb.grid), ws,
+                                               size.value, _stream()), "update_grid_r_l")
+        one = DeviceState(_falling(seed), draws="philox", seed=3 + m)
+        one.adv_step(2)
+        one.update_grid_r_l()
+        r_l = one.snapshot()["grid_scalar_fields"][5]
+        assert np.count_nonzero(r_l) == r_l.size
+        assert np.array_equal(b.snapshot(m)["grid_scalar_fields"][5], r_l)
