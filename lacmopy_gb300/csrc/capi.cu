@@ -245,7 +245,7 @@ static int adv_step_mixed(const Bt& B, const lacmo_params_t& p, const lacmo_draw
 static int adv_step(const Bt& B, const lacmo_params_t& p, const lacmo_draws_t& d, cudaStream_t s,
                     bool keep_binning = true) {
   if (p.precision == LACMO_PRECISION_MIXED) return adv_step_mixed(B, p, d, s, keep_binning);
-  LCHK(launch_records64(B, s));
+  LCHK(launch_records64(B, false, s));
   const bool col = p.act_collisions != 0;
   const int nc1 = p.no_col_per_adv == 1 ? 0 : (p.no_col_per_adv == 2 ? 1 : p.scale_dt_cond);
   const int nc2 = (p.no_col_per_adv == 1 || p.no_col_per_adv == 2) ? 1 : p.scale_dt_cond;
@@ -335,7 +335,7 @@ int lacmo_particles_only(const lacmo_sips_t* sp, const lacmo_grid_t* g, const la
   Ws w;
   if (!ws_carve(ws, bytes, sp->n, g->nx, g->nz, &w)) return LACMO_ERR_WORKSPACE;
   const Bt B = single(*sp, *g, w, 0);
-  if (p->precision == LACMO_PRECISION_MIXED) LCHK(launch_records64(B, (cudaStream_t)stream));
+  LCHK(launch_records64(B, false, (cudaStream_t)stream));   // the grid's wind as it is now
   LCHK(launch_particles(B, *p, dt_sub, dt_sub_pos, true, true, (cudaStream_t)stream));
   LCHK(launch_clear_acc64(B, (cudaStream_t)stream));
   return LACMO_OK;
@@ -455,7 +455,7 @@ int lacmo_adv_step_begin(const lacmo_sips_t* sp, const lacmo_grid_t* g, const la
   if (!ws_carve(ws, bytes, sp->n, g->nx, g->nz, &w)) return LACMO_ERR_WORKSPACE;
   cudaStream_t s = (cudaStream_t)stream;
   const Bt B = single(*sp, *g, w, 0);
-  LCHK(launch_records64(B, s));
+  LCHK(launch_records64(B, false, s));
   LCHK(launch_move(B, p->dt_sub_half, true, s));
   LCHK(launch_clear_acc64(B, s));   // the water this move took to the ground
   LCHK(launch_bin(B, s));
@@ -479,7 +479,8 @@ int lacmo_adv_substep(const lacmo_sips_t* sp, const lacmo_grid_t* g, const lacmo
   if (!ws_carve(ws, bytes, sp->n, g->nx, g->nz, &w)) return LACMO_ERR_WORKSPACE;
   cudaStream_t s = (cudaStream_t)stream;
   const Bt B = single(*sp, *g, w, 0);
-  if (p->precision == LACMO_PRECISION_MIXED) LCHK(launch_records64(B, s));
+  // the grid's wind as it is now; lacmo_adv_step_begin formed the cells' terms
+  LCHK(launch_records64(B, p->precision != LACMO_PRECISION_MIXED, s));
   LCHK(launch_particles(B, *p, p->dt_sub, dt_sub_pos, write_T_p != 0, true, s));
   LCHK(launch_cell_update(B, true, s));
   LCHK(launch_bin(B, s));
@@ -795,12 +796,14 @@ int lacmo_batch_plan_create(lacmo_batch* b, const lacmo_params_t* p, int n_steps
 
 int lacmo_batch_particles_only(lacmo_batch* b, const lacmo_params_t* p, void* stream) {
   if (!b || !prm_ok(p)) return LACMO_ERR_ARG;
-  if (p->precision == LACMO_PRECISION_MIXED)
-    LCHK(launch_particles_mixed(b->B, *p, p->dt_sub, p->dt_sub, false, false, (cudaStream_t)stream));
-  else
-    LCHK(launch_particles(b->B, *p, p->dt_sub, p->dt_sub, false, false, (cudaStream_t)stream));
-  if (p->precision != LACMO_PRECISION_MIXED)
-    LCHK(launch_clear_acc64(b->B, (cudaStream_t)stream));
+  cudaStream_t s = (cudaStream_t)stream;
+  if (p->precision == LACMO_PRECISION_MIXED) {
+    LCHK(launch_particles_mixed(b->B, *p, p->dt_sub, p->dt_sub, false, false, s));
+    return LACMO_OK;
+  }
+  LCHK(launch_records64(b->B, false, s));   // the grids' wind as it is now
+  LCHK(launch_particles(b->B, *p, p->dt_sub, p->dt_sub, false, false, s));
+  LCHK(launch_clear_acc64(b->B, s));
   return LACMO_OK;
 }
 

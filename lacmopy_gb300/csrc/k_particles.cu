@@ -541,11 +541,13 @@ __device__ __forceinline__ void interp_wind(const float4 w0, const float4 w1, co
   }
 }
 
-// The records of the FP64 kernel at the start of a step: the thermodynamic terms
-// from the cell's fields and per-cell terms (the cell update rewrites them every
-// sub-step), and its wind (grid.py:257-323): the values the bilinear interpolation starts from and the differences between its corners
-// (indices below zero wrap as in k_wind_table).
-__global__ void k_records64(const __grid_constant__ MRef mr) {
+// The records of the FP64 kernel from the grid's arrays as they are now: the
+// thermodynamic terms (the cell update rewrites them every sub-step), and the wind
+// (grid.py:257-323): the values the bilinear interpolation starts from and the
+// differences between its corners (indices below zero wrap as in k_wind_table).
+// known: the cell's six terms are the stored ones (no mixed-precision step came
+// after they were written), which leaves out most of the chain of FP64 operations.
+__global__ void k_records64(const __grid_constant__ MRef mr, int known) {
   const Member& mb = mr.get();
   const double *gsf = mb.g.scalar_fields, *gmp = mb.g.mat_prop;
   const double* in = mb.g.velocity;
@@ -570,9 +572,16 @@ __global__ void k_records64(const __grid_constant__ MRef mr) {
     w.edge = (j == 0 ? 1 : 0) | (j == nz - 1 ? 2 : 0);
     w.pad = 0;
     rec[2 * c + 1] = w;
-    write_fp64(mb.w.aux, c, C, gsf[c], gsf[6 * C + c], gmp[2 * C + c], gmp[5 * C + c],
-               gmp[6 * C + c], cell_terms64(gsf[c], gsf[C + c], gsf[7 * C + c], gmp[2 * C + c],
-                                            gmp[c], gmp[C + c]));
+    const double T = gsf[c], S = gsf[6 * C + c], L_v = gmp[2 * C + c], mu = gmp[5 * C + c],
+                 rho_f = gmp[6 * C + c];
+    if (known) {
+      const double* const a = mb.w.aux + c;
+      const CellTerms t{a[0], a[C], a[2 * C], a[3 * C], a[4 * C], a[5 * C]};
+      write_rec64(cell_rec64(mb.w.aux, C) + 2 * c, T, S, L_v, mu, rho_f, t);
+    } else {
+      write_fp64(mb.w.aux, c, C, T, S, L_v, mu, rho_f,
+                 cell_terms64(T, gsf[C + c], gsf[7 * C + c], L_v, gmp[c], gmp[C + c]));
+    }
   }
 }
 // the sum of the water removed at the ground into water_removed; one thread
@@ -1759,10 +1768,10 @@ cudaError_t launch_cell_aux(const Bt& B, cudaStream_t s) {
   k_cell_aux<<<grid2(B.nx * B.nz, 32, B.M), 32, 0, s>>>(B.ref()); note_launches(1);
   // the wind parts of the cell records too, for sub-steps run before a full step
   k_wind_table<<<grid2(B.nx * B.nz, 256, B.M), 256, 0, s>>>(B.ref()); note_launches(1);
-  return launch_records64(B, s);
+  return launch_records64(B, false, s);
 }
-cudaError_t launch_records64(const Bt& B, cudaStream_t s) {
-  k_records64<<<grid2(B.nx * B.nz, 32, B.M), 32, 0, s>>>(B.ref()); note_launches(1);
+cudaError_t launch_records64(const Bt& B, bool known, cudaStream_t s) {
+  k_records64<<<grid2(B.nx * B.nz, 32, B.M), 32, 0, s>>>(B.ref(), known ? 1 : 0); note_launches(1);
   return cudaGetLastError();
 }
 cudaError_t launch_clear_acc64(const Bt& B, cudaStream_t s) {

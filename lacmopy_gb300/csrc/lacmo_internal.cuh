@@ -179,7 +179,8 @@ cudaError_t launch_empty_bin(const Bt& B, cudaStream_t s);
 cudaError_t launch_particles(const Bt& B, const lacmo_params_t& p, double dt_sub,
                              double dt_sub_pos, bool write_Tp, bool hist, cudaStream_t s);
 cudaError_t launch_move(const Bt& B, double dt_pos, bool hist, cudaStream_t s);
-cudaError_t launch_records64(const Bt& B, cudaStream_t s);
+// the FP64 records; known: the stored cell terms hold
+cudaError_t launch_records64(const Bt& B, bool known, cudaStream_t s);
 // after a particle launch that no cell update follows: the water removed into
 // water_removed, the cells' sums emptied
 cudaError_t launch_clear_acc64(const Bt& B, cudaStream_t s);

@@ -1,6 +1,6 @@
 """The entry points between and inside advection steps: the water removed at the
-ground arrives with the call that removed it, and a member of an FP64 batch is
-binned after its step.
+ground arrives with the call that removed it, a member of an FP64 batch is binned
+after its step, and a particle pass takes the wind the grid holds at the call.
 
 Tolerance: water removed is a sum of positive products, 1e-12 (the product's and
 the reference's sums differ by their roundings only, some 1e-13 for the 300 SIPs
@@ -121,3 +121,56 @@ def test_members_of_an_fp64_batch_are_binned_after_a_step(graph):
         r_l = one.snapshot()["grid_scalar_fields"][5]
         assert np.count_nonzero(r_l) == r_l.size
         assert np.array_equal(b.snapshot(m)["grid_scalar_fields"][5], r_l)
+
+
+def _new_wind(ds, seed):
+    """Another wind of the same size into the grid's own array."""
+    v = ds.gvel.cpu().numpy()
+    ds.gvel.copy_(ds.gvel.new_tensor(v[:, ::-1].copy() + 0.1 * seed))
+
+
+@pytest.mark.parametrize("entry", ["particles_only", "substep", "batch"])
+def test_wind_changed_before_a_particle_pass(entry):
+    """Against a state that had the new wind from its start, bit for bit."""
+    from lacmopy_gb300 import BatchState, DeviceState, _lib
+    from lacmopy_gb300.device import _stream
+    if entry == "batch":
+        def make():
+            return BatchState([_falling(4), _falling(5)], [3, 4], precision="fp64", draws="philox")
+
+        def run(b):
+            _lib.check(b.lib.lacmo_batch_particles_only(b.handle, ctypes.byref(b.params),
+                                                        _stream()), "batch_particles_only")
+        one, two = make(), make()
+        for q, m in enumerate(two.members):
+            _new_wind(m, q + 1)
+        _lib.check(two.lib.lacmo_batch_prepare(two.handle, ctypes.byref(two.params), _stream()),
+                   "batch_prepare")
+        pairs = list(zip(one.members, two.members))
+    else:
+        def make():
+            return DeviceState(_falling(), draws="philox", seed=3)
+
+        def run(ds):
+            prm = ctypes.byref(ds.params)
+            if entry == "substep":
+                _call(ds, "lacmo_adv_substep", prm, 0.1, 0)
+            else:
+                _call(ds, "lacmo_particles_only", prm, 0.1, 0.1)
+        one, two = make(), make()
+        _new_wind(two, 1)
+        two.prepare()
+        pairs = [(one, two)]
+        if entry == "substep":
+            for ds in (one, two):
+                _call(ds, "lacmo_adv_step_begin", ctypes.byref(ds.params))
+    for q, (m, _) in enumerate(pairs):
+        _new_wind(m, q + 1)
+    before = pairs[0][0].snapshot()["vel"]
+    run(one)
+    run(two)
+    for m, ref in pairs:
+        a, b = m.snapshot(), ref.snapshot()
+        for k in ("vel", "pos", "m_w", "rel_pos", "cells"):
+            assert np.array_equal(a[k], b[k]), k
+    assert np.abs(pairs[0][0].snapshot()["vel"] - before).max() > 0.05
