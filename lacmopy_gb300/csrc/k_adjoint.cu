@@ -451,7 +451,7 @@ struct Args {
   double dt, ks;
   GridConst g;
   int no_iter;          // 0: implicit step to convergence, else the step's map
-  CellFF* rec;          // [C] the map's cell terms (no_iter > 0), else null
+  CellFF* rec;          // [C] the map's cell terms (no_iter > 0 and scratch), else null
   CellGrad* grad;       // [C] their derivatives (reverse sweep)
   CellFast* fast;       // [C] the terms in FP64 (forward sweep)
 };
@@ -528,8 +528,8 @@ __device__ __noinline__ double fwd_step64(const Args& a, int32_t c, double mw, d
 }
 
 // The SIPs of a forward sub-step.  MAP: the time step's map as the time step runs
-// it (newton_ff; FULL as there), else the converged step.  SIPs whose step needs
-// plain FP64 wait in the block's queue, as in the time step.  Bound by FP32 issue
+// it (newton_ff; FULL as there), else the converged step, or the map in FP64 without
+// scratch.  SIPs whose step needs plain FP64 wait in the block's queue, as in the time step.  Bound by FP32 issue
 // and the FP64 pipe; 720,000 SIPs took 1326 us a launch with the cell's ambient
 // terms and the Newton per SIP in FP64, 190 us with plain FP64 in
 // place, 140 us gathered, 117 us
@@ -794,6 +794,8 @@ __global__ void __launch_bounds__(128) k_bwd_sips(const __grid_constant__ Args a
       if (a.no_iter > REV_MAX ||
           !map_grad(a, load_cell(a.rec + c), a.grad + c, gdt, mw, ms, &g))
         g = map_grad64(a, tape_c[c], tape_c[a.C + c], a.rho_d[c], mw, ms);
+    } else if (a.no_iter > 0) {
+      g = map_grad64(a, tape_c[c], tape_c[a.C + c], a.rho_d[c], m_before[k], ms);
     } else {
       g = root_grad64(a, tape_c[c], tape_c[a.C + c], a.rho_d[c], m_after[k], ms);
     }
@@ -1082,9 +1084,10 @@ int lacmo_adj_forward(int64_t n, int64_t C, double* m_w, const double* m_s, cons
                      p_ref, V, no_iter);
   if (cudaMemsetAsync(dml, 0, 8 * C, s) != cudaSuccess) return LACMO_ERR_CUDA;
   Scratch scratch(s);
-  if (no_iter > 0 && n_sub > 0) {
+  // without scratch for the cells' terms every SIP forms its own, in FP64
+  if (no_iter > 0 && n_sub > 0)
     a.rec = (CellFF*)scratch.get((sizeof(CellFF) + sizeof(CellFast)) * (size_t)C);
-    if (!a.rec) return LACMO_ERR_CUDA;
+  if (a.rec) {
     a.fast = (CellFast*)(a.rec + C);
     k_cell_terms<<<nb(C, 32), 32, 0, s>>>(a);
     note_launches(1);
@@ -1126,11 +1129,9 @@ int lacmo_adj_backward(int64_t n, int64_t C, const double* m_s, const double* xi
                      dt_sub, kappa, p_ref, V, no_iter);
   if (cudaMemsetAsync(dml, 0, 8 * C, s) != cudaSuccess) return LACMO_ERR_CUDA;
   Scratch scratch(s);
-  if (no_iter > 0 && n_sub > 0) {
+  if (no_iter > 0 && n_sub > 0)   // as in lacmo_adj_forward
     a.rec = (CellFF*)scratch.get((sizeof(CellFF) + sizeof(CellGrad)) * (size_t)C);
-    if (!a.rec) return LACMO_ERR_CUDA;
-    a.grad = (CellGrad*)(a.rec + C);
-  }
+  if (a.rec) a.grad = (CellGrad*)(a.rec + C);
   for (int k = n_sub - 1; k >= 0; --k) {
     a.cell = cell + (size_t)k * cell_stride;
     const double* mb = tape_m + (size_t)k * n;

@@ -1,4 +1,4 @@
-"""The adjoint at the edges of its arithmetic: cells without vapour.
+"""The adjoint at the edges: cells without vapour, no scratch memory.
 
 Tolerances: the two-float partials of a sub-step are within 2^-42 (2.3e-13) of the
 terms they add up, which here stay within a factor of 100 of the largest entry:
@@ -98,3 +98,51 @@ def test_gradient_with_a_cell_that_stays_dry():
     for x, y in zip(g, r):
         assert bool(torch.isfinite(y).all())
         assert float((x.cpu() - y).abs().max()) <= 1e-9 * float(y.abs().max())
+
+
+def _without_scratch(tmp_path):
+    """The adjoint's object file with a scratch allocator that has nothing."""
+    import ctypes
+    import os
+    import subprocess
+    from lacmopy_gb300 import _lib, build
+    build.build()
+    src = tmp_path / "no_scratch.cu"
+    src.write_text('#include "lacmo_internal.cuh"\nnamespace lacmo {\nvoid note_launches(int) {}\n'
+                   'void* Scratch::get(size_t) { return nullptr; }\n}\n')
+    out = str(tmp_path / "no_scratch.so")
+    adj = os.path.join(build.BUILD, "k_adjoint.o")
+    flags = build.ARCH + ["-std=c++17", "-I" + build.CSRC, "-Xcompiler", "-fPIC"]
+    subprocess.run([build._nvcc(), "-shared", "-o", out, str(src), adj] + flags, check=True)
+    lib = ctypes.CDLL(out)
+    full = _lib.load()
+
+    class Lib:
+        def __getattr__(self, name):
+            f = getattr(full, name)
+            if name in ("lacmo_adj_forward", "lacmo_adj_backward"):
+                g = getattr(lib, name)
+                g.restype, g.argtypes = f.restype, f.argtypes
+                return g
+            return f
+    return Lib()
+
+
+@pytest.mark.parametrize("no_iter", [0, 3])
+def test_gradient_without_scratch(tmp_path, no_iter):
+    """Masses within 1e-11 (the FP64 map against the two-float one), gradients as
+    above."""
+    from lacmopy_gb300 import adjoint
+    model = adjoint.StepModel(_state(5e-3), 1)
+    w = torch.rand(model.n, generator=torch.Generator().manual_seed(4), dtype=F64).cuda()
+    out = []
+    for lib in (model.lib, _without_scratch(tmp_path)):
+        model.lib = lib
+        m_s = model.m_s0.clone().requires_grad_(True)
+        kappa = torch.tensor(0.55, dtype=F64, device="cuda", requires_grad=True)
+        s = torch.tensor(1.1, dtype=F64, device="cuda", requires_grad=True)
+        J = adjoint.objective(model, m_s, kappa, s, weights=w, no_iter=no_iter)
+        out.append((model.run(no_iter=no_iter)[0], *torch.autograd.grad(J, [m_s, kappa, s])))
+    torch.testing.assert_close(out[1][0], out[0][0], rtol=1e-11, atol=0)
+    for x, y in zip(out[1][1:], out[0][1:]):
+        assert float((x - y).abs().max()) <= 1e-9 * float(y.abs().max())
