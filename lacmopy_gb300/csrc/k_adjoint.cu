@@ -490,7 +490,7 @@ __device__ __forceinline__ void write_cell(const Args& a, int64_t c, double Th, 
                         rcp64(s.t.rhow);
     const double dT = s.T - LC_T_ALPHA_0;
     g->S_T = d2ff(s.S * (lT - les));
-    g->S_r = d2ff(div64(rho_d * s.T * LC_R_V, s.e_s));   // S / r_v, for r_v = 0 too
+    g->S_r = d2ff(rho_d * s.T * LC_R_V * rcp64(s.e_s));   // S / r_v, for r_v = 0 too
     g->lcx_T = d2ff(-lrho);
     g->lce_T = d2ff(lsig - lrho - lT);
     g->la_T = d2ff(s.t.lap0 * (LC_C_ALPHA_2 * T_T * rcp64(LC_C_ALPHA_1 + LC_C_ALPHA_2 * dT) + lK -
