@@ -760,12 +760,17 @@ __global__ void __launch_bounds__(128) k_particles(const __grid_constant__ PK x)
         }
         double m = mw, dm = 0.0;
         if (pass == 0) {
-          bool ok;
-          m = newton_ff<false, FULL>(a.sol, a.no_iter, mw, ms, cf,
-                                     d2ff(LC_FOUR_PI * 1.0E12 * a.dt_sub), 1.0, &ok);
-          dm = m - mw;   // a step below m / 8: mw + dm is m
+          // masses outside the two-float range (pure water) gain nothing from the
+          // queue where they fill the warp
+          bool ok = ff_mass_ok(mw) && ff_mass_ok(ms);
+          const bool gather = __any_sync(__activemask(), ok) != 0;
+          if (ok) {
+            m = newton_ff<false, FULL>(a.sol, a.no_iter, mw, ms, cf,
+                                       d2ff(LC_FOUR_PI * 1.0E12 * a.dt_sub), 1.0, &ok);
+            dm = m - mw;   // a step below m / 8: mw + dm is m
+          }
           if (!ok) {
-            const int at = atomicAdd(&s_n, 1);
+            const int at = gather ? atomicAdd(&s_n, 1) : PQ;
             if (at < PQ) {
               s_q[at] = (int32_t)((uint32_t)k | 0x80000000u);
               continue;
@@ -821,7 +826,7 @@ __global__ void __launch_bounds__(128) k_particles(const __grid_constant__ PK x)
         const ff duf = d2ff(du), dwf = d2ff(dw + a.dt_sub * a.g_set);
         const float dwh = d2f_int(dw);
         const float Re = 2.0E-6f * cf.rm * f_sqrt(duf.h * duf.h + dwh * dwh) * f_rcp(z.h);
-        if (Re < 0.499f && kd.h > 8.0f && (pass == 0 || (ff_mass_ok(m) && ff_mass_ok(ms)))) {
+        if (Re < 0.499f && kd.h > 8.0f && ff_mass_ok(m + ms)) {
           // (u + k uf) / (1 + k) = uf - (uf - u) / (1 + k)
           const ff inv = ff_rcp(ff_add(kd, 1.0f));
           u = uf - ff2d_of<FULL>(ff_mul(duf, inv));
