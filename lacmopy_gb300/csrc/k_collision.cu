@@ -597,9 +597,10 @@ __device__ __forceinline__ void init_exact_scratch(const CellArgs& a, Cell<BIG> 
 // the whole rest of the cell: a step of a raining 75 x 75 x 128 state (14
 // collections per cell on average, 190 in the heaviest, whose chain of events of
 // some 5 us each is what the step waits for) took 10.6 ms, 0.78 ms now.
-// Returns false when the event limit is passed (ev.pos: the first rank left).
+// Returns false when a limit is passed, of collections or of undecided pairs that
+// change nothing (ev.pos: the first rank left).
 struct PairEvents {
-  int pos, events, c0, c1;
+  int pos, events, idle, c0, c1;
   uint32_t m;
 };
 __device__ __noinline__ PhiloxBlock injected_couple(const double* rnd, int p, int P) {
@@ -618,7 +619,7 @@ template <bool BIG>
 __device__ __noinline__ bool window_events(Cell<BIG> S, int n, int P, int w0,
                                            int i, int j, PhiloxBlock x, float cmax, double Tc,
                                            bool use_E, bool injected, int event_limit,
-                                           PairEvents& ev) {
+                                           int idle_limit, PairEvents& ev) {
   const CellArgs& a = cell_args();
   constexpr unsigned FULL = 0xffffffffu;
   const int lane = threadIdx.x & 31;
@@ -663,7 +664,7 @@ __device__ __noinline__ bool window_events(Cell<BIG> S, int n, int P, int w0,
       }
       done = w0 + 2 * L + (sec ? 2 : 1);
       changed = o != 0;
-      if (changed && ++ev.events > event_limit) {
+      if (changed ? ++ev.events > event_limit : ++ev.idle > idle_limit) {
         ev.pos = done;
         return false;
       }
@@ -1018,9 +1019,14 @@ __device__ __forceinline__ int2 collide_cell(const Cell<BIG> S, int64_t c, int n
     // anti-diagonal schedule from its current position: the sequence costs a
     // chain of some 4 us per event, the 2n - 3 diagonals about as much each.
     const int event_limit = 64 + 2 * n;
+    // Undecided pairs that change nothing (multiplicities below zero, NaN) take some
+    // 2 us each where they fill a cell, the diagonals 10 us each: 250 SIPs, all of
+    // them negative, 64.7 ms a step without this limit, 5.4 ms with it.
+    const int idle_limit = min(16 + P / 64, 10 * n);
     PairEvents ev;
     ev.pos = 0;            // first rank not processed yet
-    ev.events = 0;
+    ev.events = ev.idle = 0;
+    bool diagonal = false;
     int i = 0, j = 1 + 2 * lane;   // the pair of rank w0 + 2 lane
     float4 vi = S.v()[0];
     for (int w0 = 0; w0 < P; w0 += 64, j += 64) {
@@ -1049,15 +1055,15 @@ __device__ __forceinline__ int2 collide_cell(const Cell<BIG> S, int64_t c, int n
       if (!__any_sync(0xffffffffu, m0 | m1)) continue;
       ev.m = (m0 ? 1 : 0) | (m1 ? 2 : 0);
       const bool go_on = window_events(S, n, P, w0, i, j, x, cmax, Tc, use_E, rnd != nullptr,
-                                       event_limit, ev);
+                                       event_limit, idle_limit, ev);
       c0 += ev.c0;
       c1 += ev.c1;
-      if (!go_on) break;
+      diagonal = !go_on;
+      if (diagonal) break;
       vi = S.v()[i];   // SIP i may have changed
     }
-    const int pos = ev.pos;
-    const bool diagonal = ev.events > event_limit;
     if (diagonal) {
+      const int pos = ev.pos;
       // anti-diagonal schedule of the pairs from rank pos on
       for (int s = 1; s <= 2 * n - 3; ++s) {
         const int ilo = s - (n - 1) > 0 ? s - (n - 1) : 0;
