@@ -119,7 +119,7 @@ LACMO_DEV double ff2d(ff a) { return f2d_int(a.h) + f2d_int(a.l); }
 // tens of cycles longer than the addition's).
 LACMO_DEV double ff2d_int(ff a) {
   const uint32_t hb = __float_as_uint(a.h), eh = (hb >> 23) & 0xffu;
-  if (eh - 53u >= 202u) return ff2d(a);   // 0, below 2^-74, not finite
+  if (eh - 55u >= 200u) return ff2d(a);   // 0, below 2^-72 (l may be subnormal), not finite
   const uint32_t lb = __float_as_uint(a.l) ^ (hb & 0x80000000u);   // l away from zero
   const uint32_t below = (hb & 0x007fffffu) == 0u ? lb >> 31 : 0u;
   const int k = __float2int_rn(fm(__uint_as_float(lb), __uint_as_float((306u + below - eh) << 23)));
