@@ -137,7 +137,7 @@ struct CellFF {
   ff la, lb, c1, c2;
   ff n0, n1, n3;    // NaCl solution density over rho_w: n0 + n1 w + n3 w^2
   ff mr;            // mu / rho_w
-  float rm, T;      // rho_f / mu
+  float rm, pad0;   // rho_f / mu
   double L_v;       // heat of vaporisation
   double pad[3];
 };
@@ -284,10 +284,12 @@ LACMO_DEV double newton_ff(int sol, int no_iter, double m_w, double m_s, const C
 
 // ---------------------------------------------------------------------------
 // The same Newton in plain FP64 with few instructions, for SIPs whose step needs
-// all 53 bits: reciprocals and the cube root from FP32 seeds (2^-22) refined to
-// second and third order, the differences from saturation and the factored
-// derivative of mass_rate_ff; about 100 FP64 instructions an evaluation where
-// mass_rate_and_derivative takes some 220.
+// all 53 bits: reciprocals and the cube root from FP32 seeds (2^-22) and one
+// Householder iteration (Householder, The Numerical Treatment of a Single Nonlinear
+// Equation, 1970): with the residual e of the seed, the binomial series of
+// (1 - e)^-1 and (1 - e)^(-1/3) to second and third order.  The differences from
+// saturation and the factored derivative of mass_rate_ff; about 100 FP64
+// instructions an evaluation where mass_rate_and_derivative takes some 220.
 LACMO_DEV double rcp64(double b) {
   const double y = f2d_int(f_rcp(d2f_int(b)));
   double e = fma(-b, y, 1.0);

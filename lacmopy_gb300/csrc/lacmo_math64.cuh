@@ -15,7 +15,9 @@
 
 namespace lacmo {
 
-// 1 / b (within an ulp) and a / b, a quotient's last bits from its residual
+// a / b, the quotient's last bits from its residual, and sqrt(x) by one Householder
+// iteration from the FP32 reciprocal root (as rcp64); arguments within FP32's range.
+// Compared with the library's functions by tests/test_gpu_math64.py.
 LACMO_DEV double div64(double a, double b) {
   const double r = rcp64(b), q = __dmul_rn(a, r);
   return __fma_rn(__fma_rn(-q, b, a), r, q);
@@ -210,7 +212,7 @@ static __device__ __noinline__ void write_rec64(CellFF* out, double T, double S,
   r.n3 = d2ff(__dmul_rn(LC_PAR_SOL_DENS_NACL_3, irho));
   r.mr = d2ff(__dmul_rn(mu, irho));
   r.rm = d2f_int(rho_f) * f_rcp(d2f_int(mu));
-  r.T = d2f_int(T);
+  r.pad0 = 0.0f;
   r.L_v = L_v;
   r.pad[0] = r.pad[1] = r.pad[2] = 0.0;
   *out = r;
