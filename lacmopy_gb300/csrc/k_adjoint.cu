@@ -557,12 +557,11 @@ __global__ void __launch_bounds__(128) k_fwd_sips(const __grid_constant__ Args a
     const double ms = a.m_s[k];
     double m;
     if (MAP) {
+      const CellFF cf = load_cell(a.rec + c);   // beside the loads of the masses
       bool ok = ff_mass_ok(mw) && ff_mass_ok(ms);
-      const bool gather = __any_sync(__activemask(), ok) != 0;
-      if (ok)
-        m = newton_ff<true, FULL>(SOL_AS, a.no_iter, mw, ms, load_cell(a.rec + c), gdt, a.ks, &ok);
-      if (!ok) {   // as in k_particles
-        const int at = gather ? atomicAdd(&s_n, 1) : FQ;
+      if (ok) m = newton_ff<true, FULL>(SOL_AS, a.no_iter, mw, ms, cf, gdt, a.ks, &ok);
+      if (!ok) {
+        const int at = atomicAdd(&s_n, 1);
         if (at < FQ) {
           s_q[at] = (int32_t)k;
           continue;
@@ -793,8 +792,9 @@ __global__ void __launch_bounds__(128) k_bwd_sips(const __grid_constant__ Args a
     SipGrad g;
     if (MAP) {
       const double mw = m_before[k];
+      const CellFF cf = load_cell(a.rec + c);
       if (a.no_iter > REV_MAX || !ff_mass_ok(mw) || !ff_mass_ok(ms) ||
-          !map_grad(a, load_cell(a.rec + c), a.grad + c, gdt, mw, ms, &g))
+          !map_grad(a, cf, a.grad + c, gdt, mw, ms, &g))
         g = map_grad64(a, tape_c[c], tape_c[a.C + c], a.rho_d[c], mw, ms);
     } else if (a.no_iter > 0) {
       g = map_grad64(a, tape_c[c], tape_c[a.C + c], a.rho_d[c], m_before[k], ms);
