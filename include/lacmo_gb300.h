@@ -297,9 +297,9 @@ int lacmo_batch_destroy(lacmo_batch* batch);
  * _begin: x_{n+1/2}, re-index and the first-half advective + relaxation
  *   increments kept in the workspace (integration.py:1474-1508);
  * _second_half: the second-half increments (integration.py:1536-1561);
- * _substep: one particle + grid sub-step with those increments; positions
- *   move by dt_sub_pos, T_p is written when write_T_p != 0
- *   (integration.py:1265-1281, 1593-1610). */
+ * _substep: one particle + grid sub-step with those increments, in the wind the
+ *   grid holds at the call; positions move by dt_sub_pos, T_p is written when
+ *   write_T_p != 0 (integration.py:1265-1281, 1593-1610). */
 int lacmo_adv_step_begin(const lacmo_sips_t* sips, const lacmo_grid_t* grid,
                          const lacmo_params_t* prm, void* ws, size_t ws_bytes, void* stream);
 int lacmo_adv_step_second_half(const lacmo_sips_t* sips, const lacmo_grid_t* grid,

@@ -529,11 +529,11 @@ __device__ __noinline__ double fwd_step64(const Args& a, int32_t c, double mw, d
 
 // The SIPs of a forward sub-step.  MAP: the time step's map as the time step runs
 // it (newton_ff; FULL as there), else the converged step, or the map in FP64 without
-// scratch.  SIPs whose step needs plain FP64 wait in the block's queue, as in the time step.  Bound by FP32 issue
-// and the FP64 pipe; 720,000 SIPs took 1326 us a launch with the cell's ambient
-// terms and the Newton per SIP in FP64, 190 us with plain FP64 in
-// place, 140 us gathered, 117 us
-// with the cell's FP64 terms stored beside its record.
+// scratch.  SIPs whose step needs plain FP64 wait in the block's queue, as in the
+// time step.  Bound by issue and the FP64 pipe; 720,000 SIPs took 1326 us a launch
+// with the cell's ambient terms and the Newton per SIP in FP64, 190 us with plain
+// FP64 in place, 140 us gathered, 117 us with the cell's FP64 terms stored beside its
+// record.
 constexpr int FQ = 1024;
 template <bool MAP, bool FULL>
 __global__ void __launch_bounds__(128) k_fwd_sips(const __grid_constant__ Args a, double* tape_m) {

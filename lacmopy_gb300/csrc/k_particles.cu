@@ -691,17 +691,20 @@ __device__ __noinline__ double particle_removed(const PArgs& a, int64_t k, int32
 // 670 FP64 instructions per SIP at 2 lanes an SM and clock, 478 us per launch
 // over 360,000 SIPs.  The Newton and the drag now run in two-float arithmetic
 // around the FP64 operations that decide the result's rounding (lacmo_ff.cuh;
-// about 65 a SIP are left, and some 3700 FP32 and integer instructions): 87 us.
+// about 65 a SIP are left, and some 3700 FP32 and integer instructions): 85 us once
+// few SIPs need plain FP64, 95 us averaged over 20 sub-steps from a state out of
+// equilibrium.
 // New cell indices come from the FP32 position where it is clear of the cell's
 // edges, boundaries likewise.
 // SIPs that need plain FP64 for the Newton (a step of more than an eighth of
-// the mass, a radius below 5 nm) or the drag (drops above some 30 um) wait in
-// the block's queue until its other SIPs are done: a few of them in every warp
+// the mass, a radius below 5 nm, no solute) or the drag (drops above some 30 um) wait
+// in the block's queue until its other SIPs are done: a few of them in every warp
 // would hold all warps on the FP64 pipe, gathered they fill a few warps (a
-// raining state of 545,000 SIPs, 1.3% of them large drops, averaged over 20
-// sub-steps from a state out of equilibrium: 291 us in place, 217 us gathered,
-// 144 us with newton_fast and no more blocks than are resident, 135 us when the
-// queue's second pass does only what is left of a SIP; 732 us in plain FP64).
+// raining state of 545,000 SIPs, 1.3% of them large drops, averaged the same way:
+// 291 us in place, 217 us gathered, 144 us with newton_fast and no more blocks than
+// are resident, 135 us when the queue's second pass does only what is left of a SIP;
+// 732 us in plain FP64).  Which of these ways a SIP takes follows from its own state
+// and gives the same bits in place and from the queue.
 __device__ __forceinline__ double i2d_int(int i) {   // i >= 0
   return i < (1 << 24) ? f2d_int((float)i) : (double)i;
 }
@@ -1819,7 +1822,7 @@ cudaError_t launch_move(const Bt& B, double dt_pos, bool hist, cudaStream_t s) {
 // are bound by the FP64 pipe and take FULL (the two above: 107 and 144 us); smaller
 // ones wait for one SIP's chain, which FULL lengthens (1920 SIPs: 23.6 us without,
 // 23.9 us with it).  The queue's second pass doing only what is left of a SIP
-// took all of these to 97, 135 and 19.0 us.
+// took all of these to 95, 135 and 19 us.
 cudaError_t launch_particles(const Bt& B, const lacmo_params_t& p, double dt_sub,
                              double dt_sub_pos, bool write_Tp, bool hist, cudaStream_t s) {
   PK x{B.ref(), pcall(p, dt_sub, dt_sub_pos, write_Tp, hist)};
