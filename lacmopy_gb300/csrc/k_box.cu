@@ -17,7 +17,8 @@
 //      screened again against all their later pairs, and what the screen does
 //      not rule out joins the candidates: at any time every pair to come that
 //      would collect is among them.  A collected SIP that only lost
-//      multiplicity is not screened: max(xi) falls and nothing else changed.
+//      multiplicity, and is not left below zero, is not screened: max(xi) falls and
+//      nothing else changed.
 // Bounds: the screen is limited by the Philox blocks (about 65 of some 100
 // instructions per couple of pairs); the event loop by its latency (3.6 us per
 // collection of 5000 SIPs: one exact evaluation, up to n screened pairs).
@@ -371,14 +372,17 @@ __global__ void __launch_bounds__(BOX_THREADS) k_box_step(const BoxArgs a) {
     if (t == 0) {
       int imin;
       bool split;
+      const double xi_i = S.X[i], xi_j = S.X[j];
       const int o = S.pair(a, i, j, draw_value(a, pair_draw(a, pair_rank(i, j, n))), &imin, &split);
       c0 += o == 1;
       c1 += o == 2;
       // the SIPs whose p_crit may have grown: the one that gained mass, and the
-      // other one unless it only lost multiplicity and still has some
+      // other one unless it only lost multiplicity and still has some (it gains from
+      // a SIP whose multiplicity is negative)
       const int imax = imin == i ? j : i;
+      const bool less = S.X[imax] >= 0.0 && S.X[imax] <= (imin == i ? xi_j : xi_i);
       s_chg[0] = o ? imin : -1;
-      s_chg[1] = o && (split || !(S.X[imax] >= 0.0)) ? imax : -1;
+      s_chg[1] = o && (split || !less) ? imax : -1;
     }
     __syncthreads();
     if (s_chg[0] < 0) continue;
