@@ -16,13 +16,23 @@
 namespace lacmo {
 
 // a / b, the quotient's last bits from its residual, and sqrt(x) by one Householder
-// iteration from the FP32 reciprocal root (as rcp64); arguments within FP32's range.
+// iteration from the FP32 reciprocal root (as rcp64), for |b| and x from 2^-125 to
+// 2^125 and normal quotients; the library's outside (a state that blew up).
 // Compared with the library's functions by tests/test_gpu_math64.py.
+LACMO_DEV bool ff_range(double x) {   // 2^-125 <= |x| < 2^125
+  return ((uint32_t)__double2hiint(x) & 0x7fffffffu) - (898u << 20) < (250u << 20);
+}
+static __device__ __noinline__ double div_any(double a, double b) { return a / b; }
+static __device__ __noinline__ double sqrt_any(double x) { return sqrt(x); }
+LACMO_DEV double rcp64_any(double b) { return ff_range(b) ? rcp64(b) : div_any(1.0, b); }
 LACMO_DEV double div64(double a, double b) {
   const double r = rcp64(b), q = __dmul_rn(a, r);
-  return __fma_rn(__fma_rn(-q, b, a), r, q);
+  const double d = __fma_rn(__fma_rn(-q, b, a), r, q);
+  const bool normal = ((uint32_t)__double2hiint(d) & 0x7fffffffu) - (1u << 20) < (2045u << 20);
+  return ff_range(b) && normal ? d : div_any(a, b);
 }
-LACMO_DEV double sqrt64(double x) {   // x > 0, within FP32's range
+LACMO_DEV double sqrt64(double x) {
+  if (!ff_range(x) || x < 0.0) return sqrt_any(x);
   float y;
   asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(d2f_int(x)));
   const double z = f2d_int(y), s = __dmul_rn(x, z);
@@ -165,7 +175,7 @@ LACMO_DEV CellState cell_state64_x4(double Th, double r_v, double rho_d, double 
   const double tau = __dsub_rn(1.0, __dmul_rn(T, 1.0 / 647.096));
   const double d = __dsub_rn(T, LC_PAR_WATER_DENS_2);
   a.t.rhow = __fma_rn(LC_PAR_WATER_DENS_1, __dmul_rn(d, d), LC_PAR_WATER_DENS_0);
-  *irho = rcp64(a.t.rhow);
+  *irho = rcp64_any(a.t.rhow);
   const double dT = __dsub_rn(T, LC_T_ALPHA_0);
   // -5420 / T, mu, lap0, c1
   const double q1 = div64(
@@ -193,7 +203,7 @@ LACMO_DEV CellState cell_state64_x4(double Th, double r_v, double rho_d, double 
   a.rho_f = __dmul_rn(rho_d, __dadd_rn(1.0, r_v));
   return a;
 }
-// the FP64 path's record of a cell; irho = rcp64(rho_w), kelvin: kelvin_term64
+// the FP64 path's record of a cell; irho = rcp64_any(rho_w), kelvin: kelvin_term64
 LACMO_DEV double kelvin_term64(double T, double sigw, double irho) {
   return div64(__dmul_rn(__dmul_rn(2.0E6, sigw), irho), __dmul_rn(LC_R_V, T));
 }
@@ -219,7 +229,7 @@ static __device__ __noinline__ void write_rec64(CellFF* out, double T, double S,
 }
 static __device__ __noinline__ void write_rec64(CellFF* out, double T, double S, double L_v,
                                                 double mu, double rho_f, CellTerms t) {
-  const double irho = rcp64(t.rhow);
+  const double irho = rcp64_any(t.rhow);
   write_rec64(out, T, S, L_v, mu, rho_f, t, irho, kelvin_term64(T, t.sigw, irho));
 }
 

@@ -86,6 +86,21 @@ def test_reciprocal_and_quotient(ev):
     assert _places(*ev(1, _wide(2, -100, 100, sign=True), _wide(3, -100, 100, sign=True))) <= 1
 
 
+def test_outside_the_range(ev):
+    """Infinities, NaN, zeros and numbers beyond FP32: as the library."""
+    v = np.array([0.0, -0.0, np.inf, -np.inf, np.nan, 1e-310, 5e-324, 1e-300, -1e-60, 1e-39, 1.0,
+                  -3.0, 1e37, 1e39, -1e60, 1e200, 1.7e308])
+    x, y = (t.ravel() for t in np.meshgrid(v, v))
+    a, b = ev(1, x, y)
+    nan = np.isnan(b)
+    assert np.array_equal(np.isnan(a), nan)
+    ulp = np.abs(a[~nan].view(np.int64) - b[~nan].view(np.int64))
+    assert np.array_equal(np.signbit(a[~nan]), np.signbit(b[~nan])) and ulp.max() <= 1
+    a, b = ev(2, v)
+    np.testing.assert_array_equal(a[[0, 1, 2, 3, 4, 5, 6, 7, 8, 13, 14, 15, 16]],
+                                  b[[0, 1, 2, 3, 4, 5, 6, 7, 8, 13, 14, 15, 16]])
+
+
 def test_roots(ev):
     assert _places(*ev(2, _wide(4, -120, 120))) <= 1
     a, b = ev(3, _wide(5, -100, 100))
