@@ -36,14 +36,22 @@ static cudaMemPool_t scratch_pool() {
     props.location.type = cudaMemLocationTypeDevice;
     props.location.id = dev;
     cudaMemPool_t p = nullptr;
-    if (cudaMemPoolCreate(&p, &props) != cudaSuccess) {
+    uint64_t keep = 16ull << 20;
+    int off = 0;
+    // the first call may be under a stream capture, which these calls (no stream
+    // operations) would end in the other capture modes
+    cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
+    if (cudaThreadExchangeStreamCaptureMode(&mode) != cudaSuccess) return nullptr;
+    const cudaError_t e = cudaMemPoolCreate(&p, &props);
+    if (e == cudaSuccess) {
+      cudaMemPoolSetAttribute(p, cudaMemPoolAttrReleaseThreshold, &keep);
+      cudaMemPoolSetAttribute(p, cudaMemPoolReuseAllowInternalDependencies, &off);
+    }
+    cudaThreadExchangeStreamCaptureMode(&mode);
+    if (e != cudaSuccess) {
       cudaGetLastError();
       return nullptr;
     }
-    uint64_t keep = 16ull << 20;
-    int off = 0;
-    cudaMemPoolSetAttribute(p, cudaMemPoolAttrReleaseThreshold, &keep);
-    cudaMemPoolSetAttribute(p, cudaMemPoolReuseAllowInternalDependencies, &off);
     pools[dev] = p;
   }
   return pools[dev];
