@@ -102,7 +102,8 @@ typedef struct {
  * to a few roundings (per-cell sums and water_removed are integer sums of the
  * FP64 products, exact from 2^-12 fg up and in units of 2^-64 fg below, so their
  * order does not matter; products of 2^104 fg and more, or 2^60 fg in a state of
- * 2^31 SIPs, are added in FP64).  MIXED: the Newton condensation and the drag update in FP32, with the Newton repeated in FP64 for SIPs near the
+ * 2^31 SIPs, are added in FP64).  MIXED: the Newton condensation and the
+ * drag update in FP32, with the Newton repeated in FP64 for SIPs near the
  * critical radius of activation; state, positions, per-cell condensed-mass
  * sums (into Theta / r_v), multiplicities and the collision step stay FP64;
  * the per-cell sums of dm * xi are exact integer sums (units of 2^-4 fg), so
@@ -131,7 +132,9 @@ int lacmo_abi_version(void);
 uint64_t lacmo_kernel_launches(void);
 const char* lacmo_error_string(int status);
 /* Bytes of device scratch the entry points below need for n SIPs and an
- * nx x nz grid (no allocation happens inside the library). */
+ * nx x nz grid (those that take a workspace allocate nothing; the box-model steps
+ * and the adjoint take scratch from a pool of the library's own, at most 16 MB of
+ * which outlive a synchronisation, and run without it where there is none). */
 size_t lacmo_workspace_bytes(int64_t n, int64_t nx, int64_t nz);
 /* Zero the workspace: draw cursor, collision-step counter, flags. */
 int lacmo_workspace_reset(void* ws, size_t ws_bytes, int64_t n, int64_t nx, int64_t nz,
